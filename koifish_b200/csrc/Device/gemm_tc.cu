@@ -515,10 +515,7 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
                             wreg[kin][0] = lds32(src + (((uint32_t)(boff >> 4) ^ rsw) << 4) + (boff & 15));
                         }
                     }
-                    // the bytes are in registers: hand the stage back to the loader.  One arrival per warp: 256 per-thread arrivals on
-                    // one barrier word serialise in the shared-memory atomic unit and were the bottleneck of the whole kernel
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive_a(rempty0 + rs * 8);
+                    const uint32_t rdone = rempty0 + rs * 8;
                     if (++rs == RS) rs = 0, rph ^= 1;
 #pragma unroll
                     for (int kin = 0; kin < KBR; kin += UNIT) {
@@ -570,6 +567,14 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
                             for (int u = U - 1; u < UNIT; u += U) mbar_arrive_a(sfull[u]);
                         }
                     }
+                    // Hand the stage back to the loader only now: tcgen05.wait::st above cannot complete before the weights it stores have been
+                    // computed, so every byte of the stage has reached its register.  An arrival right behind the shared-memory loads is
+                    // no such proof: it overtakes loads that still queue in the load / store unit (behind a burst of zero / step fetches at the
+                    // start of an item), the loader refills the stage and lanes expand the bytes of the stage RS further on (4-bit 8192 x 5120 at
+                    // 2048 tokens: every call wrong).  One arrival per warp: 256 per-thread arrivals on one barrier word serialise in the
+                    // shared-memory atomic unit.
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_a(rdone);
                 }
             }
         }
