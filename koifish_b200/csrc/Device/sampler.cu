@@ -10,7 +10,7 @@
 //   2. p_i = expf((l_i - l_max) / T), normalised by their sum in sorted order (sequential fp32, like the host loop);
 //   3. top-p: keep the shortest prefix whose cumulative probability exceeds top_p;
 //   4. coin = random_f32(state) * sum(kept p); first i with coin < cdf_i (else the last kept).
-// Steps 2-4 run on one thread in the reference's order of operations, so that the CPU port (oracle kfo_sample) and the kernel agree
+// The sums of steps 2-4 run on one thread in the reference's order of operations, so that the CPU port (oracle kfo_sample) and the kernel agree
 // except where expf's last ulp moves a cdf boundary across the coin.
 #include <math.h>
 
@@ -57,15 +57,13 @@ __device__ int block_exscan(int v, int* s_warp, int* total) {
     return s_warp[warp] + inc - v;
 }
 
-__global__ void __launch_bounds__(kSampThreads) kf_sample_kernel(int32_t* __restrict__ out, const uint16_t* __restrict__ logits, int vocab, float temperature,
-                                                                 int top_k, float top_p, unsigned long long* __restrict__ rng, int selection) {
+// The top_k candidates of one row in (value descending, index ascending) order, by one CTA of kSampThreads threads: any vocabulary, any top_k up to
+// kMaxTopK, both selections.
+__device__ void select_any(float* s_val, int* s_idx, const uint16_t* __restrict__ row, int vocab, int top_k, int selection) {
     __shared__ int s_hist[256];
     __shared__ int s_warp[33];
-    __shared__ float s_val[kMaxTopK];
-    __shared__ int s_idx[kMaxTopK];
     __shared__ int s_bin, s_above;
     const int tid       = threadIdx.x;
-    const uint16_t* row = logits + (size_t)blockIdx.x * vocab;
     const int chunk     = (vocab + kSampThreads - 1) / kSampThreads;  // contiguous indices per thread: tie ranks follow the index order
     const int i0 = tid * chunk, i1 = min(vocab, i0 + chunk);
     const int k  = top_k;
@@ -159,44 +157,230 @@ __global__ void __launch_bounds__(kSampThreads) kf_sample_kernel(int32_t* __rest
             }
             __syncthreads();
         }
-    // ---- softmax with temperature over the candidates, top-p, coin: one thread, the host loop's order of operations ---------------------
+}
+
+// Softmax with temperature over the candidates, top-p, coin.  The host loop's order of operations: the two running sums are formed by one thread,
+// entry after entry; what is independent per entry (exponential, quotient) by one thread each.  The cumulative probabilities of the top-p cut, the
+// sum under the coin and the cdf are one and the same running sum.  Called by a whole CTA; s_val is overwritten.
+__device__ void draw(int32_t* out, float* s_val, const int* s_idx, int k, float temperature, float top_p, unsigned long long* rng) {
+    __shared__ float s_sum;
+    __shared__ int s_last;
+    const int tid  = threadIdx.x;
+    const float mx = s_val[0];
+    __syncthreads();
+    if (tid < k) s_val[tid] = expf((s_val[tid] - mx) / temperature);
+    if (tid == 0) s_last = k - 1;
+    __syncthreads();
     if (tid == 0) {
-        const float mx = s_val[0];
-        float sum      = 0.f;
-        for (int i = 0; i < k; i++) {
-            const float p = expf((s_val[i] - mx) / temperature);
-            s_val[i]      = p;
-            sum += p;
+        float sum = 0.f;
+#pragma unroll 8
+        for (int i = 0; i < k; i++) sum += s_val[i];
+        s_sum = sum;
+    }
+    __syncthreads();
+    if (tid < k) s_val[tid] /= s_sum;
+    __syncthreads();
+    if (tid == 0) {
+        float cum = 0.f;
+#pragma unroll 8
+        for (int i = 0; i < k; i++) cum += s_val[i], s_val[i] = cum;
+    }
+    __syncthreads();
+    if (top_p < 1.0f && tid < k && s_val[tid] > top_p) atomicMin(&s_last, tid);
+    __syncthreads();
+    const int last = s_last;
+    __syncthreads();
+    unsigned long long st = *rng;
+    const float coin      = (float)(xorshift_u32(&st) >> 8) / 16777216.0f * s_val[last];
+    if (tid < last && coin < s_val[tid]) atomicMin(&s_last, tid);
+    __syncthreads();
+    if (tid == 0) *rng = st, *out = s_idx[s_last];
+}
+
+__global__ void __launch_bounds__(kSampThreads) kf_sample_kernel(int32_t* __restrict__ out, const uint16_t* __restrict__ logits, int vocab, float temperature,
+                                                                 int top_k, float top_p, unsigned long long* __restrict__ rng, int selection) {
+    __shared__ float s_val[kMaxTopK];
+    __shared__ int s_idx[kMaxTopK];
+    select_any(s_val, s_idx, logits + (size_t)blockIdx.x * vocab, vocab, top_k, selection);
+    draw(out + blockIdx.x, s_val, s_idx, top_k, temperature, top_p, rng + blockIdx.x);
+}
+
+// ---- up to kFastTopK candidates: ONE pass over the logits, held in registers by a cluster of CTAs per row --------------------------------------------
+// The single CTA above reads its row three times with 2-byte loads and sorts 1024 slots: 148 us at 8 rows of 151936 (a row is 304 KB: 0.4 us at the HBM
+// rate for all eight), all latency.  Here the row is spread over up to 8 CTAs, 24 logits per thread, loaded once.  The k-th largest of a CTA's
+// per-thread maxima bounds the k-th largest logit of the row from below (k threads hold one at least as large), so only what reaches the largest of
+// these bounds -- a few hundred logits -- is collected, and the first CTA finds the exact k-th key among them, ranks the survivors by counting and
+// draws: 152 -> 21.5 us a call.  Rows that leave too many (long runs of equal logits) or that hold NaN among the chosen take the general selection.
+constexpr int kFastTopK = 256, kFastPer = 24, kFastCtas = 8, kFastLocal = 2048, kFastTotal = 4096;
+
+// the number of threads of the CTA whose key reaches t, for the largest t that at least k reach (0: fewer than k hold a key)
+__device__ __forceinline__ uint32_t kth_bound(uint32_t key, int k) {
+    uint32_t t = 0;
+    for (int b = 16; b >= 0; b--) {
+        const uint32_t cand = t | (1u << b);
+        if (__syncthreads_count(key >= cand) >= k) t = cand;
+    }
+    return t;
+}
+__device__ __forceinline__ uint32_t ld_cluster_u32(const void* local_ptr, int cta_rank) {
+    uint32_t remote, v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"((uint32_t)__cvta_generic_to_shared(local_ptr)), "r"(cta_rank));
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(remote) : "memory");
+    return v;
+}
+
+template <bool VEC>
+__global__ void __launch_bounds__(kSampThreads) kf_sample_cluster_kernel(int32_t* __restrict__ out, const uint16_t* __restrict__ logits, int vocab, float temperature,
+                                                                         int k, float top_p, unsigned long long* __restrict__ rng, int ctas) {
+    __shared__ uint32_t s_key[kFastLocal], s_at[kFastLocal];  // this CTA's candidates: key (1 .. 65536), index
+    __shared__ uint32_t s_bound, s_n;
+    __shared__ uint32_t g_key[kFastTotal];                    // first CTA: the candidates of all
+    __shared__ float s_val[kMaxTopK];
+    __shared__ int s_idx[kMaxTopK];
+    __shared__ uint32_t s_cnt[20];
+    __shared__ int s_above, s_ties, s_nan;
+    const int tid = threadIdx.x, rank = blockIdx.x % ctas;
+    const uint16_t* row = logits + (size_t)(blockIdx.x / ctas) * vocab;
+    // ---- the one pass: keys in registers, two per word; 0 marks what lies past the end ----
+    uint32_t kk[kFastPer];
+#pragma unroll
+    for (int j = 0; j < kFastPer; j++) kk[j] = 0;
+    if (VEC) {
+#pragma unroll
+        for (int j = 0; j < kFastPer / 8; j++) {
+            const int i = ((j * ctas + rank) * kSampThreads + tid) * 8;
+            if (i < vocab) {
+                const uint4 v = __ldg(reinterpret_cast<const uint4*>(row + i));
+                const uint32_t q[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int e = 0; e < 4; e++) kk[8 * j + 2 * e] = order_key((uint16_t)q[e]) + 1, kk[8 * j + 2 * e + 1] = order_key((uint16_t)(q[e] >> 16)) + 1;
+            }
         }
-        for (int i = 0; i < k; i++) s_val[i] /= sum;
-        int n_pick = k;
-        if (top_p < 1.0f) {
-            float cum = 0.f;
-            int last  = k - 1;
-            for (int i = 0; i < k; i++) {
-                cum += s_val[i];
-                if (cum > top_p) {
-                    last = i;
-                    break;
+    } else {
+#pragma unroll
+        for (int j = 0; j < kFastPer; j++) {
+            const int i = (j * ctas + rank) * kSampThreads + tid;
+            if (i < vocab) kk[j] = order_key(__ldg(row + i)) + 1;
+        }
+    }
+    uint32_t mx = 0;
+#pragma unroll
+    for (int j = 0; j < kFastPer; j++) mx = max(mx, kk[j]);
+    uint32_t bound = max(kth_bound(mx, k), 1u);
+    if (tid == 0) s_bound = bound, s_n = 0;
+    if (tid < 20) s_cnt[tid] = 0;
+    __syncthreads();
+    if (ctas > 1) {
+        cluster_arrive();
+        cluster_wait();
+        for (int c = 0; c < ctas; c++) bound = max(bound, ld_cluster_u32(&s_bound, c));
+    }
+    // ---- what reaches the bound ----
+    if (mx >= bound) {
+#pragma unroll
+        for (int j = 0; j < kFastPer; j++)
+            if (kk[j] >= bound) {
+                const uint32_t at = atomicAdd(&s_n, 1u);
+                const int i = VEC ? (((j / 8) * ctas + rank) * kSampThreads + tid) * 8 + (j & 7) : (j * ctas + rank) * kSampThreads + tid;
+                if (at < (uint32_t)kFastLocal) s_key[at] = kk[j], s_at[at] = (uint32_t)i;
+            }
+    }
+    __syncthreads();
+    if (ctas > 1) {
+        cluster_arrive();
+        cluster_wait();
+    }
+    if (rank == 0) {
+        // ---- gather: thread t holds candidates t, t + 1024, .. of the concatenated lists ----
+        constexpr int PER = kFastTotal / kSampThreads;
+        uint32_t start[kFastCtas + 1];
+        start[0] = 0;
+        bool fits = true;
+        for (int c = 0; c < kFastCtas; c++) {
+            const uint32_t n = c < ctas ? (c ? ld_cluster_u32(&s_n, c) : s_n) : 0u;
+            fits = fits && n <= (uint32_t)kFastLocal;
+            start[c + 1] = start[c] + n;
+        }
+        const uint32_t total = start[kFastCtas];
+        fits = fits && total <= (uint32_t)kFastTotal;
+        uint32_t ck[PER], ci[PER];
+#pragma unroll
+        for (int j = 0; j < PER; j++) {
+            const uint32_t t = (uint32_t)(j * kSampThreads + tid);
+            ck[j] = 0, ci[j] = 0;
+            if (fits && t < total) {
+                int c = 0;
+#pragma unroll
+                for (int u = 1; u < kFastCtas; u++) c += t >= start[u];
+                uint32_t o = t;
+#pragma unroll
+                for (int u = 1; u < kFastCtas; u++)
+                    if (c == u) o = t - start[u];
+                ck[j] = ld_cluster_u32(&s_key[o], c), ci[j] = ld_cluster_u32(&s_at[o], c);
+            }
+        }
+        if (tid == 0) s_above = 0, s_ties = 0, s_nan = 0;
+        __syncthreads();
+        if (fits) {
+            // ---- the k-th largest key ----
+            uint32_t thr = 0;
+            for (int b = 16; b >= 0; b--) {
+                const uint32_t cand = thr | (1u << b);
+                int n = 0;
+#pragma unroll
+                for (int j = 0; j < PER; j++) n += ck[j] >= cand;
+                n = __reduce_add_sync(0xffffffffu, n);
+                if ((tid & 31) == 0 && n) atomicAdd(&s_cnt[b], (uint32_t)n);
+                __syncthreads();
+                if (s_cnt[b] >= (uint32_t)k) thr = cand;
+            }
+            // ---- everything above it (fewer than k), and the entries at it with the lowest indices ----
+            uint32_t* a_key = s_key;  // the local lists have been read
+            uint32_t* a_at  = s_at;
+            __syncthreads();
+#pragma unroll
+            for (int j = 0; j < PER; j++) {
+                if (ck[j] > thr) {
+                    const int at = atomicAdd(&s_above, 1);
+                    a_key[at] = ck[j], a_at[at] = ci[j];
+                } else if (ck[j] == thr && ck[j]) {
+                    g_key[atomicAdd(&s_ties, 1)] = ci[j];
                 }
             }
-            n_pick = last + 1;
-        }
-        float psum = 0.f;
-        for (int i = 0; i < n_pick; i++) psum += s_val[i];
-        unsigned long long st = rng[blockIdx.x];
-        const float coin      = (float)(xorshift_u32(&st) >> 8) / 16777216.0f * psum;
-        rng[blockIdx.x]       = st;
-        int q     = s_idx[n_pick - 1];
-        float cdf = 0.f;
-        for (int i = 0; i < n_pick; i++) {
-            cdf += s_val[i];
-            if (coin < cdf) {
-                q = s_idx[i];
-                break;
+            __syncthreads();
+            const int above = s_above, ties = s_ties;
+            for (int i = tid; i < ties; i += kSampThreads) {
+                const uint32_t me = g_key[i];
+                int before = 0;
+                for (int j = 0; j < ties; j++) before += g_key[j] < me;
+                if (above + before < k) a_key[above + before] = thr, a_at[above + before] = me;
             }
+            __syncthreads();
+            // ---- order by (value descending, index ascending): the two zeros are one value ----
+            if (tid < k) {
+                const uint32_t zero = 0x8001u, me = a_key[tid] == zero - 1 ? zero : a_key[tid], at = a_at[tid];
+                const uint32_t raw = a_key[tid] - 1;
+                int before = 0;
+                for (int j = 0; j < k; j++) {
+                    const uint32_t o = a_key[j] == zero - 1 ? zero : a_key[j];
+                    before += o > me || (o == me && a_at[j] < at);
+                }
+                const float v = bf16_bits_to_f32((uint16_t)((raw & 0x8000u) ? (raw & 0x7fffu) : ~raw));
+                if (v != v) s_nan = 1;
+                s_val[before] = v, s_idx[before] = (int)at;
+            }
+            __syncthreads();
+            fits = !s_nan;
         }
-        out[blockIdx.x] = q;
+        if (!fits) {
+            __syncthreads();
+            select_any(s_val, s_idx, row, vocab, k, 0);
+        }
+        draw(out + blockIdx.x / ctas, s_val, s_idx, k, temperature, top_p, rng + blockIdx.x / ctas);
+    }
+    if (ctas > 1) {  // the lists of the other CTAs stay until the first one has read them
+        cluster_arrive();
+        cluster_wait();
     }
 }
 }  // namespace
@@ -212,6 +396,22 @@ extern "C" int kf_sample(kf_ctx* ctx, int32_t* next_dev, const void* logits_bf16
     KF_REQUIRE(ctx, temperature > 0.0f && top_p > 0.0f && (selection == 0 || selection == 1), "temperature > 0, top_p > 0");
     if (top_k <= 0 || top_k > vocab) top_k = vocab;  // CHAT_SAMPLER: nCanTopK = min(top_k, n_vocab), GoPT.cpp:389
     KF_REQUIRE(ctx, top_k <= kMaxTopK && top_k < vocab / 2, "top_k <= 1024 candidates (and < vocab / 2, TOPK_heap::Select's own assert)");
+    if (selection == 0 && top_k <= kFastTopK && vocab <= kFastCtas * kSampThreads * kFastPer) {
+        // as few CTAs per row as hold 16 logits per thread: small rows in one CTA (no cluster barriers), Qwen3's 151936 in eight
+        int ctas = 1;
+        while (ctas < kFastCtas && vocab > ctas * kSampThreads * 16) ctas *= 2;
+        const bool vec = vocab % 8 == 0 && ((uintptr_t)logits_bf16_dev & 15) == 0;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)M * ctas), cfg.blockDim = dim3(kSampThreads), cfg.stream = ctx->stream;
+        cudaLaunchAttribute attr[1];
+        attr[0].id               = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)ctas, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr, cfg.numAttrs = ctas > 1 ? 1 : 0;
+        KF_CUDA(ctx, cudaLaunchKernelEx(&cfg, vec ? kf_sample_cluster_kernel<true> : kf_sample_cluster_kernel<false>, (int32_t*)next_dev, (const uint16_t*)logits_bf16_dev, vocab,
+                                        temperature, top_k, top_p, (unsigned long long*)rng_state_dev, ctas));
+        KF_LAUNCH_CHECK(ctx);
+        return KF_OK;
+    }
     kf_sample_kernel<<<M, kSampThreads, 0, ctx->stream>>>(next_dev, (const uint16_t*)logits_bf16_dev, vocab, temperature, top_k, top_p,
                                                           (unsigned long long*)rng_state_dev, selection);
     KF_LAUNCH_CHECK(ctx);

@@ -48,3 +48,42 @@ def test_tc_long_reduction(ctx, rows, cols, M):
             assert float(worst) < 1e-4, float(worst)
     finally:
         ctx.set_int("gemv_exact", exact)
+
+
+# ---------------------------------------------------------------------------------------------- sampler: one pass over the row by a cluster of CTAs
+def _rows(kind, M, vocab, rng):
+    if kind == "normal":
+        v = rng.standard_normal((M, vocab)) * 2.5
+    elif kind == "ties":  # a handful of values: the threshold falls into a long run of equal logits, lists overflow at the larger sizes
+        v = rng.integers(-3, 3, (M, vocab)).astype(np.float32)
+    elif kind == "zeros":  # the two zeros are one value, ordered by index
+        v = np.where(rng.random((M, vocab)) < 0.5, 0.0, -0.0)
+        v[:, ::7] = -1.0
+    elif kind == "few":  # the chosen ones sit side by side, the rest far below: infinities and the lowest value among it
+        v = np.full((M, vocab), -np.inf)
+        v[:, 1::3] = -3.3e38
+        v[:, 40:400] = rng.standard_normal((M, 360))
+    else:  # descending: the largest all in one thread block's part
+        v = np.tile(-np.arange(vocab, dtype=np.float64) / 64, (M, 1))
+    return ol.f32_to_bf16(v.astype(np.float32))
+
+
+@pytest.mark.parametrize("vocab,top_k", [(1000, 200), (1001, 2), (16384, 50), (16385, 256), (32768, 255), (49151, 50), (65544, 20), (151936, 50), (196608, 256),
+                                         (196609, 256), (151936, 257)])
+@pytest.mark.parametrize("kind", ["normal", "ties", "zeros", "few", "falling"])
+def test_sample_selection(ctx, kind, vocab, top_k):
+    """Tokens equal those of the CPU port (which shares no code): a high temperature makes every candidate as likely, so the token names a place in the sorted
+    list of candidates.  1 draw in 100 may differ (a coin within rounding of a boundary: the two exponentials differ in the last place)."""
+    M, rounds = 3, 12
+    rng = np.random.default_rng(vocab + top_k)
+    lg = _rows(kind, M, vocab, rng).reshape(M, vocab)
+    lgd = ctx.array(lg)
+    for T, top_p in ((1e4, 1.0), (0.8, 0.9)):
+        seeds = rng.integers(1, 2 ** 62, M).astype(np.uint64)
+        std, states, diff = ctx.array(seeds.view(np.uint16)), [[int(s)] for s in seeds], 0
+        for _ in range(rounds):
+            got = kf.sample(ctx, lgd, M, vocab, T, top_k, top_p, std, 0).numpy(np.int32)
+            for m in range(M):
+                diff += int(got[m] != ol.sample(lg[m], T, top_k, top_p, states[m], 0)[0])
+        assert diff <= 1, (T, diff)
+        assert np.array_equal(std.numpy(np.uint64), np.array([s[0] for s in states], dtype=np.uint64))
