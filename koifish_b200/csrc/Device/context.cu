@@ -163,6 +163,8 @@ extern "C" int kf_ctx_set_int(kf_ctx* ctx, const char* key, int value) {
         ctx->tp_fused = value;
     else if (!strcmp(key, "gemv_xg_min_m"))
         ctx->gemv_xg_min_m = value;
+    else if (!strcmp(key, "tc_bn"))
+        ctx->tc_bn = (value == 16 || value == 32 || value == 64 || value == 128 || value == 256) ? value : 0;
     else if (!strcmp(key, "deq_fma"))
         ctx->deq_fma = value ? 1 : 0;
     else if (!strcmp(key, "pdl"))

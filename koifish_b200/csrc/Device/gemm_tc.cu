@@ -19,7 +19,6 @@
 // bf16 weights need no expansion: warp 9 TMA-loads them straight into a swizzled A tile in shared memory (classic SS MMA).
 // The k order inside every 32-wide slot is the extraction-friendly permutation of gemv.cu; kf_tc_prepare_x permutes the activations
 // identically, so the contraction is unchanged.  Every barrier wait is bounded and traps instead of hanging the GPU.
-#include <cuda.h>
 #include <string.h>
 
 #include <algorithm>
@@ -27,6 +26,7 @@
 #include <tuple>
 
 #include "kf_common.cuh"
+#include "kf_tc.cuh"
 
 // tuning experiments (bit 0: no expansion, 1: no TMEM store, 2: no scale / zero fetch in the loop ...): debug builds only
 // (KF_NVCC_DEFS="-DKF_DEBUG_KNOBS -DKF_TC_EXP=n"); a release build compiles them out
@@ -55,6 +55,7 @@ __host__ __device__ constexpr int raw_bytes() { return (FMT == 3 || FMT == 4) ? 
 constexpr int kProducerWarps = 8, kMmaWarp = 8, kRawWarp = 9, kXWarp = 10, kEpiWarp0 = 11;
 constexpr int kThreadsTC = 15 * 32;
 
+constexpr int kEpiGlu = 2;  // epilogue: y = silu(w0 x) * (w1 x); an item takes 64 rows of either weight
 constexpr int kMaxW = 3;  // weights of one launch (Q/K/V, gate/up): same type, same K, their row tiles share one item space
 struct GemmParams {
     const uint16_t* zero[kMaxW];
@@ -68,6 +69,7 @@ struct GemmParams {
     int M, N, K;
     int qbias, gshift, epilogue;
     int n_tiles, m_tiles, splits, n_items;
+    int staged;                // outputs (and residual) may be accessed 16 bytes at a time
     uint32_t lop_mask, lop_magic;
 };
 
@@ -91,6 +93,8 @@ __host__ __device__ constexpr int tperm(int o) {
 template <int FMT>
 __global__ void __launch_bounds__(256) kf_permute_x_kernel(uint16_t* __restrict__ xp, const uint16_t* __restrict__ x, size_t n_slots) {
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;  // one 32-element slot per thread
+    kf_grid_dependency_wait();    // x comes from the kernel before us ...
+    kf_grid_launch_dependents();  // ... and only behind it may the matmul start to stream its weights (they might have been written there as well)
     if (i >= n_slots) return;
     const uint4* src = reinterpret_cast<const uint4*>(x + i * 32);
     uint32_t s[16];
@@ -116,6 +120,8 @@ template <int FMT>
 __global__ void __launch_bounds__(256) kf_rmsnorm_permute_kernel(uint16_t* __restrict__ xp, const uint16_t* __restrict__ x, const uint16_t* __restrict__ w,
                                                                   int dim, float eps) {
     __shared__ float red[32];
+    kf_grid_dependency_wait();  // as above
+    kf_grid_launch_dependents();
     const uint16_t* xr = x + (size_t)blockIdx.x * dim;
     uint16_t* orow     = xp + (size_t)blockIdx.x * dim;
     float ss = 0.f;
@@ -152,123 +158,6 @@ __global__ void __launch_bounds__(256) kf_rmsnorm_permute_kernel(uint16_t* __res
     }
 }
 
-// ---- PTX helpers ------------------------------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_a(uint32_t bar_addr) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar_addr) : "memory");
-}
-__device__ __forceinline__ uint32_t mbar_try(uint32_t a, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(a), "r"(parity)
-        : "memory");
-    return ok;
-}
-// bounded wait: a protocol bug traps (the launch fails with an error) instead of hanging the GPU
-__device__ __noinline__ void mbar_wait_slow(uint32_t a, uint32_t parity) {
-    for (uint32_t it = 0; it < (1u << 24); it++)
-        if (mbar_try(a, parity)) return;
-    __trap();
-}
-__device__ __forceinline__ void mbar_wait_a(uint32_t a, uint32_t parity) {
-    if (!mbar_try(a, parity)) mbar_wait_slow(a, parity);
-}
-__device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity) { mbar_wait_a(smem_u32(bar), parity); }
-// for the warps that wait a long time (epilogue): back off between polls so the spinning does not take issue slots from the producers
-__device__ __noinline__ void mbar_wait_sleepy(uint64_t* bar, uint32_t parity) {
-    const uint32_t a = smem_u32(bar);
-    for (uint32_t it = 0; it < (1u << 22); it++) {
-        if (mbar_try(a, parity)) return;
-        __nanosleep(200);
-    }
-    __trap();
-}
-__device__ __forceinline__ void lds128(uint32_t a, uint32_t* r) {
-    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
-}
-__device__ __forceinline__ void lds64(uint32_t a, uint32_t* r) {
-    asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(a) : "memory");
-}
-__device__ __forceinline__ uint32_t lds32(uint32_t a) {
-    uint32_t r;
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(r) : "r"(a) : "memory");
-    return r;
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* tm, int c0, int c1, uint64_t* bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)),
-                 "l"(tm), "r"(c0), "r"(c1), "r"(smem_u32(bar))
-                 : "memory");
-}
-// shared-memory matrix descriptor, K-major, SWIZZLE_128B, 8-row groups 1024 bytes apart (cute::UMMA::SmemDescriptor bit layout)
-__device__ __forceinline__ uint64_t make_desc_sw128(uint32_t smem_addr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((smem_addr & 0x3FFFF) >> 4);  // start address, 16-byte units          bits [0,14)
-    d |= (uint64_t)1 << 16;                       // leading byte offset (unused for swizzled K-major)   [16,30)
-    d |= (uint64_t)(1024 >> 4) << 32;             // stride byte offset between 8-row groups [32,46)
-    d |= (uint64_t)1 << 46;                       // descriptor version (Blackwell)           [46,48)
-    d |= (uint64_t)2 << 61;                       // layout type SWIZZLE_128B                 [61,64)
-    return d;
-}
-// instruction descriptor, kind::f16: D = fp32, A = B = bf16, both K-major, M = 128, N = n (cute::UMMA::InstrDescriptor bit layout)
-__host__ __device__ constexpr uint32_t make_idesc_bf16(int n) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
-}
-// The MMA / commit helpers are executed by the whole (converged) warp; elect.sync picks one lane -- the same one every time, so all
-// MMAs and the commits that track them come from a single thread -- and only that lane issues the instruction.
-__device__ __forceinline__ void umma_ss(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t"
-        "elect.sync _|q, 0xffffffff;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t"
-        "elect.sync _|q, 0xffffffff;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-__device__ __forceinline__ void umma_commit_a(uint32_t bar_addr) {
-    asm volatile(
-        "{\n\t.reg .pred q;\n\t"
-        "elect.sync _|q, 0xffffffff;\n\t"
-        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar_addr)
-        : "memory");
-}
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr), "r"(v[0]),
-                 "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]),
-                 "r"(v[13]), "r"(v[14]), "r"(v[15])
-                 : "memory");
-}
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]),
-                   "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-                 : "r"(taddr)
-                 : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
 __device__ __forceinline__ void epi_bar_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
 __device__ __forceinline__ uint32_t and_or3(uint32_t a, uint32_t b, uint32_t c) {
@@ -344,6 +233,7 @@ __device__ __forceinline__ int slot_offset(int q) {
 // Ring depths.  The three rings are decoupled because their latencies differ: the raw ring hides DRAM latency (bytes in flight per SM
 // = RS x 8 KB must cover ~2 us x 44 GB/s), the B ring hides the L2 round trip of the (small, L2-resident) activation tiles, the A ring
 // only the on-chip producer -> MMA hand-off.  Sized so that shared memory stays below ~210 KB and tensor memory within 512 columns.
+constexpr int kStageOut = 8 * 1024;  // one of the epilogue's two output buffers: 32 tokens x 128 rows in bf16, or 16 tokens in fp32
 template <int FMT, int BN>
 struct Rings {
     static constexpr bool A_TMEM = FMT != TF_BF16;
@@ -357,8 +247,8 @@ struct Rings {
                                            : (BN == 16 ? 10 : BN == 32 ? 10 : BN == 64 ? 8 : BN == 128 ? 6 : 4)) / U;
     static constexpr int RAWB    = raw_bytes<FMT>();
     static constexpr int RS      = !A_TMEM ? 0 : (BN <= 64 ? 128 : BN == 128 ? 112 : 80) * 1024 / (BM * RAWB);
-    static constexpr size_t SMEM = (size_t)SB * STAGE + (size_t)RS * BM * RAWB + 1024;
-    static_assert(SMEM <= 216 * 1024, "shared memory budget");
+    static constexpr size_t SMEM = (size_t)SB * STAGE + (size_t)RS * BM * RAWB + 2 * kStageOut + 1024;
+    static_assert(SMEM <= 226 * 1024, "shared memory budget");
 };
 
 struct Item {
@@ -373,8 +263,8 @@ __device__ __forceinline__ Item decode_item(const GemmParams& p, int item) {
     const int t  = item / p.m_tiles;
     it.z         = t % p.splits;
     const int tn = t / p.splits;
-    it.wi = (tn >= p.tile0[1] ? 1 : 0) + (tn >= p.tile0[2] ? 1 : 0);
-    it.n0 = (tn - p.tile0[it.wi]) * BM, it.m0 = mt, it.tile = tn * p.m_tiles + mt;  // m0 = token-tile index (the caller scales it by BN)
+    it.wi = p.epilogue == kEpiGlu ? 0 : (tn >= p.tile0[1] ? 1 : 0) + (tn >= p.tile0[2] ? 1 : 0);
+    it.n0 = p.epilogue == kEpiGlu ? tn * (BM / 2) : (tn - p.tile0[it.wi]) * BM, it.m0 = mt, it.tile = tn * p.m_tiles + mt;  // m0 = token-tile index (the caller scales it by BN)
     const int nkb  = p.K / BK;
     const int nraw = (nkb + KBR - 1) / KBR;
     const int base = nraw / p.splits, rem = nraw % p.splits;
@@ -437,6 +327,8 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     uint8_t* raws  = tiles + (size_t)SB * STAGE;
+    uint8_t* outs  = raws + (size_t)RS * RAW_BYTES;
+    const bool glu = p.epilogue == kEpiGlu;
     __shared__ uint64_t a_full[SA1], a_empty[SA1], b_full[SB], b_empty[SB], raw_full[RS1], raw_empty[RS1], tmem_full[NACC], tmem_empty[NACC];
     __shared__ uint32_t tmem_base_smem;
     __shared__ int last_flag;
@@ -479,9 +371,10 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
             uint32_t s = 0, eph = 1, rs = 0, rph = 0;  // ring positions and the parities to wait for
             for (int item = blockIdx.x; item < p.n_items; item += gridDim.x) {
                 const Item w = decode_item<KBR>(p, item);
-                const int grow       = min(w.n0 + row, p.Nw[w.wi] - 1);
-                const uint16_t* zrow = MODE == TM_PLAIN ? nullptr : p.zero[w.wi] + (size_t)grow * gpr;
-                const uint16_t* srow = MODE == TM_PLAIN ? nullptr : p.step[w.wi] + (size_t)grow * gpr;
+                const int seg        = glu ? row >> 6 : w.wi;
+                const int grow       = min(w.n0 + (glu ? row & 63 : row), p.Nw[seg] - 1);
+                const uint16_t* zrow = MODE == TM_PLAIN ? nullptr : p.zero[seg] + (size_t)grow * gpr;
+                const uint16_t* srow = MODE == TM_PLAIN ? nullptr : p.step[seg] + (size_t)grow * gpr;
                 // scale / zero of the current group and of the next two (register queue; the loads run 1-2 groups ahead of their use)
                 int gcur = 0;
                 uint32_t zq0 = 0, sq0 = 0, zq1 = 0, sq1 = 0, zq2 = 0, sq2 = 0;
@@ -594,6 +487,7 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
 #else
                         mbar_arrive_expect_tx(&raw_full[rs], RAW_BYTES);
                         tma_load_2d(raws + (size_t)rs * RAW_BYTES, tm_w, r * RAWB, w.n0, &raw_full[rs]);
+                        if (glu) tma_load_2d(raws + (size_t)rs * RAW_BYTES + RAW_BYTES / 2, &tm_w1, r * RAWB, w.n0, &raw_full[rs]);
 #endif
                         it++;
                     }
@@ -603,7 +497,10 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
                         mbar_wait(&b_empty[s], ((it / SB) & 1) ^ 1);
                         mbar_arrive_expect_tx(&b_full[s], U * A_BYTES);
 #pragma unroll
-                        for (int u = 0; u < U; u++) tma_load_2d(tiles + (size_t)s * STAGE + u * SUB, tm_w, (kb + u) * BK, w.n0, &b_full[s]);
+                        for (int u = 0; u < U; u++) {
+                            tma_load_2d(tiles + (size_t)s * STAGE + u * SUB, tm_w, (kb + u) * BK, w.n0, &b_full[s]);
+                            if (glu) tma_load_2d(tiles + (size_t)s * STAGE + u * SUB + A_BYTES / 2, &tm_w1, (kb + u) * BK, w.n0, &b_full[s]);
+                        }
                         it++;
                     }
                 }
@@ -684,12 +581,17 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
             ait++;
         }
     } else {
-        // ============ epilogue: TMEM -> registers -> Y (or split-K partial + ordered reduction by the last CTA) ============
+        // ============ epilogue: TMEM -> registers -> output buffer in shared memory -> Y in 16-byte accesses, 32 tokens at a time (fp32: 16); with split-K an
+        // fp32 partial + ordered reduction by the last CTA, through the same output buffers.  Straight from the registers (one 2-byte store per token and
+        // lane) the 256 tokens of an item took 10 us and another 12 with a residual, whose loads waited in front of every 16 tokens: 1024 x 4096 at 700
+        // tokens 19 / 31 us, of which the matrix instructions are 4 ============
         kf_grid_dependency_wait();  // residual / workspace / counters may still be in use by the previous kernel
         const int quad = warp & 3;
         const int row  = quad * 32 + lane;
         const int et   = (warp - kEpiWarp0) * 32 + lane;  // 0..127
-        uint32_t ait   = 0;
+        const bool f32out = p.epilogue == 4;
+        const int ch      = f32out ? 16 : 32;             // tokens per output buffer
+        uint32_t ait = 0, obuf = 0;
         for (int item = blockIdx.x; item < p.n_items; item += gridDim.x) {
             const Item w  = decode_item<KBR>(p, item);
             const int buf = ait % NACC;
@@ -699,6 +601,57 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
             const int N = p.Nw[w.wi];
             void* const y = p.y[w.wi];
             const bool row_ok = grow < N;
+            uint4 res[4];
+            // the residual of a buffer's four 16-byte pieces of this thread: piece i = token et / 16 + 8 i, rows 8 (et % 16) ..
+            auto fetch_res = [&](int c0) {
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const int t = c0 + (et >> 4) + 8 * i, n = w.n0 + (et & 15) * 8;
+                    res[i]      = t < cnt && n < N ? *reinterpret_cast<const uint4*>(p.residual + (size_t)(m0 + t) * N + n) : make_uint4(0, 0, 0, 0);
+                }
+            };
+            // output buffer -> Y
+            auto copy_out = [&](const uint8_t* o, int c0) {
+                if (glu) {
+#pragma unroll
+                    for (int i = 0; i < 2; i++) {
+                        const int t = (et >> 3) + 16 * i, n = w.n0 + (et & 7) * 8;
+                        if (c0 + t >= cnt || n >= N) continue;
+                        const uint4 g4 = *reinterpret_cast<const uint4*>(o + t * 256 + (et & 7) * 16), u4 = *reinterpret_cast<const uint4*>(o + t * 256 + 128 + (et & 7) * 16);
+                        const uint32_t g[4] = {g4.x, g4.y, g4.z, g4.w}, u[4] = {u4.x, u4.y, u4.z, u4.w};
+                        uint32_t v[4];
+#pragma unroll
+                        for (int j = 0; j < 4; j++) {  // CU_swiglu_v0 on the bf16 gate / up (Activation.cu:86-93), as kf_swiglu computes it
+                            const float g0 = bf16lo(g[j]), g1 = bf16hi(g[j]), u0 = bf16lo(u[j]), u1 = bf16hi(u[j]);
+                            v[j] = pack_bf16x2((g0 * u0) / (1.0f + expf(-g0)), (g1 * u1) / (1.0f + expf(-g1)));
+                        }
+                        *reinterpret_cast<uint4*>((uint16_t*)y + (size_t)(m0 + c0 + t) * N + n) = make_uint4(v[0], v[1], v[2], v[3]);
+                    }
+                } else if (f32out) {
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        const int t = (et >> 5) + 4 * i, n = w.n0 + lane * 4;
+                        if (c0 + t < cnt && n < N)
+                            *reinterpret_cast<uint4*>((float*)y + (size_t)(m0 + c0 + t) * N + n) = *reinterpret_cast<const uint4*>(o + t * 512 + lane * 16);
+                    }
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        const int t = (et >> 4) + 8 * i, n = w.n0 + (et & 15) * 8;
+                        if (c0 + t >= cnt || n >= N) continue;
+                        uint4 v4 = *reinterpret_cast<const uint4*>(o + t * 256 + (et & 15) * 16);
+                        if (p.epilogue == 1) {
+                            const uint32_t r[4] = {res[i].x, res[i].y, res[i].z, res[i].w};
+                            uint32_t v[4]       = {v4.x, v4.y, v4.z, v4.w};
+#pragma unroll
+                            for (int j = 0; j < 4; j++) v[j] = pack_bf16x2(bf16lo(r[j]) + bf16lo(v[j]), bf16hi(r[j]) + bf16hi(v[j]));
+                            v4 = make_uint4(v[0], v[1], v[2], v[3]);
+                        }
+                        *reinterpret_cast<uint4*>((uint16_t*)y + (size_t)(m0 + c0 + t) * N + n) = v4;
+                    }
+                }
+            };
+            if (p.staged && p.splits == 1 && p.epilogue == 1) fetch_res(0);
             if (NACC == 2)
                 mbar_wait_sleepy(&tmem_full[buf], (ait / NACC) & 1);  // a whole main loop away: poll politely
             else
@@ -706,23 +659,51 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
             tc_fence_after();
             const uint32_t tbase = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * BN);
             float* wsp = p.ws + ((size_t)w.tile * p.splits + w.z) * (size_t)(BN * BM);
-            for (int c0 = 0; c0 < cnt; c0 += 16) {
-                uint32_t v[16];
-                tmem_ld16(tbase + (uint32_t)c0, v);
-                if (p.splits > 1) {
+            auto release = [&]() {  // the accumulator buffer may be overwritten by the next item
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&tmem_empty[buf]);
+            };
+            if (p.splits == 1 && p.staged) {
+                for (int c0 = 0; c0 < cnt; c0 += ch, obuf ^= 1) {
+                    uint8_t* o = outs + obuf * kStageOut;
+                    if (f32out || BN < 32) {
+                        uint32_t v[16];
+                        tmem_ld16(tbase + (uint32_t)c0, v);
+                        if (c0 + ch >= cnt) release();
 #pragma unroll
-                    for (int j = 0; j < 16; j++)
-                        if (c0 + j < cnt) wsp[(size_t)(c0 + j) * BM + row] = __uint_as_float(v[j]);
-                } else if (row_ok) {
-                    float acc[16];
+                        for (int j = 0; j < 16; j++) {
+                            if (f32out) *reinterpret_cast<uint32_t*>(o + j * 512 + row * 4) = v[j];
+                            else *reinterpret_cast<uint16_t*>(o + j * 256 + row * 2) = f32_to_bf16_bits(__uint_as_float(v[j]));
+                        }
+                    } else {
+                        uint32_t v[32];
+                        tmem_ld32(tbase + (uint32_t)c0, v);
+                        if (c0 + ch >= cnt) release();
 #pragma unroll
-                    for (int j = 0; j < 16; j++) acc[j] = __uint_as_float(v[j]);
-                    store_cols<16>(p, y, N, acc, m0 + c0, cnt - c0, grow);
+                        for (int j = 0; j < 32; j++) *reinterpret_cast<uint16_t*>(o + j * 256 + row * 2) = f32_to_bf16_bits(__uint_as_float(v[j]));  // the reference's GEMM output is bf16 (gemm.cu:124-126)
+                    }
+                    epi_bar_sync();  // also: everybody has left the copy of the buffer before this one, which the next 32 tokens overwrite
+                    copy_out(o, c0);
+                    if (p.epilogue == 1 && c0 + ch < cnt) fetch_res(c0 + ch);
                 }
+            } else {
+                for (int c0 = 0; c0 < cnt; c0 += 16) {
+                    uint32_t v[16];
+                    tmem_ld16(tbase + (uint32_t)c0, v);
+                    if (p.splits > 1) {
+#pragma unroll
+                        for (int j = 0; j < 16; j++)
+                            if (c0 + j < cnt) wsp[(size_t)(c0 + j) * BM + row] = __uint_as_float(v[j]);
+                    } else if (row_ok) {
+                        float acc[16];
+#pragma unroll
+                        for (int j = 0; j < 16; j++) acc[j] = __uint_as_float(v[j]);
+                        store_cols<16>(p, y, N, acc, m0 + c0, cnt - c0, grow);
+                    }
+                }
+                release();
             }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&tmem_empty[buf]);  // the accumulator buffer may be overwritten by the next item
             ait++;
             if (p.splits > 1) {
                 __threadfence();
@@ -736,26 +717,39 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
                 if (last_flag) {
                     __threadfence();
                     const float* base = p.ws + (size_t)w.tile * p.splits * (size_t)(BN * BM);
-                    if (row_ok) {
-                        // 8 tokens x 2 partials in flight per thread; the partials are added in split order (deterministic)
-                        for (int j0 = 0; j0 < cnt; j0 += 8) {
-                            float acc[8];
-#pragma unroll
-                            for (int u = 0; u < 8; u++) acc[u] = 0.f;
-                            for (int z = 0; z < p.splits; z += 2) {
-                                float t0[8], t1[8];
-                                const float* b0 = base + (size_t)z * (BN * BM) + (size_t)j0 * BM + row;
-                                const bool two  = z + 1 < p.splits;
-#pragma unroll
-                                for (int u = 0; u < 8; u++) {
-                                    const bool ok = j0 + u < cnt;
-                                    t0[u] = ok ? __ldcg(b0 + u * BM) : 0.f;
-                                    t1[u] = (ok && two) ? __ldcg(b0 + BN * BM + u * BM) : 0.f;
-                                }
-#pragma unroll
-                                for (int u = 0; u < 8; u++) acc[u] = (acc[u] + t0[u]) + t1[u];
+                    // a thread sums four rows of one token (16-byte loads), two tokens and four partials in flight; the partials are added in split order
+                    for (int c0 = 0; c0 < cnt; c0 += ch, obuf ^= 1) {
+                        uint8_t* o = outs + obuf * kStageOut;
+                        if (p.epilogue == 1 && p.staged) fetch_res(c0);
+                        for (int t = et >> 5; t < ch && c0 + t < cnt; t += 8) {
+                            const bool two  = t + 4 < ch && c0 + t + 4 < cnt;
+                            const float* b0 = base + (size_t)(c0 + t) * BM + lane * 4;
+                            float4 s0 = make_float4(0.f, 0.f, 0.f, 0.f), s1 = s0;
+#pragma unroll 4
+                            for (int z = 0; z < p.splits; z++) {
+                                const float4 a = __ldcg(reinterpret_cast<const float4*>(b0 + (size_t)z * (BN * BM)));
+                                const float4 c = two ? __ldcg(reinterpret_cast<const float4*>(b0 + (size_t)z * (BN * BM) + 4 * BM)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                                s0.x += a.x, s0.y += a.y, s0.z += a.z, s0.w += a.w;
+                                s1.x += c.x, s1.y += c.y, s1.z += c.z, s1.w += c.w;
                             }
-                            store_cols<8>(p, y, N, acc, m0 + j0, cnt - j0, grow);
+                            auto put = [&](int tt, const float4& f) {
+                                if (p.staged) {
+                                    if (f32out) *reinterpret_cast<float4*>(o + tt * 512 + lane * 16) = f;
+                                    else *reinterpret_cast<uint2*>(o + tt * 256 + lane * 8) = make_uint2(pack_bf16x2(f.x, f.y), pack_bf16x2(f.z, f.w));
+                                    return;
+                                }
+                                const float v[4] = {f.x, f.y, f.z, f.w};
+                                for (int j = 0; j < 4; j++) {
+                                    const float one[1] = {v[j]};
+                                    if (w.n0 + lane * 4 + j < N) store_cols<1>(p, y, N, one, m0 + c0 + tt, 1, w.n0 + lane * 4 + j);
+                                }
+                            };
+                            put(t, s0);
+                            if (two) put(t + 4, s1);
+                        }
+                        if (p.staged) {
+                            epi_bar_sync();
+                            copy_out(o, c0);
                         }
                     }
                 }
@@ -793,7 +787,8 @@ EncodeTiledFn encode_fn() {
     }();
     return fn;
 }
-int make_map_2d(kf_ctx* ctx, CUtensorMap* tm, CUtensorMapDataType dt, int esize, const void* base, uint64_t inner, uint64_t outer, uint32_t box_inner,
+}  // namespace
+int kf_tmap_2d(kf_ctx* ctx, CUtensorMap* tm, CUtensorMapDataType dt, int esize, const void* base, uint64_t inner, uint64_t outer, uint32_t box_inner,
                 uint32_t box_outer, CUtensorMapSwizzle sw) {
     // a tensor map depends only on (address, geometry, box, swizzle): encode each once per context and reuse it (weights and the context's
     // activation scratch keep their addresses from token to token)
@@ -824,9 +819,17 @@ int make_map_2d(kf_ctx* ctx, CUtensorMap* tm, CUtensorMapDataType dt, int esize,
     (*cache)[key] = *tm;
     return KF_OK;
 }
+namespace {
 
+// Row tiles of a launch: 128 rows of one weight each, or (SwiGLU) 64 rows of gate and the same 64 of up
+int row_tiles(const GemmParams& p, int nw) {
+    if (p.epilogue == kEpiGlu) return (p.Nw[0] + BM / 2 - 1) / (BM / 2);
+    int n = 0;
+    for (int i = 0; i < nw; i++) n += (p.Nw[i] + BM - 1) / BM;
+    return n;
+}
 template <int FMT, int MODE, int BN>
-int launch_tc(kf_ctx* ctx, GemmParams& p, const void* const* wdata, int nw, const void* xp) {
+int launch_tc(kf_ctx* ctx, GemmParams& p, const void* const* wdata, int nw, const void* xp, int splits) {
     using F              = Fmt<FMT>;
     constexpr bool A_TMEM = FMT != TF_BF16;
     const size_t smem    = Rings<FMT, BN>::SMEM;
@@ -837,27 +840,14 @@ int launch_tc(kf_ctx* ctx, GemmParams& p, const void* const* wdata, int nw, cons
         attr_set[ctx->device] = true;
     }
     // ---- decomposition: row tiles x token tiles x split-K, walked round-robin by one CTA per SM ----
-    p.n_tiles = 0;
-    for (int i = 0; i <= kMaxW; i++) p.tile0[i] = 0x7fffffff;
-    for (int i = 0; i < nw; i++) p.tile0[i] = p.n_tiles, p.n_tiles += (p.Nw[i] + BM - 1) / BM;
-    p.m_tiles = (p.M + BN - 1) / BN;
-    const int nkb = p.K / BK, nraw = (nkb + F::KBR - 1) / F::KBR;
-    const int base_items = p.n_tiles * p.m_tiles;
-    int splits = 1;
-    if (ctx->gemv_splitk > 0) {
-        splits = ctx->gemv_splitk;
-    } else {
-        double best = 1e30;
-        for (int s = 1; s <= 16; s++) {
-            if (s > nraw) break;
-            const int waves  = (base_items * s + ctx->sm_count - 1) / ctx->sm_count;
-            // k-blocks per item + restart of the pipeline + (split) partial write / ordered fix-up, which grows with the token tile
-            const double len = (double)((nraw + s - 1) / s) * F::KBR + 2.0 + (s > 1 ? BN / 16.0 : 0.0);
-            const double c   = waves * len;
-            if (c < best * 0.95) best = c, splits = s;
-        }
+    const bool glu = p.epilogue == kEpiGlu;
+    for (int i = 0, n = 0; i <= kMaxW; i++) {
+        p.tile0[i] = i < nw && !(glu && i) ? n : 0x7fffffff;
+        if (i < nw) n += (p.Nw[i] + BM - 1) / BM;
     }
-    splits = std::max(1, std::min(splits, nraw));
+    p.n_tiles = row_tiles(p, nw);
+    p.m_tiles = (p.M + BN - 1) / BN;
+    const int base_items = p.n_tiles * p.m_tiles;
     p.splits = splits, p.n_items = base_items * splits;
     if (splits > 1) {
         int rc = kf_ensure_gemv_ws(ctx, (size_t)p.n_items * BN * BM * sizeof(float), base_items);
@@ -869,26 +859,55 @@ int launch_tc(kf_ctx* ctx, GemmParams& p, const void* const* wdata, int nw, cons
     for (int i = 0; i < kMaxW && !rc; i++) {
         const int j = i < nw ? i : 0;  // unused slots repeat the first weight (never dereferenced)
         if (A_TMEM)
-            rc = make_map_2d(ctx, &tm_w[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, wdata[j], (uint64_t)p.K * F::BITS / 8, (uint64_t)p.Nw[j], F::RAWB, BM,
-                             F::RAWB == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B);
+            rc = kf_tmap_2d(ctx, &tm_w[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, wdata[j], (uint64_t)p.K * F::BITS / 8, (uint64_t)p.Nw[j], F::RAWB, glu ? BM / 2 : BM,
+                            F::RAWB == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B);
         else
-            rc = make_map_2d(ctx, &tm_w[i], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, wdata[j], (uint64_t)p.K, (uint64_t)p.Nw[j], BK, BM,
-                             CU_TENSOR_MAP_SWIZZLE_128B);
+            rc = kf_tmap_2d(ctx, &tm_w[i], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, wdata[j], (uint64_t)p.K, (uint64_t)p.Nw[j], BK, glu ? BM / 2 : BM,
+                            CU_TENSOR_MAP_SWIZZLE_128B);
     }
-    if (!rc) rc = make_map_2d(ctx, &tm_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, xp, (uint64_t)p.K, (uint64_t)p.M, BK, BN, CU_TENSOR_MAP_SWIZZLE_128B);
+    if (!rc) rc = kf_tmap_2d(ctx, &tm_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, xp, (uint64_t)p.K, (uint64_t)p.M, BK, BN, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc) return rc;
     const int grid = std::min(p.n_items, ctx->sm_count);
     KF_CUDA(ctx, kf_launch_pdl(ctx, kern, dim3(grid), dim3(kThreadsTC), smem, tm_w[0], tm_w[1], tm_w[2], tm_x, p));
     KF_LAUNCH_CHECK(ctx);
     return KF_OK;
 }
+// Token tile and k-split by their modelled time: waves x (k-blocks x time per k-block + epilogue) + the fix-up of split sums.  The times per k-block of 64 are
+// measured ones (us; below 64 tokens the weights' bytes or their expansion, above the matrix instructions).  Splitting pays for few row tiles and a
+// handful of tokens only: 1024 x 3072 at 16 tokens 9.9 us in 8 parts against 15.7 whole, at 256 tokens 34 against 17.  (The rule before it charged BN / 16
+// k-blocks for the fix-up: 1024 x 3072 at 256 tokens went into 12 parts and took 91 us, now 17.5.)  The reference-exact arithmetic keeps that rule and the
+// order of sums it was compared in.
 template <int FMT, int MODE>
 int launch_tc_bn(kf_ctx* ctx, GemmParams& p, const void* const* wdata, int nw, const void* xp) {
-    if (p.M > 128) return launch_tc<FMT, MODE, 256>(ctx, p, wdata, nw, xp);
-    if (p.M > 64) return launch_tc<FMT, MODE, 128>(ctx, p, wdata, nw, xp);
-    if (p.M > 32) return launch_tc<FMT, MODE, 64>(ctx, p, wdata, nw, xp);
-    if (p.M > 16) return launch_tc<FMT, MODE, 32>(ctx, p, wdata, nw, xp);
-    return launch_tc<FMT, MODE, 16>(ctx, p, wdata, nw, xp);
+    constexpr int KBR = Fmt<FMT>::KBR;
+    const int nkb = p.K / BK, nraw = (nkb + KBR - 1) / KBR, tiles = row_tiles(p, nw);
+    int bn = 256, splits = 1;
+    double best = 1e30;
+    for (int b = 16, i = 0; b <= 256; b *= 2, i++) {
+        const int by_m = p.M > 128 ? 256 : p.M > 64 ? 128 : p.M > 32 ? 64 : p.M > 16 ? 32 : 16;  // one token tile where the panel fits one
+        if (ctx->tc_bn > 0 ? b != ctx->tc_bn : ctx->gemv_exact ? b != by_m : ((b < 256 && p.M > 8 * b) || (b > 16 && p.M <= b / 2))) continue;
+        static const double kb_packed[5] = {0.235, 0.235, 0.24, 0.26, 0.42}, kb_bf16[5] = {0.09, 0.10, 0.16, 0.24, 0.39};
+        const double t_kb = FMT == TF_BF16 ? kb_bf16[i] : kb_packed[i];
+        const int items   = tiles * ((p.M + b - 1) / b);
+        for (int s = 1; s <= 16 && s <= nraw; s++) {
+            if (ctx->gemv_splitk > 0 && s != std::min(ctx->gemv_splitk, nraw)) continue;
+            const int waves = (items * s + ctx->sm_count - 1) / ctx->sm_count, len = (nraw + s - 1) / s * KBR;
+            if (ctx->gemv_exact) {
+                const double c = waves * (len + 2.0 + (s > 1 ? b / 16.0 : 0.0));
+                if (c < best * 0.95) best = c, bn = b, splits = s;
+                continue;
+            }
+            const double t = waves * (len * t_kb + 0.5 + 0.006 * b + (s > 1 ? 0.5 + 0.02 * b : 0.0)) + (s > 1 ? b * (0.03 + 0.008 * s) : 0.0);
+            if (t < best * 0.98) best = t, bn = b, splits = s;
+        }
+    }
+    switch (bn) {
+        case 256: return launch_tc<FMT, MODE, 256>(ctx, p, wdata, nw, xp, splits);
+        case 128: return launch_tc<FMT, MODE, 128>(ctx, p, wdata, nw, xp, splits);
+        case 64: return launch_tc<FMT, MODE, 64>(ctx, p, wdata, nw, xp, splits);
+        case 32: return launch_tc<FMT, MODE, 32>(ctx, p, wdata, nw, xp, splits);
+        default: return launch_tc<FMT, MODE, 16>(ctx, p, wdata, nw, xp, splits);
+    }
 }
 
 int tc_format(const kf_tensor_desc* w, int* fmt, int* mode, int deq_fma) {
@@ -925,11 +944,11 @@ int kf_tc_prepare_x(kf_ctx* ctx, const kf_tensor_desc* w, const void* x, int M, 
     const size_t n_slots  = (size_t)M * K / 32;
     const unsigned blocks = (unsigned)((n_slots + 255) / 256);
     if (fmt == TF_Q4)
-        kf_permute_x_kernel<TF_Q4><<<blocks, 256, 0, ctx->stream>>>((uint16_t*)ctx->xperm, (const uint16_t*)x, n_slots);
+        KF_CUDA(ctx, kf_launch_pdl(ctx, kf_permute_x_kernel<TF_Q4>, dim3(blocks), dim3(256), 0, (uint16_t*)ctx->xperm, (const uint16_t*)x, n_slots));
     else if (fmt == TF_Q2)
-        kf_permute_x_kernel<TF_Q2><<<blocks, 256, 0, ctx->stream>>>((uint16_t*)ctx->xperm, (const uint16_t*)x, n_slots);
+        KF_CUDA(ctx, kf_launch_pdl(ctx, kf_permute_x_kernel<TF_Q2>, dim3(blocks), dim3(256), 0, (uint16_t*)ctx->xperm, (const uint16_t*)x, n_slots));
     else
-        kf_permute_x_kernel<TF_Q1><<<blocks, 256, 0, ctx->stream>>>((uint16_t*)ctx->xperm, (const uint16_t*)x, n_slots);
+        KF_CUDA(ctx, kf_launch_pdl(ctx, kf_permute_x_kernel<TF_Q1>, dim3(blocks), dim3(256), 0, (uint16_t*)ctx->xperm, (const uint16_t*)x, n_slots));
     KF_LAUNCH_CHECK(ctx);
     *xp_out = ctx->xperm;
     return KF_OK;
@@ -949,11 +968,11 @@ int kf_tc_prepare_x_norm(kf_ctx* ctx, const kf_tensor_desc* w, const void* x, co
     int rc = kf_ensure_buf(ctx, &ctx->xperm, &ctx->xperm_bytes, (size_t)M * K * 2);
     if (rc) return rc;
     if (fmt == TF_Q4)
-        kf_rmsnorm_permute_kernel<TF_Q4><<<M, 256, 0, ctx->stream>>>((uint16_t*)ctx->xperm, (const uint16_t*)x, (const uint16_t*)norm_w, K, eps);
+        KF_CUDA(ctx, kf_launch_pdl(ctx, kf_rmsnorm_permute_kernel<TF_Q4>, dim3(M), dim3(256), 0, (uint16_t*)ctx->xperm, (const uint16_t*)x, (const uint16_t*)norm_w, K, eps));
     else if (fmt == TF_Q2)
-        kf_rmsnorm_permute_kernel<TF_Q2><<<M, 256, 0, ctx->stream>>>((uint16_t*)ctx->xperm, (const uint16_t*)x, (const uint16_t*)norm_w, K, eps);
+        KF_CUDA(ctx, kf_launch_pdl(ctx, kf_rmsnorm_permute_kernel<TF_Q2>, dim3(M), dim3(256), 0, (uint16_t*)ctx->xperm, (const uint16_t*)x, (const uint16_t*)norm_w, K, eps));
     else
-        kf_rmsnorm_permute_kernel<TF_Q1><<<M, 256, 0, ctx->stream>>>((uint16_t*)ctx->xperm, (const uint16_t*)x, (const uint16_t*)norm_w, K, eps);
+        KF_CUDA(ctx, kf_launch_pdl(ctx, kf_rmsnorm_permute_kernel<TF_Q1>, dim3(M), dim3(256), 0, (uint16_t*)ctx->xperm, (const uint16_t*)x, (const uint16_t*)norm_w, K, eps));
     KF_LAUNCH_CHECK(ctx);
     *xp_out = ctx->xperm;
     return KF_OK;
@@ -999,6 +1018,9 @@ int kf_gemm_tc_multi(kf_ctx* ctx, int n, void* const* y, const kf_tensor_desc* w
         p.gshift = gs;
     }
     if (epilogue == 1) KF_REQUIRE(ctx, residual && n == 1, "residual: single weight");
+    p.staged = ((uintptr_t)residual & 15) == 0;
+    for (int i = 0; i < n; i++) p.staged = p.staged && ((uintptr_t)y[i] & 15) == 0;
+    if (epilogue == kEpiGlu) KF_REQUIRE(ctx, n == 2 && w[0].rows == w[1].rows && y[0] == y[1] && p.staged, "SwiGLU: gate and up of equal shape, one 16-byte aligned output");
 #define KF_TC_CASE(F, MD) \
     if (fmt == F && mode == MD) return launch_tc_bn<F, MD>(ctx, p, wdata, n, xp);
     KF_TC_CASE(TF_Q4, TM_AFFINE_FMA)

@@ -142,6 +142,10 @@ static int linear_any(kf_ctx* ctx, int n, void* const* y, const kf_tensor_desc* 
         rc = kf_tc_prepare_x(ctx, &w[0], xin, M, &xp);
         if (rc) return rc;
     }
+    if (epilogue == 2 && tc_fusable(&w[0], &w[1]) && ((uintptr_t)y[0] & 15) == 0) {  // gate, up and CU_swiglu_v0 in one launch
+        void* yy[2] = {y[0], y[0]};
+        return kf_gemm_tc_multi(ctx, 2, yy, w, xp, M, 2, nullptr);
+    }
     if (epilogue == 2) {
         const size_t bytes = (size_t)M * w[0].rows * 2;
         rc = kf_ensure_buf(ctx, &ctx->tmp0, &ctx->tmp0_bytes, bytes);

@@ -87,3 +87,58 @@ def test_sample_selection(ctx, kind, vocab, top_k):
                 diff += int(got[m] != ol.sample(lg[m], T, top_k, top_p, states[m], 0)[0])
         assert diff <= 1, (T, diff)
         assert np.array_equal(std.numpy(np.uint64), np.array([s[0] for s in states], dtype=np.uint64))
+
+
+# ---------------------------------------------------------------------------------------------- tcgen05 matmul: token tiles, k-splits, epilogues
+def _ptr(t):
+    return t.data_ptr()
+
+
+@pytest.mark.parametrize("typ", [kf.KF_T_Q4, kf.KF_T_BINARY, kf.KF_T_F8E5M2, kf.KF_T_BF16])
+@pytest.mark.parametrize("M,tc_bn,splits", [(9, 16, 1), (9, 32, 3), (17, 16, 2), (33, 64, 0), (64, 32, 5), (65, 128, 1), (129, 64, 1), (130, 256, 2), (255, 128, 3),
+                                            (257, 0, 0), (300, 256, 1)])
+@pytest.mark.parametrize("rows,cols", [(16, 128), (144, 1152), (272, 640)])
+def test_tc_tiles_and_epilogues(ctx, typ, M, tc_bn, splits, rows, cols):
+    """Every epilogue (plain, residual in place, fp32, SwiGLU) over ragged token and row tiles, whole and split reductions, aligned and misaligned outputs.
+    Weights and activations are exact on both sides and the sums are fp32 (1e-5 of the rms covers their order), so a bf16 result (8 significant bits) is off by one rounding,
+    2^-8 of itself, the residual form by two; SwiGLU rounds gate and up as well, whose errors pass through |d silu| < 1.1."""
+    import torch
+    torch.backends.cuda.matmul.allow_tf32 = False
+    mk = lambda seed: (make_q(ctx, typ, rows, cols, seed) if typ != kf.KF_T_BF16 else _bf16_weight(ctx, rows, cols, seed))  # noqa: E731
+    (w, wd), (u, ud) = mk(5), mk(6)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(M)
+    x = torch.randn(M, cols, generator=g, device="cuda").bfloat16()
+    r = torch.randn(M, rows, generator=g, device="cuda").bfloat16()
+    acc, up = x.float() @ wd.T, x.float() @ ud.T
+    eps, tiny = 2.0 ** -8 * 1.001, 1e-5 * float(acc.square().mean().sqrt())
+    want_glu = acc * torch.sigmoid(acc) * up
+    import ctypes as C
+    dw, du = w.desc(), u.desc()
+    gu = (kf.TensorDesc * 2)(dw, du)
+    ctx.set_int("tc_min_m", 1), ctx.set_int("tc_bn", tc_bn), ctx.set_int("gemv_splitk", splits)
+    try:
+        for off in (0, 1):  # elements that the output lies behind a 16-byte boundary
+            def out(dtype):
+                return torch.zeros(M * rows + off, dtype=dtype, device="cuda")[off:].view(M, rows)
+            y, yr, yf, yg = out(torch.bfloat16), out(torch.bfloat16), out(torch.float32), out(torch.bfloat16)
+            yr.copy_(r)
+            torch.cuda.synchronize()
+            ctx.check(ctx.lib.kf_linear(ctx.h, _ptr(y), C.byref(dw), _ptr(x), M, kf.KF_EPI_NONE, None), "none")
+            ctx.check(ctx.lib.kf_linear(ctx.h, _ptr(yr), C.byref(dw), _ptr(x), M, kf.KF_EPI_RESIDUAL, _ptr(yr)), "residual")
+            ctx.check(ctx.lib.kf_linear(ctx.h, _ptr(yf), C.byref(dw), _ptr(x), M, kf.KF_EPI_F32, None), "f32")
+            ctx.check(ctx.lib.kf_linear_swiglu(ctx.h, _ptr(yg), C.byref(gu[0]), C.byref(gu[1]), _ptr(x), M), "swiglu")
+            ctx.sync()
+            assert bool(((yf - acc).abs() <= tiny).all())
+            assert bool(((y.float() - acc).abs() <= eps * acc.abs() + tiny).all())
+            assert bool(((yr.float() - (r.float() + acc)).abs() <= eps * (acc.abs() + (r.float() + acc).abs()) * 1.02 + tiny).all())
+            bound = 1.1 * eps * acc.abs() * up.abs() + 2.1 * eps * want_glu.abs() + tiny * (up.abs() + acc.abs() + 1)
+            assert bool(((yg.float() - want_glu).abs() <= bound * 1.02).all())
+    finally:
+        ctx.set_int("tc_min_m", -1), ctx.set_int("tc_bn", 0), ctx.set_int("gemv_splitk", 0)
+
+
+def _bf16_weight(ctx, rows, cols, seed):
+    d = kf.fill_normal(ctx, rows * cols, seed, 0.02)
+    bits = d.numpy(np.uint16)
+    return kf.QTensor.from_packed(ctx, bits.view(np.uint8), None, rows, cols, kf.KF_T_BF16), bf16_tensor(d, rows, cols).float()
