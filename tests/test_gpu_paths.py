@@ -142,3 +142,36 @@ def _bf16_weight(ctx, rows, cols, seed):
     d = kf.fill_normal(ctx, rows * cols, seed, 0.02)
     bits = d.numpy(np.uint16)
     return kf.QTensor.from_packed(ctx, bits.view(np.uint8), None, rows, cols, kf.KF_T_BF16), bf16_tensor(d, rows, cols).float()
+
+
+# ---------------------------------------------------------------------------------------------- panel attention on tcgen05
+@pytest.mark.parametrize("n_head,n_kv", [(2, 1), (16, 8), (32, 8)])
+@pytest.mark.parametrize("M,pos0,behind", [(65, 0, 0), (128, 0, 300), (129, 0, 1), (200, 1, 57), (127, 128, 1), (256, 127, 129), (100, 700, 60), (513, 255, 0), (300, 4000, 90)])
+@pytest.mark.parametrize("sharp", [1.0, 12.0])
+def test_prefill_tc(ctx, n_head, n_kv, M, pos0, behind, sharp):
+    """Ragged query and key tiles, cache rows behind the last position that hold no numbers, flat and peaked scores (maxima that grow along the keys: the
+    rescaling of the output).  A weight is rounded to bf16 once (2^-8 of itself), the result once, scores and sums are fp32:
+    |error| <= 2^-8 (sum p |v| + |out|) + 1e-4 of that for the fp32 parts."""
+    import torch
+    hd, max_seq = 128, pos0 + M + behind
+    g = torch.Generator(device="cuda")
+    g.manual_seed(M + pos0 + n_head)
+    q = (torch.randn(M, n_head, hd, generator=g, device="cuda") * sharp).bfloat16()
+    k, v = (torch.randn(max_seq, n_kv, hd, generator=g, device="cuda") for _ in range(2))
+    k = (k * torch.linspace(0.2, 1.5, max_seq, device="cuda")[:, None, None]).bfloat16()
+    v = v.bfloat16()
+    k[pos0 + M:], v[pos0 + M:] = float("nan"), float("inf")
+    pos = torch.arange(pos0, pos0 + M, dtype=torch.int32, device="cuda")
+    out = torch.full((M, n_head, hd), 7.0, device="cuda").bfloat16()
+    torch.cuda.synchronize()
+    ctx.check(ctx.lib.kf_attn_prefill(ctx.h, _ptr(out), _ptr(q), _ptr(k), _ptr(v), _ptr(pos), M, n_head, n_kv, hd, max_seq), "prefill")
+    ctx.sync()
+    assert ctx.get_int("attn_tc_error") == 0
+    keys = torch.arange(pos0 + M, device="cuda")
+    for h in range(n_head):
+        kk, vv = k[:pos0 + M, h // (n_head // n_kv)].double(), v[:pos0 + M, h // (n_head // n_kv)].double()
+        s = q[:, h].double() @ kk.T / hd ** 0.5
+        p = torch.softmax(s.masked_fill(keys[None] > pos[:, None], float("-inf")), -1)
+        want, mass = p @ vv, p @ vv.abs()
+        err = (out[:, h].double() - want).abs()
+        assert bool((err <= 2.0 ** -8 * 1.01 * (mass + want.abs()) + 1e-6).all()), (h, float((err / (mass + want.abs())).max()))
