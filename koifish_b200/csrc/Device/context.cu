@@ -146,6 +146,8 @@ extern "C" int kf_ctx_get_int(kf_ctx* ctx, const char* key, int* value_out) {
         *value_out = ctx->gemv_xg_min_m;
     else if (!strcmp(key, "attn_tc_error"))
         *value_out = kf_attn_prefill_tc_error();
+    else if (!strcmp(key, "attn_gqa_error"))
+        *value_out = kf_attn_gqa_error();
     else
         return KF_ERR_BAD_ARG;
     return KF_OK;

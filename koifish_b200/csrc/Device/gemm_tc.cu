@@ -772,9 +772,10 @@ struct TmapKey {
     const void* base;
     uint64_t inner, outer;
     uint32_t box_inner, box_outer, dt, sw, esize;
+    uint64_t planes, plane_stride;  // third dimension (1: a matrix)
     bool operator<(const TmapKey& o) const {
-        return std::tie(base, inner, outer, box_inner, box_outer, dt, sw, esize) <
-               std::tie(o.base, o.inner, o.outer, o.box_inner, o.box_outer, o.dt, o.sw, o.esize);
+        return std::tie(base, inner, outer, box_inner, box_outer, dt, sw, esize, planes, plane_stride) <
+               std::tie(o.base, o.inner, o.outer, o.box_inner, o.box_outer, o.dt, o.sw, o.esize, o.planes, o.plane_stride);
     }
 };
 using TmapCache = std::map<TmapKey, CUtensorMap>;
@@ -788,11 +789,11 @@ EncodeTiledFn encode_fn() {
     return fn;
 }
 }  // namespace
-int kf_tmap_2d(kf_ctx* ctx, CUtensorMap* tm, CUtensorMapDataType dt, int esize, const void* base, uint64_t inner, uint64_t outer, uint32_t box_inner,
-                uint32_t box_outer, CUtensorMapSwizzle sw) {
+static int tmap_encode(kf_ctx* ctx, CUtensorMap* tm, CUtensorMapDataType dt, int esize, const void* base, uint64_t inner, uint64_t outer, uint32_t box_inner,
+                       uint32_t box_outer, CUtensorMapSwizzle sw, uint64_t planes, uint64_t plane_stride) {
     // a tensor map depends only on (address, geometry, box, swizzle): encode each once per context and reuse it (weights and the context's
     // activation scratch keep their addresses from token to token)
-    TmapKey key = {base, inner, outer, box_inner, box_outer, (uint32_t)dt, (uint32_t)sw, (uint32_t)esize};
+    TmapKey key = {base, inner, outer, box_inner, box_outer, (uint32_t)dt, (uint32_t)sw, (uint32_t)esize, planes, plane_stride};
     TmapCache* cache = reinterpret_cast<TmapCache*>(ctx->tmap_cache);
     if (!cache) ctx->tmap_cache = cache = new TmapCache();
     auto hit = cache->find(key);
@@ -803,11 +804,11 @@ int kf_tmap_2d(kf_ctx* ctx, CUtensorMap* tm, CUtensorMapDataType dt, int esize, 
     EncodeTiledFn fn = encode_fn();
     KF_REQUIRE(ctx, fn != nullptr, "cuTensorMapEncodeTiled not available from the driver");
     KF_REQUIRE(ctx, ((uintptr_t)base & 15) == 0 && (inner * esize) % 16 == 0, "TMA needs 16-byte aligned rows");
-    cuuint64_t dims[2]    = {inner, outer};
-    cuuint64_t strides[1] = {inner * (uint64_t)esize};
-    cuuint32_t box[2]     = {box_inner, box_outer};
-    cuuint32_t estr[2]    = {1, 1};
-    CUresult r = fn(tm, dt, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+    cuuint64_t dims[3]    = {inner, outer, planes};
+    cuuint64_t strides[2] = {inner * (uint64_t)esize, plane_stride};
+    cuuint32_t box[3]     = {box_inner, box_outer, 1};
+    cuuint32_t estr[3]    = {1, 1, 1};
+    CUresult r = fn(tm, dt, plane_stride ? 3 : 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) {
         char b[128];
@@ -818,6 +819,14 @@ int kf_tmap_2d(kf_ctx* ctx, CUtensorMap* tm, CUtensorMapDataType dt, int esize, 
     if (cache->size() > 4096) cache->clear();  // models hold a few hundred weights; bound it anyway
     (*cache)[key] = *tm;
     return KF_OK;
+}
+int kf_tmap_2d(kf_ctx* ctx, CUtensorMap* tm, CUtensorMapDataType dt, int esize, const void* base, uint64_t inner, uint64_t outer, uint32_t box_inner,
+               uint32_t box_outer, CUtensorMapSwizzle sw) {
+    return tmap_encode(ctx, tm, dt, esize, base, inner, outer, box_inner, box_outer, sw, 1, 0);
+}
+int kf_tmap_rows(kf_ctx* ctx, CUtensorMap* tm, const void* base, uint64_t inner, uint64_t rows, uint64_t planes, uint64_t plane_stride, uint32_t box_inner,
+                 uint32_t box_rows) {
+    return tmap_encode(ctx, tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, inner, rows, box_inner, box_rows, CU_TENSOR_MAP_SWIZZLE_128B, planes, plane_stride);
 }
 namespace {
 

@@ -167,6 +167,7 @@ int kf_gemm_tc(kf_ctx* ctx, void* y, const kf_tensor_desc* w, const void* xp, in
 int kf_attn_prefill_tc_ok(const kf_ctx* ctx, const void* out, const void* q, const void* kc, const void* vc, int M, int n_head, int n_kv, int hd);
 int kf_attn_prefill_tc(kf_ctx* ctx, void* out, const void* q, const void* kc, const void* vc, const int32_t* pos_dev, int M, int n_head, int n_kv, int max_seq);
 int kf_attn_prefill_tc_error();
+int kf_attn_gqa_error();  // attn_gqa.cu
 int kf_gemm_tc_multi(kf_ctx* ctx, int n, void* const* y, const kf_tensor_desc* w, const void* xp, int M, int epilogue, const void* residual);
 
 #ifdef __CUDACC__

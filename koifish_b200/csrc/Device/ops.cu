@@ -75,6 +75,7 @@ __global__ void kf_qknorm_rope_kv_kernel(uint16_t* __restrict__ q, const uint16_
                                          uint16_t* __restrict__ vcache, const float2* __restrict__ table, const int32_t* __restrict__ pos_dev,
                                          int n_head, int n_kv, int hd, float eps, size_t seq_stride) {
     __shared__ float red[32];
+    kf_grid_launch_dependents();  // the attention behind us may set itself up; it waits for our end before it reads anything
     const int m = blockIdx.y, h = blockIdx.x, j = threadIdx.x, half = hd / 2;
     const int pos   = pos_dev[m];
     const bool is_q = h < n_head;

@@ -175,3 +175,43 @@ def test_prefill_tc(ctx, n_head, n_kv, M, pos0, behind, sharp):
         want, mass = p @ vv, p @ vv.abs()
         err = (out[:, h].double() - want).abs()
         assert bool((err <= 2.0 ** -8 * 1.01 * (mass + want.abs()) + 1e-6).all()), (h, float((err / (mass + want.abs())).max()))
+
+
+# ---------------------------------------------------------------------------------------------- grouped decode attention
+@pytest.mark.parametrize("hd,n_head,n_kv", [(128, 8, 8), (128, 16, 8), (128, 16, 1), (128, 24, 2), (64, 8, 2)])
+@pytest.mark.parametrize("lens,hint", [((1,), 0), ((63, 64, 65, 1, 128, 129), 128), ((256, 257, 511, 513, 40), 512), ((2000, 3, 700, 1300), 1999), ((9000,), 8999), ((9000,), 100),
+                                       ((5000, 17), 300), ((40000,), 65535)])
+def test_gqa_runs(ctx, hd, n_head, n_kv, lens, hint):
+    """Edges of tiles and runs, lengths of their own, hints that are too small or too large, cache rows behind the last position that hold no numbers, again on
+    used workspaces.  Bound as for the panel kernel: one rounding of the weights, one of the result."""
+    import torch
+    M, max_seq = len(lens), max(lens) + 70
+    g = torch.Generator(device="cuda")
+    g.manual_seed(sum(lens) + n_head)
+    q = (torch.randn(M, n_head, hd, generator=g, device="cuda") * 2).bfloat16()
+    k, v = (torch.randn(M, max_seq, n_kv, hd, generator=g, device="cuda").bfloat16() for _ in range(2))
+    for i, n in enumerate(lens):
+        k[i, n:], v[i, n:] = float("nan"), float("inf")
+    pos = torch.tensor([n - 1 for n in lens], dtype=torch.int32, device="cuda")
+    out = torch.full((M, n_head, hd), 7.0, device="cuda").bfloat16()
+    stride = max_seq * n_kv * hd
+    torch.cuda.synchronize()
+    first = None
+    for split in (0, 0, 3):
+        ctx.set_int("attn_split", split)
+        try:
+            ctx.check(ctx.lib.kf_attn_decode_gqa(ctx.h, _ptr(out), _ptr(q), _ptr(k), _ptr(v), _ptr(pos), M, n_head, n_kv, hd, max_seq, hint, stride), "gqa")
+            ctx.sync()
+        finally:
+            ctx.set_int("attn_split", 0)
+        assert ctx.get_int("attn_gqa_error") == 0
+        if split == 0 and first is not None:
+            assert torch.equal(out, first)
+        first = out.clone() if split == 0 else first
+        for i, n in enumerate(lens):
+            for h in range(n_head):
+                kk, vv = k[i, :n, h // (n_head // n_kv)].double(), v[i, :n, h // (n_head // n_kv)].double()
+                p = torch.softmax(kk @ q[i, h].double() / hd ** 0.5, 0)
+                want, mass = p @ vv, p @ vv.abs()
+                err = (out[i, h].double() - want).abs()
+                assert bool((err <= 2.0 ** -8 * 1.01 * (mass + want.abs()) + 1e-6).all()), (split, i, h, float((err / (mass + want.abs())).max()))
