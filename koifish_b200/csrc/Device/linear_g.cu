@@ -7,8 +7,8 @@
 //   * DUAL form: two weight tables A, B of equal shape and y = silu(A x) * (B x), the gate / up pair of a gated feed-forward, or its clamped
 //     form y = g sigmoid(alpha g) (u + shift) with g = min(A x, limit), u = clamp(B x, -limit, limit);
 //   * "batch" form for a handful of rows: several weights, each with an input and an output of its own, in one launch.
-// Two kernels: a warp-per-output GEMV for a handful of rows (decode: every weight row is read once, 16-byte loads when the row length
-// allows) and a 64 x 64 x 32 shared-memory tile kernel for panels (mma.sync m16n8k16 for bf16 activations, FFMA for float ones).
+// A warp-per-output GEMV for a handful of rows (decode: every weight row is read once, 16-byte loads when the row length allows) and 64 x 64 shared-memory tile
+// kernels for panels: a cp.async ring with mma.sync m16n8k16 for bf16 activations, FFMA for float ones (which also takes bf16 rows of odd lengths).
 // No reference equivalent: the reference's SLP::Forw hands every shape to cuBLASLt (src/Device/CUDA/NeuronFuse.cu:305-381).
 #include <algorithm>
 
@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(256) kf_lin_skinny_mma_kernel(LinArgs a) {
 }
 
 template <typename TA, bool DUAL>
-__global__ void __launch_bounds__(256) kf_lin_tile_kernel(LinArgs a) {
+__global__ void __launch_bounds__(256) kf_lin_tile_any_kernel(LinArgs a) {
     const int g    = blockIdx.z;
     const int lo   = a.offsets ? a.offsets[g] : 0;
     const int hi   = a.offsets ? a.offsets[g + 1] : a.M;
@@ -457,6 +457,138 @@ __global__ void __launch_bounds__(256) kf_lin_tile_kernel(LinArgs a) {
     }
 }
 
+// bf16 activations: 64 slots x 64 outputs (of either weight, DUAL) per CTA, k in steps of 64 through a ring of stages filled by cp.async, 8 warps as 4 (m) x 2 (n) on
+// mma.sync m16n8k16.  The weights of a routed panel are the traffic (64 experts of 2 x 1408 x 2048: 738 MB), so the ring is there to keep bytes on their way: two
+// CTAs per SM with three of four stages in flight, 128 KB an SM.  Fetching the next step through registers had 24 KB on its way: 291 us for those, 0.39 of the HBM
+// rate, 176 here (0.64); the down projections 194 and 114.  A warp whose 16 slots lie past the group's end only helps to load.
+// Rows lie as 128 bytes, 16-byte chunk c of row r at c ^ (r & 7): ldmatrix without conflicts.  A weight that is not 16-byte aligned (the table is on the device: only
+// the kernel sees it) is fetched element by element into the same places.
+template <bool DUAL>
+struct TileRing {
+    static constexpr int BK = 64, TILE = 64 * BK * 2, STAGE = (DUAL ? 3 : 2) * TILE, N = DUAL ? 4 : 6;
+    static constexpr size_t SMEM = (size_t)N * STAGE;
+};
+__device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool ok) {
+    asm volatile("cp.async.cg.shared.global.L2::256B [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+template <bool DUAL>
+__global__ void __launch_bounds__(256, 2) kf_lin_tile_kernel(LinArgs a) {
+    using R = TileRing<DUAL>;
+    constexpr int BK = R::BK;
+    extern __shared__ __align__(128) uint8_t tile_smem[];
+    const uint32_t ring = (uint32_t)__cvta_generic_to_shared(tile_smem);
+    const int g  = blockIdx.z;
+    const int lo = a.offsets ? a.offsets[g] : 0, hi = a.offsets ? a.offsets[g + 1] : a.M;
+    const int n0 = blockIdx.x * BN, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int wm = warp & 3, wn = warp >> 2;             // warp tile: rows wm * 16, columns wn * 32
+    const int lr = tid >> 3, lc = tid & 7;                // this thread's loads: rows lr and lr + 32, chunk lc of each tile
+    const int steps = (a.K + BK - 1) / BK;
+    // a CTA walks the slot tiles blockIdx.y, blockIdx.y + gridDim.y, ... of its group: the grid is sized for the average group, not the worst
+    for (int m0 = lo + blockIdx.y * BM; m0 < hi; m0 += gridDim.y * BM) {
+        const uint16_t* W[2] = {a.Wt0 ? a.Wt0[g] : a.W0, DUAL ? (a.Wt1 ? a.Wt1[g] : a.W1) : nullptr};
+        const bool wvec = ((uintptr_t)W[0] & 15) == 0 && (!DUAL || ((uintptr_t)W[1] & 15) == 0);
+        const uint16_t* xr[2];
+        bool xok[2], wok[2];
+        size_t woff[2];
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int s = m0 + lr + 32 * i, n = n0 + lr + 32 * i;
+            xok[i]  = s < hi, wok[i] = n < a.N;
+            xr[i]   = (const uint16_t*)a.x + (size_t)(xok[i] ? (a.src_row ? a.src_row[s] : s) : 0) * a.ldx + lc * 8;
+            woff[i] = (size_t)(wok[i] ? n : 0) * a.K + lc * 8;
+        }
+        auto load = [&](int step) {
+            const uint32_t st = ring + (uint32_t)(step % R::N) * R::STAGE;
+            const int k       = step * BK + lc * 8;
+            const bool kok    = k < a.K;  // K is a multiple of 8
+            const size_t kof  = (size_t)(kok ? step * BK : 0);
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const int r        = lr + 32 * i;
+                const uint32_t dst = st + (uint32_t)(r * 128 + ((lc ^ (r & 7)) << 4));
+                cp16(dst, xok[i] && kok ? xr[i] + kof : (const uint16_t*)a.x, xok[i] && kok);
+#pragma unroll
+                for (int w = 0; w < (DUAL ? 2 : 1); w++) {
+                    const bool ok = wok[i] && kok;
+                    if (wvec) {
+                        cp16(dst + (1 + w) * R::TILE, ok ? W[w] + woff[i] + kof : W[w], ok);
+                    } else {
+                        uint16_t* d = reinterpret_cast<uint16_t*>(tile_smem + (dst - ring) + (1 + w) * R::TILE);
+                        for (int e = 0; e < 8; e++) d[e] = ok ? W[w][woff[i] + kof + e] : (uint16_t)0;
+                    }
+                }
+            }
+        };
+        float acc[DUAL ? 2 : 1][16];
+#pragma unroll
+        for (int w = 0; w < (DUAL ? 2 : 1); w++)
+#pragma unroll
+            for (int i = 0; i < 16; i++) acc[w][i] = 0.f;
+#pragma unroll
+        for (int i = 0; i < R::N - 1; i++) {
+            if (i < steps) load(i);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        }
+        const bool busy = m0 + wm * 16 < hi;
+        for (int step = 0; step < steps; step++) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(R::N - 2) : "memory");
+            __syncthreads();  // this step's bytes are there for everybody, and everybody has left the stage that is filled next
+            if (step + R::N - 1 < steps) load(step + R::N - 1);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            if (!busy) continue;
+            const uint8_t* xs = tile_smem + (size_t)(step % R::N) * R::STAGE;
+            auto at = [](const uint8_t* base, int row, int c) { return base + row * 128 + ((c ^ (row & 7)) << 4); };
+#pragma unroll
+            for (int kk = 0; kk < BK / 16; kk++) {
+                uint32_t af[4];
+                ldsm_x4(af, at(xs, wm * 16 + (lane & 15), kk * 2 + (lane >> 4)));
+#pragma unroll
+                for (int j = 0; j < 4; j += 2) {
+                    const int nr = wn * 32 + j * 8 + (lane & 7) + (lane >> 4) * 8, c = kk * 2 + ((lane >> 3) & 1);
+#pragma unroll
+                    for (int w = 0; w < (DUAL ? 2 : 1); w++) {
+                        uint32_t bf[4];
+                        ldsm_x4(bf, at(xs + (1 + w) * R::TILE, nr, c));
+                        mma_bf16_16816(&acc[w][j * 4], af, bf);
+                        mma_bf16_16816(&acc[w][(j + 1) * 4], af, bf + 2);
+                    }
+                }
+            }
+        }
+        const int gr = lane >> 2, tg = lane & 3;
+        const bool pairs = a.ldy % 2 == 0 && ((uintptr_t)a.y & 7) == 0;
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int s = m0 + wm * 16 + gr + 8 * h, n = n0 + wn * 32 + j * 8 + tg * 2;
+                if (s >= hi || n >= a.N) continue;
+                float v[2];
+#pragma unroll
+                for (int e = 0; e < 2; e++) v[e] = DUAL ? lin_pair(a, acc[0][j * 4 + 2 * h + e], acc[DUAL ? 1 : 0][j * 4 + 2 * h + e]) : lin_act(acc[0][j * 4 + 2 * h + e], a.act);
+                const size_t at = (size_t)s * a.ldy + n;
+                const bool two  = n + 1 < a.N;
+                if ((DUAL || a.act) && a.out_act == 1) {
+                    uint16_t* y = (uint16_t*)a.y + at;
+                    if (two && pairs) *reinterpret_cast<uint32_t*>(y) = pack_bf16x2(v[0], v[1]);
+                    else {
+                        y[0] = f32_to_bf16_bits(v[0]);
+                        if (two) y[1] = f32_to_bf16_bits(v[1]);
+                    }
+                } else {
+                    float* y = (float*)a.y + at;
+                    if (two && pairs) *reinterpret_cast<float2*>(y) = make_float2(v[0], v[1]);
+                    else {
+                        y[0] = v[0];
+                        if (two) y[1] = v[1];
+                    }
+                }
+            }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();  // the ring is free for the next slot tile
+    }
+}
+
 template <typename TA, bool DUAL>
 int launch(kf_ctx* ctx, const LinArgs& a, int slots, int groups, bool gemv) {
     if (gemv) {
@@ -466,7 +598,16 @@ int launch(kf_ctx* ctx, const LinArgs& a, int slots, int groups, bool gemv) {
         const int tiles = (slots + BM - 1) / BM;
         const int gy    = groups > 1 ? std::min(tiles, std::max(1, (2 * slots / groups + BM - 1) / BM)) : tiles;
         dim3 grid((a.N + BN - 1) / BN, gy, groups);
-        kf_lin_tile_kernel<TA, DUAL><<<grid, 256, 0, ctx->stream>>>(a);
+        if (sizeof(TA) == 2 && a.K % 8 == 0 && a.ldx % 8 == 0 && ((uintptr_t)a.x & 15) == 0) {  // rows that can be fetched 16 bytes at a time
+            static bool set[kf_ctx::kMaxDevices] = {};  // function attributes are per device (one flag per instantiation and device)
+            if (!set[ctx->device]) {
+                KF_CUDA(ctx, cudaFuncSetAttribute(kf_lin_tile_kernel<DUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TileRing<DUAL>::SMEM));
+                set[ctx->device] = true;
+            }
+            kf_lin_tile_kernel<DUAL><<<grid, 256, TileRing<DUAL>::SMEM, ctx->stream>>>(a);
+        } else {
+            kf_lin_tile_any_kernel<TA, DUAL><<<grid, 256, 0, ctx->stream>>>(a);
+        }
     }
     KF_LAUNCH_CHECK(ctx);
     return KF_OK;
