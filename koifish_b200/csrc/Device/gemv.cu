@@ -262,22 +262,42 @@ template <int FMT, int MODE, int MX>
 __device__ __forceinline__ void gemv_stage_x(uint4* __restrict__ dstx, float4* __restrict__ dstsx, const GemvParams& p, int s_begin, int nsteps,
                                              float* s_red, float* s_scale) {
     const int tid = threadIdx.x, lane = tid & 31;
-    // ---- optional fused RMSNorm: the same arithmetic, in the same order, as kf_rmsnorm_kernel (ops.cu) --------------------------
+    // ---- optional fused RMSNorm: the same arithmetic, in the same order, as kf_rmsnorm_kernel (ops.cu).  Bound by latency: a token is two loads a thread.  The sums of
+    //      up to eight tokens are formed side by side, their loads travel together and they share two block barriers; one token after the other cost a memory
+    //      round trip and two barriers each (28 layers of 1024 x 3072, 8 tokens, 112 of these matmuls: step 1579 -> 1254 us; bits unchanged) ------------------
     if (p.norm_w) {
-        for (int m = 0; m < p.M; m++) {
-            const uint16_t* xr = p.x + (size_t)m * p.K;
-            float ss = 0.f;
-            for (int i = tid * 8; i < p.K; i += kThreads * 8) {
-                const uint4 v = __ldg(reinterpret_cast<const uint4*>(xr + i));
-                const uint32_t q[4] = {v.x, v.y, v.z, v.w};
+        constexpr int TB8 = MX < 8 ? MX : 8;
+        const int warp = tid >> 5;
+        for (int m0 = 0; m0 < p.M; m0 += TB8) {
+            float ss[TB8];
 #pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const float a = bf16lo(q[j]), b = bf16hi(q[j]);
-                    ss = fmaf(a, a, ss), ss = fmaf(b, b, ss);
+            for (int m = 0; m < TB8; m++) ss[m] = 0.f;
+            for (int i = tid * 8; i < p.K; i += kThreads * 8) {
+                uint4 v[TB8];
+#pragma unroll
+                for (int m = 0; m < TB8; m++) v[m] = m0 + m < p.M ? __ldg(reinterpret_cast<const uint4*>(p.x + (size_t)(m0 + m) * p.K + i)) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+                for (int m = 0; m < TB8; m++) {
+                    const uint32_t q[4] = {v[m].x, v[m].y, v[m].z, v[m].w};
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        const float a = bf16lo(q[j]), b = bf16hi(q[j]);
+                        ss[m] = fmaf(a, a, ss[m]), ss[m] = fmaf(b, b, ss[m]);
+                    }
                 }
             }
-            ss = block_sum(ss, s_red);
-            if (tid == 0) s_scale[m] = 1.0f / sqrtf(fmaf(ss, 1.0f / (float)p.K, p.norm_eps));
+#pragma unroll
+            for (int m = 0; m < TB8; m++) ss[m] = warp_sum(ss[m]);
+            __syncthreads();
+            if (lane == 0)
+#pragma unroll
+                for (int m = 0; m < TB8; m++) s_red[m * 8 + warp] = ss[m];
+            __syncthreads();
+            if (tid < TB8 && m0 + tid < p.M) {  // the warps in index order, as block_sum adds them
+                float t = 0.f;
+                for (int w = 0; w < kThreads / 32; w++) t += s_red[tid * 8 + w];
+                s_scale[m0 + tid] = 1.0f / sqrtf(fmaf(t, 1.0f / (float)p.K, p.norm_eps));
+            }
         }
         __syncthreads();
     }
@@ -388,7 +408,7 @@ __global__ void __launch_bounds__(kThreads, (NT >= 4 ? 1 : NT == 1 ? KF_GEMV_OCC
     static_assert(TB == CPB * NCH, "ring chunking");
     extern __shared__ uint4 smem[];
     __shared__ int s_last;
-    __shared__ float s_red[32];
+    __shared__ float s_red[64];
     __shared__ float s_scale[64];
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
@@ -825,7 +845,7 @@ __global__ void __launch_bounds__(kThreads, (NT >= 4 ? 1 : NT == 1 ? KF_GEMV_OCC
 // RMSNorm (optional) + fragment-order fp16 staging of ALL of x, once, for the XG variants of the kernel above: grid = ceil(k-steps / prep_steps)
 template <int FMT, int MX>
 __global__ void __launch_bounds__(kThreads) kf_gemv_xprep_kernel(const GemvParams p) {
-    __shared__ float s_red[32];
+    __shared__ float s_red[64];
     __shared__ float s_scale[64];
     kf_grid_launch_dependents();  // the matmul behind us may start streaming its weights
     kf_grid_dependency_wait();    // x comes from the kernel before us

@@ -216,3 +216,50 @@ def test_gqa_runs(ctx, hd, n_head, n_kv, lens, hint):
                 want, mass = p @ vv, p @ vv.abs()
                 err = (out[i, h].double() - want).abs()
                 assert bool((err <= 2.0 ** -8 * 1.01 * (mass + want.abs()) + 1e-6).all()), (split, i, h, float((err / (mass + want.abs())).max()))
+
+
+# ---------------------------------------------------------------------------------------------- tile matmul over expert-sorted slots
+@pytest.mark.parametrize("N,K", [(64, 64), (65, 72), (8, 8), (130, 200), (192, 448), (33, 512)])
+@pytest.mark.parametrize("counts", [(64, 0, 1, 63, 65, 17), (200, 3, 0, 0, 1, 0), (16, 16, 16, 16, 16, 16)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_grouped_tiles(ctx, N, K, counts, shift):
+    """Ragged outputs, reductions and slot tiles, empty experts, gathered rows, weights that do not start on 16 bytes.  Products are exact in fp32 and the sums fp32:
+    2^-24 * K terms of the rms, stated as 1e-5; the gate / up form rounds its result to bf16 once (2^-8)."""
+    import torch
+    torch.backends.cuda.matmul.allow_tf32 = False
+    g = torch.Generator(device="cuda")
+    g.manual_seed(N * K + sum(counts))
+    X, slots, M = len(counts), sum(counts), 50
+    x = torch.randn(M, K, generator=g, device="cuda").bfloat16()
+    flat = [torch.randn(X * N * K + shift, generator=g, device="cuda").bfloat16()[shift:].view(X, N, K) for _ in range(2)]
+    tabs = [torch.tensor([t[e].data_ptr() for e in range(X)], dtype=torch.int64, device="cuda") for t in flat]
+    group = torch.repeat_interleave(torch.arange(X), torch.tensor(counts)).int().cuda()
+    off = torch.cumsum(torch.tensor((0,) + counts), 0).int().cuda()
+    src = torch.randint(0, M, (slots,), generator=g, device="cuda", dtype=torch.int32)
+    y, h = torch.full((slots, N), 9.0, device="cuda"), torch.full((slots, N), 9.0, device="cuda").bfloat16()
+    torch.cuda.synchronize()
+    ctx.check(ctx.lib.kf_linear_grouped(ctx.h, _ptr(y), N, _ptr(tabs[0]), None, X, N, K, _ptr(x), 0, K, _ptr(off), _ptr(group), _ptr(src), slots), "single")
+    ctx.check(ctx.lib.kf_linear_grouped(ctx.h, _ptr(h), N, _ptr(tabs[0]), _ptr(tabs[1]), X, N, K, _ptr(x), 0, K, _ptr(off), _ptr(group), _ptr(src), slots), "dual")
+    ctx.sync()
+    xs = x[src.long()].double()
+    a, u = (torch.einsum("sk,snk->sn", xs, t[group.long()].double()) for t in flat)
+    tiny = 1e-5 * float(a.square().mean().sqrt())
+    assert bool(((y.double() - a).abs() <= tiny).all())
+    want = a * torch.sigmoid(a) * u
+    assert bool(((h.double() - want).abs() <= 2.0 ** -8 * 1.01 * want.abs() + tiny * (1 + a.abs() + u.abs())).all())
+
+
+# ---------------------------------------------------------------------------------------------- RMSNorm inside the skinny matmul
+@pytest.mark.parametrize("typ", [kf.KF_T_Q4, kf.KF_T_Q2, kf.KF_T_BF16])
+@pytest.mark.parametrize("M", [2, 3, 4, 7, 8, 9, 15, 17, 32, 33, 64])
+@pytest.mark.parametrize("K", [256, 1152, 4096])
+def test_norm_of_several_tokens(ctx, typ, M, K):
+    """The sums of the tokens are formed eight at a time, each in the order of kf_rmsnorm: the fused call has the bits of the two calls."""
+    x, nw = kf.fill_normal(ctx, M * K, M * K, 2.0), kf.fill_normal(ctx, K, 3, 0.5)
+    xn = kf.rmsnorm(ctx, x, nw, M, K, 1e-6)
+    if typ == kf.KF_T_BF16:
+        ws = [kf.QTensor.from_packed(ctx, ol.fill_normal(n * K, n, 0.02).view(np.uint8), None, n, K, typ) for n in (256, 128)]
+    else:
+        ws = [make_q(ctx, typ, n, K, n)[0] for n in (256, 128)]
+    for a, b in zip(kf.rmsnorm_linear(ctx, ws, x, nw, M, 1e-6), kf.linear_multi(ctx, ws, xn, M)):
+        assert np.array_equal(a.numpy(np.uint16), b.numpy(np.uint16))
