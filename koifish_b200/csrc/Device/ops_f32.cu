@@ -748,26 +748,33 @@ __device__ __forceinline__ void route_grouped_warp(int* taken, int32_t* idx, flo
     if (E <= 32 * kRouteCache) route_grouped_body<true>(taken, idx, wgt, lg, bias, E, top, md, lane);
     else route_grouped_body<false>(taken, idx, wgt, lg, bias, E, top, md, lane);
 }
-// one warp per token: `top` rounds of arg-max over the E router logits (+ bias), ties to the lower index; weights = softmax over the
-// chosen logits only, or (full) the chosen entries of the softmax over ALL experts, not renormalised.  All in fp32.
-__global__ void __launch_bounds__(128) kf_moe_route_kernel(int32_t* __restrict__ idx, float* __restrict__ wgt, const float* __restrict__ logits, int ldl,
-                                                           const uint16_t* __restrict__ bias, int M, int E, int top, int full, const RouteMode md) {
-    const int m = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (m >= M) return;
-    const float* lg = logits + (size_t)m * ldl;
-    if (md.kind) {
-        route_grouped_warp(idx + (size_t)m * top, idx + (size_t)m * top, wgt + (size_t)m * top, lg, bias, E, top, md, lane);
-        return;
+// One warp per token: `top` rounds of arg-max over the E router logits (+ bias), ties to the lower index; weights = softmax over the chosen logits
+// only, or (full) the chosen entries of the softmax over ALL experts, not renormalised.  All in fp32.  Bound by latency.  CACHED: the lane keeps its
+// logits and a mask of the chosen ones in registers, so that a round is its compares and shuffles (512 tokens, 6 of 64: 6.4 us; reading
+// the logits and the choices again in every round, 8.8); otherwise taken[0 .. j) names the choices so far.
+template <bool CACHED>
+__device__ __forceinline__ void route_plain_body(int* taken, int32_t* idx, float* __restrict__ wgt, const float* __restrict__ lg, const uint16_t* __restrict__ bias,
+                                                 int E, int top, int full, int lane) {
+    const int n = CACHED ? kRouteCache : (E + 31) / 32;
+    float vals[kRouteCache];
+    unsigned gone = 0;
+    auto value = [&](int e) { return lg[e] + (bias ? bf16_bits_to_f32(bias[e]) : 0.f); };
+    if (CACHED) {
+#pragma unroll
+        for (int i = 0; i < kRouteCache; i++) vals[i] = 32 * i + lane < E ? value(32 * i + lane) : 0.f;
     }
     float first = 0.f, den = 0.f;
     for (int j = 0; j < top; j++) {
         float best = -INFINITY;
         int bi     = 0x7fffffff;
-        for (int e = lane; e < E; e += 32) {
-            bool taken = false;
-            for (int q = 0; q < j; q++) taken = taken || idx[(size_t)m * top + q] == e;
-            if (taken) continue;
-            const float v = lg[e] + (bias ? bf16_bits_to_f32(bias[e]) : 0.f);
+#pragma unroll
+        for (int i = 0; i < n; i++) {
+            const int e = 32 * i + lane;
+            bool skip   = e >= E;
+            if (CACHED) skip = skip || ((gone >> i) & 1u);
+            else for (int q = 0; q < j; q++) skip = skip || taken[q] == e;
+            if (skip) continue;
+            const float v = CACHED ? vals[i] : value(e);
             if (v > best || (v == best && e < bi)) best = v, bi = e;
         }
 #pragma unroll
@@ -779,17 +786,33 @@ __global__ void __launch_bounds__(128) kf_moe_route_kernel(int32_t* __restrict__
         if (j == 0) first = best;
         const float p = expf(best - first);
         den += p;
-        if (lane == 0) idx[(size_t)m * top + j] = bi, wgt[(size_t)m * top + j] = p;
-        __syncwarp();
+        if (CACHED && (bi & 31) == lane && bi < E) gone |= 1u << (bi >> 5);
+        if (lane == 0) taken[j] = bi, idx[j] = bi, wgt[j] = p;
+        if (!CACHED) __syncwarp();
     }
     if (full) {  // the denominator runs over every expert (first = the largest logit)
         float d = 0.f;
-        for (int e = lane; e < E; e += 32) d += expf(lg[e] + (bias ? bf16_bits_to_f32(bias[e]) : 0.f) - first);
+#pragma unroll
+        for (int i = 0; i < n; i++)
+            if (32 * i + lane < E) d += expf((CACHED ? vals[i] : value(32 * i + lane)) - first);
         den = warp_sum(d);
     }
-    if (lane < top) {
-        for (int j = lane; j < top; j += 32) wgt[(size_t)m * top + j] /= den;
-    }
+    __syncwarp();
+    for (int j = lane; j < top; j += 32) wgt[j] /= den;
+}
+__device__ __forceinline__ void route_plain_warp(int* taken, int32_t* idx, float* __restrict__ wgt, const float* __restrict__ lg, const uint16_t* __restrict__ bias,
+                                                 int E, int top, int full, int lane) {
+    if (E <= 32 * kRouteCache) route_plain_body<true>(taken, idx, wgt, lg, bias, E, top, full, lane);
+    else route_plain_body<false>(taken, idx, wgt, lg, bias, E, top, full, lane);
+}
+__global__ void __launch_bounds__(128) kf_moe_route_kernel(int32_t* __restrict__ idx, float* __restrict__ wgt, const float* __restrict__ logits, int ldl,
+                                                           const uint16_t* __restrict__ bias, int M, int E, int top, int full, const RouteMode md) {
+    const int m = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (m >= M) return;
+    const float* lg = logits + (size_t)m * ldl;
+    int32_t* choice = idx + (size_t)m * top;
+    if (md.kind) route_grouped_warp(choice, choice, wgt + (size_t)m * top, lg, bias, E, top, md, lane);
+    else route_plain_warp(choice, choice, wgt + (size_t)m * top, lg, bias, E, top, full, lane);
 }
 // The dispatch tables of a few entries by ONE block of 256 threads: entry i = (token i / top, choice i % top) goes to expert sidx[i]; thread i
 // ranks its entry among the earlier ones of its expert, the lanes of warp 0 count one expert each and scan the counts.  Entries of outputs
@@ -844,39 +867,8 @@ __global__ void __launch_bounds__(256) kf_moe_route_small_kernel(int32_t* __rest
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n = M * top;
     for (int m = warp; m < M; m += 8) {
         const float* lg = logits + (size_t)m * ldl;
-        if (md.kind) {
-            route_grouped_warp(sidx + m * top, idx + (size_t)m * top, wgt + (size_t)m * top, lg, bias, E, top, md, lane);
-            continue;
-        }
-        float first = 0.f, den = 0.f;
-        for (int j = 0; j < top; j++) {
-            float best = -INFINITY;
-            int bi     = 0x7fffffff;
-            for (int e = lane; e < E; e += 32) {
-                bool taken = false;
-                for (int q = 0; q < j; q++) taken = taken || sidx[m * top + q] == e;
-                if (taken) continue;
-                const float v = lg[e] + (bias ? bf16_bits_to_f32(bias[e]) : 0.f);
-                if (v > best || (v == best && e < bi)) best = v, bi = e;
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-                const int oi   = __shfl_xor_sync(0xffffffffu, bi, o);
-                if (ob > best || (ob == best && oi < bi)) best = ob, bi = oi;
-            }
-            if (j == 0) first = best;
-            const float p = expf(best - first);
-            den += p;
-            if (lane == 0) sidx[m * top + j] = bi, idx[(size_t)m * top + j] = bi, wgt[(size_t)m * top + j] = p;
-            __syncwarp();
-        }
-        if (full) {
-            float d = 0.f;
-            for (int e = lane; e < E; e += 32) d += expf(lg[e] + (bias ? bf16_bits_to_f32(bias[e]) : 0.f) - first);
-            den = warp_sum(d);
-        }
-        for (int j = lane; j < top; j += 32) wgt[(size_t)m * top + j] /= den;
+        if (md.kind) route_grouped_warp(sidx + m * top, idx + (size_t)m * top, wgt + (size_t)m * top, lg, bias, E, top, md, lane);
+        else route_plain_warp(sidx + m * top, idx + (size_t)m * top, wgt + (size_t)m * top, lg, bias, E, top, full, lane);
     }
     dispatch_small(sidx, srank, n, E - md.pass, top, offsets, entry_slot, slot_row, slot_group);
 }
@@ -906,30 +898,40 @@ __device__ __forceinline__ void rank_expert(int32_t* rank, int32_t* count, const
     }
     if (threadIdx.x == 0) count[e] = base;
 }
-__global__ void __launch_bounds__(256) kf_moe_rank_kernel(int32_t* __restrict__ rank, int32_t* __restrict__ count, const int32_t* __restrict__ idx, int n) {
-    rank_expert(rank, count, idx, n, blockIdx.x);
-}
-// offsets = exclusive scan of the counts (one thread: E is small); then each entry learns its slot
-__global__ void kf_moe_offsets_kernel(int32_t* __restrict__ offsets, const int32_t* __restrict__ count, int E) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        int s = 0;
-        for (int e = 0; e < E; e++) offsets[e] = s, s += count[e];
-        offsets[E] = s;
+// The dispatch tables of a panel in one launch: block e counts the entries of the experts before e (its first slot) and hands its slots to its own in
+// entry order; block X (one more than the experts) takes the entries of outputs beyond the experts, which get no slot, and marks as many slots behind
+// the last expert as free.  A warp owns a run of entries, so one scan over the warps places them all.  Bound by latency: two passes over n indices that
+// sit in L2 (3072 entries of 64 experts: 4.3 us; rank, scan and slots as three launches 13.0).
+constexpr int kTabThreads = 512;
+__global__ void __launch_bounds__(kTabThreads) kf_moe_tables_kernel(int32_t* __restrict__ offsets, int32_t* __restrict__ entry_slot, int32_t* __restrict__ slot_row,
+                                                                    int32_t* __restrict__ slot_group, const int32_t* __restrict__ idx, int n, int top, int X) {
+    constexpr int W = kTabThreads / 32;
+    __shared__ int hits[W], less[W];
+    const int e = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int run = ((n + W - 1) / W + 31) & ~31, i0 = min(n, warp * run), i1 = min(n, i0 + run);
+    auto mine = [&](int k) { return e < X ? k == e : k >= X; };
+    int h = 0, l = 0;
+#pragma unroll 4
+    for (int i = i0 + lane; i < i1; i += 32) {
+        const int k = idx[i];
+        h += mine(k), l += k < e;
     }
-}
-__global__ void kf_moe_slots_kernel(int32_t* __restrict__ entry_slot, int32_t* __restrict__ slot_row, int32_t* __restrict__ slot_group,
-                                    const int32_t* __restrict__ idx, const int32_t* __restrict__ rank, const int32_t* __restrict__ offsets, int n, int top,
-                                    int E) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (i >= offsets[E]) slot_row[i] = 0, slot_group[i] = -1;  // no entry has this slot
-    const int e = idx[i];
-    if (e >= E) {
-        entry_slot[i] = -1;
-        return;
+    for (int o = 16; o > 0; o >>= 1) h += __shfl_xor_sync(0xffffffffu, h, o), l += __shfl_xor_sync(0xffffffffu, l, o);
+    if (lane == 0) hits[warp] = h, less[warp] = l;
+    __syncthreads();
+    int first = 0, before = 0;
+    for (int w = 0; w < W; w++) first += less[w], before += w < warp ? hits[w] : 0;
+    if (threadIdx.x == 0) offsets[e] = first;
+    int slot = first + before;
+    for (int i = i0; i < i1; i += 32) {
+        const bool hit   = i + lane < i1 && mine(idx[i + lane]);
+        const unsigned b = __ballot_sync(0xffffffffu, hit);
+        if (hit) {
+            const int s = slot + __popc(b & ((1u << lane) - 1));
+            entry_slot[i + lane] = e < X ? s : -1, slot_row[s] = e < X ? (i + lane) / top : 0, slot_group[s] = e < X ? e : -1;
+        }
+        slot += __popc(b);
     }
-    const int s = offsets[e] + rank[i];
-    entry_slot[i] = s, slot_row[s] = i / top, slot_group[s] = e;
 }
 // Routing from a table of token ids: row tokens[m] names the token's `top` experts, each with weight 1 / top -- no logits.  It depends on
 // the token ids alone, so ONE launch fills the tables of several layers (blockIdx.y / .x picks the layer).
@@ -983,18 +985,50 @@ __global__ void kf_moe_table_slots_kernel(const kf_table_route* __restrict__ rou
     const int e = r.idx[i], sl = soff[e] + r.work[i];
     r.entry_slot[i] = sl, r.slot_row[sl] = i / r.top, r.slot_group[sl] = e;
 }
-// out[m] = sum_j wgt[m][j] * y[slot(m, j)]  (+ sigmoid(sg[m]) * shared[m]), choices added in their routing order
-__global__ void kf_moe_combine_kernel(float* __restrict__ out, const float* __restrict__ y, const int32_t* __restrict__ entry_slot,
+// out[m] = sum_j wgt[m][j] * y[slot(m, j)]  (+ sigmoid(sg[m]) * shared[m]), choices added in their routing order; a choice without a slot adds nothing.
+// Bound by bytes (every slot's row once), as long as enough of them are in flight: V floats a thread, one pass over the row by as many blocks as it
+// needs, the rows of eight choices requested together.  One float at a time, one request after the other: 14.0 us for 512 tokens of six choices of
+// 2048 floats, 7.5 us so.  V = 1: rows or buffers that are not made of 16-byte pieces.
+template <int V>
+__global__ void __launch_bounds__(256) kf_moe_combine_kernel(float* __restrict__ out, const float* __restrict__ y, const int32_t* __restrict__ entry_slot,
                                       const float* __restrict__ wgt, const float* __restrict__ shared, const float* __restrict__ sg, int ldsg, int dim, int top,
                                       int accumulate) {
-    const int m = blockIdx.x;
+    constexpr int kBatch = 8;
+    struct alignas(4 * V) Vec { float f[V]; };
+    const int m = blockIdx.x, d = (blockIdx.y * blockDim.x + threadIdx.x) * V;
+    if (d >= dim) return;
     const float gate = shared ? (sg ? sigmoid_f(sg[(size_t)m * ldsg]) : 1.f) : 0.f;
-    for (int d = threadIdx.x; d < dim; d += blockDim.x) {
-        float s = 0.f;
-        for (int j = 0; j < top; j++) s = fmaf(wgt[(size_t)m * top + j], y[(size_t)entry_slot[(size_t)m * top + j] * dim + d], s);
-        if (shared) s = fmaf(gate, shared[(size_t)m * dim + d], s);
-        out[(size_t)m * dim + d] = accumulate ? out[(size_t)m * dim + d] + s : s;
+    const int32_t* slots = entry_slot + (size_t)m * top;
+    const float* w       = wgt + (size_t)m * top;
+    Vec s = {};
+    for (int j0 = 0; j0 < top; j0 += kBatch) {
+        Vec v[kBatch];
+        int sl[kBatch];
+#pragma unroll
+        for (int j = 0; j < kBatch; j++) sl[j] = j0 + j < top ? slots[j0 + j] : -1;
+#pragma unroll
+        for (int j = 0; j < kBatch; j++)
+            if (sl[j] >= 0) v[j] = *reinterpret_cast<const Vec*>(y + (size_t)sl[j] * dim + d);
+#pragma unroll
+        for (int j = 0; j < kBatch; j++)
+            if (sl[j] >= 0) {
+                const float wj = w[j0 + j];
+#pragma unroll
+                for (int i = 0; i < V; i++) s.f[i] = fmaf(wj, v[j].f[i], s.f[i]);
+            }
     }
+    if (shared) {
+        const Vec h = *reinterpret_cast<const Vec*>(shared + (size_t)m * dim + d);
+#pragma unroll
+        for (int i = 0; i < V; i++) s.f[i] = fmaf(gate, h.f[i], s.f[i]);
+    }
+    Vec* o = reinterpret_cast<Vec*>(out + (size_t)m * dim + d);
+    if (accumulate) {
+        const Vec r = *o;
+#pragma unroll
+        for (int i = 0; i < V; i++) s.f[i] = r.f[i] + s.f[i];
+    }
+    *o = s;
 }
 }  // namespace
 
@@ -1263,15 +1297,10 @@ static int moe_route_impl(kf_ctx* ctx, int32_t* idx, float* wgt, int32_t* offset
         KF_LAUNCH_CHECK(ctx);
         return KF_OK;
     }
-    int32_t *rank = work, *count = work + n;
     kf_moe_route_kernel<<<(M + 3) / 4, 128, 0, ctx->stream>>>(idx, wgt, logits, ldl, (const uint16_t*)bias_bf16, M, E, top, full_softmax, md);
     KF_LAUNCH_CHECK(ctx);
     const int X = E - md.pass;
-    kf_moe_rank_kernel<<<X, 256, 0, ctx->stream>>>(rank, count, idx, n);
-    KF_LAUNCH_CHECK(ctx);
-    kf_moe_offsets_kernel<<<1, 32, 0, ctx->stream>>>(offsets, count, X);
-    KF_LAUNCH_CHECK(ctx);
-    kf_moe_slots_kernel<<<(n + 255) / 256, 256, 0, ctx->stream>>>(entry_slot, slot_row, slot_group, idx, rank, offsets, n, top, X);
+    kf_moe_tables_kernel<<<X + 1, kTabThreads, 0, ctx->stream>>>(offsets, entry_slot, slot_row, slot_group, idx, n, top, X);
     KF_LAUNCH_CHECK(ctx);
     return KF_OK;
 }
@@ -1334,7 +1363,11 @@ extern "C" int kf_moe_route_table(kf_ctx* ctx, const kf_table_route* routes_dev,
 extern "C" int kf_moe_combine_ex(kf_ctx* ctx, float* out, const float* y_slots, const int32_t* entry_slot, const float* wgt, const float* shared,
                                  const float* shared_gate_logit, int ld_gate, int M, int dim, int top, int accumulate) {
     if (!ctx || !out || !y_slots || !entry_slot || !wgt) return KF_ERR_BAD_ARG;
-    kf_moe_combine_kernel<<<M, 256, 0, ctx->stream>>>(out, y_slots, entry_slot, wgt, shared, shared_gate_logit, ld_gate, dim, top, accumulate);
+    const bool vec = dim % 4 == 0 && (((uintptr_t)out | (uintptr_t)y_slots | (uintptr_t)shared) & 15) == 0;
+    if (vec)
+        kf_moe_combine_kernel<4><<<dim3(M, (dim / 4 + 255) / 256), 256, 0, ctx->stream>>>(out, y_slots, entry_slot, wgt, shared, shared_gate_logit, ld_gate, dim, top, accumulate);
+    else
+        kf_moe_combine_kernel<1><<<dim3(M, (dim + 255) / 256), 256, 0, ctx->stream>>>(out, y_slots, entry_slot, wgt, shared, shared_gate_logit, ld_gate, dim, top, accumulate);
     KF_LAUNCH_CHECK(ctx);
     return KF_OK;
 }

@@ -263,3 +263,69 @@ def test_norm_of_several_tokens(ctx, typ, M, K):
         ws = [make_q(ctx, typ, n, K, n)[0] for n in (256, 128)]
     for a, b in zip(kf.rmsnorm_linear(ctx, ws, x, nw, M, 1e-6), kf.linear_multi(ctx, ws, xn, M)):
         assert np.array_equal(a.numpy(np.uint16), b.numpy(np.uint16))
+
+
+# ---------------------------------------------------------------------------------------------- routing of a panel, weighted sum of the experts
+@pytest.mark.parametrize("M,E,top,full", [(33, 8, 8, 0), (300, 7, 2, 1), (512, 64, 6, 0), (129, 256, 4, 1), (129, 257, 4, 1), (70, 300, 40, 0), (2049, 33, 1, 0), (5, 64, 6, 1)])
+def test_panel_routing(ctx, M, E, top, full):
+    """Ties, rows of -inf, more outputs than a warp's registers hold, more choices than lanes, one block and panels; whole numbers are exact, a weight is
+    one expf (2 units) over a sum of up to E of them: 1e-5."""
+    rng = np.random.default_rng(M + E)
+    lg, bias = np.round(rng.standard_normal((M, E + 3)) * 8).astype(np.float32) / 4, np.round(rng.standard_normal(E) * 4).astype(np.float32) / 4
+    lg[1, top:E] = -np.inf
+    n = M * top
+    idx, wgt, offs, es, sr, sg, work = (ctx.zeros(4 * k) for k in (n, n, E + 1, n, n, n, 2 * n + E))
+    lgd, bd = ctx.array(lg), ctx.array(ol.f32_to_bf16(bias))
+    ctx.check(ctx.lib.kf_moe_route_ex(ctx.h, idx.ptr, wgt.ptr, offs.ptr, es.ptr, sr.ptr, sg.ptr, work.ptr, lgd.ptr, E + 3, bd.ptr, M, E, top, full), "route")
+    v = (lg[:, :E] + bias).astype(np.float64)
+    want = np.argsort(-v, axis=1, kind="stable")[:, :top]
+    gi = idx.numpy(np.int32, (M, top))
+    assert np.array_equal(gi, want)
+    chosen = np.exp(np.take_along_axis(v, want, 1) - v.max(1, keepdims=True))
+    den = np.exp(v - v.max(1, keepdims=True)).sum(1, keepdims=True) if full else chosen.sum(1, keepdims=True)
+    assert np.allclose(wgt.numpy(np.float32, (M, top)), chosen / den, rtol=1e-5, atol=1e-30)
+    flat = gi.reshape(-1)
+    order = np.argsort(flat, kind="stable")
+    assert np.array_equal(offs.numpy(np.int32, (E + 1,)), np.concatenate([[0], np.cumsum(np.bincount(flat, minlength=E))]))
+    assert np.array_equal(es.numpy(np.int32, (n,))[order], np.arange(n))
+    assert np.array_equal(sr.numpy(np.int32, (n,)), order // top) and np.array_equal(sg.numpy(np.int32, (n,)), flat[order])
+
+
+@pytest.mark.parametrize("M,X,spare,top", [(200, 12, 4, 5), (513, 30, 34, 2), (100, 3, 61, 8)])
+def test_panel_routing_past_the_experts(ctx, M, X, spare, top):
+    """Entries of outputs beyond the experts take no slot; as many slots stay free behind the last expert."""
+    n, E = M * top, X + spare
+    idx, wgt, offs, es, sr, sg, work = (ctx.zeros(4 * k) for k in (n, n, E + 1, n, n, n, 2 * n + E))
+    lgd = ctx.array(np.random.default_rng(M).standard_normal((M, E)).astype(np.float32))
+    ctx.check(ctx.lib.kf_moe_route_softmax_grouped(ctx.h, idx.ptr, wgt.ptr, offs.ptr, es.ptr, sr.ptr, sg.ptr, work.ptr, lgd.ptr, E, None, M, X, spare, top, 1, 1), "route")
+    flat = idx.numpy(np.int32, (n,))
+    real = int((flat < X).sum())
+    order = np.argsort(np.minimum(flat, X), kind="stable")
+    assert np.array_equal(offs.numpy(np.int32)[:X + 1], np.concatenate([[0], np.cumsum(np.bincount(flat[flat < X], minlength=X))]))
+    assert np.array_equal(es.numpy(np.int32, (n,))[order], np.where(np.arange(n) < real, np.arange(n), -1))
+    assert np.array_equal(sr.numpy(np.int32, (n,)), np.where(np.arange(n) < real, order // top, 0))
+    assert np.array_equal(sg.numpy(np.int32, (n,)), np.where(np.arange(n) < real, flat[order], -1))
+
+
+@pytest.mark.parametrize("M,dim,top,shift", [(1, 8, 1, 0), (3, 1028, 7, 0), (3, 1028, 8, 1), (5, 1023, 9, 0), (40, 2304, 17, 0), (2, 3, 2, 0)])
+@pytest.mark.parametrize("shared,accumulate", [(0, 0), (1, 0), (2, 1)])
+def test_combine(ctx, M, dim, top, shift, shared, accumulate):
+    """Rows that are and are not made of 16-byte pieces, more choices than one batch holds; fp32 sums of top + 2 terms: 2^-24 (top + 2) of their masses."""
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(M * dim + top)
+    y = torch.randn(M * top * dim + shift, generator=g, device="cuda")[shift:].view(M * top, dim)
+    w, sh, sg, out = torch.rand(M, top, generator=g, device="cuda"), torch.randn(M, dim, generator=g, device="cuda"), torch.randn(M, 2, generator=g, device="cuda"), torch.randn(M, dim, generator=g, device="cuda")
+    slot = torch.randperm(M * top, generator=g, device="cuda").int()
+    before = out.double()
+    torch.cuda.synchronize()
+    ctx.check(ctx.lib.kf_moe_combine_ex(ctx.h, _ptr(out), _ptr(y), _ptr(slot), _ptr(w), _ptr(sh) if shared else None, _ptr(sg) if shared == 2 else None, 2, M, dim, top,
+                                        accumulate), "combine")
+    ctx.sync()
+    terms = [w[:, j, None].double() * y[slot.view(M, top)[:, j].long()].double() for j in range(top)]
+    if shared:
+        terms.append((torch.sigmoid(sg[:, :1].double()) if shared == 2 else 1.0) * sh.double())
+    if accumulate:
+        terms.append(before)
+    mass = sum(t.abs() for t in terms)
+    assert bool(((out.double() - sum(terms)).abs() <= 2.0 ** -24 * (top + 6) * mass + 1e-30).all())
