@@ -100,9 +100,10 @@ uint64_t kf_scratch_generation(kf_ctx* ctx);
  * for sm_90+; 0: twice, as its -fmad=false / pre-sm_90 builds), "gemv_tma" (1, default: decode GEMVs of 4-bit weights take the persistent
  * TMA-fed stream-K kernel; 0: the round-1 cp.async kernel), "gemv_tma_occ" (CTAs per SM, 1 or 2), "gemv_tma_smem_kb" (shared-memory budget),
  * "gqa_min_ctx" (single-sequence decode: context length beyond which the kv-group tensor-core attention replaces the fused per-head
- * kernel; default 1024), "tc_min_m" (token count from which kf_linear* use the tcgen05 GEMM: -1 = measured per-type crossover, 0 = never, n = from n) */
+ * kernel; default 1024), "tc_min_m" (token count from which kf_linear* use the tcgen05 GEMM: -1 = measured per-type crossover, 0 = never, n = from n),
+ * "tc_bn" (token tile of the tcgen05 GEMM: 16, 32, 64, 128 or 256; 0 = by modelled time) */
 int kf_ctx_set_int(kf_ctx* ctx, const char* key, int value);
-int kf_ctx_get_int(kf_ctx* ctx, const char* key, int* value_out); /* gqa_min_ctx, tc_min_m, pdl, attn_split */
+int kf_ctx_get_int(kf_ctx* ctx, const char* key, int* value_out); /* gqa_min_ctx, tc_min_m, pdl, attn_split; attn_tc_error, attn_gqa_error: not 0 when a bounded wait of these kernels ran out */
 
 /* ---- device memory (huTensor::Alloc_1, src/Device/CUDA/huTensor.cu:70-103) ---- */
 int kf_malloc(kf_ctx* ctx, size_t bytes, void** dev_out);
@@ -193,12 +194,14 @@ int kf_qkv_attention(kf_ctx* ctx, void* out_dev, const void* q_dev, const void* 
 /* ---- prefill attention: causal attention of a panel of M CONSECUTIVE tokens of one sequence (positions pos_dev[0] + m) over the
  *      cache rows [0, pos_dev[0] + M).  q_dev must already be normalised + rotated and the panel's K / V rows appended
  *      (kf_qknorm_rope_kvappend).  Replaces the reference's token-by-token prompt loop (src/Manifold/GoPT.cpp:1111-1235) through
- *      attention_qk / softmax / attention_v (src/Device/CUDA/kernel/operator.cuh:573-668); flash-attention on mma.sync tensor cores. ---- */
+ *      attention_qk / softmax / attention_v (src/Device/CUDA/kernel/operator.cuh:573-668); flash-attention: panels of more than 64 tokens with
+ *      head_dim 128, an even n_head / n_kv and 16-byte aligned buffers on tcgen05, others on mma.sync. ---- */
 int kf_attn_prefill(kf_ctx* ctx, void* out_dev, const void* q_dev, const void* kcache_layer_dev, const void* vcache_layer_dev,
                     const int32_t* pos_dev, int M, int n_head, int n_kv, int head_dim, int max_seq);
 /* ---- decode attention for many sequences per step: same contract as kf_attn_decode, but the query heads that share a kv head are
  *      processed together on the tensor cores, so every cached row is read once per kv head instead of once per query head
- *      (batched decode; replaces the same reference kernels, operator.cuh:573-668).  n_head / n_kv <= 16. ---- */
+ *      (batched decode; replaces the same reference kernels, operator.cuh:573-668).  n_head / n_kv <= 16; q and the caches
+ *      16-byte aligned, seq_stride a multiple of 8 when M > 1. ---- */
 int kf_attn_decode_gqa(kf_ctx* ctx, void* out_dev, const void* q_dev, const void* kcache_layer_dev, const void* vcache_layer_dev,
                        const int32_t* pos_dev, int M, int n_head, int n_kv, int head_dim, int max_seq, int max_pos_hint, size_t seq_stride);
 /* ---- CU_swiglu_v0 (Activation.cu:86-93), CU_add3 (packedN.cuh:867-875) as stand-alone ops ---- */
