@@ -52,6 +52,26 @@ __device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], 
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+// Stages of the ring: what shared memory holds beside the warps' areas (SETS 1: two CTAs per SM), at most ten per set.  With two sets, whose tiles alternate, their
+// number is a multiple of 4 (K and V of a tile of either), so that a stage always comes back to the set that used it last: a wait tells a phase of a barrier from
+// the one before by a single bit, so the warps that wait for a use of a stage have to have waited for the use before.  With ten stages tile 5 lay where tile 0
+// had, for the other set, which would have taken it for landed while the copies of tile 0 were still under way (copies may overtake each other).
+constexpr int gqa_area(int hd, int sets, int group) { return 4 * sets * ((group + 1) & ~1) * hd * 4; }
+constexpr int gqa_stages(int hd, int sets, int group) {
+    const int fit = ((sets == 1 ? 97 : 200) * 1024 - gqa_area(hd, sets, group)) / (kTok * hd * 2), most = fit < 10 * sets ? fit : 10 * sets;
+    return sets == 1 ? most : most & ~3;
+}
+constexpr bool gqa_rings_fit() {
+    for (int hd = 64; hd <= 128; hd += 64)
+        for (int sets = 1; sets <= 2; sets++)
+            for (int group = 1; group <= 16; group++) {
+                const int n = gqa_stages(hd, sets, group);
+                if (n < 4 * sets || (sets == 2 && n % 4)) return false;
+            }
+    return true;
+}
+static_assert(gqa_rings_fit(), "two tiles of every set in flight, and a stage stays with its set");
+
 struct GqaItem {
     int m, run, kvh, t0, t1, runs;
 };
@@ -382,9 +402,8 @@ int gqa_launch(kf_ctx* ctx, void* out, const void* q, const void* kc, const void
     int rc = kf_tmap_rows(ctx, &tk, kc, (uint64_t)n_kv * HD, (uint64_t)max_seq, (uint64_t)M, stride, 64, kTok);
     if (!rc) rc = kf_tmap_rows(ctx, &tv, vc, (uint64_t)n_kv * HD, (uint64_t)max_seq, (uint64_t)M, stride, 64, kTok);
     if (rc) return rc;
-    const size_t area = (size_t)4 * SETS * ((group + 1) & ~1) * HD * 4, tile = (size_t)kTok * HD * 2;
-    const int stages  = (int)std::min<size_t>(10 * SETS, ((SETS == 1 ? 97 : 200) * 1024 - area) / tile);
-    const size_t smem = stages * tile + area + 1024;
+    const int stages  = gqa_stages(HD, SETS, group);
+    const size_t smem = (size_t)stages * kTok * HD * 2 + gqa_area(HD, SETS, group) + 1024;
     auto kern         = kf_attn_gqa_kernel<HD, SETS>;
     static bool set[kf_ctx::kMaxDevices] = {};  // function attributes are per device
     if (!set[ctx->device]) {
@@ -424,6 +443,8 @@ extern "C" int kf_attn_decode_gqa(kf_ctx* ctx, void* out, const void* q, const v
     if (hd == 128) return gqa_any<128>(ctx, out, q, kc, vc, pos_dev, M, n_head, n_kv, max_seq, len, seq_stride);
     return gqa_any<64>(ctx, out, q, kc, vc, pos_dev, M, n_head, n_kv, max_seq, len, seq_stride);
 }
+// Ring stages of a launch: host arithmetic for the test of the protocol, no device
+extern "C" int kf_attn_gqa_stages(int hd, int sets, int group) { return gqa_stages(hd, sets, group); }
 int kf_attn_gqa_error() {
     int v = 0;
     cudaMemcpyFromSymbol(&v, g_gqa_error, sizeof(v));

@@ -401,3 +401,20 @@ def test_bench_reference_arm_under_torchrun_two_ranks():
     if d["cpu_baseline"]["kind"] == "reference":  # oracle/_ref present: the reference's own primitives, exactly --steps timed samples
         assert "3 timed" in d["cpu_baseline"]["sample"]
     assert d["e2e"] == {"value": d["value"], "unit": "tokens/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0}
+
+
+def test_attention_ring_phases_are_told_apart():
+    """The decode attention's ring of shared-memory stages, followed use by use for every shape it is launched with: K and V of tile T are uses 2T and 2T + 1, use n lies
+    in stage n % stages, tile T belongs to set T % sets.  A wait names the phase of a stage's barrier by its parity alone, so it also passes while the stage is one
+    use behind: whoever waits for a use of a stage must have waited for the use before it.  The loader runs at most a ring ahead, so no stage is further behind."""
+    lib = kf.load()
+    for hd in (64, 128):
+        for sets in (1, 2):
+            for group in range(1, 17):
+                stages = lib.kf_attn_gqa_stages(hd, sets, group)
+                assert stages >= 4 * sets, (hd, sets, group, stages)
+                waited = {}  # stage -> set that waited for its last use
+                for use in range(8 * stages):
+                    mine = use // 2 % sets
+                    assert waited.get(use % stages, mine) == mine, "head size %d, %d sets, group %d: use %d of %d stages" % (hd, sets, group, use, stages)
+                    waited[use % stages] = mine

@@ -178,10 +178,14 @@ def test_prefill_tc(ctx, n_head, n_kv, M, pos0, behind, sharp):
 
 
 # ---------------------------------------------------------------------------------------------- grouped decode attention
-@pytest.mark.parametrize("hd,n_head,n_kv", [(128, 8, 8), (128, 16, 8), (128, 16, 1), (128, 24, 2), (64, 8, 2)])
-@pytest.mark.parametrize("lens,hint", [((1,), 0), ((63, 64, 65, 1, 128, 129), 128), ((256, 257, 511, 513, 40), 512), ((2000, 3, 700, 1300), 1999), ((9000,), 8999), ((9000,), 100),
-                                       ((5000, 17), 300), ((40000,), 65535), (tuple(1 + 37 * i % 190 for i in range(40)), 189),
-                                       (tuple(1 + 37 * i % 190 for i in range(300)), 100)])
+_GQA_SHAPES = [(128, 8, 8), (128, 16, 8), (128, 16, 1), (128, 24, 2), (64, 8, 2)]
+_GQA_LENS = [((1,), 0), ((63, 64, 65, 1, 128, 129), 128), ((256, 257, 511, 513, 40), 512), ((2000, 3, 700, 1300), 1999), ((9000,), 8999), ((9000,), 100),
+             ((5000, 17), 300), ((40000,), 65535), (tuple(1 + 37 * i % 190 for i in range(40)), 189), (tuple(1 + 37 * i % 190 for i in range(300)), 100)]
+# four and eight heads per kv head, each run several rings long
+_GQA_RINGS = [(128, 32, 8, (40000,), 39999), (128, 64, 8, (40000,), 39999), (128, 8, 2, (9000, 30000), 29999), (64, 32, 8, (40000,), 39999)]
+
+
+@pytest.mark.parametrize("hd,n_head,n_kv,lens,hint", [a + b for a in _GQA_SHAPES for b in _GQA_LENS] + _GQA_RINGS)
 def test_gqa_runs(ctx, hd, n_head, n_kv, lens, hint):
     """Edges of tiles and runs, lengths of their own, hints that are too small or too large, cache rows behind the last position that hold no numbers, again on
     used workspaces.  Bound as for the panel kernel: one rounding of the weights, one of the result."""
