@@ -72,6 +72,12 @@ constexpr bool gqa_rings_fit() {
 }
 static_assert(gqa_rings_fit(), "two tiles of every set in flight, and a stage stays with its set");
 
+// two results; out may start at any element
+__device__ __forceinline__ void put2(uint16_t* p, float a, float b, bool pairs) {
+    if (pairs) *reinterpret_cast<uint32_t*>(p) = pack_bf16x2(a, b);
+    else p[0] = f32_to_bf16_bits(a), p[1] = f32_to_bf16_bits(b);
+}
+
 struct GqaItem {
     int m, run, kvh, t0, t1, runs;
 };
@@ -183,6 +189,7 @@ __global__ void __launch_bounds__((4 * SETS + 1) * 32, 3 - SETS)
         return;
     }
     const int set = warp >> 2, w4 = warp & 3;
+    const bool pairs = ((uintptr_t)out & 3) == 0;
     uint32_t mph = 0, done = 0;  // done: tiles of this CTA before the current item
     bool live = true;
     auto meet = [&]() {  // all computing warps; bounded like every wait
@@ -311,7 +318,7 @@ __global__ void __launch_bounds__((4 * SETS + 1) * 32, 3 - SETS)
             }
             if (it.runs == 1) {
                 uint16_t* op = out + (head0 * group + r) * HD + c;
-                *reinterpret_cast<uint32_t*>(op) = pack_bf16x2(a.x / L_, a.y / L_), *reinterpret_cast<uint32_t*>(op + 2) = pack_bf16x2(a.z / L_, a.w / L_);
+                put2(op, a.x / L_, a.y / L_, pairs), put2(op + 2, a.z / L_, a.w / L_, pairs);
             } else {
                 __stcg(reinterpret_cast<float4*>(ws + (part0 + (size_t)it.run * group + r) * HD + c), a);
                 if (c == 0) __stcg(ws_ml + part0 + (size_t)it.run * group + r, make_float2(M_, L_));
@@ -375,7 +382,7 @@ __global__ void __launch_bounds__((4 * SETS + 1) * 32, 3 - SETS)
                             const float2 v = *reinterpret_cast<const float2*>(s_o + ((size_t)sl * per + r) * HD + d);
                             a0 += v.x, a1 += v.y;
                         }
-                        *reinterpret_cast<uint32_t*>(out + (head0 * group + r0 + r) * HD + d) = pack_bf16x2(a0 * s_i[r0 + r], a1 * s_i[r0 + r]);
+                        put2(out + (head0 * group + r0 + r) * HD + d, a0 * s_i[r0 + r], a1 * s_i[r0 + r], pairs);
                     }
                     if (r0 + per < group) meet();
                 }

@@ -222,6 +222,27 @@ def test_gqa_runs(ctx, hd, n_head, n_kv, lens, hint):
                 assert bool((err <= 2.0 ** -8 * 1.01 * (mass + want.abs()) + 1e-6).all()), (split, i, h, float((err / (mass + want.abs())).max()))
 
 
+@pytest.mark.parametrize("hd,n_head,n_kv,lens", [(128, 16, 8, (700, 3, 64)), (128, 16, 8, tuple(range(1, 41))), (64, 8, 2, (9000,))])
+def test_gqa_output_at_any_element(ctx, hd, n_head, n_kv, lens):
+    """The result may start at an odd element (whole sequences, and runs merged by the last): the same bits as an aligned one, nothing written around it."""
+    import torch
+    M, max_seq = len(lens), max(lens)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(hd + M)
+    q = torch.randn(M, n_head, hd, generator=g, device="cuda").bfloat16()
+    k, v = (torch.randn(M, max_seq, n_kv, hd, generator=g, device="cuda").bfloat16() for _ in range(2))
+    pos = torch.tensor([n - 1 for n in lens], dtype=torch.int32, device="cuda")
+    size, got = M * n_head * hd, []
+    for off in (0, 1):
+        buf = torch.full((size + 8,), 7.0, device="cuda").bfloat16()
+        torch.cuda.synchronize()
+        ctx.check(ctx.lib.kf_attn_decode_gqa(ctx.h, _ptr(buf[off:]), _ptr(q), _ptr(k), _ptr(v), _ptr(pos), M, n_head, n_kv, hd, max_seq, max_seq - 1, max_seq * n_kv * hd), "gqa")
+        ctx.sync()
+        assert bool((buf[:off] == 7).all()) and bool((buf[off + size:] == 7).all())
+        got.append(buf[off:off + size].clone())
+    assert torch.equal(got[0], got[1])
+
+
 # ---------------------------------------------------------------------------------------------- tile matmul over expert-sorted slots
 @pytest.mark.parametrize("N,K", [(64, 64), (65, 72), (8, 8), (130, 200), (192, 448), (33, 512)])
 @pytest.mark.parametrize("counts", [(64, 0, 1, 63, 65, 17), (200, 3, 0, 0, 1, 0), (16, 16, 16, 16, 16, 16)])
