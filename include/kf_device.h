@@ -101,9 +101,11 @@ uint64_t kf_scratch_generation(kf_ctx* ctx);
  * TMA-fed stream-K kernel; 0: the round-1 cp.async kernel), "gemv_tma_occ" (CTAs per SM, 1 or 2), "gemv_tma_smem_kb" (shared-memory budget),
  * "gqa_min_ctx" (single-sequence decode: context length beyond which the kv-group tensor-core attention replaces the fused per-head
  * kernel; default 1024), "tc_min_m" (token count from which kf_linear* use the tcgen05 GEMM: -1 = measured per-type crossover, 0 = never, n = from n),
- * "tc_bn" (token tile of the tcgen05 GEMM: 16, 32, 64, 128 or 256; 0 = by modelled time) */
+ * "tc_bn" (token tile of the tcgen05 GEMM: 16, 32, 64, 128 or 256; 0 = by modelled time), "attn_wait_us" (how long a wait inside kf_attn_prefill /
+ * kf_attn_decode_gqa may take, default 4 s; when one runs out the kernel ends and kf_ctx_sync -- or the next of these calls -- returns KF_ERR_CUDA, once, and the
+ * context is usable again), "attn_drop" (n > 0: the n-th thread block of these kernels loads nothing, so that its waits run out; for tests) */
 int kf_ctx_set_int(kf_ctx* ctx, const char* key, int value);
-int kf_ctx_get_int(kf_ctx* ctx, const char* key, int* value_out); /* gqa_min_ctx, tc_min_m, pdl, attn_split; attn_tc_error, attn_gqa_error: not 0 when a bounded wait of these kernels ran out */
+int kf_ctx_get_int(kf_ctx* ctx, const char* key, int* value_out); /* gqa_min_ctx, tc_min_m, pdl, attn_split; attn_tc_error, attn_gqa_error (waits for the stream): not 0 when a bounded wait of these kernels ran out and has not been reported yet */
 
 /* ---- device memory (huTensor::Alloc_1, src/Device/CUDA/huTensor.cu:70-103) ---- */
 int kf_malloc(kf_ctx* ctx, size_t bytes, void** dev_out);

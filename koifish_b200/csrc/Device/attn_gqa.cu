@@ -22,19 +22,6 @@
 namespace {
 constexpr int kTok = 64, kMaxRuns = 128, kMaxSeqs = 512;
 
-__device__ int g_gqa_error;
-__device__ __noinline__ bool gqa_wait_slow(uint32_t bar, uint32_t parity, volatile int* dead) {
-    for (int it = 0; it < (1 << 20); it++) {
-        if (mbar_try(bar, parity)) return true;
-        if (*dead) return false;
-    }
-    *dead = 1;
-    atomicExch(&g_gqa_error, 1);
-    return false;
-}
-__device__ __forceinline__ bool gqa_wait(uint32_t bar, uint32_t parity, volatile int* dead) {
-    return __all_sync(0xffffffffu, mbar_try(bar, parity) || gqa_wait_slow(bar, parity, dead));
-}
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* tm, int c0, int c1, int c2, uint64_t* bar) {
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_u32(dst)), "l"(tm), "r"(c0),
                  "r"(c1), "r"(c2), "r"(smem_u32(bar))
@@ -86,7 +73,7 @@ template <int HD, int SETS>
 __global__ void __launch_bounds__((4 * SETS + 1) * 32, 3 - SETS)
     kf_attn_gqa_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, uint16_t* __restrict__ out, float* __restrict__ ws,
                        float2* __restrict__ ws_ml, unsigned* __restrict__ cnt, const uint16_t* __restrict__ q, const int32_t* __restrict__ pos_dev, int M, int n_head, int n_kv,
-                       int max_seq, int min_chunk, int max_runs, int stages, float sc2 /* log2(e) / sqrt(hd) */) {
+                       int max_seq, int min_chunk, int max_runs, int stages, float sc2 /* log2(e) / sqrt(hd) */, const __grid_constant__ KfBound bound) {
     constexpr int HALVES = HD / 64, TILE = kTok * HD * 2, HALF = kTok * 128;  // a tile lies as halves of 64 dims: 64 rows of 128 bytes (SWIZZLE_128B)
     constexpr int kWarps = 4 * SETS, kComp = kWarps * 32, kMaxStages = 20;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -165,6 +152,7 @@ __global__ void __launch_bounds__((4 * SETS + 1) * 32, 3 - SETS)
     };
     uint32_t st = 0, ph = 0;  // ring position and its phase
     if (warp == kWarps) {
+        if (bound.drop == (int)blockIdx.x + 1) return;
         bool live = true;
         uint32_t asked = 0;
         for (int k = 0; live && k * grid < n_items; k++) {
@@ -172,7 +160,7 @@ __global__ void __launch_bounds__((4 * SETS + 1) * 32, 3 - SETS)
             if (nth(k) >= n_items || !item_of(nth(k), it)) continue;
             for (int t = it.t0; live && t < it.t1; t += kTok)
                 for (int kv = 0; kv < 2; kv++) {
-                    if (!(live = gqa_wait(smem_u32(&empty[st]), ph ^ 1, &dead))) break;
+                    if (!(live = mbar_wait_warp(smem_u32(&empty[st]), ph ^ 1, &dead, bound))) break;
                     if (lane == 0) {
                         mbar_arrive_expect_tx(&full[st], TILE);
 #pragma unroll
@@ -184,8 +172,7 @@ __global__ void __launch_bounds__((4 * SETS + 1) * 32, 3 - SETS)
                 }
         }
         if (!live)  // copies in flight write shared memory
-            for (uint32_t k = asked > (uint32_t)stages ? asked - stages : 0; k < asked; k++)
-                for (int n = 0; n < (1 << 14) && !mbar_try(smem_u32(&full[k % stages]), (k / stages) & 1); n++) {}
+            for (uint32_t k = asked > (uint32_t)stages ? asked - stages : 0; k < asked; k++) mbar_drain(smem_u32(&full[k % stages]), (k / stages) & 1, bound);
         return;
     }
     const int set = warp >> 2, w4 = warp & 3;
@@ -195,7 +182,7 @@ __global__ void __launch_bounds__((4 * SETS + 1) * 32, 3 - SETS)
     auto meet = [&]() {  // all computing warps; bounded like every wait
         __syncwarp();
         if (lane == 0) mbar_arrive(&meet_bar);
-        live = gqa_wait(smem_u32(&meet_bar), mph, &dead) && live;
+        live = mbar_wait_warp(smem_u32(&meet_bar), mph, &dead, bound) && live;
         mph ^= 1;
     };
     // 16-byte chunk c (0 .. HD / 8 - 1) of a row: half c / 8, chunk c % 8 swizzled by the row
@@ -221,7 +208,7 @@ __global__ void __launch_bounds__((4 * SETS + 1) * 32, 3 - SETS)
         for (int kt = set; kt < ntiles; kt += SETS) {
             const uint32_t n = 2 * (done + kt);
             const uint32_t sk = n % stages, pk = (n / stages) & 1, sv = (n + 1) % stages, pv = ((n + 1) / stages) & 1;
-            if (!(live = gqa_wait(smem_u32(&full[sk]), pk, &dead))) break;
+            if (!(live = mbar_wait_warp(smem_u32(&full[sk]), pk, &dead, bound))) break;
             const uint32_t kb = smem_u32(ring + (size_t)sk * TILE), vb = smem_u32(ring + (size_t)sv * TILE);
             const int tok0 = it.t0 + kt * kTok + w4 * 16;  // this warp's 16 positions
             const bool mine = tok0 < it.t1;
@@ -240,7 +227,7 @@ __global__ void __launch_bounds__((4 * SETS + 1) * 32, 3 - SETS)
             // a stage goes back when every ldmatrix of it has delivered: the matrix instructions behind them were issued with its registers
             __syncwarp();
             if (lane == 0) mbar_arrive(&empty[sk]);
-            if (!(live = gqa_wait(smem_u32(&full[sv]), pv, &dead))) break;
+            if (!(live = mbar_wait_warp(smem_u32(&full[sv]), pv, &dead, bound))) break;
             if (mine) {
                 if (tok0 + 16 > it.t1) {  // the run's last positions: no weight, and no value that might not be a number
 #pragma unroll
@@ -420,7 +407,7 @@ int gqa_launch(kf_ctx* ctx, void* out, const void* q, const void* kc, const void
     const long long items = (long long)M * runs * n_kv, slots = (long long)(3 - SETS) * ctx->sm_count;
     KF_CUDA(ctx, kf_launch_pdl(ctx, kern, dim3((unsigned)std::min(items, slots)), dim3((4 * SETS + 1) * 32), smem, tk, tv, (uint16_t*)out, ws,
                                reinterpret_cast<float2*>(ws ? ws + rows * HD : nullptr), ctx->attn_cnt, (const uint16_t*)q, pos_dev, M, n_head, n_kv, max_seq, chunk, runs, stages,
-                               1.4426950408889634f / sqrtf((float)HD)));
+                               1.4426950408889634f / sqrtf((float)HD), KfBound{ctx->wait_flags + 1, (unsigned)ctx->attn_wait_us, ctx->attn_drop}));
     KF_LAUNCH_CHECK(ctx);
     return KF_OK;
 }
@@ -446,14 +433,11 @@ extern "C" int kf_attn_decode_gqa(kf_ctx* ctx, void* out, const void* q, const v
     KF_REQUIRE(ctx, (hd == 128 || hd == 64) && n_head % n_kv == 0 && n_head / n_kv <= 16 && M >= 1 && max_seq >= 1, "head_dim 64/128, group <= 16");
     KF_REQUIRE(ctx, M == 1 || seq_stride > 0, "one sequence per token");
     KF_REQUIRE(ctx, (((uintptr_t)q | (uintptr_t)kc | (uintptr_t)vc) & 15) == 0 && (M == 1 || seq_stride % 8 == 0), "16-byte aligned rows");
+    const int rc = kf_wait_status(ctx);
+    if (rc) return rc;
     const int len = std::max(1, std::min(max_seq, max_pos_hint + 1));
     if (hd == 128) return gqa_any<128>(ctx, out, q, kc, vc, pos_dev, M, n_head, n_kv, max_seq, len, seq_stride);
     return gqa_any<64>(ctx, out, q, kc, vc, pos_dev, M, n_head, n_kv, max_seq, len, seq_stride);
 }
 // Ring stages of a launch: host arithmetic for the test of the protocol, no device
 extern "C" int kf_attn_gqa_stages(int hd, int sets, int group) { return gqa_stages(hd, sets, group); }
-int kf_attn_gqa_error() {
-    int v = 0;
-    cudaMemcpyFromSymbol(&v, g_gqa_error, sizeof(v));
-    return v;
-}

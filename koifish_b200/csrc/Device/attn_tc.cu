@@ -25,19 +25,6 @@ constexpr int kTile = kKV * kHD * 2, kHalf = kTile / 2;  // a tile lies as two h
 constexpr int kMmaW = 8, kLoadW = 9, kThreads = 10 * 32;
 constexpr size_t kSmem = 2 * kTile + 2 * kStages * kTile + 1024;
 
-__device__ int g_attn_tc_error;
-__device__ __noinline__ bool wait_slow(uint32_t bar, uint32_t parity, volatile int* dead) {
-    for (int it = 0; it < (1 << 20); it++) {
-        if (mbar_try(bar, parity)) return true;
-        if (*dead) return false;
-    }
-    *dead = 1;
-    atomicExch(&g_attn_tc_error, 1);
-    return false;
-}
-__device__ __forceinline__ bool wait1(uint32_t bar, uint32_t parity, volatile int* dead) { return mbar_try(bar, parity) || wait_slow(bar, parity, dead); }
-__device__ __forceinline__ bool wait_all(uint32_t bar, uint32_t parity, volatile int* dead) { return __all_sync(0xffffffffu, wait1(bar, parity, dead)); }
-
 // 32 columns of this lane's row; the caller waits (tcgen05.wait::ld) before it uses them
 __device__ __forceinline__ void ld32_async(uint32_t taddr, uint32_t* v) {
     asm volatile(
@@ -98,7 +85,8 @@ __device__ __forceinline__ uint64_t make_desc_v(uint32_t smem_addr) {
 
 __global__ void __launch_bounds__(kThreads, 1)
     kf_attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
-                              uint16_t* __restrict__ out, const int32_t* __restrict__ pos_dev, int M, int n_head, int n_kv, int max_seq, float sc2 /* log2(e) / sqrt(hd) */) {
+                              uint16_t* __restrict__ out, const int32_t* __restrict__ pos_dev, int M, int n_head, int n_kv, int max_seq, float sc2 /* log2(e) / sqrt(hd) */,
+                              const __grid_constant__ KfBound bound) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* sq = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     uint8_t* sk = sq + 2 * kTile;
@@ -137,7 +125,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         unsigned long long l2 = 0ull;  // the denominator, even and odd positions apart
         bool live = true;
         for (int kt = 0; kt < n_tiles; kt++) {
-            if (!(live = wait_all(sfull, kt & 1, &dead))) break;
+            if (!(live = mbar_wait_warp(sfull, kt & 1, &dead, bound))) break;
             tc_fence_after();
             // The scores are read twice, 64 positions at a time: 128 of them beside the weights do not fit the registers.  The second half is still there when the
             // maximum is known, so it goes first.
@@ -167,7 +155,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 m = mn;
             } else if (__any_sync(0xffffffffu, mn > m)) {
                 const float n = fmaxf(m, mn), f = ex2((m - n) * sc2);
-                if (!(live = wait_all(odone, (kt - 1) & 1, &dead))) break;  // the last O += P V is through
+                if (!(live = mbar_wait_warp(odone, (kt - 1) & 1, &dead, bound))) break;  // the last O += P V is through
                 tc_fence_after();
 #pragma unroll
                 for (int c = 0; c < 4; c++) {
@@ -200,7 +188,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 if (lane == 0) mbar_arrive_a(pfull + 8 * c);
             }
         }
-        if (live) live = wait_all(odone, (n_tiles - 1) & 1, &dead);
+        if (live) live = mbar_wait_warp(odone, (n_tiles - 1) & 1, &dead, bound);
         if (live) {
             tc_fence_after();
             const float2 l  = unpack2(l2);
@@ -225,7 +213,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     } else if (warp == kMmaW) {
         constexpr uint32_t id_s = make_idesc_bf16(128), id_o = make_idesc_bf16(128) | (1u << 16);  // bit 16: B is MN-major
         const uint32_t q_addr = smem_u32(sq), k_addr = smem_u32(sk), v_addr = smem_u32(sv);
-        bool live = wait_all(smem_u32(&q_full), 0, &dead);
+        bool live = mbar_wait_warp(smem_u32(&q_full), 0, &dead, bound);
         auto score = [&](int t, int stage) {  // S_t = Q_t K^T, 16 of the 128 dims per instruction
 #pragma unroll
             for (int k = 0; k < 8; k++) {
@@ -234,7 +222,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
             umma_commit_a(smem_u32(&s_full[t]));
         };
-        if (live) live = wait_all(smem_u32(&k_full[0]), 0, &dead);
+        if (live) live = mbar_wait_warp(smem_u32(&k_full[0]), 0, &dead, bound);
         if (live) {
             tc_fence_after();
             score(0, 0), score(1, 0);
@@ -244,12 +232,12 @@ __global__ void __launch_bounds__(kThreads, 1)
             const int st = kt % kStages, sn = (kt + 1) % kStages;
 #pragma unroll
             for (int t = 0; t < 2; t++) {
-                if (t == 0 && !(live = wait_all(smem_u32(&v_full[st]), (kt / kStages) & 1, &dead))) break;
+                if (t == 0 && !(live = mbar_wait_warp(smem_u32(&v_full[st]), (kt / kStages) & 1, &dead, bound))) break;
 #pragma unroll
                 for (int i = 0; i < 8; i++) {  // O_t += P_t V, 16 positions per instruction, the second half of the positions first
                     const int k = i ^ 4;
                     if (i % 4 == 0) {
-                        live = live && wait_all(smem_u32(&p_full[t][k / 4]), kt & 1, &dead);
+                        live = live && mbar_wait_warp(smem_u32(&p_full[t][k / 4]), kt & 1, &dead, bound);
                         tc_fence_after();
                     }
                     if (live) umma_ts(tmem + 256 + t * 128, tmem + t * 128 + 64 + k * 8, make_desc_v(v_addr + st * kTile + k * 2048), id_o, kt > 0 || i > 0);
@@ -258,7 +246,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 umma_commit_a(smem_u32(&o_done[t]));
                 if (kt + 1 < n_tiles) {
                     if (t == 0) {
-                        if (!(live = wait_all(smem_u32(&k_full[sn]), ((kt + 1) / kStages) & 1, &dead))) break;
+                        if (!(live = mbar_wait_warp(smem_u32(&k_full[sn]), ((kt + 1) / kStages) & 1, &dead, bound))) break;
                         tc_fence_after();
                     }
                     score(t, sn);  // behind the O above, which reads the weights from the same columns
@@ -270,9 +258,9 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         if (!live) {
             umma_commit_a(smem_u32(&done_bar));
-            for (int it = 0; it < (1 << 16) && !mbar_try(smem_u32(&done_bar), 0); it++) {}
+            mbar_drain(smem_u32(&done_bar), 0, bound);
         }
-    } else if (warp == kLoadW) {
+    } else if (warp == kLoadW && bound.drop != (int)(blockIdx.y * gridDim.x + blockIdx.x) + 1) {
         bool live = true;
         if (lane == 0) {
             mbar_arrive_expect_tx(&q_full, 2 * kTile);
@@ -283,13 +271,13 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (; kt < n_tiles; kt++) {
             const int st = kt % kStages;
             const uint32_t ph = ((kt / kStages) & 1) ^ 1;
-            if (!(live = wait_all(smem_u32(&k_empty[st]), ph, &dead))) break;
+            if (!(live = mbar_wait_warp(smem_u32(&k_empty[st]), ph, &dead, bound))) break;
             if (lane == 0) {
                 mbar_arrive_expect_tx(&k_full[st], kTile);
 #pragma unroll
                 for (int i = 0; i < 2; i++) tma_load_2d(sk + st * kTile + i * kHalf, &tm_k, kvh * kHD + i * 64, kt * kKV, &k_full[st]);
             }
-            if (!(live = wait_all(smem_u32(&v_empty[st]), ph, &dead))) break;
+            if (!(live = mbar_wait_warp(smem_u32(&v_empty[st]), ph, &dead, bound))) break;
             const bool ragged = (kt + 1) * kKV > kv_len;  // the last tile, unless it ends with a position
             uint64_t* bar = ragged ? &v_land : &v_full[st];
             if (lane == 0) {
@@ -298,7 +286,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 for (int i = 0; i < 2; i++) tma_load_2d(sv + st * kTile + i * kHalf, &tm_v, kvh * kHD + i * 64, kt * kKV, bar);
             }
             if (ragged) {
-                if (!(live = wait_all(smem_u32(&v_land), 0, &dead))) break;
+                if (!(live = mbar_wait_warp(smem_u32(&v_land), 0, &dead, bound))) break;
                 const int r0 = kv_len - kt * kKV;
                 for (int i = lane; i < (kKV - r0) * 16; i += 32)
                     *reinterpret_cast<uint4*>(sv + st * kTile + (i & 1) * kHalf + (r0 + (i >> 4)) * 128 + ((i >> 1) & 7) * 16) = make_uint4(0, 0, 0, 0);
@@ -308,9 +296,9 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
         }
         if (!live) {  // copies in flight write shared memory: wait for what was asked for
-            auto drain = [](uint64_t* bar, uint32_t parity) { for (int it = 0; it < (1 << 14) && !mbar_try(smem_u32(bar), parity); it++) {} };
-            drain(&q_full, 0);
-            for (int k = kt > 0 ? kt - 1 : 0; k <= kt && k < n_tiles; k++) drain(&k_full[k % kStages], (k / kStages) & 1), drain(&v_full[k % kStages], (k / kStages) & 1);
+            mbar_drain(smem_u32(&q_full), 0, bound);
+            for (int k = kt > 0 ? kt - 1 : 0; k <= kt && k < n_tiles; k++)
+                mbar_drain(smem_u32(&k_full[k % kStages]), (k / kStages) & 1, bound), mbar_drain(smem_u32(&v_full[k % kStages]), (k / kStages) & 1, bound);
         }
     }
     tc_fence_before();
@@ -329,7 +317,8 @@ int kf_attn_prefill_tc_ok(const kf_ctx* ctx, const void* out, const void* q, con
 }
 int kf_attn_prefill_tc(kf_ctx* ctx, void* out, const void* q, const void* kc, const void* vc, const int32_t* pos_dev, int M, int n_head, int n_kv, int max_seq) {
     CUtensorMap tq, tk, tv;
-    int rc = kf_tmap_2d(ctx, &tq, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, q, (uint64_t)n_head * kHD, (uint64_t)M, 64, kQ, CU_TENSOR_MAP_SWIZZLE_128B);
+    int rc = kf_wait_status(ctx);
+    if (!rc) rc = kf_tmap_2d(ctx, &tq, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, q, (uint64_t)n_head * kHD, (uint64_t)M, 64, kQ, CU_TENSOR_MAP_SWIZZLE_128B);
     if (!rc) rc = kf_tmap_2d(ctx, &tk, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, kc, (uint64_t)n_kv * kHD, (uint64_t)max_seq, 64, kKV, CU_TENSOR_MAP_SWIZZLE_128B);
     if (!rc) rc = kf_tmap_2d(ctx, &tv, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, vc, (uint64_t)n_kv * kHD, (uint64_t)max_seq, 64, kKV, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc) return rc;
@@ -339,12 +328,7 @@ int kf_attn_prefill_tc(kf_ctx* ctx, void* out, const void* q, const void* kc, co
         set[ctx->device] = true;
     }
     KF_CUDA(ctx, kf_launch_pdl(ctx, kf_attn_prefill_tc_kernel, dim3((M + kQ - 1) / kQ, n_head / 2), dim3(kThreads), kSmem, tq, tk, tv, (uint16_t*)out, pos_dev, M, n_head, n_kv,
-                               max_seq, 1.4426950408889634f / sqrtf((float)kHD)));
+                               max_seq, 1.4426950408889634f / sqrtf((float)kHD), KfBound{ctx->wait_flags, (unsigned)ctx->attn_wait_us, ctx->attn_drop}));
     KF_LAUNCH_CHECK(ctx);
     return KF_OK;
-}
-int kf_attn_prefill_tc_error() {
-    int v = 0;
-    cudaMemcpyFromSymbol(&v, g_attn_tc_error, sizeof(v));
-    return v;
 }

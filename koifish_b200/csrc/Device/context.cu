@@ -63,6 +63,13 @@ extern "C" int kf_ctx_create(int device, void* cuda_stream, kf_ctx** out) {
         }
         ctx->own_stream = true;
     }
+    if (cudaHostAlloc((void**)&ctx->wait_flags, 2 * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {  // one address for host and device
+        (void)cudaGetLastError();
+        if (ctx->own_stream) cudaStreamDestroy(ctx->stream);
+        delete ctx;
+        return KF_ERR_OOM;
+    }
+    ctx->wait_flags[0] = ctx->wait_flags[1] = 0;
     *out = ctx;
     return KF_OK;
 }
@@ -103,6 +110,8 @@ extern "C" int kf_ctx_destroy(kf_ctx* ctx) {
     for (void* b : scratch)
         if (b)
             cudaFree(b);
+    if (ctx->wait_flags)
+        cudaFreeHost(ctx->wait_flags);
     if (ctx->own_stream)
         cudaStreamDestroy(ctx->stream);
     delete ctx;
@@ -117,7 +126,20 @@ extern "C" int kf_ctx_sync(kf_ctx* ctx) {
     if (!ctx)
         return KF_ERR_BAD_ARG;
     KF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    return KF_OK;
+    return kf_wait_status(ctx);
+}
+int kf_wait_status(kf_ctx* ctx) {
+    volatile int* flag = ctx->wait_flags;
+    if (!flag[0] && !flag[1]) return KF_OK;
+    ctx->last_error = std::string("a bounded wait ran out in the ") + (flag[0] ? "prefill" : "grouped decode") + " attention kernel: results since the last synchronisation are not valid";
+    if (ctx->capturing) return KF_ERR_CUDA;  // nothing can be cleared here: told again by the next call
+    KF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    if (ctx->attn_cnt) {  // runs that arrived before the kernel gave up are still counted
+        KF_CUDA(ctx, cudaMemsetAsync(ctx->attn_cnt, 0, sizeof(unsigned) * ctx->attn_cnt_n, ctx->stream));
+        KF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    }
+    flag[0] = flag[1] = 0;
+    return KF_ERR_CUDA;
 }
 extern "C" void* kf_ctx_stream(kf_ctx* ctx) { return ctx ? (void*)ctx->stream : nullptr; }
 extern "C" int kf_ctx_sm_count(kf_ctx* ctx) { return ctx ? ctx->sm_count : 0; }
@@ -144,11 +166,10 @@ extern "C" int kf_ctx_get_int(kf_ctx* ctx, const char* key, int* value_out) {
         *value_out = ctx->tp_fused;
     else if (!strcmp(key, "gemv_xg_min_m"))
         *value_out = ctx->gemv_xg_min_m;
-    else if (!strcmp(key, "attn_tc_error"))
-        *value_out = kf_attn_prefill_tc_error();
-    else if (!strcmp(key, "attn_gqa_error"))
-        *value_out = kf_attn_gqa_error();
-    else
+    else if (!strcmp(key, "attn_tc_error") || !strcmp(key, "attn_gqa_error")) {
+        if (!ctx->capturing) KF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        *value_out = ((volatile int*)ctx->wait_flags)[key[5] == 'g'];
+    } else
         return KF_ERR_BAD_ARG;
     return KF_OK;
 }
@@ -179,6 +200,10 @@ extern "C" int kf_ctx_set_int(kf_ctx* ctx, const char* key, int value) {
         ctx->attn_split = value;
     else if (!strcmp(key, "gqa_min_ctx"))
         ctx->gqa_min_ctx = value;
+    else if (!strcmp(key, "attn_wait_us"))
+        ctx->attn_wait_us = value > 0 ? value : 4000000;
+    else if (!strcmp(key, "attn_drop"))
+        ctx->attn_drop = value;
     else if (!strcmp(key, "attn_warps"))
         ctx->attn_warps = value;
     else if (!strcmp(key, "gemv_tma"))

@@ -59,6 +59,10 @@ struct kf_ctx {
     int deq_fma      = 1;
     int attn_split   = 0;
     int gqa_min_ctx  = 1024;  // single-sequence decode: contexts beyond this use the kv-group tensor-core attention (Transformer layer reads it)
+    // bounded waits of the attention kernels that run on copies and barriers: a kernel that gives up sets its flag ([0] prefill, [1] grouped decode; host memory)
+    int* wait_flags  = nullptr;
+    int attn_wait_us = 4000000;  // how long a wait may take
+    int attn_drop    = 0;        // n > 0: the n-th CTA of these kernels issues no copies, so that a wait of it runs out (tests)
     int attn_warps   = 0;  // warps per CTA of the cluster attention (0 = default)
     int debug_skip   = 0;  // only honoured in builds with -DKF_DEBUG_KNOBS (timing experiments: bit 0 skips attention, bit 1 the skinny GEMVs)
     // persistent TMA-fed stream-K GEMV (gemv_tma.cu): on / CTAs per SM / shared-memory budget per SM in KB
@@ -142,6 +146,8 @@ void kf_tmap_cache_destroy(kf_ctx* ctx);  // gemm_tc.cu
 int kf_gemv_tma(kf_ctx* ctx, int n, void* const* y, const kf_tensor_desc* w, const void* x, int M, int epilogue, const void* residual,
                 const void* norm_w, float norm_eps);
 int kf_ensure_gemv_ws(kf_ctx* ctx, size_t bytes, int counters);
+// KF_ERR_CUDA when a bounded wait of a kernel ran out since the last time it was asked; the counters such a kernel left half way are cleared first
+int kf_wait_status(kf_ctx* ctx);
 // awq.cu
 int kf_awq_dequant(kf_ctx* ctx, const kf_tensor_desc* w, void* out_bf16, int transposed);
 int kf_awq_gemv(kf_ctx* ctx, void* y, const kf_tensor_desc* w, const void* x, int M, int epilogue, const void* residual);
@@ -166,10 +172,13 @@ int kf_gemm_tc(kf_ctx* ctx, void* y, const kf_tensor_desc* w, const void* xp, in
 // attn_tc.cu: panels of more than 64 queries on tcgen05
 int kf_attn_prefill_tc_ok(const kf_ctx* ctx, const void* out, const void* q, const void* kc, const void* vc, int M, int n_head, int n_kv, int hd);
 int kf_attn_prefill_tc(kf_ctx* ctx, void* out, const void* q, const void* kc, const void* vc, const int32_t* pos_dev, int M, int n_head, int n_kv, int max_seq);
-int kf_attn_prefill_tc_error();
-int kf_attn_gqa_error();  // attn_gqa.cu
 int kf_gemm_tc_multi(kf_ctx* ctx, int n, void* const* y, const kf_tensor_desc* w, const void* xp, int M, int epilogue, const void* residual);
 
+struct KfBound {  // kernel parameter: see wait_flags
+    int* flag;
+    unsigned us;
+    int drop;
+};
 #ifdef __CUDACC__
 // Launch with the programmatic-dependent-launch attribute (when ctx->pdl): the kernel may start while its predecessor in the stream
 // is still draining; it must execute kf_grid_dependency_wait() before touching anything the predecessor writes.

@@ -57,6 +57,33 @@ __device__ __noinline__ void mbar_wait_sleepy(uint64_t* bar, uint32_t parity) {
     }
     __trap();
 }
+// Bounded waits that report (attn_tc.cu, attn_gqa.cu): when one has waited for `us` microseconds, `dead` (shared memory) ends all roles of the CTA and `flag` (host
+// memory of the context) tells the host, which returns an error where it synchronises (kf_wait_status).
+__device__ __forceinline__ unsigned long long global_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
+__device__ __noinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity, volatile int* dead, volatile int* flag, uint32_t us) {
+    const unsigned long long t0 = global_ns();
+    do {
+        if (mbar_try(bar, parity)) return true;
+        if (*dead) return false;
+    } while (global_ns() - t0 < us * 1000ull);
+    *dead = 1;
+    *flag = 1;
+    __threadfence_system();
+    return false;
+}
+// one warp, the same answer in every lane
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* dead, const KfBound& b) {
+    return __all_sync(0xffffffffu, mbar_try(bar, parity) || mbar_wait_bounded(bar, parity, dead, b.flag, b.us));
+}
+// copies or matrix instructions in flight, after a wait has run out
+__device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t parity, const KfBound& b) {
+    const unsigned long long t0 = global_ns();
+    while (!mbar_try(bar, parity) && global_ns() - t0 < b.us * 1000ull) {}
+}
 __device__ __forceinline__ void lds128(uint32_t a, uint32_t* r) {
     asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
 }

@@ -243,6 +243,46 @@ def test_gqa_output_at_any_element(ctx, hd, n_head, n_kv, lens):
     assert torch.equal(got[0], got[1])
 
 
+@pytest.mark.parametrize("kind,lens", [("decode", (5000, 900)), ("decode", tuple(range(1, 41))), ("prefill", (300,))])
+def test_attention_wait_that_runs_out(ctx, kind, lens):
+    """One thread block loads nothing, its waits end after 2 ms: the call that synchronises (or the next attention call) says so, once, and the call after that has
+    the bits of the one before: no arrival of the other blocks is left counted."""
+    import torch
+    lib, hd, n_head, n_kv, n = ctx.lib, 128, 16, 8, len(lens)
+    M, max_seq = (n, max(lens)) if kind == "decode" else (lens[0], lens[0])
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n)
+    q = torch.randn(M, n_head, hd, generator=g, device="cuda").bfloat16()
+    k, v = (torch.randn(n, max_seq, n_kv, hd, generator=g, device="cuda").bfloat16() for _ in range(2))
+    pos = torch.tensor([x - 1 for x in lens] if kind == "decode" else list(range(M)), dtype=torch.int32, device="cuda")
+    out = torch.zeros(M, n_head, hd, device="cuda").bfloat16()
+    torch.cuda.synchronize()
+
+    def call():
+        if kind == "decode":
+            return lib.kf_attn_decode_gqa(ctx.h, _ptr(out), _ptr(q), _ptr(k), _ptr(v), _ptr(pos), M, n_head, n_kv, hd, max_seq, max_seq - 1, max_seq * n_kv * hd)
+        return lib.kf_attn_prefill(ctx.h, _ptr(out), _ptr(q), _ptr(k), _ptr(v), _ptr(pos), M, n_head, n_kv, hd, max_seq)
+
+    key = "attn_gqa_error" if kind == "decode" else "attn_tc_error"
+    assert call() == 0 and lib.kf_ctx_sync(ctx.h) == 0
+    good = out.clone()
+    torch.cuda.synchronize()
+    for told_by in ("sync", "call"):
+        ctx.set_int("attn_wait_us", 2000), ctx.set_int("attn_drop", 1)
+        try:
+            assert call() == 0
+        finally:
+            ctx.set_int("attn_wait_us", 0), ctx.set_int("attn_drop", 0)
+        assert ctx.get_int(key) == 1
+        assert (lib.kf_ctx_sync(ctx.h) if told_by == "sync" else call()) != 0
+        assert b"wait ran out" in lib.kf_last_error(ctx.h)
+        assert ctx.get_int(key) == 0 and lib.kf_ctx_sync(ctx.h) == 0
+        out.zero_()
+        torch.cuda.synchronize()
+        assert call() == 0 and lib.kf_ctx_sync(ctx.h) == 0
+        assert torch.equal(out, good)
+
+
 # ---------------------------------------------------------------------------------------------- tile matmul over expert-sorted slots
 @pytest.mark.parametrize("N,K", [(64, 64), (65, 72), (8, 8), (130, 200), (192, 448), (33, 512)])
 @pytest.mark.parametrize("counts", [(64, 0, 1, 63, 65, 17), (200, 3, 0, 0, 1, 0), (16, 16, 16, 16, 16, 16)])
