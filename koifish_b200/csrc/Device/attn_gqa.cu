@@ -93,11 +93,12 @@ __global__ void __launch_bounds__((4 * SETS + 1) * 32, 3 - SETS)
     }
     kf_grid_launch_dependents();
     kf_grid_dependency_wait();  // queries, the rows of the current position, positions, workspace
-    // the launch was sized from a hint: a sequence that needs them takes longer runs, so any length is covered
+    // the launch was sized from a hint: a sequence that needs them takes longer runs, so any length is covered; one without positions has one empty run, whose
+    // result is what an empty softmax gives (0 / 0)
     auto shape = [&](int m, int& chunk, int& len) {
-        len   = min(pos_dev[m] + 1, max_seq);
+        len   = max(0, min(pos_dev[m] + 1, max_seq));
         chunk = max(min_chunk, ((len + max_runs - 1) / max_runs + kTok - 1) / kTok * kTok);
-        return (len + chunk - 1) / chunk;
+        return max(1, (len + chunk - 1) / chunk);
     };
     const bool whole = max_runs == 1, dealt = M <= (whole ? kMaxSeqs / 2 : kMaxSeqs);
     if (dealt && whole) {

@@ -283,6 +283,35 @@ def test_attention_wait_that_runs_out(ctx, kind, lens):
         assert torch.equal(out, good)
 
 
+@pytest.mark.parametrize("split", [0, 3])
+@pytest.mark.parametrize("lens", [(70, 0, 300, 1), (0,), tuple(i % 5 * 30 for i in range(40))])
+def test_gqa_sequence_without_positions(ctx, lens, split):
+    """Position -1: no key, so the softmax has no value; the rows are written all the same (not a number), those of the other sequences are right."""
+    import torch
+    hd, n_head, n_kv, M, max_seq = 128, 16, 8, len(lens), 320
+    g = torch.Generator(device="cuda")
+    g.manual_seed(M)
+    q = torch.randn(M, n_head, hd, generator=g, device="cuda").bfloat16()
+    k, v = (torch.randn(M, max_seq, n_kv, hd, generator=g, device="cuda").bfloat16() for _ in range(2))
+    pos = torch.tensor([n - 1 for n in lens], dtype=torch.int32, device="cuda")
+    out = torch.full((M, n_head, hd), 7.0, device="cuda").bfloat16()
+    torch.cuda.synchronize()
+    ctx.set_int("attn_split", split)
+    try:
+        ctx.check(ctx.lib.kf_attn_decode_gqa(ctx.h, _ptr(out), _ptr(q), _ptr(k), _ptr(v), _ptr(pos), M, n_head, n_kv, hd, max_seq, max(lens), max_seq * n_kv * hd), "gqa")
+        ctx.sync()
+    finally:
+        ctx.set_int("attn_split", 0)
+    for i, n in enumerate(lens):
+        if n == 0:
+            assert bool(out[i].isnan().all())
+            continue
+        kk, vv = (t[i, :n].double().repeat_interleave(n_head // n_kv, 1) for t in (k, v))
+        p = torch.softmax(torch.einsum("thd,hd->ht", kk, q[i].double()) / hd ** 0.5, -1)
+        want, mass = torch.einsum("ht,thd->hd", p, vv), torch.einsum("ht,thd->hd", p, vv.abs())
+        assert bool(((out[i].double() - want).abs() <= 2.0 ** -8 * 1.01 * (mass + want.abs()) + 1e-6).all())
+
+
 # ---------------------------------------------------------------------------------------------- tile matmul over expert-sorted slots
 @pytest.mark.parametrize("N,K", [(64, 64), (65, 72), (8, 8), (130, 200), (192, 448), (33, 512)])
 @pytest.mark.parametrize("counts", [(64, 0, 1, 63, 65, 17), (200, 3, 0, 0, 1, 0), (16, 16, 16, 16, 16, 16)])
