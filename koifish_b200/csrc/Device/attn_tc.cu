@@ -52,6 +52,8 @@ __device__ __forceinline__ float ex2(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+// the maximum of scores that are all -inf so far is taken as 0, so that their weights are 0
+__device__ __forceinline__ float finite_or_0(float m) { return m == -INFINITY ? 0.f : m; }
 __device__ __forceinline__ unsigned long long pack2(float a, float b) {
     unsigned long long r;
     asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
@@ -154,7 +156,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (kt == 0) {
                 m = mn;
             } else if (__any_sync(0xffffffffu, mn > m)) {
-                const float n = fmaxf(m, mn), f = ex2((m - n) * sc2);
+                const float n = fmaxf(m, mn), f = ex2((m - finite_or_0(n)) * sc2);
                 if (!(live = mbar_wait_warp(odone, (kt - 1) & 1, &dead, bound))) break;  // the last O += P V is through
                 tc_fence_after();
 #pragma unroll
@@ -169,7 +171,8 @@ __global__ void __launch_bounds__(kThreads, 1)
                 wait_st();
                 l2 = mul2(l2, pack2(f, f)), m = n;
             }
-            const unsigned long long sc22 = pack2(sc2, sc2), nm2 = pack2(-m * sc2, -m * sc2);
+            const float base = finite_or_0(m) * sc2;
+            const unsigned long long sc22 = pack2(sc2, sc2), nm2 = pack2(-base, -base);
 #pragma unroll
             for (int c = 1; c >= 0; c--) {  // one half's O += P V runs while the other half's weights are formed
                 if (c == 0) fetch(0);

@@ -177,6 +177,32 @@ def test_prefill_tc(ctx, n_head, n_kv, M, pos0, behind, sharp):
         assert bool((err <= 2.0 ** -8 * 1.01 * (mass + want.abs()) + 1e-6).all()), (h, float((err / (mass + want.abs())).max()))
 
 
+@pytest.mark.parametrize("M,pos0,gone", [(100, 256, (0, 128)), (100, 256, (0, 250)), (300, 130, (0, 130)), (200, 300, (128, 256))])
+def test_prefill_scores_of_minus_infinity(ctx, M, pos0, gone):
+    """Whole key tiles whose scores are -inf, the first ones among them: their weights are 0, the keys behind them count."""
+    import torch
+    hd, n_head, n_kv, n = 128, 16, 8, pos0 + M
+    g = torch.Generator(device="cuda")
+    g.manual_seed(M + pos0)
+    q = torch.randn(M, n_head, hd, generator=g, device="cuda").bfloat16()
+    q[..., 0] = q[..., 0].abs() + 0.25
+    k, v = (torch.randn(n, n_kv, hd, generator=g, device="cuda").bfloat16() for _ in range(2))
+    k[gone[0]:gone[1], :, 0] = float("-inf")
+    pos = torch.arange(pos0, n, dtype=torch.int32, device="cuda")
+    out = torch.zeros(M, n_head, hd, device="cuda").bfloat16()
+    torch.cuda.synchronize()
+    ctx.check(ctx.lib.kf_attn_prefill(ctx.h, _ptr(out), _ptr(q), _ptr(k), _ptr(v), _ptr(pos), M, n_head, n_kv, hd, n), "prefill")
+    ctx.sync()
+    keys = torch.arange(n, device="cuda")
+    unseen = (keys[None] > pos[:, None]) | ((keys >= gone[0]) & (keys < gone[1]))[None]
+    k[gone[0]:gone[1], :, 0] = 0
+    for h in range(n_head):
+        kk, vv = k[:, h // 2].double(), v[:, h // 2].double()
+        p = torch.softmax((q[:, h].double() @ kk.T / hd ** 0.5).masked_fill(unseen, float("-inf")), -1)
+        want, mass = p @ vv, p @ vv.abs()
+        assert bool(((out[:, h].double() - want).abs() <= 2.0 ** -8 * 1.01 * (mass + want.abs()) + 1e-6).all()), h
+
+
 # ---------------------------------------------------------------------------------------------- grouped decode attention
 _GQA_SHAPES = [(128, 8, 8), (128, 16, 8), (128, 16, 1), (128, 24, 2), (64, 8, 2)]
 _GQA_LENS = [((1,), 0), ((63, 64, 65, 1, 128, 129), 128), ((256, 257, 511, 513, 40), 512), ((2000, 3, 700, 1300), 1999), ((9000,), 8999), ((9000,), 100),
