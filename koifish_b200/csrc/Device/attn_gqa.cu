@@ -248,15 +248,17 @@ __global__ void __launch_bounds__((4 * SETS + 1) * 32, 3 - SETS)
                 float mx_lo = fmaxf(fmaxf(sc[0][0], sc[0][1]), fmaxf(sc[1][0], sc[1][1])), mx_hi = fmaxf(fmaxf(sc[0][2], sc[0][3]), fmaxf(sc[1][2], sc[1][3]));
                 mx_lo = fmaxf(mx_lo, __shfl_xor_sync(0xffffffffu, mx_lo, 1)), mx_lo = fmaxf(mx_lo, __shfl_xor_sync(0xffffffffu, mx_lo, 2));
                 mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 1)), mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 2));
-                const float mn_lo = fmaxf(m_lo, mx_lo * sc2), mn_hi = fmaxf(m_hi, mx_hi * sc2);  // finite: position tok0 is seen
-                const float c_lo = exp2f(m_lo - mn_lo), c_hi = exp2f(m_hi - mn_hi);
+                const float mn_lo = fmaxf(m_lo, mx_lo * sc2), mn_hi = fmaxf(m_hi, mx_hi * sc2);
+                // where all scores so far are -inf their weights are 0, whichever positions a run starts with
+                const float b_lo = mn_lo == -INFINITY ? 0.f : mn_lo, b_hi = mn_hi == -INFINITY ? 0.f : mn_hi;
+                const float c_lo = exp2f(m_lo - b_lo), c_hi = exp2f(m_hi - b_hi);
                 m_lo = mn_lo, m_hi = mn_hi;
                 float rs_lo = 0.f, rs_hi = 0.f;
                 uint32_t pa[4];
 #pragma unroll
                 for (int j = 0; j < 2; j++) {
-                    const float p0 = exp2f(fmaf(sc[j][0], sc2, -mn_lo)), p1 = exp2f(fmaf(sc[j][1], sc2, -mn_lo));
-                    const float p2 = exp2f(fmaf(sc[j][2], sc2, -mn_hi)), p3 = exp2f(fmaf(sc[j][3], sc2, -mn_hi));
+                    const float p0 = exp2f(fmaf(sc[j][0], sc2, -b_lo)), p1 = exp2f(fmaf(sc[j][1], sc2, -b_lo));
+                    const float p2 = exp2f(fmaf(sc[j][2], sc2, -b_hi)), p3 = exp2f(fmaf(sc[j][3], sc2, -b_hi));
                     rs_lo += p0 + p1, rs_hi += p2 + p3;
                     pa[j * 2 + 0] = pack_bf16x2(p0, p1), pa[j * 2 + 1] = pack_bf16x2(p2, p3);
                 }

@@ -338,6 +338,36 @@ def test_gqa_sequence_without_positions(ctx, lens, split):
         assert bool(((out[i].double() - want).abs() <= 2.0 ** -8 * 1.01 * (mass + want.abs()) + 1e-6).all())
 
 
+@pytest.mark.parametrize("split", [0, 3])
+@pytest.mark.parametrize("lens", [(700, 129, 400), tuple(129 + i for i in range(40))])
+@pytest.mark.parametrize("gone", [(0, 16), (0, 64), (64, 128), (17, 111)])
+def test_gqa_scores_of_minus_infinity(ctx, lens, split, gone):
+    """Positions whose scores are -inf, all of a warp's or of a run's first ones among them: their weights are 0, the others count."""
+    import torch
+    hd, n_head, n_kv, M, max_seq = 128, 16, 8, len(lens), max(lens)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(M + gone[1])
+    q = torch.randn(M, n_head, hd, generator=g, device="cuda").bfloat16()
+    q[..., 0] = q[..., 0].abs() + 0.25
+    k, v = (torch.randn(M, max_seq, n_kv, hd, generator=g, device="cuda").bfloat16() for _ in range(2))
+    k[:, gone[0]:gone[1], :, 0] = float("-inf")
+    pos = torch.tensor([n - 1 for n in lens], dtype=torch.int32, device="cuda")
+    out = torch.full((M, n_head, hd), 7.0, device="cuda").bfloat16()
+    torch.cuda.synchronize()
+    ctx.set_int("attn_split", split)
+    try:
+        ctx.check(ctx.lib.kf_attn_decode_gqa(ctx.h, _ptr(out), _ptr(q), _ptr(k), _ptr(v), _ptr(pos), M, n_head, n_kv, hd, max_seq, max_seq - 1, max_seq * n_kv * hd), "gqa")
+        ctx.sync()
+    finally:
+        ctx.set_int("attn_split", 0)
+    for i, n in enumerate(lens):
+        at = torch.tensor([t for t in range(n) if not gone[0] <= t < gone[1]], device="cuda")
+        kk, vv = (t[i, at].double().repeat_interleave(n_head // n_kv, 1) for t in (k, v))
+        p = torch.softmax(torch.einsum("thd,hd->ht", kk, q[i].double()) / hd ** 0.5, -1)
+        want, mass = torch.einsum("ht,thd->hd", p, vv), torch.einsum("ht,thd->hd", p, vv.abs())
+        assert bool(((out[i].double() - want).abs() <= 2.0 ** -8 * 1.01 * (mass + want.abs()) + 1e-6).all()), i
+
+
 # ---------------------------------------------------------------------------------------------- tile matmul over expert-sorted slots
 @pytest.mark.parametrize("N,K", [(64, 64), (65, 72), (8, 8), (130, 200), (192, 448), (33, 512)])
 @pytest.mark.parametrize("counts", [(64, 0, 1, 63, 65, 17), (200, 3, 0, 0, 1, 0), (16, 16, 16, 16, 16, 16)])
