@@ -985,7 +985,8 @@ __global__ void kf_moe_table_slots_kernel(const kf_table_route* __restrict__ rou
     const int e = r.idx[i], sl = soff[e] + r.work[i];
     r.entry_slot[i] = sl, r.slot_row[sl] = i / r.top, r.slot_group[sl] = e;
 }
-// out[m] = sum_j wgt[m][j] * y[slot(m, j)]  (+ sigmoid(sg[m]) * shared[m]), choices added in their routing order; a choice without a slot adds nothing.
+// out[m] = sum_j wgt[m][j] * y[slot(m, j)]  (+ sigmoid(sg[m]) * shared[m]), choices added in their routing order; a choice without a slot (a token whose logits are
+// no numbers has no other) counts as a row of zeros, so a weight that is not a number still shows in the result.
 // Bound by bytes (every slot's row once), as long as enough of them are in flight: V floats a thread, one pass over the row by as many blocks as it
 // needs, the rows of eight choices requested together.  One float at a time, one request after the other: 14.0 us for 512 tokens of six choices of
 // 2048 floats, 7.5 us so.  V = 1: rows or buffers that are not made of 16-byte pieces.
@@ -1008,10 +1009,10 @@ __global__ void __launch_bounds__(256) kf_moe_combine_kernel(float* __restrict__
         for (int j = 0; j < kBatch; j++) sl[j] = j0 + j < top ? slots[j0 + j] : -1;
 #pragma unroll
         for (int j = 0; j < kBatch; j++)
-            if (sl[j] >= 0) v[j] = *reinterpret_cast<const Vec*>(y + (size_t)sl[j] * dim + d);
+            v[j] = sl[j] >= 0 ? *reinterpret_cast<const Vec*>(y + (size_t)sl[j] * dim + d) : Vec{};
 #pragma unroll
         for (int j = 0; j < kBatch; j++)
-            if (sl[j] >= 0) {
+            if (j0 + j < top) {
                 const float wj = w[j0 + j];
 #pragma unroll
                 for (int i = 0; i < V; i++) s.f[i] = fmaf(wj, v[j].f[i], s.f[i]);

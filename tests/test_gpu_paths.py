@@ -479,3 +479,24 @@ def test_combine(ctx, M, dim, top, shift, shared, accumulate):
         terms.append(before)
     mass = sum(t.abs() for t in terms)
     assert bool(((out.double() - sum(terms)).abs() <= 2.0 ** -24 * (top + 6) * mass + 1e-30).all())
+
+
+@pytest.mark.parametrize("M,dim", [(9, 64), (100, 1023)])
+def test_router_row_that_is_no_number(ctx, M, dim):
+    """A token whose router logits are all NaN chooses nothing: its result is NaN, not a sum of nothing, and the other tokens do not notice."""
+    E, top, bad = 8, 4, 3
+    n = M * top
+    idx, wgt, offs, es, sr, sg, work = (ctx.zeros(4 * k) for k in (n, n, E + 1, n, n, n, 2 * n + E))
+    lg = np.random.default_rng(M).standard_normal((M, E)).astype(np.float32)
+    lg[bad] = np.nan
+    lgd, out = ctx.array(lg), ctx.zeros(4 * M * dim)
+    y = np.random.default_rng(dim).standard_normal((n, dim)).astype(np.float32)
+    yd = ctx.array(y)
+    ctx.check(ctx.lib.kf_moe_route(ctx.h, idx.ptr, wgt.ptr, offs.ptr, es.ptr, sr.ptr, sg.ptr, work.ptr, lgd.ptr, E, None, M, E, top), "route")
+    ctx.check(ctx.lib.kf_moe_combine(ctx.h, out.ptr, yd.ptr, es.ptr, wgt.ptr, None, None, 0, M, dim, top), "combine")
+    got, slot, w = out.numpy(np.float32, (M, dim)), es.numpy(np.int32, (M, top)), wgt.numpy(np.float32, (M, top)).astype(np.float64)
+    assert np.isnan(got[bad]).all() and (slot[bad] == -1).all()
+    for m in range(M):
+        if m != bad:
+            terms = w[m, :, None] * y[slot[m]].astype(np.float64)
+            assert (np.abs(got[m] - terms.sum(0)) <= 2.0 ** -24 * (top + 6) * np.abs(terms).sum(0) + 1e-30).all()
