@@ -142,7 +142,11 @@ static int linear_any(kf_ctx* ctx, int n, void* const* y, const kf_tensor_desc* 
         rc = kf_tc_prepare_x(ctx, &w[0], xin, M, &xp);
         if (rc) return rc;
     }
-    if (epilogue == 2 && tc_fusable(&w[0], &w[1]) && ((uintptr_t)y[0] & 15) == 0) {  // gate, up and CU_swiglu_v0 in one launch
+    // gate, up and CU_swiglu_v0 in one launch; not where the matmul reads x itself (bf16 and 8-bit weights without a norm) and the result lies over it: an item
+    // would overwrite activations that others have yet to read
+    const char *x0 = (const char*)x, *y0 = (const char*)y[0];
+    const bool over_x = xp == x && y0 < x0 + (size_t)M * K * 2 && x0 < y0 + (size_t)M * w[0].rows * 2;
+    if (epilogue == 2 && tc_fusable(&w[0], &w[1]) && ((uintptr_t)y[0] & 15) == 0 && !over_x) {
         void* yy[2] = {y[0], y[0]};
         return kf_gemm_tc_multi(ctx, 2, yy, w, xp, M, 2, nullptr);
     }

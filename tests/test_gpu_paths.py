@@ -138,6 +138,28 @@ def test_tc_tiles_and_epilogues(ctx, typ, M, tc_bn, splits, rows, cols):
         ctx.set_int("tc_min_m", -1), ctx.set_int("tc_bn", 0), ctx.set_int("gemv_splitk", 0)
 
 
+@pytest.mark.parametrize("typ", [kf.KF_T_BF16, kf.KF_T_F8E5M2, kf.KF_T_Q4])
+@pytest.mark.parametrize("M,rows,cols,at", [(16, 512, 1024, 0), (300, 4096, 1024, 0), (300, 1024, 4096, 16), (700, 3072, 3072, -64)])
+def test_tc_swiglu_over_its_input(ctx, typ, M, rows, cols, at):
+    """The result may lie over the activations, `at` elements behind their start: the bits of a result in a buffer of its own."""
+    import ctypes as C
+
+    import torch
+    mk = lambda seed: (make_q(ctx, typ, rows, cols, seed) if typ != kf.KF_T_BF16 else _bf16_weight(ctx, rows, cols, seed))[0]  # noqa: E731
+    wg, wu = mk(5), mk(6)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(M)
+    x = torch.randn(M * cols, generator=g, device="cuda").bfloat16()
+    own, buf = torch.zeros(M * rows, device="cuda").bfloat16(), torch.zeros(M * max(rows, cols) + 256, device="cuda").bfloat16()
+    buf[64:64 + M * cols] = x
+    torch.cuda.synchronize()
+    dg, du = wg.desc(), wu.desc()
+    ctx.check(ctx.lib.kf_linear_swiglu(ctx.h, _ptr(own), C.byref(dg), C.byref(du), _ptr(x), M), "swiglu")
+    ctx.check(ctx.lib.kf_linear_swiglu(ctx.h, _ptr(buf[64 + at:]), C.byref(dg), C.byref(du), _ptr(buf[64:]), M), "swiglu over x")
+    ctx.sync()
+    assert torch.equal(own, buf[64 + at:64 + at + M * rows])
+
+
 def _bf16_weight(ctx, rows, cols, seed):
     d = kf.fill_normal(ctx, rows * cols, seed, 0.02)
     bits = d.numpy(np.uint16)
