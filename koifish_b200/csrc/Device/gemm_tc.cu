@@ -898,8 +898,8 @@ int launch_tc_bn(kf_ctx* ctx, GemmParams& p, const void* const* wdata, int nw, c
         static const double kb_packed[5] = {0.235, 0.235, 0.24, 0.26, 0.42}, kb_bf16[5] = {0.09, 0.10, 0.16, 0.24, 0.39};
         const double t_kb = FMT == TF_BF16 ? kb_bf16[i] : kb_packed[i];
         const int items   = tiles * ((p.M + b - 1) / b);
-        for (int s = 1; s <= 16 && s <= nraw; s++) {
-            if (ctx->gemv_splitk > 0 && s != std::min(ctx->gemv_splitk, nraw)) continue;
+        const int given = std::min(ctx->gemv_splitk, nraw);  // > 0: the split asked for
+        for (int s = given > 0 ? given : 1; s <= (given > 0 ? given : std::min(16, nraw)); s++) {
             const int waves = (items * s + ctx->sm_count - 1) / ctx->sm_count, len = (nraw + s - 1) / s * KBR;
             if (ctx->gemv_exact) {
                 const double c = waves * (len + 2.0 + (s > 1 ? b / 16.0 : 0.0));

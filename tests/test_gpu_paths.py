@@ -160,6 +160,28 @@ def test_tc_swiglu_over_its_input(ctx, typ, M, rows, cols, at):
     assert torch.equal(own, buf[64 + at:64 + at + M * rows])
 
 
+@pytest.mark.parametrize("tc_bn", [0, 64])
+def test_tc_split_as_asked(ctx, tc_bn):
+    """gemv_splitk is taken as it is, up to the number of k stages (K = 5120 in 4 bits: 20 of 256), and so is the token tile beside it.  Sums of parts differ in
+    their last bits from one pass: 17 and more parts must not give the bits of one, and stay within 1e-4 of the result's rms (320 partial sums on tensor cores, each off by up to 2^-23)."""
+    import torch
+    rows, cols, M = 256, 5120, 40
+    w, wd = make_q(ctx, kf.KF_T_Q4, rows, cols)
+    x = kf.fill_normal(ctx, M * cols, 7, 1.0)
+    want = bf16_tensor(x, M, cols).double() @ wd.double().T
+    got = {}
+    ctx.set_int("tc_bn", tc_bn)
+    try:
+        for s in (1, 17, 20, 1000):
+            ctx.set_int("gemv_splitk", s)
+            got[s] = torch.from_numpy(kf.linear(ctx, w, x, M, kf.KF_EPI_F32).numpy(np.float32, (M, rows))).cuda()
+            assert float(((got[s].double() - want).abs().max() / want.square().mean().sqrt())) < 1e-4
+    finally:
+        ctx.set_int("gemv_splitk", 0), ctx.set_int("tc_bn", 0)
+    assert not torch.equal(got[1], got[17]) and not torch.equal(got[17], got[20])
+    assert torch.equal(got[20], got[1000])
+
+
 def _bf16_weight(ctx, rows, cols, seed):
     d = kf.fill_normal(ctx, rows * cols, seed, 0.02)
     bits = d.numpy(np.uint16)
