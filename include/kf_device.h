@@ -97,8 +97,8 @@ uint64_t kf_scratch_generation(kf_ctx* ctx);
 /* tuning knobs for sweeps: "gemv_splitk" (0 = heuristic), "gemv_variant", "gemv_exact" (0: factored dequant, NOT reference-exact),
  * "gemv_cluster" (single-token split-K merged inside a thread-block cluster), "attn_split", "attn_warps", "pdl" (programmatic
  * dependent launch), "deq_fma" (1, default: the dequant expression step*k - zero rounds ONCE in bf16, as the reference's kernel does when built
- * for sm_90+; 0: twice, as its -fmad=false / pre-sm_90 builds), "gemv_tma" (1, default: decode GEMVs of 4-bit weights take the persistent
- * TMA-fed stream-K kernel; 0: the round-1 cp.async kernel), "gemv_tma_occ" (CTAs per SM, 1 or 2), "gemv_tma_smem_kb" (shared-memory budget),
+ * for sm_90+; 0: twice, as its -fmad=false / pre-sm_90 builds), "gemv_tma" (1: decode GEMVs of 4-bit weights take the persistent
+ * TMA-fed stream-K kernel; 0, default: the cp.async kernel, which is faster), "gemv_tma_occ" (CTAs per SM, 1 or 2), "gemv_tma_smem_kb" (shared-memory budget),
  * "gqa_min_ctx" (single-sequence decode: context length beyond which the kv-group tensor-core attention replaces the fused per-head
  * kernel; default 1024), "tc_min_m" (token count from which kf_linear* use the tcgen05 GEMM: -1 = measured per-type crossover, 0 = never, n = from n),
  * "tc_bn" (token tile of the tcgen05 GEMM: 16, 32, 64, 128 or 256; 0 = by modelled time), "attn_wait_us" (how long a wait inside kf_attn_prefill /

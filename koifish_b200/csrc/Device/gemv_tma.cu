@@ -438,10 +438,6 @@ kf_gemv_tma_kernel(const __grid_constant__ TMaps tm, const TParams p) {
                     lds128(ring0 + stage * SBYTES + woff + (jp + jj) * UBYTES, ra[jj]);
                     lds128(ring0 + stage * SBYTES + woff + (jp + jj) * UBYTES + 512, rb8[jj]);
                 }
-                if (jp + 2 >= UPW) {  // last read of the stage: hand it back to the producer (one arrival per warp)
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(empty0 + 8 * stage);
-                }
 #pragma unroll
                 for (int jj = 0; jj < 2; jj++) {
                     const int u = uc + j0 + jj;
@@ -508,6 +504,10 @@ kf_gemv_tma_kernel(const __grid_constant__ TMaps tm, const TParams p) {
                     }
                 }
             }
+            // Hand the stage back to the producer only now: the matrix instructions above were issued with its bytes in their registers (in issue order, so before
+            // this).  An arrival right behind the shared-memory loads can overtake them, and the producer would refill what is still being read.  One per warp.
+            __syncwarp();
+            if (lane == 0) mbar_arrive(empty0 + 8 * stage);
             if (++stage == NS) stage = 0, phase ^= 1;
             // ---- end of a row block (always the end of a stage) or of this CTA's share: hand the sums over ----
             if (ks0 + CHUNK == p.ksteps || uc + CHUNK >= u1) {
