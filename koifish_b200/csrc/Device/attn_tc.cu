@@ -321,9 +321,9 @@ int kf_attn_prefill_tc_ok(const kf_ctx* ctx, const void* out, const void* q, con
 int kf_attn_prefill_tc(kf_ctx* ctx, void* out, const void* q, const void* kc, const void* vc, const int32_t* pos_dev, int M, int n_head, int n_kv, int max_seq) {
     CUtensorMap tq, tk, tv;
     int rc = kf_wait_status(ctx);
-    if (!rc) rc = kf_tmap_2d(ctx, &tq, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, q, (uint64_t)n_head * kHD, (uint64_t)M, 64, kQ, CU_TENSOR_MAP_SWIZZLE_128B);
-    if (!rc) rc = kf_tmap_2d(ctx, &tk, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, kc, (uint64_t)n_kv * kHD, (uint64_t)max_seq, 64, kKV, CU_TENSOR_MAP_SWIZZLE_128B);
-    if (!rc) rc = kf_tmap_2d(ctx, &tv, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, vc, (uint64_t)n_kv * kHD, (uint64_t)max_seq, 64, kKV, CU_TENSOR_MAP_SWIZZLE_128B);
+    if (!rc) rc = kf_tmap_2d(ctx, &tq, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, q, (uint64_t)n_head * kHD, (uint64_t)M, 64, kQ, CU_TENSOR_MAP_SWIZZLE_128B, false);
+    if (!rc) rc = kf_tmap_2d(ctx, &tk, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, kc, (uint64_t)n_kv * kHD, (uint64_t)max_seq, 64, kKV, CU_TENSOR_MAP_SWIZZLE_128B, false);
+    if (!rc) rc = kf_tmap_2d(ctx, &tv, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, vc, (uint64_t)n_kv * kHD, (uint64_t)max_seq, 64, kKV, CU_TENSOR_MAP_SWIZZLE_128B, false);
     if (rc) return rc;
     static bool set[kf_ctx::kMaxDevices] = {};  // function attributes are per device
     if (!set[ctx->device]) {

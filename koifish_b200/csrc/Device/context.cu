@@ -166,6 +166,8 @@ extern "C" int kf_ctx_get_int(kf_ctx* ctx, const char* key, int* value_out) {
         *value_out = ctx->tp_fused;
     else if (!strcmp(key, "gemv_xg_min_m"))
         *value_out = ctx->gemv_xg_min_m;
+    else if (!strcmp(key, "tmap_weights"))
+        *value_out = kf_tmap_count(ctx, true);
     else if (!strcmp(key, "attn_tc_error") || !strcmp(key, "attn_gqa_error")) {
         if (!ctx->capturing) KF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         *value_out = ((volatile int*)ctx->wait_flags)[key[5] == 'g'];

@@ -778,7 +778,12 @@ struct TmapKey {
                std::tie(o.base, o.inner, o.outer, o.box_inner, o.box_outer, o.dt, o.sw, o.esize, o.planes, o.plane_stride);
     }
 };
-using TmapCache = std::map<TmapKey, CUtensorMap>;
+// Maps of weights apart from those of what changes from call to call (activations and queries by their number of tokens, the cache by the number of sequences): a
+// 64-layer model in steps of varying size makes 128 of the latter for every size, which must not cost the weights theirs.  Each is dropped when it is full.
+struct TmapCache {
+    std::map<TmapKey, CUtensorMap> maps[2];  // [0] weights: models hold a few hundred; [1] the others
+};
+constexpr size_t kTmapMost[2] = {4096, 16384};
 EncodeTiledFn encode_fn() {
     static EncodeTiledFn fn = [] {
         void* f = nullptr;
@@ -790,14 +795,14 @@ EncodeTiledFn encode_fn() {
 }
 }  // namespace
 static int tmap_encode(kf_ctx* ctx, CUtensorMap* tm, CUtensorMapDataType dt, int esize, const void* base, uint64_t inner, uint64_t outer, uint32_t box_inner,
-                       uint32_t box_outer, CUtensorMapSwizzle sw, uint64_t planes, uint64_t plane_stride) {
+                       uint32_t box_outer, CUtensorMapSwizzle sw, uint64_t planes, uint64_t plane_stride, bool weight) {
     // a tensor map depends only on (address, geometry, box, swizzle): encode each once per context and reuse it (weights and the context's
     // activation scratch keep their addresses from token to token)
     TmapKey key = {base, inner, outer, box_inner, box_outer, (uint32_t)dt, (uint32_t)sw, (uint32_t)esize, planes, plane_stride};
-    TmapCache* cache = reinterpret_cast<TmapCache*>(ctx->tmap_cache);
-    if (!cache) ctx->tmap_cache = cache = new TmapCache();
-    auto hit = cache->find(key);
-    if (hit != cache->end()) {
+    if (!ctx->tmap_cache) ctx->tmap_cache = new TmapCache();
+    auto& cache = reinterpret_cast<TmapCache*>(ctx->tmap_cache)->maps[weight ? 0 : 1];
+    auto hit    = cache.find(key);
+    if (hit != cache.end()) {
         *tm = hit->second;
         return KF_OK;
     }
@@ -816,17 +821,21 @@ static int tmap_encode(kf_ctx* ctx, CUtensorMap* tm, CUtensorMapDataType dt, int
         ctx->last_error = b;
         return KF_ERR_CUDA;
     }
-    if (cache->size() > 4096) cache->clear();  // models hold a few hundred weights; bound it anyway
-    (*cache)[key] = *tm;
+    if (cache.size() >= kTmapMost[weight ? 0 : 1]) cache.clear();
+    cache[key] = *tm;
     return KF_OK;
 }
 int kf_tmap_2d(kf_ctx* ctx, CUtensorMap* tm, CUtensorMapDataType dt, int esize, const void* base, uint64_t inner, uint64_t outer, uint32_t box_inner,
-               uint32_t box_outer, CUtensorMapSwizzle sw) {
-    return tmap_encode(ctx, tm, dt, esize, base, inner, outer, box_inner, box_outer, sw, 1, 0);
+               uint32_t box_outer, CUtensorMapSwizzle sw, bool weight) {
+    return tmap_encode(ctx, tm, dt, esize, base, inner, outer, box_inner, box_outer, sw, 1, 0, weight);
+}
+int kf_tmap_count(const kf_ctx* ctx, bool weights) {
+    return ctx->tmap_cache ? (int)reinterpret_cast<const TmapCache*>(ctx->tmap_cache)->maps[weights ? 0 : 1].size() : 0;
 }
 int kf_tmap_rows(kf_ctx* ctx, CUtensorMap* tm, const void* base, uint64_t inner, uint64_t rows, uint64_t planes, uint64_t plane_stride, uint32_t box_inner,
                  uint32_t box_rows) {
-    return tmap_encode(ctx, tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, inner, rows, box_inner, box_rows, CU_TENSOR_MAP_SWIZZLE_128B, planes, plane_stride);
+    return tmap_encode(ctx, tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, inner, rows, box_inner, box_rows, CU_TENSOR_MAP_SWIZZLE_128B, planes, plane_stride,
+                       false);
 }
 namespace {
 
@@ -869,12 +878,12 @@ int launch_tc(kf_ctx* ctx, GemmParams& p, const void* const* wdata, int nw, cons
         const int j = i < nw ? i : 0;  // unused slots repeat the first weight (never dereferenced)
         if (A_TMEM)
             rc = kf_tmap_2d(ctx, &tm_w[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, wdata[j], (uint64_t)p.K * F::BITS / 8, (uint64_t)p.Nw[j], F::RAWB, glu ? BM / 2 : BM,
-                            F::RAWB == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B);
+                            F::RAWB == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, true);
         else
             rc = kf_tmap_2d(ctx, &tm_w[i], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, wdata[j], (uint64_t)p.K, (uint64_t)p.Nw[j], BK, glu ? BM / 2 : BM,
-                            CU_TENSOR_MAP_SWIZZLE_128B);
+                            CU_TENSOR_MAP_SWIZZLE_128B, true);
     }
-    if (!rc) rc = kf_tmap_2d(ctx, &tm_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, xp, (uint64_t)p.K, (uint64_t)p.M, BK, BN, CU_TENSOR_MAP_SWIZZLE_128B);
+    if (!rc) rc = kf_tmap_2d(ctx, &tm_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, xp, (uint64_t)p.K, (uint64_t)p.M, BK, BN, CU_TENSOR_MAP_SWIZZLE_128B, false);
     if (rc) return rc;
     const int grid = std::min(p.n_items, ctx->sm_count);
     KF_CUDA(ctx, kf_launch_pdl(ctx, kern, dim3(grid), dim3(kThreadsTC), smem, tm_w[0], tm_w[1], tm_w[2], tm_x, p));

@@ -5,9 +5,10 @@
 
 #include "kf_common.cuh"
 
-// 2-D tensor map over rows of `inner` elements (outer rows, dense), box [box_outer][box_inner]; encoded once per geometry and context (gemm_tc.cu)
+// 2-D tensor map over rows of `inner` elements (outer rows, dense), box [box_outer][box_inner]; encoded once per geometry and context (gemm_tc.cu), weights kept
+// apart from the rest
 int kf_tmap_2d(kf_ctx* ctx, CUtensorMap* tm, CUtensorMapDataType dt, int esize, const void* base, uint64_t inner, uint64_t outer, uint32_t box_inner,
-               uint32_t box_outer, CUtensorMapSwizzle sw);
+               uint32_t box_outer, CUtensorMapSwizzle sw, bool weight);
 // planes of bf16 rows (dense rows, planes plane_stride bytes apart), box [1][box_rows][box_inner], SWIZZLE_128B
 int kf_tmap_rows(kf_ctx* ctx, CUtensorMap* tm, const void* base, uint64_t inner, uint64_t rows, uint64_t planes, uint64_t plane_stride, uint32_t box_inner,
                  uint32_t box_rows);

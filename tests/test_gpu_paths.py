@@ -436,6 +436,28 @@ def test_gqa_scores_of_minus_infinity(ctx, lens, split, gone):
         assert bool(((out[i].double() - want).abs() <= 2.0 ** -8 * 1.01 * (mass + want.abs()) + 1e-6).all()), i
 
 
+def test_maps_of_steps_leave_those_of_weights(ctx):
+    """Steps of ever new buffers (the cache of a sequence moves on by 16 bytes each time) make new tensor maps; those of a weight stay."""
+    import torch
+    hd, n = 128, 3000
+    w = make_q(ctx, kf.KF_T_Q4, 256, 512)[0]
+    x = kf.fill_normal(ctx, 16 * 512, 7, 1.0)
+    kf.linear(ctx, w, x, 16)
+    held = ctx.get_int("tmap_weights")
+    assert held > 0
+    q, out = torch.ones(1, 1, hd, device="cuda").bfloat16(), torch.zeros(1, 1, hd, device="cuda").bfloat16()
+    kv = torch.ones(8 * n + 4 * hd, device="cuda").bfloat16()
+    pos = torch.zeros(1, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    for i in range(n):
+        p = _ptr(kv) + 16 * i
+        ctx.check(ctx.lib.kf_attn_decode_gqa(ctx.h, _ptr(out), _ptr(q), p, p + 16, _ptr(pos), 1, 1, 1, hd, 2, 1, 0), "gqa")
+    kf.linear(ctx, w, x, 16)
+    ctx.sync()
+    assert ctx.get_int("tmap_weights") == held
+    assert bool((out == 1).all())
+
+
 # ---------------------------------------------------------------------------------------------- tile matmul over expert-sorted slots
 @pytest.mark.parametrize("N,K", [(64, 64), (65, 72), (8, 8), (130, 200), (192, 448), (33, 512)])
 @pytest.mark.parametrize("counts", [(64, 0, 1, 63, 65, 17), (200, 3, 0, 0, 1, 0), (16, 16, 16, 16, 16, 16)])
