@@ -29,18 +29,19 @@ def make_q(ctx, typ, rows, cols, seed=5):
 
 
 # ---------------------------------------------------------------------------------------------- long reductions in the tcgen05 matmul
-@pytest.mark.parametrize("rows,cols,M", [(5120, 8192, 2048), (10240, 25600, 45), (2560, 25600, 128)])
-def test_tc_long_reduction(ctx, rows, cols, M):
+@pytest.mark.parametrize("plan", [0, 1])
+@pytest.mark.parametrize("rows,cols,M", [(5120, 8192, 2048), (10240, 25600, 45), (2560, 25600, 128), (51200, 5120, 45), (1024, 25600, 300)])
+def test_tc_long_reduction(ctx, rows, cols, M, plan):
     """Items of 32 and more raw stages: a stage that is handed back before its bytes were read shows as whole rows that used another stage's weights.
     The weights are exact on both sides, so what is left is the order of fp32 sums: 2^-24 * sqrt(cols) of the result, far below 1e-4; a stage that went
-    wrong moves a row by 0.1 of it."""
+    wrong moves a row by 0.1 of it.  plan 0: token tile and split by modelled time; 1: those of gemv_exact."""
     import torch
     torch.backends.cuda.matmul.allow_tf32 = False
     w, wd = make_q(ctx, kf.KF_T_Q4, rows, cols)
     x = kf.fill_normal(ctx, M * cols, 7, 1.0)
     want = bf16_tensor(x, M, cols).float() @ wd.T
     exact = ctx.get_int("gemv_exact")
-    ctx.set_int("gemv_exact", 1)
+    ctx.set_int("gemv_exact", plan)
     try:
         for _ in range(4):
             y = torch.from_numpy(kf.linear(ctx, w, x, M, kf.KF_EPI_F32).numpy(np.float32, (M, rows))).cuda()
@@ -98,7 +99,7 @@ def _rows(kind, M, vocab, rng):
 def test_sample_selection(ctx, kind, vocab, top_k):
     """Tokens equal those of the CPU port (which shares no code): a high temperature makes every candidate as likely, so the token names a place in the sorted
     list of candidates.  1 draw in 100 may differ (a coin within rounding of a boundary: the two exponentials differ in the last place)."""
-    M, rounds = 3, 12
+    M, rounds = 3, 34
     rng = np.random.default_rng(vocab + top_k)
     lg = _rows(kind, M, vocab, rng).reshape(M, vocab)
     lgd = ctx.array(lg)
@@ -277,9 +278,11 @@ _GQA_LENS = [((1,), 0), ((63, 64, 65, 1, 128, 129), 128), ((256, 257, 511, 513, 
              ((5000, 17), 300), ((40000,), 65535), (tuple(1 + 37 * i % 190 for i in range(40)), 189), (tuple(1 + 37 * i % 190 for i in range(300)), 100)]
 # four and eight heads per kv head, each run several rings long
 _GQA_RINGS = [(128, 32, 8, (40000,), 39999), (128, 64, 8, (40000,), 39999), (128, 8, 2, (9000, 30000), 29999), (64, 32, 8, (40000,), 39999)]
+# more sequences than the dealing tables hold, cut into runs
+_GQA_MANY = [(128, 2, 1, tuple(1 + 37 * i % 190 for i in range(600)), 189), (64, 1, 1, tuple(1 + 37 * i % 190 for i in range(513)), 50)]
 
 
-@pytest.mark.parametrize("hd,n_head,n_kv,lens,hint", [a + b for a in _GQA_SHAPES for b in _GQA_LENS] + _GQA_RINGS)
+@pytest.mark.parametrize("hd,n_head,n_kv,lens,hint", [a + b for a in _GQA_SHAPES for b in _GQA_LENS] + _GQA_RINGS + _GQA_MANY)
 def test_gqa_runs(ctx, hd, n_head, n_kv, lens, hint):
     """Edges of tiles and runs, lengths of their own, hints that are too small or too large, cache rows behind the last position that hold no numbers, again on
     used workspaces.  Bound as for the panel kernel: one rounding of the weights, one of the result."""
