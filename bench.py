@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""bench.py -- decode throughput of the quantized-inference hot path (BASELINE.json metric: decode tokens/s, Qwen3 4-bit).
+"""bench.py -- decode throughput of the quantized-inference hot path (decode tokens/s, Qwen3 4-bit).
 
     python bench.py --gpus N --steps K --warmup W [--impl reference] [--workload qwen3-32b-q4] [--ctx 512]
     python bench.py --compare-arch sipazen|kivorax|sedotar|fazolorn|gadilix|zadinex [--arch-sizes s,m] [--prompt 2048] [--panel 512]     (another architecture beside Qwen3; own output)
@@ -110,7 +110,7 @@ def kernel_digest():
 
 
 def gemv_algorithmic_bytes(rows, cols, bits, group, M):
-    """SURVEY.md 8d / BASELINE.md 3: N*K*bits/8 + (N*K/G)*4 [packed types] + 2*M*K + 2*M*N"""
+    """N*K*bits/8 + (N*K/G)*4 [packed types] + 2*M*K + 2*M*N"""
     b = rows * cols * bits / 8.0 + 2.0 * M * cols + 2.0 * M * rows
     if bits in (4, 2, 1):
         b += (rows * cols / group) * 4.0

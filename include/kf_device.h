@@ -2,7 +2,7 @@
  * kf_device.h -- the C ABI of koifish_b200's device layer (the drop-in boundary for Koifish's quantized-inference
  * hot path on B200 / sm_100a).
  *
- * The reference has no FFI layer: the path sits behind C++ neuron/tensor calls (SURVEY.md section 8b).  Each entry
+ * The reference has no FFI layer: the path sits behind C++ neuron/tensor calls.  Each entry
  * point below names the reference interface it replaces (file:line relative to the reference tree).  Conventions:
  *   - plain pointers and sizes only; every pointer called "dev" is a CUDA device pointer, "host" a host pointer;
  *   - all bf16 tensors are raw uint16 bit patterns (floatX == floatGama == __nv_bfloat16, src/g_float.hpp:246-261);
@@ -225,7 +225,7 @@ int kf_argmax(kf_ctx* ctx, int32_t* out_tokens_dev, const void* logits_bf16_dev,
 int kf_sample(kf_ctx* ctx, int32_t* out_tokens_dev, const void* logits_bf16_dev, int M, int vocab, float temperature, int top_k, float top_p,
               uint64_t* rng_state_dev, int selection);
 
-/* ---- tensor parallel: no reference equivalent (multi_gpu.cuh is dead code, SURVEY.md 2.1 row 21).  One process per GPU;
+/* ---- tensor parallel: no reference equivalent (multi_gpu.cuh is dead code).  One process per GPU;
  *      the unique id is exchanged by the caller (torch.distributed / MPI) ---- */
 int kf_nccl_unique_id(void* id_out_128_bytes);
 int kf_ctx_init_nccl(kf_ctx* ctx, const void* id_128_bytes, int rank, int world);

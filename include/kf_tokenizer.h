@@ -1,5 +1,5 @@
 /*
- * kf_tokenizer.h -- C ABI of the text side of the chat loop (SURVEY.md 8f N3): what a Koifish maintainer binds instead of
+ * kf_tokenizer.h -- C ABI of the text side of the chat loop: what a Koifish maintainer binds instead of
  * AutoTokenizer::from_pretrained / HF_Tokenizer::encode / decode / T2STR / eos_token_id (reference src/TokenSet/HF_Tokenizer.cpp:1723-1830)
  * and CHAT_SAMPLER::InitPrefillTemplate / toChatML (reference src/Utils/CLI_params.cpp:1990-2031).  Host only: no device, no CUDA.
  * Strings are UTF-8; every returned string is malloc'ed and freed with kf_string_free (kf_model.h).  Status codes are kf_device.h's.

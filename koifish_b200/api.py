@@ -139,7 +139,7 @@ class DevArray:
 
 
 class QTensor:
-    """A weight in the reference's storage form: packed data || gama (SURVEY.md A.1)."""
+    """A weight in the reference's storage form: packed data || gama."""
 
     def __init__(self, ctx, rows, cols, type_, group=128, qbias=0):
         self.ctx, self.rows, self.cols, self.type, self.group, self.qbias = ctx, rows, cols, type_, group, qbias
@@ -594,7 +594,7 @@ def qwen3_config(n_layer, n_embd, n_ff, n_head, n_kv_head, head_dim=128, vocab=1
     return cfg
 
 
-QWEN3_DIMS = {  # SURVEY.md section 8 table (HF Qwen3 configs)
+QWEN3_DIMS = {  # the HF Qwen3 configs
     "0.6B": dict(n_layer=28, n_embd=1024, n_ff=3072, n_head=16, n_kv_head=8, tie=True),
     "8B": dict(n_layer=36, n_embd=4096, n_ff=12288, n_head=32, n_kv_head=8, tie=False),
     "32B": dict(n_layer=64, n_embd=5120, n_ff=25600, n_head=64, n_kv_head=8, tie=False),

@@ -6,7 +6,7 @@
 //     w[ic][oc] = bf16( float(q - z) * float(scale) )
 // kf_tensor_desc for it: type KF_T_AWQ4, rows = OC, cols = IC, data_dev = qweight, zero_dev = qzeros, step_dev = scales, group = 128.
 // AWQ tensors come from vendor checkpoints (the reference has no AWQ quantiser, and neither has this library): this is the device-level
-// entry (dequant + matmul); the model runtime's loader for such checkpoints is a 'next' row.
+// entry (dequant + matmul); the model runtime's loader for such checkpoints is in csrc/Transformer/QWen3.cpp.
 //
 // Matmul: up to 8 tokens a coalesced column-walking GEMV (a thread owns one int32 word = 8 output columns and strides over the input rows;
 // k-slices reduced in a fixed order by a second small launch), more tokens dequantise into [OC][IC] bf16 + the tcgen05 GEMM.  Functional

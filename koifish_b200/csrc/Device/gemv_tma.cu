@@ -5,7 +5,7 @@
 // CU_Q128toX_ T.cu:245-294) + CU_mm_blasLt (cuBLASLt GEMM, src/Device/CUDA/kernel/gemm.cu:93-214) as called from SLP::Forw
 // (src/Device/CUDA/NeuronFuse.cu:305-381), with the neighbouring CU_rms_infer / CU_swiglu_v0 / CU_add3 launches folded in.
 //
-// The op is HBM-bound on paper (0.53 B / weight, every packed byte read once).  What actually limited round 1's kernel (gemv.cu) was the
+// The op is HBM-bound on paper (0.53 B / weight, every packed byte read once).  What actually limited the first form of the cp.async kernel (gemv.cu) was the
 // ALU pipe: tools/ubench/deq_rate*.cu measure, from registers only, 432 clk per [128 rows x 128 k] tile and SM for the bit-exact bf16
 // unpack (SHF + LOP3 + HSUB2 + HFMA2 per pair of weights; a funnel shift alone costs ~5 clk per warp instruction and scheduler on this
 // part) -- MORE than the 392 clk the tile's bytes take at the measured HBM rate.  Hence two arithmetic modes (template MODE):

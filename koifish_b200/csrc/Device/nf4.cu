@@ -10,7 +10,7 @@
 //
 // Matmul: up to 8 tokens take a warp-per-row GEMV with a per-row 256-entry (byte -> two weights) table in shared memory; more tokens dequantise
 // into a context scratch and take the bf16 tcgen05 GEMM, as the reference does for every format (GTensor::GetDataX + cuBLASLt).  This is the
-// functional path of the format, not a tuned one: see DESIGN.md.
+// functional path of the format, not a tuned one.
 #include "kf_common.cuh"
 
 namespace {

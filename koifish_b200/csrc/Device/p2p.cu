@@ -1,7 +1,7 @@
 // p2p.cu -- the tensor-parallel exchange step of decode over NVLink / NVSwitch PEER MEMORY, fused with the residual add.
 //
 // After the row-parallel matmuls (O and down) every rank holds an fp32 partial of the M x hidden activations; the reference has no
-// counterpart (its multi_gpu.cuh is dead code, SURVEY.md 2.1 row 21).  The library path (ncclAllReduce + a residual-add kernel) costs
+// counterpart (its multi_gpu.cuh is dead code).  The library path (ncclAllReduce + a residual-add kernel) costs
 // two launches and ~15 us of latency per exchange -- 128 exchanges per Qwen3-32B token.  Here ONE kernel per exchange does
 //     push : every rank stores its partial into slot [rank] of EVERY peer's symmetric buffer (remote stores over NVLink),
 //     flag : publishes an epoch flag on every peer (release at system scope),

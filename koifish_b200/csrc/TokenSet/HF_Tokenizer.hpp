@@ -1,4 +1,4 @@
-// HF_Tokenizer.hpp -- the text side of the chat loop (SURVEY 8f N3): a reader of HF "tokenizer.json" files of the Qwen family and the ChatML
+// HF_Tokenizer.hpp -- the text side of the chat loop: a reader of HF "tokenizer.json" files of the Qwen family and the ChatML
 // prompt templates.  Mirrors the surface the reference's chat path uses:
 //   HF_Tokenizer::encode / decode / T2STR / token_to_id / id_to_token / eos_token_id   (reference src/TokenSet/HF_Tokenizer.cpp:1723-1771)
 //   AutoTokenizer::from_pretrained(dir) -> dir/tokenizer.json                           (:1813-1830)

@@ -415,7 +415,7 @@ static void shard_window(const Fish& f, const std::string& name, int rows_l, int
 
 // Host-only shard plan (no device): full shape of a tensor by its HF name and the window rank `rank` of `world` holds.
 // Megatron-style: Q/K/V/gate/up split by output rows (heads / ffn), O/down by input columns in whole 128-wide quant groups, the
-// rest replicated (SURVEY.md 8e).  Returns false for an unknown name or an indivisible configuration.
+// rest replicated.  Returns false for an unknown name or an indivisible configuration.
 bool ShardPlan(const MODEL_CARD& c, const std::string& name, int rank, int world, int* rows_g, int* cols_g, int* rows_l, int* cols_l, int* row0,
                int* col0) {
     if (world < 1 || rank < 0 || rank >= world) return false;
@@ -535,7 +535,7 @@ int Fish::SetTensorIds(const std::string& name, const int32_t* ids, int rows, in
     return rc;
 }
 // The window [out r0, r0 + OCl) x [in c0, c0 + ICl) of a full AWQ triple as ONE blob qweight || qzeros || scales (GTensor::AllocAWQ).  r0 and OCl
-// are multiples of 8 (whole int32 words), c0 and ICl of 128 (whole groups).  Pure host code (the tensor-parallel shard plan of SURVEY 8e applied
+// are multiples of 8 (whole int32 words), c0 and ICl of 128 (whole groups).  Pure host code (the tensor-parallel shard plan applied
 // to the vendor layout); out_blob holds ICl * OCl / 2 + (ICl / 128) * (OCl / 8) * 4 + (ICl / 128) * OCl * 2 bytes.
 void AwqShardWindow(const void* qweight, const void* qzeros, const void* scales, int IC, int OC, int r0, int OCl, int c0, int ICl, uint8_t* out_blob) {
     (void)IC;

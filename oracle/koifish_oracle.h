@@ -6,7 +6,7 @@
  * --impl reference legs -- always as the checker, never as the product.  Nothing under koifish_b200/
  * links it.
  *
- * Parity pinning: the reference ships NO golden vectors / known-answer tests for this path (SURVEY.md section 8c), so the oracle
+ * Parity pinning: the reference ships NO golden vectors / known-answer tests for this path, so the oracle
  * is pinned against the reference's own code compiled where it lies under /root/reference (recipe: oracle/Makefile):
  *   - 128-bit word layout: the PACK_/UNPACK_ macros of src/PackedQ.hpp (oracle/ref_shim.cpp -> oracle/_ref/libkoifish_ref.so,
  *     tests/test_oracle_vs_ref.py, fixtures tests/golden/packq_ref.npz);
@@ -115,7 +115,7 @@ void kfo_add(uint16_t* out, const uint16_t* a, const uint16_t* b, size_t n);
 void kfo_attention_decode(uint16_t* out, const uint16_t* q, const uint16_t* kcache, const uint16_t* vcache, int pos, int n_head, int n_kv,
                           int head_dim, int score_bf16);
 
-/* ---- whole model (op order: SURVEY.md appendix A.6; src/Device/CUDA/QKV.cu:617-706, NeuronFuse.cu:615-656, 842-862,
+/* ---- whole model (op order: src/Device/CUDA/QKV.cu:617-706, NeuronFuse.cu:615-656, 842-862,
  *      Generate.cu:180-346) ---- */
 typedef struct {
     int n_layer, n_embd, n_ff, n_head, n_kv_head, head_dim, vocab, max_seq;

@@ -1,6 +1,6 @@
 """Generate tests/golden/packq_ref.npz from the REFERENCE's own PackedQ.hpp macros (oracle/_ref, built from
 /root/reference by oracle/Makefile).  Run in the build container only:  python tests/golden/make_golden.py
-The fixture pins the 128-bit word layout (SURVEY.md A.2) for the oracle and for the CUDA unpackers on the GPU box,
+The fixture pins the 128-bit word layout for the oracle and for the CUDA unpackers on the GPU box,
 where /root/reference does not exist."""
 import os
 import sys
@@ -24,7 +24,7 @@ for bits in (4, 2, 1):
         oh[j * per + j] = (1 << bits) - 1
     out[f"onehot_codes{bits}"] = oh
     out[f"onehot_bytes{bits}"] = ol.ref_pack(oh, bits)
-# the probe quoted in SURVEY.md 8c: codes (3+7i) mod 16
+# a probe: codes (3+7i) mod 16
 kat = np.array([(3 + 7 * i) % 16 for i in range(32)], dtype=np.int32)
 out["kat4_codes"] = kat
 out["kat4_bytes"] = ol.ref_pack(kat, 4)

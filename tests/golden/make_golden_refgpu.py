@@ -2,7 +2,7 @@
 """Golden vectors from the reference's OWN CUDA kernels (oracle/_ref/libkoifish_refgpu*.so, libkoifish_refq.so: built from
 /root/reference/src/Device/CUDA/T.cu and kernel/quantizer.cu by oracle/Makefile), run on a B200:
 
-    gpurun -- 'python tests/golden/make_golden_refgpu.py gpurun_out/refgpu_golden.npz'      (then copy the file into tests/golden/)
+    python tests/golden/make_golden_refgpu.py [refgpu_golden.npz]      (on a machine with a B200; then copy the file into tests/golden/)
 
 Inputs are regenerated from seeds by tests/test_oracle_golden_refgpu.py (the oracle's own generator / numpy default_rng), so the file
 holds only the reference kernels' OUTPUTS.  The CPU test then checks the oracle against them without a GPU and without /root/reference."""
@@ -67,4 +67,4 @@ def main(path):
 
 
 if __name__ == "__main__":
-    main(sys.argv[1] if len(sys.argv) > 1 else "gpurun_out/refgpu_golden.npz")
+    main(sys.argv[1] if len(sys.argv) > 1 else "refgpu_golden.npz")

@@ -1,4 +1,4 @@
-"""Golden vectors for csrc/TokenSet (SURVEY 8f N3), produced with the HF `tokenizers` library -- the crate the reference's
+"""Golden vectors for csrc/TokenSet, produced with the HF `tokenizers` library -- the crate the reference's
 src/TokenSet/HF_Tokenizer.cpp ports.  No Qwen3 tokenizer.json exists offline, so this script TRAINS a small byte-level BPE with exactly the
 pipeline a Qwen3 tokenizer.json declares (NFC; Split(<pattern>, Isolated) + ByteLevel(use_regex = false); BPE; ByteLevel decoder; the ChatML
 added tokens) and writes

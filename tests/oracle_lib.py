@@ -513,7 +513,7 @@ def tensor_seed(model_seed, tid):
 
 
 class OracleModel:
-    """Whole-model CPU decode following the reference op order (SURVEY.md appendix A.6)."""
+    """Whole-model CPU decode following the reference op order."""
 
     def __init__(self, **kw):
         d = dict(n_layer=2, n_embd=256, n_ff=512, n_head=4, n_kv_head=2, head_dim=64, vocab=1024, max_seq=64,

@@ -470,7 +470,7 @@ def test_linear_rejects_bad_shapes(ctx):
 
 
 def test_gemv_full_size_properties_qwen3_32b_down_proj(ctx):
-    # BASELINE full size: K = 25600, N = 5120, 4-bit.  Size-independent properties: one-hot columns reproduce the dequantised
+    # full size: K = 25600, N = 5120, 4-bit.  Size-independent properties: one-hot columns reproduce the dequantised
     # weights bit-exactly; x = ones gives the row sums; linearity y(a+b) ~ y(a)+y(b).
     N, K = 5120, 25600
     w = kf.fill_normal(ctx, N * K, 4242, 0.02)
@@ -540,7 +540,7 @@ def test_qknorm_rope_kvappend(ctx, hd, n_head, n_kv, theta, M):
 @pytest.mark.parametrize("hd,n_head,n_kv", [(128, 16, 8), (128, 64, 8), (64, 4, 2)])
 @pytest.mark.parametrize("pos", [0, 1, 31, 200, 1500])
 def test_attention_decode(ctx, hd, n_head, n_kv, pos):
-    # includes pos >= 1024, which the reference's attention_qk_kernel silently truncates (SURVEY.md 5.7)
+    # includes pos >= 1024, which the reference's attention_qk_kernel silently truncates
     rng = np.random.default_rng(pos + hd)
     max_seq = 2048
     q = rand_bf16(rng, (1, n_head * hd))
@@ -907,7 +907,7 @@ def test_nf4_linear_matches_oracle(ctx, M):
     assert np.abs(got - want).max() <= 2e-2 * np.abs(want).max()
 
 
-# ---------------------------------------------------------------------------------------------- round-2 regressions
+# ---------------------------------------------------------------------------------------------- regressions
 @pytest.mark.parametrize("M", [1, 5, 40])
 def test_mixed_storage_types_share_a_call(ctx, M):
     # the quantizer card selects the type per tensor-name substring (Init4Neuron), so Q / K / V or gate / up of one block may differ:

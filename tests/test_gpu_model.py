@@ -1,5 +1,5 @@
 """GPU parity tests of the whole decode path through the reference-facing C ABI (kf_model_*), against the CPU oracle's model on
-the same synthetic weights (same generator definition, same quantiser).  Gates (SURVEY.md 8d): dequantised weights bit-exact;
+the same synthetic weights (same generator definition, same quantiser).  Gates: dequantised weights bit-exact;
 logits max error <= 1e-2 of the logit scale; top-1 agreement on teacher-forced tokens."""
 import numpy as np
 import pytest
@@ -9,7 +9,7 @@ import oracle_lib as ol
 
 pytestmark = pytest.mark.gpu
 
-# north_star: "logits within a stated relative tolerance (e.g. 1e-2 bf16 / top-1 token agreement)".  Every test below runs twice:
+# The target: "logits within a stated relative tolerance (e.g. 1e-2 bf16 / top-1 token agreement)".  Every test below runs twice:
 #   exact -- gemv_exact = 1: each weight dequantised in-kernel to the reference's bf16 value (bit-exact, test_gpu_refkernels.py);
 #            logits within 1e-2 of the largest logit, i.e. about one bf16 ulp of it (an ulp is 3.9e-3 .. 7.8e-3 of the value);
 #   fast  -- the default decode arithmetic for 4-bit weights (MODE_FAST in gemv.cu: group sums in fp32, the affine map applied per
@@ -203,7 +203,7 @@ def test_set_tensor_quantises_external_weights(ctx):
 
 
 def test_qwen3_0p6b_dims_two_layers_full_vocab(ctx):
-    # BASELINE config 1 shapes (E 1024, FFN 3072, H16/KV8, hd 128, vocab 151936, tied bf16 head, 4-bit blocks), 2 of the 28 layers
+    # Qwen3-0.6B shapes (E 1024, FFN 3072, H16/KV8, hd 128, vocab 151936, tied bf16 head, 4-bit blocks), 2 of the 28 layers
     model, oracle = build_pair(ctx, n_layer=2, n_embd=1024, n_ff=3072, n_head=16, n_kv_head=8, head_dim=128, vocab=151936, max_seq=64,
                                norm_sigma=0.0)
     toks = prompt(6, 151936)
@@ -301,7 +301,7 @@ def test_long_context_decode_switches_to_kv_group_attention(ctx):
 
 
 def test_qwen3_32b_dims_one_layer(ctx):
-    # BASELINE headline shapes (E 5120, FFN 25600, H64/KV8, hd 128, 4-bit blocks, untied bf16 head), ONE of the 64 layers and a
+    # Qwen3-32B shapes (E 5120, FFN 25600, H64/KV8, hd 128, 4-bit blocks, untied bf16 head), ONE of the 64 layers and a
     # 16 K-row vocabulary so that the CPU oracle stays in seconds: the full-size GEMV shapes, the 64-head cluster attention and the
     # bf16 tensor-core head against the oracle, then a 24-token panel through the tcgen05 dequant-GEMM and the flash attention
     model, oracle = build_pair(ctx, n_layer=1, n_embd=5120, n_ff=25600, n_head=64, n_kv_head=8, head_dim=128, vocab=16384, max_seq=64,
@@ -322,7 +322,7 @@ def test_qwen3_32b_dims_one_layer(ctx):
 
 @pytest.mark.parametrize("bits,name", [(2, "ternary"), (1, "binary")])
 def test_qwen3_8b_dims_one_layer_low_bit(ctx, bits, name):
-    # BASELINE configs[3] shapes (Qwen3-8B: E 4096, FFN 12288, H32/KV8, hd 128), every block linear 2-bit ternary / 1-bit (yyang, g=128),
+    # Qwen3-8B shapes (E 4096, FFN 12288, H32/KV8, hd 128), every block linear 2-bit ternary / 1-bit (yyang, g=128),
     # ONE of the 36 layers and a 16 K-row vocabulary: the full-size low-bit GEMV shapes token by token, then a 24-token panel through the
     # tcgen05 dequant-GEMM, against the oracle
     model, oracle = build_pair(ctx, n_layer=1, n_embd=4096, n_ff=12288, n_head=32, n_kv_head=8, head_dim=128, vocab=16384, max_seq=64,
@@ -343,7 +343,7 @@ def test_qwen3_8b_dims_one_layer_low_bit(ctx, bits, name):
 
 
 def test_context_512_prefill_then_decode_matches_oracle(ctx):
-    # "ctx 512".  A 500-token prompt through the prefill panels (tcgen05 linears + flash prefill attention), then 24
+    # Context 512: a 500-token prompt through the prefill panels (tcgen05 linears + flash prefill attention), then 24
     # teacher-forced decode steps across position 512 (split-context decode attention over 500..523 cached rows), every step against the
     # oracle fed the same 524 tokens one by one.  Qwen3-0.6B head geometry (16 heads / 8 KV heads of 128), two layers.
     model, oracle = build_pair(ctx, n_layer=2, n_embd=1024, n_ff=3072, n_head=16, n_kv_head=8, head_dim=128, vocab=4096, max_seq=640)
@@ -368,7 +368,7 @@ def test_context_512_prefill_then_decode_matches_oracle(ctx):
 # oracle's sequential loop) flips individual activations by one bf16 ulp (0.4 .. 0.8 % of the value).  Those flips random-walk through the
 # depth: measured rms logit error 7e-3 of the rms logit after 2 layers, 1.4e-2 after 28 (tools/greedy_gate.py ->
 # profiles/r02_greedy_gate.txt), in the bit-faithful arithmetic as well as in the fast one.  The per-layer gate stays 1e-2 (the tests above);
-# the 28-layer gate is the measured worst case (1.8e-2 exact, 2.2e-2 fast) plus a third, and -- the other half of north_star's gate -- top-1
+# the 28-layer gate is the measured worst case (1.8e-2 exact, 2.2e-2 fast) plus a third, and -- the other half of the target -- top-1
 # agreement at every position where the oracle's best two logits are further apart than DECISIVE_GAP.
 DEEP_RTOL_BY_ARITH = {"exact": 2.5e-2, "fast": 3e-2}
 DECISIVE_GAP = 1.5e-2
@@ -376,7 +376,7 @@ DECISIVE_GAP = 1.5e-2
 
 @pytest.mark.parametrize("theta", [1e6, 1e4])
 def test_qwen3_0p6b_greedy_128_tokens_top1(ctx, theta):
-    # BASELINE configs[0] / SURVEY.md 8(d) config 1 in full: Qwen3-0.6B (28 layers, E 1024, FFN 3072, H16/KV8, hd 128, vocab 151936, tied
+    # Qwen3-0.6B in full (28 layers, E 1024, FFN 3072, H16/KV8, hd 128, vocab 151936, tied
     # bf16 head), 4-bit RTN blocks, seed 42; prompt (1000 + 37 i) mod 151936 for 16 tokens, then 128 greedy tokens chosen by the ORACLE and
     # teacher-forced into the GPU path.  Gates at every one of the 144 positions: see above.
     steps = 128 if theta == 1e6 else 32
@@ -540,7 +540,7 @@ def test_load_safetensors_equals_set_tensor(ctx, tmp_path):
         a.load_safetensors(tmp_path / "awq.safetensors")
 
 
-# ---------------------------------------------------------------------------------------------- vendor AWQ checkpoints (SURVEY N2)
+# ---------------------------------------------------------------------------------------------- vendor AWQ checkpoints
 AWQ_VENDOR_BLOCK = {"bits": 4, "group_size": 128, "modules_to_not_convert": None, "quant_method": "awq", "version": "gemm", "zero_point": True}
 
 

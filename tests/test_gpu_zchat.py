@@ -1,4 +1,4 @@
-"""GPU tests of the chat loop (SURVEY 8f N3): kf_model_generate -- the generation loop of Fish::Chat, reference src/Manifold/GoPT.cpp:1111-1235 --
+"""GPU tests of the chat loop: kf_model_generate -- the generation loop of Fish::Chat, reference src/Manifold/GoPT.cpp:1111-1235 --
 against the same steps made one kf_model_forward call at a time, its three stop conditions, and one text-in / text-out turn through the tokenizer."""
 import os
 

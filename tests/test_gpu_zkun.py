@@ -1,4 +1,4 @@
-"""GPU tests of the fish.kun container at the model level (SURVEY 8f N1): kf_model_save_kun / kf_model_load_kun -- what the reference's
+"""GPU tests of the fish.kun container at the model level: kf_model_save_kun / kf_model_load_kun -- what the reference's
 Fish::SAFETENSOR_Serialize writes and SAFETENSOR2Gensors + GTensor::LoadParam + Serial_Quant_MMAP read (reference src/Manifold/Serialize.cpp:
 145-230, 770-1010; src/Device/CUDA/huTensor.cu:413-458, 487-588).  The container code itself is covered on the CPU (tests/test_kun_host.py)."""
 import json

@@ -1,4 +1,4 @@
-"""CPU tests of the fish.kun container code (csrc/Tensor/KunFile.cpp; SURVEY 8f N1) through the host-only C ABI entries: files laid out the
+"""CPU tests of the fish.kun container code (csrc/Tensor/KunFile.cpp) through the host-only C ABI entries: files laid out the
 way the reference's writer lays them out (K_SafeTensors::Save / GTensor::jDesc / insertJS, reference src/Manifold/Serialize.cpp:61-100, 880-1010,
 src/Tensor/Safetensors.hpp:87-102) are read back, files this library writes are checked byte for byte with plain Python, and the msgpack config
 entry goes both ways against the `msgpack` package."""

@@ -1,5 +1,5 @@
 """CPU tests: the oracle against the reference's own macros (oracle/_ref), the committed golden fixtures, the
-in-code invariants the reference asserts (SURVEY.md section 4), and exact bf16 arithmetic."""
+in-code invariants the reference asserts, and exact bf16 arithmetic."""
 import os
 
 import numpy as np
@@ -21,7 +21,7 @@ def test_pack_matches_golden_from_reference_macros(bits):
 
 
 def test_survey_probe_bytes():
-    # SURVEY.md 8c probe of PACK_4to128_: codes (3+7i)%16 -> low half "5c 7e 90 b2 d4 f6 18 3a", same for the high half
+    # probe of PACK_4to128_: codes (3+7i)%16 -> low half "5c 7e 90 b2 d4 f6 18 3a", same for the high half
     b = ol.pack_codes(GOLD["kat4_codes"], 4)
     want = bytes.fromhex("5c7e90b2d4f6183a") * 2
     assert bytes(b) == want
@@ -30,7 +30,7 @@ def test_survey_probe_bytes():
 
 @pytest.mark.parametrize("bits", [4, 2, 1])
 def test_layout_table_A2(bits):
-    # SURVEY.md appendix A.2: code j of a word -> byte / bit field
+    # code j of a word -> byte / bit field
     per = 128 // bits
     for j in range(per):
         codes = np.zeros(per, dtype=np.int32)

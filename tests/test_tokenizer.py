@@ -1,4 +1,4 @@
-"""CPU tests of csrc/TokenSet through the C ABI (include/kf_tokenizer.h; SURVEY 8f N3) against
+"""CPU tests of csrc/TokenSet through the C ABI (include/kf_tokenizer.h) against
   * golden vectors computed by the HF `tokenizers` library (tests/golden/make_tokenizer_golden.py -> tests/golden/tokenizer/),
   * CPython's unicodedata for Unicode NFC,
   * the `tokenizers` library itself, live, on random strings -- when it is importable (it is in this image).

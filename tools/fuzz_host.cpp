@@ -3,7 +3,7 @@
 // refused or parsed, never crash.  From the repo root:
 //   g++ -std=c++17 -O1 -g -fsanitize=address,undefined -fno-sanitize-recover=undefined -Ikoifish_b200/csrc -Iinclude tools/fuzz_host.cpp \
 //       koifish_b200/csrc/TokenSet/HF_Tokenizer.cpp koifish_b200/csrc/Tensor/KunFile.cpp -o /tmp/fuzz_host && /tmp/fuzz_host
-// Last run (round 2): "ok tokens=360691", no sanitizer report.
+// Last run: "ok tokens=360691", no sanitizer report.
 #include <cstdio>
 #include <cstdlib>
 #include <random>

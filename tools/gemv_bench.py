@@ -1,10 +1,10 @@
 #!/usr/bin/env python
-"""Microbench sweep of the fused dequant GEMV / skinny GEMM (BASELINE.json config 5):
+"""Microbench sweep of the fused dequant GEMV / skinny GEMM:
     y[M,N] = x[M,K] . deq(W[N,K])^T,  K,N in {4096, 5120, 25600}, bits {16, 8, 4, 2, 1}, M in {1, 16, ...}
 Reports achieved algorithmic GB/s against the measured HBM peak and 8 TB/s.  Weights rotate through buffers larger than the
 126 MB L2 so every launch streams from HBM.  One JSON line per case (also appended to --out).
 
-    python tools/gemv_bench.py [--quick] [--splitk 0,1,2,4] [--out gpurun_out/gemv_sweep.jsonl]
+    python tools/gemv_bench.py [--quick] [--splitk 0,1,2,4] [--out gemv_sweep.jsonl]
 """
 import argparse
 import ctypes as C

@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Batched-decode and prefill throughput of the Qwen3 workloads of SURVEY.md 8(d) (configs 2-4) on one GPU.
+"""Batched-decode and prefill throughput of the Qwen3 workloads (0.6B, 8B, 32B) on one GPU.
 
     python tools/throughput_bench.py --workload qwen3-32b-q4 --batch 1,8,16,32,64 --ctx 512 --prefill 4096 --panel 2048
 

@@ -105,7 +105,7 @@ void run(const char* name) {
     cudaFree(out), cudaFree(cyc);
 }
 int main() {
-    run<0>("factor, LOP3 r,r,r (round 1 form)");
+    run<0>("factor, LOP3 r,r,r (first form)");
     run<1>("factor, LOP3 r,imm,r");
     run<2>("factor, fp16 trick: 2 SHF + 8 LOP3 per 8 pairs");
     run<4>("exact sub+fma, LOP3 r,r,r");
