@@ -10,10 +10,10 @@
 //   warp 9           TMA: both Q tiles once, then the K and V tiles through two stages each
 // Tensor memory: S0 S1 O0 O1, 128 columns each.  What bounds it: a tile pair needs 2 x 1024 clocks of matrix instructions and 2 x 16384 exponentials, 2048 clocks
 // of the special-function units.  Measured: 1999 queries of 32 heads behind 4096 positions 575 us with the mma.sync kernel (64 queries of one head per CTA,
-// fragments through ldmatrix: 290 TFLOP/s), 187 us here (890 TFLOP/s).  A chain on its own
+// fragments through ldmatrix: 290 TFLOP/s), 199 us here (840 TFLOP/s; tensor pipe half busy).  A chain on its own
 // (few heads and queries) advances a tile in 1.7 us.
 // The output is rescaled whenever a maximum of the warp's rows grows, so the largest weight of a row is 1 and has no rounding error: waiting until it has grown by
-// 2^8 takes 167 us instead of 187 here, but its error against 64 bits is 3 % (flat) to 20 % (sharp scores) above the mma.sync kernel's.  The denominator adds the unrounded weights.
+// 2^8 is 20 us faster here, but its error against 64 bits is 3 % (flat) to 20 % (sharp scores) above the mma.sync kernel's.  The denominator adds the unrounded weights.
 // Rows of V behind the last position are zeroed in shared memory: their weight is zero, but whatever the cache holds there need not be a number.
 // Every wait is bounded: when one runs out, `dead` ends all roles, copies and matrix instructions in flight are awaited and tensor memory is freed.
 #include "kf_common.cuh"

@@ -232,7 +232,7 @@ __device__ __forceinline__ int slot_offset(int q) {
 
 // Ring depths.  The three rings are decoupled because their latencies differ: the raw ring hides DRAM latency (bytes in flight per SM
 // = RS x 8 KB must cover ~2 us x 44 GB/s), the B ring hides the L2 round trip of the (small, L2-resident) activation tiles, the A ring
-// only the on-chip producer -> MMA hand-off.  Sized so that shared memory stays below ~210 KB and tensor memory within 512 columns.
+// only the on-chip producer -> MMA hand-off.  Sized so that shared memory, the epilogue's two output buffers included, stays below 226 KB and tensor memory within 512 columns.
 constexpr int kStageOut = 8 * 1024;  // one of the epilogue's two output buffers: 32 tokens x 128 rows in bf16, or 16 tokens in fp32
 template <int FMT, int BN>
 struct Rings {
@@ -891,7 +891,7 @@ int launch_tc(kf_ctx* ctx, GemmParams& p, const void* const* wdata, int nw, cons
     return KF_OK;
 }
 // Token tile and k-split by their modelled time: waves x (k-blocks x time per k-block + epilogue) + the fix-up of split sums.  The times per k-block of 64 are
-// measured ones (us; below 64 tokens the weights' bytes or their expansion, above the matrix instructions).  Splitting pays for few row tiles and a
+// measured ones (us; 4-bit and bf16 weights, the former stand for all that are expanded; below 64 tokens the weights' bytes or their expansion, above the matrix instructions).  Splitting pays for few row tiles and a
 // handful of tokens only: 1024 x 3072 at 16 tokens 9.9 us in 8 parts against 15.7 whole, at 256 tokens 34 against 17.  (The rule before it charged BN / 16
 // k-blocks for the fix-up: 1024 x 3072 at 256 tokens went into 12 parts and took 91 us, now 17.5.)  The reference-exact arithmetic keeps that rule and the
 // order of sums it was compared in.

@@ -459,8 +459,8 @@ __global__ void __launch_bounds__(256) kf_lin_tile_any_kernel(LinArgs a) {
 
 // bf16 activations: 64 slots x 64 outputs (of either weight, DUAL) per CTA, k in steps of 64 through a ring of stages filled by cp.async, 8 warps as 4 (m) x 2 (n) on
 // mma.sync m16n8k16.  The weights of a routed panel are the traffic (64 experts of 2 x 1408 x 2048: 738 MB), so the ring is there to keep bytes on their way: two
-// CTAs per SM with three of four stages in flight, 128 KB an SM.  Fetching the next step through registers had 24 KB on its way: 291 us for those, 0.39 of the HBM
-// rate, 176 here (0.64); the down projections 194 and 114.  A warp whose 16 slots lie past the group's end only helps to load.
+// CTAs per SM, each with three of four 24 KB stages in flight (DUAL; 144 KB an SM, 96 of them weights) or five of six 16 KB stages (160 KB, 80 of them weights).
+// Fetching the next step through registers had 24 KB on its way: 291 us for those, 0.39 of the HBM rate, 177 here (0.64); the down projections 194 and 113 (0.50).  A warp whose 16 slots lie past the group's end only helps to load.
 // Rows lie as 128 bytes, 16-byte chunk c of row r at c ^ (r & 7): ldmatrix without conflicts.  A weight that is not 16-byte aligned (the table is on the device: only
 // the kernel sees it) is fetched element by element into the same places.
 template <bool DUAL>

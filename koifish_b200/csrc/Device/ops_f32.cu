@@ -1281,7 +1281,7 @@ extern "C" int kf_f32_to_bf16(kf_ctx* ctx, void* out_bf16, const float* in, size
 
 // Router of a mixture of experts over fp32 logits [M][ldl] (+ bf16 bias [E] or NULL): idx / wgt [M][top]; then the dispatch tables:
 // offsets [E + 1], entry_slot [M * top] (where each (token, choice) sits among the expert-sorted slots), slot_row / slot_group [M * top].
-// work: device int32 scratch of 2 * M * top + E entries.
+// work: not used any more (the tables of a panel are one launch), but part of the interface: it must not be NULL.
 // full_softmax 0: weights = softmax over the chosen logits; 1: the chosen entries of the softmax over all E experts (not renormalised).
 static int moe_route_impl(kf_ctx* ctx, int32_t* idx, float* wgt, int32_t* offsets, int32_t* entry_slot, int32_t* slot_row, int32_t* slot_group,
                           int32_t* work, const float* logits, int ldl, const void* bias_bf16, int M, int E, int top, int full_softmax, const RouteMode md) {

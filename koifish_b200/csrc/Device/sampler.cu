@@ -1,4 +1,4 @@
-// sampler.cu -- temperature / top-k / top-p sampling ON THE DEVICE, one CTA per sequence: the step right after the logits
+// sampler.cu -- temperature / top-k / top-p sampling ON THE DEVICE, one cluster of CTAs (or one CTA) per sequence: the step right after the logits
 // (GeneratOnPrompt::Sample, reference src/Manifold/GoPT.cpp:614-630, with LogitsInfo::TopK :632-640, UpdateLogits :751-766, TopP :729-748,
 // Qu_FlipCoin :768-786 and the xorshift64* generator :594-600).  The reference copies the [vocab] logits to the host every token and samples
 // there; here only the 4-byte token leaves the GPU (or nothing at all inside the device-resident decode loop).
@@ -10,8 +10,9 @@
 //   2. p_i = expf((l_i - l_max) / T), normalised by their sum in sorted order (sequential fp32, like the host loop);
 //   3. top-p: keep the shortest prefix whose cumulative probability exceeds top_p;
 //   4. coin = random_f32(state) * sum(kept p); first i with coin < cdf_i (else the last kept).
-// The sums of steps 2-4 run on one thread in the reference's order of operations, so that the CPU port (oracle kfo_sample) and the kernel agree
-// except where expf's last ulp moves a cdf boundary across the coin.
+// The two running sums of steps 2-4 (of the exponentials, of the probabilities) are formed by one thread in the reference's order; exponentials, quotients and the
+// search for the cut and the coin by one thread per candidate.  So the CPU port (oracle kfo_sample) and the kernel agree except where expf's last ulp moves
+// a cdf boundary across the coin.
 #include <math.h>
 
 #include "kf_common.cuh"
@@ -241,7 +242,7 @@ __global__ void __launch_bounds__(kSampThreads) kf_sample_cluster_kernel(int32_t
     __shared__ int s_above, s_ties, s_nan;
     const int tid = threadIdx.x, rank = blockIdx.x % ctas;
     const uint16_t* row = logits + (size_t)(blockIdx.x / ctas) * vocab;
-    // ---- the one pass: keys in registers, two per word; 0 marks what lies past the end ----
+    // ---- the one pass: keys in registers, one each; 0 marks what lies past the end ----
     uint32_t kk[kFastPer];
 #pragma unroll
     for (int j = 0; j < kFastPer; j++) kk[j] = 0;
