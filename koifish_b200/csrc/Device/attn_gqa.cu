@@ -42,7 +42,8 @@ __device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], 
 // Stages of the ring: what shared memory holds beside the warps' areas (SETS 1: two CTAs per SM), at most ten per set.  With two sets, whose tiles alternate, their
 // number is a multiple of 4 (K and V of a tile of either), so that a stage always comes back to the set that used it last: a wait tells a phase of a barrier from
 // the one before by a single bit, so the warps that wait for a use of a stage have to have waited for the use before.  With ten stages tile 5 lay where tile 0
-// had, for the other set, which would have taken it for landed while the copies of tile 0 were still under way (copies may overtake each other).
+// had, for the other set, which would have taken it for landed while the copies of tile 0 were still under way (copies may overtake each other).  Between two
+// items of a CTA all its warps meet, behind every wait of the first.
 constexpr int gqa_area(int hd, int sets, int group) { return 4 * sets * ((group + 1) & ~1) * hd * 4; }
 constexpr int gqa_stages(int hd, int sets, int group) {
     const int fit = ((sets == 1 ? 97 : 200) * 1024 - gqa_area(hd, sets, group)) / (kTok * hd * 2), most = fit < 10 * sets ? fit : 10 * sets;
@@ -420,6 +421,10 @@ int gqa_any(kf_ctx* ctx, void* out, const void* q, const void* kc, const void* v
     const int pairs = n_kv * M, sms = ctx->sm_count;
     const bool few  = pairs < sms;
     int chunk = 2 * kTok, runs = few ? sms / pairs : 1;
+    // between a half and two thirds as many pairs as SMs: thirds make two passes over nearly all SMs, where whole ones leave a third or more of the SMs idle (12 ragged
+    // sequences of 8 kv heads and 64 heads, norm and append in front: 58 against 65 us up to 6000 positions, 107 against 145 up to 16000; 49 against
+    // 47 up to 4200 and 34 against 27 up to 2000, where the merges cost more).  From there on whole ones again (16 sequences: 56 against 71 us, 146 against 156)
+    if (few && 2 * pairs > sms && 3 * pairs <= 2 * sms && len >= 5120) runs = 3;
     if (ctx->attn_split > 0) chunk = kTok, runs = ctx->attn_split;
     runs = std::max(1, std::min(runs, std::min(kMaxRuns, (len + chunk - 1) / chunk)));
     if (runs == 1) chunk = std::max(chunk, (max_seq + kTok - 1) / kTok * kTok);

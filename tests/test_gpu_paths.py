@@ -278,11 +278,12 @@ _GQA_LENS = [((1,), 0), ((63, 64, 65, 1, 128, 129), 128), ((256, 257, 511, 513, 
              ((5000, 17), 300), ((40000,), 65535), (tuple(1 + 37 * i % 190 for i in range(40)), 189), (tuple(1 + 37 * i % 190 for i in range(300)), 100)]
 # four and eight heads per kv head, each run several rings long
 _GQA_RINGS = [(128, 32, 8, (40000,), 39999), (128, 64, 8, (40000,), 39999), (128, 8, 2, (9000, 30000), 29999), (64, 32, 8, (40000,), 39999)]
-# more sequences than the dealing tables hold, cut into runs
+# whole sequences in thirds, two items per thread block; more sequences than the dealing tables hold, cut into runs
+_GQA_THIRDS = [(128, 16, 8, tuple(6000 - 397 * i for i in range(12)), 5999), (128, 80, 10, tuple(300 + 1237 * i % 5200 for i in range(9)), 5499)]
 _GQA_MANY = [(128, 2, 1, tuple(1 + 37 * i % 190 for i in range(600)), 189), (64, 1, 1, tuple(1 + 37 * i % 190 for i in range(513)), 50)]
 
 
-@pytest.mark.parametrize("hd,n_head,n_kv,lens,hint", [a + b for a in _GQA_SHAPES for b in _GQA_LENS] + _GQA_RINGS + _GQA_MANY)
+@pytest.mark.parametrize("hd,n_head,n_kv,lens,hint", [a + b for a in _GQA_SHAPES for b in _GQA_LENS] + _GQA_RINGS + _GQA_THIRDS + _GQA_MANY)
 def test_gqa_runs(ctx, hd, n_head, n_kv, lens, hint):
     """Edges of tiles and runs, lengths of their own, hints that are too small or too large, cache rows behind the last position that hold no numbers, again on
     used workspaces.  Bound as for the panel kernel: one rounding of the weights, one of the result."""
