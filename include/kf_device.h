@@ -101,7 +101,8 @@ uint64_t kf_scratch_generation(kf_ctx* ctx);
  * TMA-fed stream-K kernel; 0, default: the cp.async kernel, which is faster), "gemv_tma_occ" (CTAs per SM, 1 or 2), "gemv_tma_smem_kb" (shared-memory budget),
  * "gqa_min_ctx" (single-sequence decode: context length beyond which the kv-group tensor-core attention replaces the fused per-head
  * kernel; default 1024), "tc_min_m" (token count from which kf_linear* use the tcgen05 GEMM: -1 = measured per-type crossover, 0 = never, n = from n),
- * "tc_bn" (token tile of the tcgen05 GEMM: 16, 32, 64, 128 or 256; 0 = by modelled time), "attn_wait_us" (how long a wait inside kf_attn_prefill /
+ * "tc_bn" (token tile of the tcgen05 GEMM: 16, 32, 64, 128 or 256; 0 = by modelled time), "attn_tc_min_m" (panel size from which
+ * kf_attn_prefill takes the tcgen05 kernel, at least 65 tokens; 0 = where it is the faster one), "attn_wait_us" (how long a wait inside kf_attn_prefill /
  * kf_attn_decode_gqa may take, default 4 s; when one runs out the kernel ends and kf_ctx_sync -- or the next of these calls -- returns KF_ERR_CUDA, once, and the
  * context is usable again), "attn_drop" (n > 0: the n-th thread block of these kernels loads nothing, so that its waits run out; for tests) */
 int kf_ctx_set_int(kf_ctx* ctx, const char* key, int value);
@@ -197,7 +198,7 @@ int kf_qkv_attention(kf_ctx* ctx, void* out_dev, const void* q_dev, const void* 
  *      cache rows [0, pos_dev[0] + M).  q_dev must already be normalised + rotated and the panel's K / V rows appended
  *      (kf_qknorm_rope_kvappend).  Replaces the reference's token-by-token prompt loop (src/Manifold/GoPT.cpp:1111-1235) through
  *      attention_qk / softmax / attention_v (src/Device/CUDA/kernel/operator.cuh:573-668); flash-attention: panels of more than 64 tokens with
- *      head_dim 128, an even n_head / n_kv and 16-byte aligned buffers on tcgen05, others on mma.sync. ---- */
+ *      head_dim 128, an even n_head / n_kv and 16-byte aligned buffers on tcgen05, others -- and small ones with little room in front of them -- on mma.sync. ---- */
 int kf_attn_prefill(kf_ctx* ctx, void* out_dev, const void* q_dev, const void* kcache_layer_dev, const void* vcache_layer_dev,
                     const int32_t* pos_dev, int M, int n_head, int n_kv, int head_dim, int max_seq);
 /* ---- decode attention for many sequences per step: same contract as kf_attn_decode, but the query heads that share a kv head are

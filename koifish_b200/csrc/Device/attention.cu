@@ -951,7 +951,7 @@ extern "C" int kf_attn_prefill(kf_ctx* ctx, void* out, const void* q, const void
                                int n_kv, int hd, int max_seq) {
     if (!ctx || !out || !q || !kc || !vc || !pos_dev) return KF_ERR_BAD_ARG;
     KF_REQUIRE(ctx, (hd == 128 || hd == 64) && n_head % n_kv == 0 && M >= 1 && max_seq >= 1, "head_dim 64/128, GQA");
-    if (kf_attn_prefill_tc_ok(ctx, out, q, kc, vc, M, n_head, n_kv, hd)) return kf_attn_prefill_tc(ctx, out, q, kc, vc, pos_dev, M, n_head, n_kv, max_seq);
+    if (kf_attn_prefill_tc_ok(ctx, out, q, kc, vc, M, n_head, n_kv, hd, max_seq)) return kf_attn_prefill_tc(ctx, out, q, kc, vc, pos_dev, M, n_head, n_kv, max_seq);
     const size_t smem = (size_t)(kPfQ + 4 * KF_PF_BKV) * hd * 2;
     dim3 grid((M + kPfQ - 1) / kPfQ, n_head);
     const float sq = sqrtf((float)hd);

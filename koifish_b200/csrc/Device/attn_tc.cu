@@ -313,10 +313,14 @@ __global__ void __launch_bounds__(kThreads, 1)
 }
 }  // namespace
 
-// Panels the kernel takes: head size 128, an even number of query heads per kv head, 16-byte aligned rows, and more than 64 queries (one tile of the mma.sync
-// kernel).  With the append in front, 16 heads: 65 queries 13.9 us here / 14.0 there, behind 500 positions 19.0 / 18.9, behind 4000 63 / 82; 700 queries 23 / 31.
-int kf_attn_prefill_tc_ok(const kf_ctx* ctx, const void* out, const void* q, const void* kc, const void* vc, int M, int n_head, int n_kv, int hd) {
-    return hd == kHD && M > 64 && (n_head / n_kv) % 2 == 0 && n_head / 2 <= 65535 && (((uintptr_t)out | (uintptr_t)q | (uintptr_t)kc | (uintptr_t)vc) & 15) == 0;
+// Panels the kernel takes: head size 128, an even number of query heads per kv head, 16-byte aligned rows, and more than 64 queries -- but not those of up to 512
+// queries for whose blocks (64 queries of a head) the mma.sync kernel has an SM each and that cannot lie deep in their context, the cache having room for no more than
+// 512 positions in front of them (where they do lie is known on the device only).  There that kernel's finer tiles win.  With norm and append in front, here / there in us:
+// 16 heads, 96 queries 11.0 / 10.4, behind 300 positions 18.6 / 16.5, behind 700 24.8 / 22.7; 300 queries 16.5 / 16.5, behind 700 28.8 / 28.7; 513 behind 4000 78 / 92; 700 queries
+// 24.7 / 30.8.  32 heads, 256 queries 16.5 / 14.5, 300 queries 17.4 / 18.6.  64 heads, 128 queries 13.0 / 12.4, 129 queries 14.5 / 16.5.  2 heads, 512 queries 18.6 / 17.5.
+int kf_attn_prefill_tc_ok(const kf_ctx* ctx, const void* out, const void* q, const void* kc, const void* vc, int M, int n_head, int n_kv, int hd, int max_seq) {
+    const bool gains = ctx->attn_tc_min_m > 0 ? M >= ctx->attn_tc_min_m : M > 512 || max_seq - M > 512 || (long long)((M + 63) / 64) * n_head > ctx->sm_count;
+    return hd == kHD && M > 64 && gains && (n_head / n_kv) % 2 == 0 && n_head / 2 <= 65535 && (((uintptr_t)out | (uintptr_t)q | (uintptr_t)kc | (uintptr_t)vc) & 15) == 0;
 }
 int kf_attn_prefill_tc(kf_ctx* ctx, void* out, const void* q, const void* kc, const void* vc, const int32_t* pos_dev, int M, int n_head, int n_kv, int max_seq) {
     CUtensorMap tq, tk, tv;

@@ -202,6 +202,8 @@ extern "C" int kf_ctx_set_int(kf_ctx* ctx, const char* key, int value) {
         ctx->attn_split = value;
     else if (!strcmp(key, "gqa_min_ctx"))
         ctx->gqa_min_ctx = value;
+    else if (!strcmp(key, "attn_tc_min_m"))
+        ctx->attn_tc_min_m = value;
     else if (!strcmp(key, "attn_wait_us"))
         ctx->attn_wait_us = value > 0 ? value : 4000000;
     else if (!strcmp(key, "attn_drop"))

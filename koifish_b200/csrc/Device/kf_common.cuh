@@ -61,6 +61,7 @@ struct kf_ctx {
     int gqa_min_ctx  = 1024;  // single-sequence decode: contexts beyond this use the kv-group tensor-core attention (Transformer layer reads it)
     // bounded waits of the attention kernels that run on copies and barriers: a kernel that gives up sets its flag ([0] prefill, [1] grouped decode; host memory)
     int* wait_flags  = nullptr;
+    int attn_tc_min_m = 0;       // panels from which the tcgen05 prefill attention is taken (from 65 queries); 0 = where it gains (attn_tc.cu)
     int attn_wait_us = 4000000;  // how long a wait may take
     int attn_drop    = 0;        // n > 0: the n-th CTA of these kernels issues no copies, so that a wait of it runs out (tests)
     int attn_warps   = 0;  // warps per CTA of the cluster attention (0 = default)
@@ -171,7 +172,7 @@ int kf_tc_same_order(const kf_tensor_desc* a, const kf_tensor_desc* b);  // 0: o
 int kf_gemm_tc(kf_ctx* ctx, void* y, const kf_tensor_desc* w, const void* xp, int M, int epilogue, const void* residual);
 // up to 3 weights of the same type / K / group in ONE launch (Q/K/V, gate/up)
 // attn_tc.cu: panels of more than 64 queries on tcgen05
-int kf_attn_prefill_tc_ok(const kf_ctx* ctx, const void* out, const void* q, const void* kc, const void* vc, int M, int n_head, int n_kv, int hd);
+int kf_attn_prefill_tc_ok(const kf_ctx* ctx, const void* out, const void* q, const void* kc, const void* vc, int M, int n_head, int n_kv, int hd, int max_seq);
 int kf_attn_prefill_tc(kf_ctx* ctx, void* out, const void* q, const void* kc, const void* vc, const int32_t* pos_dev, int M, int n_head, int n_kv, int max_seq);
 int kf_gemm_tc_multi(kf_ctx* ctx, int n, void* const* y, const kf_tensor_desc* w, const void* xp, int M, int epilogue, const void* residual);
 

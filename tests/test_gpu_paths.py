@@ -233,7 +233,11 @@ def test_prefill_tc(ctx, n_head, n_kv, M, pos0, behind, sharp):
     pos = torch.arange(pos0, pos0 + M, dtype=torch.int32, device="cuda")
     out = torch.full((M, n_head, hd), 7.0, device="cuda").bfloat16()
     torch.cuda.synchronize()
-    ctx.check(ctx.lib.kf_attn_prefill(ctx.h, _ptr(out), _ptr(q), _ptr(k), _ptr(v), _ptr(pos), M, n_head, n_kv, hd, max_seq), "prefill")
+    ctx.set_int("attn_tc_min_m", 65)
+    try:
+        ctx.check(ctx.lib.kf_attn_prefill(ctx.h, _ptr(out), _ptr(q), _ptr(k), _ptr(v), _ptr(pos), M, n_head, n_kv, hd, max_seq), "prefill")
+    finally:
+        ctx.set_int("attn_tc_min_m", 0)
     ctx.sync()
     assert ctx.get_int("attn_tc_error") == 0
     keys = torch.arange(pos0 + M, device="cuda")
@@ -244,6 +248,33 @@ def test_prefill_tc(ctx, n_head, n_kv, M, pos0, behind, sharp):
         want, mass = p @ vv, p @ vv.abs()
         err = (out[:, h].double() - want).abs()
         assert bool((err <= 2.0 ** -8 * 1.01 * (mass + want.abs()) + 1e-6).all()), (h, float((err / (mass + want.abs())).max()))
+
+
+@pytest.mark.parametrize("n_head,M,room,tc", [(16, 96, 0, False), (16, 96, 512, False), (16, 96, 513, True), (16, 512, 0, False), (16, 600, 0, True), (32, 256, 0, False),
+                                              (32, 257, 0, True), (64, 128, 0, False), (64, 129, 0, True), (2, 512, 300, False), (2, 513, 300, True)])
+def test_prefill_takes_the_kernel_that_gains(ctx, n_head, M, room, tc):
+    """Panels that the mma.sync kernel has SMs for (148: one 64-query tile of a head each), of up to 512 tokens and with room for up to 512 in front, go there: the
+    bits name the kernel."""
+    import torch
+    hd, n_kv = 128, max(1, n_head // 4)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(M)
+    q = torch.randn(M, n_head, hd, generator=g, device="cuda").bfloat16()
+    k, v = (torch.randn(M + room, n_kv, hd, generator=g, device="cuda").bfloat16() for _ in range(2))
+    pos, got = torch.arange(M, dtype=torch.int32, device="cuda"), []
+    torch.cuda.synchronize()
+    for least in (0, 65, 1 << 30):
+        out = torch.zeros(M, n_head, hd, device="cuda").bfloat16()
+        torch.cuda.synchronize()
+        ctx.set_int("attn_tc_min_m", least)
+        try:
+            ctx.check(ctx.lib.kf_attn_prefill(ctx.h, _ptr(out), _ptr(q), _ptr(k), _ptr(v), _ptr(pos), M, n_head, n_kv, hd, M + room), "prefill")
+        finally:
+            ctx.set_int("attn_tc_min_m", 0)
+        ctx.sync()
+        got.append(out)
+    assert not torch.equal(got[1], got[2])
+    assert torch.equal(got[0], got[1 if tc else 2])
 
 
 @pytest.mark.parametrize("M,pos0,gone", [(100, 256, (0, 128)), (100, 256, (0, 250)), (300, 130, (0, 130)), (200, 300, (128, 256))])
@@ -260,7 +291,11 @@ def test_prefill_scores_of_minus_infinity(ctx, M, pos0, gone):
     pos = torch.arange(pos0, n, dtype=torch.int32, device="cuda")
     out = torch.zeros(M, n_head, hd, device="cuda").bfloat16()
     torch.cuda.synchronize()
-    ctx.check(ctx.lib.kf_attn_prefill(ctx.h, _ptr(out), _ptr(q), _ptr(k), _ptr(v), _ptr(pos), M, n_head, n_kv, hd, n), "prefill")
+    ctx.set_int("attn_tc_min_m", 65)
+    try:
+        ctx.check(ctx.lib.kf_attn_prefill(ctx.h, _ptr(out), _ptr(q), _ptr(k), _ptr(v), _ptr(pos), M, n_head, n_kv, hd, n), "prefill")
+    finally:
+        ctx.set_int("attn_tc_min_m", 0)
     ctx.sync()
     keys = torch.arange(n, device="cuda")
     unseen = (keys[None] > pos[:, None]) | ((keys >= gone[0]) & (keys < gone[1]))[None]
@@ -341,7 +376,7 @@ def test_gqa_output_at_any_element(ctx, hd, n_head, n_kv, lens):
     assert torch.equal(got[0], got[1])
 
 
-@pytest.mark.parametrize("kind,lens", [("decode", (5000, 900)), ("decode", tuple(range(1, 41))), ("prefill", (300,))])
+@pytest.mark.parametrize("kind,lens", [("decode", (5000, 900)), ("decode", tuple(range(1, 41))), ("prefill", (700,))])
 def test_attention_wait_that_runs_out(ctx, kind, lens):
     """One thread block loads nothing, its waits end after 2 ms: the call that synchronises (or the next attention call) says so, once, and the call after that has
     the bits of the one before: no arrival of the other blocks is left counted."""
