@@ -13,9 +13,10 @@
 //     two-rounding arithmetic as gemv.cu) -> tcgen05.st into the A ring that lives in TENSOR MEMORY (lane = row, 2 weights / column);
 //     the expanded weights never touch shared memory, which stays free for the B operand;
 //   * warp 8  (1 thread): tcgen05.mma [D], [A in TMEM], B-descriptor; tcgen05.commit frees the stage / publishes the accumulator;
-//   * warps 11-14 (epilogue): tcgen05.ld the accumulator (double-buffered, so the next item's main loop overlaps), then either the
-//     final store (bf16 / +residual / fp32) or, with split-K, an fp32 partial + arrival counter; the last CTA to arrive reduces the
-//     partials in fixed order (deterministic) and stores.
+//   * warps 11-14 (epilogue): tcgen05.ld the accumulator into shared memory (it then goes back to the MMA warp), then the final store (bf16 / +residual /
+//     SwiGLU / fp32) under the next item's main loop; the producers help with a CTA's last item.  With split-K the parts of a tile are the CTAs of a
+//     cluster, which add up through distributed shared memory, or, where these do not fit on the GPU at once, fp32 partials in global memory + an
+//     arrival counter; either way in the order of the parts (deterministic).
 // bf16 weights need no expansion: warp 9 TMA-loads them straight into a swizzled A tile in shared memory (classic SS MMA).
 // The k order inside every 32-wide slot is the extraction-friendly permutation of gemv.cu; kf_tc_prepare_x permutes the activations
 // identically, so the contraction is unchanged.  Every barrier wait is bounded and traps instead of hanging the GPU.
@@ -70,6 +71,7 @@ struct GemmParams {
     int qbias, gshift, epilogue;
     int n_tiles, m_tiles, splits, n_items;
     int staged;                // outputs (and residual) may be accessed 16 bytes at a time
+    int cluster;               // the parts of a split are the CTAs of a cluster, one item each
     uint32_t lop_mask, lop_magic;
 };
 
@@ -158,7 +160,18 @@ __global__ void __launch_bounds__(256) kf_rmsnorm_permute_kernel(uint16_t* __res
     }
 }
 
-__device__ __forceinline__ void epi_bar_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+// the warps that finish an item: the four of the epilogue, or these and the eight producers
+__device__ __forceinline__ void epi_bar_sync(int nthr) {
+    if (nthr == 128) asm volatile("bar.sync 1, 128;" ::: "memory");
+    else asm volatile("bar.sync 2, 384;" ::: "memory");
+}
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t local, int cta_rank) {
+    uint32_t remote;
+    float4 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(cta_rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(remote) : "memory");
+    return v;
+}
 
 __device__ __forceinline__ uint32_t and_or3(uint32_t a, uint32_t b, uint32_t c) {
     uint32_t d;
@@ -233,7 +246,6 @@ __device__ __forceinline__ int slot_offset(int q) {
 // Ring depths.  The three rings are decoupled because their latencies differ: the raw ring hides DRAM latency (bytes in flight per SM
 // = RS x 8 KB must cover ~2 us x 44 GB/s), the B ring hides the L2 round trip of the (small, L2-resident) activation tiles, the A ring
 // only the on-chip producer -> MMA hand-off.  Sized so that shared memory, the epilogue's two output buffers included, stays below 226 KB and tensor memory within 512 columns.
-constexpr int kStageOut = 8 * 1024;  // one of the epilogue's two output buffers: 32 tokens x 128 rows in bf16, or 16 tokens in fp32
 template <int FMT, int BN>
 struct Rings {
     static constexpr bool A_TMEM = FMT != TF_BF16;
@@ -243,11 +255,14 @@ struct Rings {
     static constexpr int SUB     = A_BYTES + BN * 128;  // one k-block of a stage: [A tile (bf16 weights only)][B tile]
     static constexpr int STAGE   = U * SUB;
     static constexpr int SA      = !A_TMEM ? 0 : (BN <= 64 ? 12 : 8) / U;
-    static constexpr int SB      = (A_TMEM ? (BN == 16 ? 32 : BN == 32 ? 16 : BN == 64 ? 10 : BN == 128 ? 6 : 4)
+    static constexpr int SB      = (A_TMEM ? (BN == 16 ? 32 : BN == 32 ? 16 : BN == 64 ? 10 : BN == 128 ? 6 : 3)
                                            : (BN == 16 ? 10 : BN == 32 ? 10 : BN == 64 ? 8 : BN == 128 ? 6 : 4)) / U;
     static constexpr int RAWB    = raw_bytes<FMT>();
-    static constexpr int RS      = !A_TMEM ? 0 : (BN <= 64 ? 128 : BN == 128 ? 112 : 80) * 1024 / (BM * RAWB);
-    static constexpr size_t SMEM = (size_t)SB * STAGE + (size_t)RS * BM * RAWB + 2 * kStageOut + 1024;
+    static constexpr int RS      = !A_TMEM ? 0 : (BN <= 64 ? 128 : BN == 128 ? 96 : 64) * 1024 / (BM * RAWB);
+    // output buffer: the item's whole accumulator in bf16 where there is only one in tensor memory, which then goes back to the MMA warp after ~1.5 us of draining
+    static constexpr int OUT     = BN == 16 ? 8 * 1024 : A_TMEM && BN > 64 ? BN * 256 : 16 * 1024;  // at least one read of tensor memory in fp32
+    static constexpr size_t SMEM = (size_t)SB * STAGE + (size_t)RS * BM * RAWB + OUT + 1024;
+    static_assert((size_t)SB * STAGE + (size_t)RS * BM * RAWB >= (size_t)BN * BM * 4, "the rings take the partial sums of a split over a cluster");
     static_assert(SMEM <= 226 * 1024, "shared memory budget");
 };
 
@@ -259,10 +274,11 @@ struct Item {
 template <int KBR>
 __device__ __forceinline__ Item decode_item(const GemmParams& p, int item) {
     Item it;
-    const int mt = item % p.m_tiles;
-    const int t  = item / p.m_tiles;
-    it.z         = t % p.splits;
-    const int tn = t / p.splits;
+    const int u  = p.cluster ? item / p.splits : item;
+    const int mt = u % p.m_tiles;
+    const int t  = u / p.m_tiles;
+    it.z         = p.cluster ? item % p.splits : t % p.splits;
+    const int tn = p.cluster ? t : t / p.splits;
     it.wi = p.epilogue == kEpiGlu ? 0 : (tn >= p.tile0[1] ? 1 : 0) + (tn >= p.tile0[2] ? 1 : 0);
     it.n0 = p.epilogue == kEpiGlu ? tn * (BM / 2) : (tn - p.tile0[it.wi]) * BM, it.m0 = mt, it.tile = tn * p.m_tiles + mt;  // m0 = token-tile index (the caller scales it by BN)
     const int nkb  = p.K / BK;
@@ -335,7 +351,30 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-    if (tid == 0) {
+    // weight stage `it` of the CTA (k-block kb of item w): packed bytes or, for bf16 weights, the A tiles themselves
+    auto load_w = [&](const Item& w, int kb, uint32_t it) {
+        const CUtensorMap* tm_w = w.wi == 0 ? &tm_w0 : w.wi == 1 ? &tm_w1 : &tm_w2;
+        if constexpr (A_TMEM) {
+            const int rs = it % RS1, r = kb / KBR;
+#if KF_TC_EXP & 8
+            mbar_arrive(&raw_full[rs]);
+#else
+            mbar_arrive_expect_tx(&raw_full[rs], RAW_BYTES);
+            tma_load_2d(raws + (size_t)rs * RAW_BYTES, tm_w, r * RAWB, w.n0, &raw_full[rs]);
+            if (glu) tma_load_2d(raws + (size_t)rs * RAW_BYTES + RAW_BYTES / 2, &tm_w1, r * RAWB, w.n0, &raw_full[rs]);
+#endif
+        } else {
+            const int s = it % SB;
+            mbar_arrive_expect_tx(&b_full[s], U * A_BYTES);
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                tma_load_2d(tiles + (size_t)s * STAGE + u * SUB, tm_w, (kb + u) * BK, w.n0, &b_full[s]);
+                if (glu) tma_load_2d(tiles + (size_t)s * STAGE + u * SUB + A_BYTES / 2, &tm_w1, (kb + u) * BK, w.n0, &b_full[s]);
+            }
+        }
+    };
+    constexpr int WKB = A_TMEM ? KBR : U, WRING = A_TMEM ? RS1 : SB;  // k-blocks of a weight stage, stages of its ring
+    if (warp == kRawWarp && lane == 0) {
         for (int s = 0; s < SA; s++) mbar_init(&a_full[s], kProducerWarps), mbar_init(&a_empty[s], 1);  // one arrival per producer WARP
         for (int s = 0; s < SB; s++) mbar_init(&b_full[s], A_TMEM ? 1 : 2), mbar_init(&b_empty[s], 1);
         for (int s = 0; s < RS; s++) mbar_init(&raw_full[s], 1), mbar_init(&raw_empty[s], kProducerWarps);
@@ -347,18 +386,218 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    if (warp == kXWarp && lane == 0) asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_x) : "memory");
+    // producers: this thread's row of zero / step; scale / zero of the current group and of the next two (register queue; the loads run 1-2 groups ahead of
+    // their use).  Those of the first item are asked for here: they take a DRAM round trip, as long as the first weights
+    const int prow = (warp & 3) * 32 + lane, gpr = (p.K >> 7) >> p.gshift;
+    const uint16_t *zrow = nullptr, *srow = nullptr;
+    int gcur = 0;
+    uint32_t zq0 = 0, sq0 = 0, zq1 = 0, sq1 = 0, zq2 = 0, sq2 = 0;
+    auto fetch_gama = [&](const Item& w) {
+        if constexpr (MODE != TM_PLAIN) {
+            const int seg  = glu ? prow >> 6 : w.wi;
+            const int grow = min(w.n0 + (glu ? prow & 63 : prow), p.Nw[seg] - 1);
+            zrow = p.zero[seg] + (size_t)grow * gpr, srow = p.step[seg] + (size_t)grow * gpr;
+            gcur = (w.kb0 >> 1) >> p.gshift;
+            const int g1 = min(gcur + 1, gpr - 1), g2 = min(gcur + 2, gpr - 1);
+            zq0 = __ldg(zrow + gcur), sq0 = __ldg(srow + gcur);
+            zq1 = __ldg(zrow + g1), sq1 = __ldg(srow + g1);
+            zq2 = __ldg(zrow + g2), sq2 = __ldg(srow + g2);
+        }
+    };
+    if (warp < kProducerWarps) fetch_gama(decode_item<KBR>(p, blockIdx.x));
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = tmem_base_smem;
     kf_grid_launch_dependents();
 
+    // ============ the end of an item: TMEM -> registers -> output buffer in shared memory -> Y in 16-byte accesses, or partial sums of a split.  Runs on the
+    // four epilogue warps while the other roles work on the next item, and on these and the eight producer warps (three to a quarter of the lanes) for the
+    // CTA's last item, where nothing else is left to do.  Four warps took 4 us for the 256 tokens of an item and 10 with SwiGLU, in front of which the matrix
+    // instructions of the next item waited: there is no second accumulator beside 256 columns and the A ring (4-bit SwiGLU 51200 x 5120 at 2048 tokens 842 -> 757 us,
+    // 6144 x 1024 at 700, one item per CTA, 22.2 -> 17.8) ============
+    const int last_ait  = (p.n_items - 1 - (int)blockIdx.x) / (int)gridDim.x, last_item = blockIdx.x + last_ait * gridDim.x;
+    const bool finisher = warp < kProducerWarps || warp >= kEpiWarp0;
+    const int fin_t     = warp < kProducerWarps ? 128 + tid : tid - kEpiWarp0 * 32;  // 0 .. 127: epilogue warps
+    const bool f32out   = p.epilogue == 4;
+    constexpr int kRes  = 4;  // residual pieces in flight per thread
+    // the residual of pieces j0 .. j0 + kRes - 1 of this thread: piece i = token t0 + i / 16, rows 8 (i % 16) ..
+    auto fetch_res = [&](uint4 (&res)[kRes], const Item& w, int m0, int N, int t0, int t1, int j0, int nthr) {
+#pragma unroll
+        for (int j = 0; j < kRes; j++) {
+            const int i = fin_t + (j0 + j) * nthr, t = t0 + (i >> 4), n = w.n0 + (i & 15) * 8;
+            res[j]      = t < t1 && n < N ? *reinterpret_cast<const uint4*>(p.residual + (size_t)(m0 + t) * N + n) : make_uint4(0, 0, 0, 0);
+        }
+    };
+    // output buffer (tokens t0 .. t1 of the item) -> Y ; res: the first kRes pieces of the residual
+    auto copy_out = [&](uint4 (&res)[kRes], const Item& w, int m0, int N, int t0, int t1, int nthr) {
+        void* const y = p.y[w.wi];
+        if (glu) {
+            for (int i = fin_t; i < (t1 - t0) * 8; i += nthr) {
+                const int t = i >> 3, n = w.n0 + (i & 7) * 8;
+                if (n >= N) continue;
+                const uint4 g4 = *reinterpret_cast<const uint4*>(outs + t * 256 + (i & 7) * 16), u4 = *reinterpret_cast<const uint4*>(outs + t * 256 + 128 + (i & 7) * 16);
+                const uint32_t g[4] = {g4.x, g4.y, g4.z, g4.w}, u[4] = {u4.x, u4.y, u4.z, u4.w};
+                uint32_t v[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) {  // CU_swiglu_v0 on the bf16 gate / up (Activation.cu:86-93), as kf_swiglu computes it
+                    const float g0 = bf16lo(g[j]), g1 = bf16hi(g[j]), u0 = bf16lo(u[j]), u1 = bf16hi(u[j]);
+                    v[j] = pack_bf16x2((g0 * u0) / (1.0f + expf(-g0)), (g1 * u1) / (1.0f + expf(-g1)));
+                }
+                *reinterpret_cast<uint4*>((uint16_t*)y + (size_t)(m0 + t0 + t) * N + n) = make_uint4(v[0], v[1], v[2], v[3]);
+            }
+        } else if (f32out) {
+            for (int i = fin_t; i < (t1 - t0) * 32; i += nthr) {
+                const int t = i >> 5, n = w.n0 + (i & 31) * 4;
+                if (n < N) *reinterpret_cast<uint4*>((float*)y + (size_t)(m0 + t0 + t) * N + n) = *reinterpret_cast<const uint4*>(outs + i * 16);
+            }
+        } else {
+            for (int j0 = 0; j0 * nthr < (t1 - t0) * 16; j0 += kRes) {
+                if (p.epilogue == 1 && j0 > 0) fetch_res(res, w, m0, N, t0, t1, j0, nthr);
+#pragma unroll
+                for (int j = 0; j < kRes; j++) {
+                    const int i = fin_t + (j0 + j) * nthr, t = t0 + (i >> 4), n = w.n0 + (i & 15) * 8;
+                    if (t >= t1 || n >= N) continue;
+                    uint4 v4 = *reinterpret_cast<const uint4*>(outs + i * 16);
+                    if (p.epilogue == 1) {
+                        const uint32_t r[4] = {res[j].x, res[j].y, res[j].z, res[j].w};
+                        uint32_t v[4]       = {v4.x, v4.y, v4.z, v4.w};
+#pragma unroll
+                        for (int q = 0; q < 4; q++) v[q] = pack_bf16x2(bf16lo(r[q]) + bf16lo(v[q]), bf16hi(r[q]) + bf16hi(v[q]));
+                        v4 = make_uint4(v[0], v[1], v[2], v[3]);
+                    }
+                    *reinterpret_cast<uint4*>((uint16_t*)y + (size_t)(m0 + t) * N + n) = v4;
+                }
+            }
+        }
+    };
+    // the sums of rows 4 lane .. 4 lane + 3 of token t -> output buffer that starts at token t0, or Y
+    auto put4 = [&](const Item& w, int m0, int N, int t0, int t, const float4& f) {
+        if (p.staged) {
+            if (f32out) *reinterpret_cast<float4*>(outs + (t - t0) * 512 + lane * 16) = f;
+            else *reinterpret_cast<uint2*>(outs + (t - t0) * 256 + lane * 8) = make_uint2(pack_bf16x2(f.x, f.y), pack_bf16x2(f.z, f.w));
+            return;
+        }
+        const float v[4] = {f.x, f.y, f.z, f.w};
+        for (int j = 0; j < 4; j++) {
+            const float one[1] = {v[j]};
+            if (w.n0 + lane * 4 + j < N) store_cols<1>(p, p.y[w.wi], N, one, m0 + t, 1, w.n0 + lane * 4 + j);
+        }
+    };
+    auto finish = [&](const Item& w, uint32_t ait, int et, int nthr) {
+        constexpr int TC = BN < 32 ? 16 : 32;  // tokens of one read of tensor memory
+        const int quad = warp & 3, row = quad * 32 + lane, part = et >> 7, nparts = nthr >> 7;
+        const int buf = ait % NACC, m0 = w.m0 * BN, cnt = min(BN, p.M - m0), N = p.Nw[w.wi];
+        const int round = C::OUT / (f32out ? 512 : 256);  // tokens that the output buffer takes
+        const uint32_t tbase = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * BN);
+        const bool direct = p.splits == 1 && p.staged;
+        uint4 res[kRes];
+        if (direct && p.epilogue == 1) fetch_res(res, w, m0, N, 0, min(cnt, round), 0, nthr);
+        if (warp >= kEpiWarp0) {
+            if (NACC == 2 && nthr == 128) mbar_wait_sleepy(&tmem_full[buf], (ait / NACC) & 1);  // a whole main loop away: poll politely
+            else mbar_wait(&tmem_full[buf], (ait / NACC) & 1);
+        }
+        epi_bar_sync(nthr);  // the output buffer is free; producers learn here that the accumulator is complete
+        tc_fence_after();
+        auto release = [&]() {  // the accumulator buffer may be overwritten by the next item
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0 && warp >= kEpiWarp0) mbar_arrive(&tmem_empty[buf]);
+        };
+        if (p.cluster) {
+            float* sums = reinterpret_cast<float*>(tiles);  // the rings are idle: this is the CTA's only item and its MMAs have completed
+            for (int c0 = part * 16; c0 < cnt; c0 += nparts * 16) {
+                uint32_t v[16];
+                tmem_ld16(tbase + (uint32_t)c0, v);
+#pragma unroll
+                for (int j = 0; j < 16; j++) sums[(c0 + j) * BM + row] = __uint_as_float(v[j]);
+            }
+            return;
+        }
+        if (direct) {
+            for (int r0 = 0; r0 < cnt; r0 += round) {
+                const int r1 = min(cnt, r0 + round);
+                if (r0 > 0) {
+                    epi_bar_sync(nthr);
+                    if (p.epilogue == 1) fetch_res(res, w, m0, N, r0, r1, 0, nthr);
+                }
+                for (int c0 = r0 + part * TC; c0 < r1; c0 += nparts * TC) {
+                    uint32_t v[TC];
+                    if constexpr (TC == 16) tmem_ld16(tbase + (uint32_t)c0, v);
+                    else tmem_ld32(tbase + (uint32_t)c0, v);
+#pragma unroll
+                    for (int j = 0; j < TC; j++) {
+                        if (f32out) *reinterpret_cast<uint32_t*>(outs + (c0 - r0 + j) * 512 + row * 4) = v[j];
+                        else *reinterpret_cast<uint16_t*>(outs + (c0 - r0 + j) * 256 + row * 2) = f32_to_bf16_bits(__uint_as_float(v[j]));  // the reference's GEMM output is bf16 (gemm.cu:124-126)
+                    }
+                }
+                if (r1 == cnt) release();
+                epi_bar_sync(nthr);
+                copy_out(res, w, m0, N, r0, r1, nthr);
+            }
+            return;
+        }
+        float* wsp = p.ws + ((size_t)w.tile * p.splits + w.z) * (size_t)(BN * BM);
+        for (int c0 = part * 16; c0 < cnt; c0 += nparts * 16) {
+            uint32_t v[16];
+            tmem_ld16(tbase + (uint32_t)c0, v);
+            if (p.splits > 1) {
+#pragma unroll
+                for (int j = 0; j < 16; j++)
+                    if (c0 + j < cnt) wsp[(size_t)(c0 + j) * BM + row] = __uint_as_float(v[j]);
+            } else if (w.n0 + row < N) {
+                float acc[16];
+#pragma unroll
+                for (int j = 0; j < 16; j++) acc[j] = __uint_as_float(v[j]);
+                store_cols<16>(p, p.y[w.wi], N, acc, m0 + c0, cnt - c0, w.n0 + row);
+            }
+        }
+        release();
+        if (p.splits == 1) return;
+        __threadfence();
+        epi_bar_sync(nthr);
+        if (et == 0) {
+            const unsigned old = atomicAdd(&p.cnt[w.tile], 1u);
+            last_flag          = (old == (unsigned)(p.splits - 1));
+            if (last_flag) p.cnt[w.tile] = 0;  // self-reset for the next launch
+        }
+        epi_bar_sync(nthr);
+        if (!last_flag) return;
+        __threadfence();
+        const float* base = p.ws + (size_t)w.tile * p.splits * (size_t)(BN * BM);
+        // a thread sums four rows of one token (16-byte loads), two tokens and four partials in flight; the partials are added in split order
+        for (int r0 = 0; r0 < cnt; r0 += round) {
+            const int r1 = min(cnt, r0 + round), nw = nthr >> 5;
+            if (r0 > 0) epi_bar_sync(nthr);
+            if (p.epilogue == 1 && p.staged) fetch_res(res, w, m0, N, r0, r1, 0, nthr);
+            for (int t = r0 + (et >> 5); t < r1; t += 2 * nw) {
+                const bool two  = t + nw < r1;
+                const float* b0 = base + (size_t)t * BM + lane * 4;
+                float4 s0 = make_float4(0.f, 0.f, 0.f, 0.f), s1 = s0;
+#pragma unroll 4
+                for (int z = 0; z < p.splits; z++) {
+                    const float4 a = __ldcg(reinterpret_cast<const float4*>(b0 + (size_t)z * (BN * BM)));
+                    const float4 c = two ? __ldcg(reinterpret_cast<const float4*>(b0 + (size_t)z * (BN * BM) + nw * BM)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    s0.x += a.x, s0.y += a.y, s0.z += a.z, s0.w += a.w;
+                    s1.x += c.x, s1.y += c.y, s1.z += c.z, s1.w += c.w;
+                }
+                put4(w, m0, N, r0, t, s0);
+                if (two) put4(w, m0, N, r0, t + nw, s1);
+            }
+            if (p.staged) {
+                epi_bar_sync(nthr);
+                copy_out(res, w, m0, N, r0, r1, nthr);
+            }
+        }
+        epi_bar_sync(nthr);  // last_flag is rewritten by the next item
+    };
+
     if (warp < kProducerWarps) {
         if constexpr (A_TMEM) {
             // ============ producers: thread = (weight row, 32-weight slot of the k-block): raw bytes -> bf16 -> TMEM ============
             const int quad = warp & 3, slot = warp >> 2;
-            const int row  = quad * 32 + lane;
-            const int gpr  = (p.K >> 7) >> p.gshift;
+            const int row  = prow;
             const uint32_t bias2 = pack_bf16x2((float)(128 + p.qbias), (float)(128 + p.qbias));
             // TMA swizzle of the raw stage: the 16-byte chunk index is XORed with address bits [7,9) (64-byte rows) / [7,10) (128-byte rows)
             const uint32_t rsw   = RAWB == 64 ? (uint32_t)((row >> 1) & 3) : (uint32_t)(row & 7);
@@ -371,20 +610,9 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
             uint32_t s = 0, eph = 1, rs = 0, rph = 0;  // ring positions and the parities to wait for
             for (int item = blockIdx.x; item < p.n_items; item += gridDim.x) {
                 const Item w = decode_item<KBR>(p, item);
-                const int seg        = glu ? row >> 6 : w.wi;
-                const int grow       = min(w.n0 + (glu ? row & 63 : row), p.Nw[seg] - 1);
-                const uint16_t* zrow = MODE == TM_PLAIN ? nullptr : p.zero[seg] + (size_t)grow * gpr;
-                const uint16_t* srow = MODE == TM_PLAIN ? nullptr : p.step[seg] + (size_t)grow * gpr;
-                // scale / zero of the current group and of the next two (register queue; the loads run 1-2 groups ahead of their use)
-                int gcur = 0;
-                uint32_t zq0 = 0, sq0 = 0, zq1 = 0, sq1 = 0, zq2 = 0, sq2 = 0;
+                if (item != (int)blockIdx.x) fetch_gama(w);
                 uint32_t step2 = 0, zero2 = 0, nb2 = 0;
                 if (MODE != TM_PLAIN) {
-                    gcur = (w.kb0 >> 1) >> p.gshift;
-                    zq0 = __ldg(zrow + gcur), sq0 = __ldg(srow + gcur);
-                    const int g1 = min(gcur + 1, gpr - 1), g2 = min(gcur + 2, gpr - 1);
-                    zq1 = __ldg(zrow + g1), sq1 = __ldg(srow + g1);
-                    zq2 = __ldg(zrow + g2), sq2 = __ldg(srow + g2);
                     step2 = __byte_perm(sq0, 0u, 0x1010), zero2 = __byte_perm(zq0, 0u, 0x1010) ^ (MODE == TM_AFFINE_FMA ? 0x80008000u : 0u);
                     if (MODE == TM_AFFINE) nb2 = bf162_as_u32(__hmul2_rn(u32_as_bf162(step2), u32_as_bf162(0xC300C300u)));
                 }
@@ -477,32 +705,9 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
             uint32_t it = 0;
             for (int item = blockIdx.x; item < p.n_items; item += gridDim.x) {
                 const Item w = decode_item<KBR>(p, item);
-                const CUtensorMap* tm_w = w.wi == 0 ? &tm_w0 : w.wi == 1 ? &tm_w1 : &tm_w2;
-                if constexpr (A_TMEM) {
-                    for (int r = w.kb0 / KBR; r * KBR < w.kb1; r++) {
-                        const int rs = it % RS;
-                        mbar_wait(&raw_empty[rs], ((it / RS) & 1) ^ 1);
-#if KF_TC_EXP & 8
-                        mbar_arrive(&raw_full[rs]);
-#else
-                        mbar_arrive_expect_tx(&raw_full[rs], RAW_BYTES);
-                        tma_load_2d(raws + (size_t)rs * RAW_BYTES, tm_w, r * RAWB, w.n0, &raw_full[rs]);
-                        if (glu) tma_load_2d(raws + (size_t)rs * RAW_BYTES + RAW_BYTES / 2, &tm_w1, r * RAWB, w.n0, &raw_full[rs]);
-#endif
-                        it++;
-                    }
-                } else {
-                    for (int kb = w.kb0; kb < w.kb1; kb += U) {
-                        const int s = it % SB;
-                        mbar_wait(&b_empty[s], ((it / SB) & 1) ^ 1);
-                        mbar_arrive_expect_tx(&b_full[s], U * A_BYTES);
-#pragma unroll
-                        for (int u = 0; u < U; u++) {
-                            tma_load_2d(tiles + (size_t)s * STAGE + u * SUB, tm_w, (kb + u) * BK, w.n0, &b_full[s]);
-                            if (glu) tma_load_2d(tiles + (size_t)s * STAGE + u * SUB + A_BYTES / 2, &tm_w1, (kb + u) * BK, w.n0, &b_full[s]);
-                        }
-                        it++;
-                    }
+                for (int kb = w.kb0; kb < w.kb1; kb += WKB, it++) {
+                    mbar_wait(A_TMEM ? &raw_empty[it % RS1] : &b_empty[it % SB], ((it / WRING) & 1) ^ 1);
+                    load_w(w, kb, it);
                 }
             }
         }
@@ -581,181 +786,55 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
             ait++;
         }
     } else {
-        // ============ epilogue: TMEM -> registers -> output buffer in shared memory -> Y in 16-byte accesses, 32 tokens at a time (fp32: 16); with split-K an
-        // fp32 partial + ordered reduction by the last CTA, through the same output buffers.  Straight from the registers (one 2-byte store per token and
-        // lane) the 256 tokens of an item took 10 us and another 12 with a residual, whose loads waited in front of every 16 tokens: 1024 x 4096 at 700
-        // tokens 19 / 31 us, of which the matrix instructions are 4 ============
         kf_grid_dependency_wait();  // residual / workspace / counters may still be in use by the previous kernel
-        const int quad = warp & 3;
-        const int row  = quad * 32 + lane;
-        const int et   = (warp - kEpiWarp0) * 32 + lane;  // 0..127
-        const bool f32out = p.epilogue == 4;
-        const int ch      = f32out ? 16 : 32;             // tokens per output buffer
-        uint32_t ait = 0, obuf = 0;
-        for (int item = blockIdx.x; item < p.n_items; item += gridDim.x) {
-            const Item w  = decode_item<KBR>(p, item);
-            const int buf = ait % NACC;
-            const int m0  = w.m0 * BN;
-            const int cnt = min(BN, p.M - m0);
-            const int grow = w.n0 + row;
-            const int N = p.Nw[w.wi];
-            void* const y = p.y[w.wi];
-            const bool row_ok = grow < N;
-            uint4 res[4];
-            // the residual of a buffer's four 16-byte pieces of this thread: piece i = token et / 16 + 8 i, rows 8 (et % 16) ..
-            auto fetch_res = [&](int c0) {
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    const int t = c0 + (et >> 4) + 8 * i, n = w.n0 + (et & 15) * 8;
-                    res[i]      = t < cnt && n < N ? *reinterpret_cast<const uint4*>(p.residual + (size_t)(m0 + t) * N + n) : make_uint4(0, 0, 0, 0);
-                }
-            };
-            // output buffer -> Y
-            auto copy_out = [&](const uint8_t* o, int c0) {
-                if (glu) {
-#pragma unroll
-                    for (int i = 0; i < 2; i++) {
-                        const int t = (et >> 3) + 16 * i, n = w.n0 + (et & 7) * 8;
-                        if (c0 + t >= cnt || n >= N) continue;
-                        const uint4 g4 = *reinterpret_cast<const uint4*>(o + t * 256 + (et & 7) * 16), u4 = *reinterpret_cast<const uint4*>(o + t * 256 + 128 + (et & 7) * 16);
-                        const uint32_t g[4] = {g4.x, g4.y, g4.z, g4.w}, u[4] = {u4.x, u4.y, u4.z, u4.w};
-                        uint32_t v[4];
-#pragma unroll
-                        for (int j = 0; j < 4; j++) {  // CU_swiglu_v0 on the bf16 gate / up (Activation.cu:86-93), as kf_swiglu computes it
-                            const float g0 = bf16lo(g[j]), g1 = bf16hi(g[j]), u0 = bf16lo(u[j]), u1 = bf16hi(u[j]);
-                            v[j] = pack_bf16x2((g0 * u0) / (1.0f + expf(-g0)), (g1 * u1) / (1.0f + expf(-g1)));
-                        }
-                        *reinterpret_cast<uint4*>((uint16_t*)y + (size_t)(m0 + c0 + t) * N + n) = make_uint4(v[0], v[1], v[2], v[3]);
-                    }
-                } else if (f32out) {
-#pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        const int t = (et >> 5) + 4 * i, n = w.n0 + lane * 4;
-                        if (c0 + t < cnt && n < N)
-                            *reinterpret_cast<uint4*>((float*)y + (size_t)(m0 + c0 + t) * N + n) = *reinterpret_cast<const uint4*>(o + t * 512 + lane * 16);
-                    }
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        const int t = (et >> 4) + 8 * i, n = w.n0 + (et & 15) * 8;
-                        if (c0 + t >= cnt || n >= N) continue;
-                        uint4 v4 = *reinterpret_cast<const uint4*>(o + t * 256 + (et & 15) * 16);
-                        if (p.epilogue == 1) {
-                            const uint32_t r[4] = {res[i].x, res[i].y, res[i].z, res[i].w};
-                            uint32_t v[4]       = {v4.x, v4.y, v4.z, v4.w};
-#pragma unroll
-                            for (int j = 0; j < 4; j++) v[j] = pack_bf16x2(bf16lo(r[j]) + bf16lo(v[j]), bf16hi(r[j]) + bf16hi(v[j]));
-                            v4 = make_uint4(v[0], v[1], v[2], v[3]);
-                        }
-                        *reinterpret_cast<uint4*>((uint16_t*)y + (size_t)(m0 + c0 + t) * N + n) = v4;
-                    }
-                }
-            };
-            if (p.staged && p.splits == 1 && p.epilogue == 1) fetch_res(0);
-            if (NACC == 2)
-                mbar_wait_sleepy(&tmem_full[buf], (ait / NACC) & 1);  // a whole main loop away: poll politely
-            else
-                mbar_wait(&tmem_full[buf], (ait / NACC) & 1);
-            tc_fence_after();
-            const uint32_t tbase = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * BN);
-            float* wsp = p.ws + ((size_t)w.tile * p.splits + w.z) * (size_t)(BN * BM);
-            auto release = [&]() {  // the accumulator buffer may be overwritten by the next item
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&tmem_empty[buf]);
-            };
-            if (p.splits == 1 && p.staged) {
-                for (int c0 = 0; c0 < cnt; c0 += ch, obuf ^= 1) {
-                    uint8_t* o = outs + obuf * kStageOut;
-                    if (f32out || BN < 32) {
-                        uint32_t v[16];
-                        tmem_ld16(tbase + (uint32_t)c0, v);
-                        if (c0 + ch >= cnt) release();
-#pragma unroll
-                        for (int j = 0; j < 16; j++) {
-                            if (f32out) *reinterpret_cast<uint32_t*>(o + j * 512 + row * 4) = v[j];
-                            else *reinterpret_cast<uint16_t*>(o + j * 256 + row * 2) = f32_to_bf16_bits(__uint_as_float(v[j]));
-                        }
-                    } else {
-                        uint32_t v[32];
-                        tmem_ld32(tbase + (uint32_t)c0, v);
-                        if (c0 + ch >= cnt) release();
-#pragma unroll
-                        for (int j = 0; j < 32; j++) *reinterpret_cast<uint16_t*>(o + j * 256 + row * 2) = f32_to_bf16_bits(__uint_as_float(v[j]));  // the reference's GEMM output is bf16 (gemm.cu:124-126)
-                    }
-                    epi_bar_sync();  // also: everybody has left the copy of the buffer before this one, which the next 32 tokens overwrite
-                    copy_out(o, c0);
-                    if (p.epilogue == 1 && c0 + ch < cnt) fetch_res(c0 + ch);
-                }
-            } else {
-                for (int c0 = 0; c0 < cnt; c0 += 16) {
-                    uint32_t v[16];
-                    tmem_ld16(tbase + (uint32_t)c0, v);
-                    if (p.splits > 1) {
-#pragma unroll
-                        for (int j = 0; j < 16; j++)
-                            if (c0 + j < cnt) wsp[(size_t)(c0 + j) * BM + row] = __uint_as_float(v[j]);
-                    } else if (row_ok) {
-                        float acc[16];
-#pragma unroll
-                        for (int j = 0; j < 16; j++) acc[j] = __uint_as_float(v[j]);
-                        store_cols<16>(p, y, N, acc, m0 + c0, cnt - c0, grow);
-                    }
-                }
-                release();
-            }
-            ait++;
-            if (p.splits > 1) {
-                __threadfence();
-                epi_bar_sync();
-                if (et == 0) {
-                    const unsigned old = atomicAdd(&p.cnt[w.tile], 1u);
-                    last_flag          = (old == (unsigned)(p.splits - 1));
-                    if (last_flag) p.cnt[w.tile] = 0;  // self-reset for the next launch
-                }
-                epi_bar_sync();
-                if (last_flag) {
-                    __threadfence();
-                    const float* base = p.ws + (size_t)w.tile * p.splits * (size_t)(BN * BM);
-                    // a thread sums four rows of one token (16-byte loads), two tokens and four partials in flight; the partials are added in split order
-                    for (int c0 = 0; c0 < cnt; c0 += ch, obuf ^= 1) {
-                        uint8_t* o = outs + obuf * kStageOut;
-                        if (p.epilogue == 1 && p.staged) fetch_res(c0);
-                        for (int t = et >> 5; t < ch && c0 + t < cnt; t += 8) {
-                            const bool two  = t + 4 < ch && c0 + t + 4 < cnt;
-                            const float* b0 = base + (size_t)(c0 + t) * BM + lane * 4;
-                            float4 s0 = make_float4(0.f, 0.f, 0.f, 0.f), s1 = s0;
+        uint32_t ait = 0;
+        for (int item = blockIdx.x; item < last_item; item += gridDim.x, ait++) {
+            const Item w = decode_item<KBR>(p, item);
+            finish(w, ait, (warp - kEpiWarp0) * 32 + lane, 128);
+        }
+    }
+    if (finisher) {  // the last item: all twelve warps
+        if (warp < kProducerWarps) kf_grid_dependency_wait();
+        finish(decode_item<KBR>(p, last_item), last_ait, fin_t, 384);
+    }
+    // ============ split over a cluster: every CTA has its partial sums in shared memory and adds up its share of the tokens, in the order of the parts.  Takes
+    // 3 us, of which the reads from the other CTAs are half; through global memory, where the last CTA to arrive did it all, 4-bit 4096 x 12288 at 300 tokens
+    // took 75.5 us (now 50.4), 6144 x 4096 at 64 21.7 (15.9), 4096 x 4096 at 64 17.0 (13.5) ============
+    if (p.cluster) {
+        __syncwarp();
+        cluster_arrive(), cluster_wait();
+        if (finisher) {
+            const Item w  = decode_item<KBR>(p, last_item);
+            const int m0 = w.m0 * BN, cnt = min(BN, p.M - m0), N = p.Nw[w.wi];
+            const int t0 = cnt * w.z / p.splits, t1 = cnt * (w.z + 1) / p.splits;
+            const int round = C::OUT / (f32out ? 512 : 256);  // tokens that the output buffer takes
+            const uint32_t part = smem_u32(tiles);
+            uint4 res[kRes];
+            for (int r0 = t0; r0 < t1; r0 += round) {
+                const int r1 = min(t1, r0 + round);
+                if (r0 > t0) epi_bar_sync(384);
+                if (p.epilogue == 1 && p.staged) fetch_res(res, w, m0, N, r0, r1, 0, 384);
+                for (int t = r0 + (fin_t >> 5); t < r1; t += 24) {  // a warp adds up two tokens at a time
+                    const bool two = t + 12 < r1;
+                    float4 s0 = make_float4(0.f, 0.f, 0.f, 0.f), s1 = s0;
 #pragma unroll 4
-                            for (int z = 0; z < p.splits; z++) {
-                                const float4 a = __ldcg(reinterpret_cast<const float4*>(b0 + (size_t)z * (BN * BM)));
-                                const float4 c = two ? __ldcg(reinterpret_cast<const float4*>(b0 + (size_t)z * (BN * BM) + 4 * BM)) : make_float4(0.f, 0.f, 0.f, 0.f);
-                                s0.x += a.x, s0.y += a.y, s0.z += a.z, s0.w += a.w;
-                                s1.x += c.x, s1.y += c.y, s1.z += c.z, s1.w += c.w;
-                            }
-                            auto put = [&](int tt, const float4& f) {
-                                if (p.staged) {
-                                    if (f32out) *reinterpret_cast<float4*>(o + tt * 512 + lane * 16) = f;
-                                    else *reinterpret_cast<uint2*>(o + tt * 256 + lane * 8) = make_uint2(pack_bf16x2(f.x, f.y), pack_bf16x2(f.z, f.w));
-                                    return;
-                                }
-                                const float v[4] = {f.x, f.y, f.z, f.w};
-                                for (int j = 0; j < 4; j++) {
-                                    const float one[1] = {v[j]};
-                                    if (w.n0 + lane * 4 + j < N) store_cols<1>(p, y, N, one, m0 + c0 + tt, 1, w.n0 + lane * 4 + j);
-                                }
-                            };
-                            put(t, s0);
-                            if (two) put(t + 4, s1);
-                        }
-                        if (p.staged) {
-                            epi_bar_sync();
-                            copy_out(o, c0);
-                        }
+                    for (int z = 0; z < p.splits; z++) {
+                        const float4 a = ld_cluster_f4(part + (uint32_t)(t * BM + lane * 4) * 4, z);
+                        const float4 c = ld_cluster_f4(part + (uint32_t)((two ? t + 12 : t) * BM + lane * 4) * 4, z);
+                        s0.x += a.x, s0.y += a.y, s0.z += a.z, s0.w += a.w;
+                        s1.x += c.x, s1.y += c.y, s1.z += c.z, s1.w += c.w;
                     }
+                    put4(w, m0, N, r0, t, s0);
+                    if (two) put4(w, m0, N, r0, t + 12, s1);
                 }
-                epi_bar_sync();  // last_flag is rewritten by the next item
+                if (p.staged) {
+                    epi_bar_sync(384);
+                    copy_out(res, w, m0, N, r0, r1, 384);
+                }
             }
         }
+        __syncwarp();
+        cluster_arrive(), cluster_wait();  // nobody leaves while others still read its sums
     }
     tc_fence_before();
     __syncthreads();
@@ -846,8 +925,45 @@ int row_tiles(const GemmParams& p, int nw) {
     for (int i = 0; i < nw; i++) n += (p.Nw[i] + BM - 1) / BM;
     return n;
 }
+struct TcPlan {
+    int bn, splits;
+    bool cluster;
+};
+// CTAs of the kernel that can be resident in clusters of s (2 .. 8); 0 where the driver cannot say.  A property of the device: asked once.
 template <int FMT, int MODE, int BN>
-int launch_tc(kf_ctx* ctx, GemmParams& p, const void* const* wdata, int nw, const void* xp, int splits) {
+int cluster_ctas(const kf_ctx* ctx, int s) {
+    static int known[kf_ctx::kMaxDevices][9] = {};  // + 1
+    int& k = known[ctx->device][s];
+    if (k == 0) {
+        auto kern = kf_gemm_tc_kernel<FMT, MODE, BN>;
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr[1];
+        attr[0].id               = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)s, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
+        cfg.gridDim = dim3((unsigned)(ctx->sm_count / s * s)), cfg.blockDim = dim3(kThreadsTC), cfg.dynamicSmemBytes = Rings<FMT, BN>::SMEM;
+        cfg.attrs = attr, cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Rings<FMT, BN>::SMEM) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+            (void)cudaGetLastError();
+            n = 0;
+        }
+        k = n * s + 1;
+    }
+    return k - 1;
+}
+template <int FMT, int MODE>
+int cluster_ctas(const kf_ctx* ctx, int bn, int s) {
+    switch (bn) {
+        case 256: return cluster_ctas<FMT, MODE, 256>(ctx, s);
+        case 128: return cluster_ctas<FMT, MODE, 128>(ctx, s);
+        case 64: return cluster_ctas<FMT, MODE, 64>(ctx, s);
+        case 32: return cluster_ctas<FMT, MODE, 32>(ctx, s);
+        default: return cluster_ctas<FMT, MODE, 16>(ctx, s);
+    }
+}
+template <int FMT, int MODE, int BN>
+int launch_tc(kf_ctx* ctx, GemmParams& p, const void* const* wdata, int nw, const void* xp, const TcPlan& plan) {
     using F              = Fmt<FMT>;
     constexpr bool A_TMEM = FMT != TF_BF16;
     const size_t smem    = Rings<FMT, BN>::SMEM;
@@ -866,8 +982,8 @@ int launch_tc(kf_ctx* ctx, GemmParams& p, const void* const* wdata, int nw, cons
     p.n_tiles = row_tiles(p, nw);
     p.m_tiles = (p.M + BN - 1) / BN;
     const int base_items = p.n_tiles * p.m_tiles;
-    p.splits = splits, p.n_items = base_items * splits;
-    if (splits > 1) {
+    p.splits = plan.splits, p.n_items = base_items * plan.splits, p.cluster = plan.cluster;
+    if (plan.splits > 1 && !plan.cluster) {
         int rc = kf_ensure_gemv_ws(ctx, (size_t)p.n_items * BN * BM * sizeof(float), base_items);
         if (rc) return rc;
         p.ws = ctx->gemv_ws, p.cnt = ctx->gemv_cnt;
@@ -886,20 +1002,33 @@ int launch_tc(kf_ctx* ctx, GemmParams& p, const void* const* wdata, int nw, cons
     if (!rc) rc = kf_tmap_2d(ctx, &tm_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, xp, (uint64_t)p.K, (uint64_t)p.M, BK, BN, CU_TENSOR_MAP_SWIZZLE_128B, false);
     if (rc) return rc;
     const int grid = std::min(p.n_items, ctx->sm_count);
-    KF_CUDA(ctx, kf_launch_pdl(ctx, kern, dim3(grid), dim3(kThreadsTC), smem, tm_w[0], tm_w[1], tm_w[2], tm_x, p));
+    if (plan.cluster) {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr[2];
+        attr[0].id               = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)plan.splits, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
+        attr[1].id               = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.gridDim = dim3(p.n_items), cfg.blockDim = dim3(kThreadsTC), cfg.dynamicSmemBytes = smem, cfg.stream = ctx->stream;
+        cfg.attrs = attr, cfg.numAttrs = ctx->pdl ? 2 : 1;
+        KF_CUDA(ctx, cudaLaunchKernelEx(&cfg, kern, tm_w[0], tm_w[1], tm_w[2], tm_x, p));
+    } else {
+        KF_CUDA(ctx, kf_launch_pdl(ctx, kern, dim3(grid), dim3(kThreadsTC), smem, tm_w[0], tm_w[1], tm_w[2], tm_x, p));
+    }
     KF_LAUNCH_CHECK(ctx);
     return KF_OK;
 }
 // Token tile and k-split by their modelled time: waves x (k-blocks x time per k-block + epilogue) + the fix-up of split sums.  The times per k-block of 64 are
 // measured ones (us; 4-bit and bf16 weights, the former stand for all that are expanded; below 64 tokens the weights' bytes or their expansion, above the matrix instructions).  Splitting pays for few row tiles and a
 // handful of tokens only: 1024 x 3072 at 16 tokens 9.9 us in 8 parts against 15.7 whole, at 256 tokens 34 against 17.  (The rule before it charged BN / 16
-// k-blocks for the fix-up: 1024 x 3072 at 256 tokens went into 12 parts and took 91 us, now 17.5.)  The reference-exact arithmetic keeps that rule and the
-// order of sums it was compared in.
+// k-blocks for the fix-up: 1024 x 3072 at 256 tokens went into 12 parts and took 91 us, now 17.5.)  Parts that fit on the GPU as clusters cost 1 us more and
+// no second pass: swept over six shapes of the 0.6B and 8B blocks at 12 to 2000 tokens, the choice is within 8 % of the best tile and split.  The
+// reference-exact arithmetic keeps the earlier rule and the order of sums it was compared in.
 template <int FMT, int MODE>
 int launch_tc_bn(kf_ctx* ctx, GemmParams& p, const void* const* wdata, int nw, const void* xp) {
     constexpr int KBR = Fmt<FMT>::KBR;
     const int nkb = p.K / BK, nraw = (nkb + KBR - 1) / KBR, tiles = row_tiles(p, nw);
-    int bn = 256, splits = 1;
+    TcPlan plan = {256, 1, false};
     double best = 1e30;
     for (int b = 16, i = 0; b <= 256; b *= 2, i++) {
         const int by_m = p.M > 128 ? 256 : p.M > 64 ? 128 : p.M > 32 ? 64 : p.M > 16 ? 32 : 16;  // one token tile where the panel fits one
@@ -912,19 +1041,22 @@ int launch_tc_bn(kf_ctx* ctx, GemmParams& p, const void* const* wdata, int nw, c
             const int waves = (items * s + ctx->sm_count - 1) / ctx->sm_count, len = (nraw + s - 1) / s * KBR;
             if (ctx->gemv_exact) {
                 const double c = waves * (len + 2.0 + (s > 1 ? b / 16.0 : 0.0));
-                if (c < best * 0.95) best = c, bn = b, splits = s;
+                if (c < best * 0.95) best = c, plan = {b, s, false};
                 continue;
             }
             const double t = waves * (len * t_kb + 0.5 + 0.006 * b + (s > 1 ? 0.5 + 0.02 * b : 0.0)) + (s > 1 ? b * (0.03 + 0.008 * s) : 0.0);
-            if (t < best * 0.98) best = t, bn = b, splits = s;
+            if (t < best * 0.98) best = t, plan = {b, s, false};
+            if (s == 1 || s > 8 || items * s > ctx->sm_count) continue;
+            const double tc = len * t_kb + 0.5 + 0.003 * b + 1.0 + 0.006 * b;
+            if (tc < best * 0.98 && items * s <= cluster_ctas<FMT, MODE>(ctx, b, s)) best = tc, plan = {b, s, true};
         }
     }
-    switch (bn) {
-        case 256: return launch_tc<FMT, MODE, 256>(ctx, p, wdata, nw, xp, splits);
-        case 128: return launch_tc<FMT, MODE, 128>(ctx, p, wdata, nw, xp, splits);
-        case 64: return launch_tc<FMT, MODE, 64>(ctx, p, wdata, nw, xp, splits);
-        case 32: return launch_tc<FMT, MODE, 32>(ctx, p, wdata, nw, xp, splits);
-        default: return launch_tc<FMT, MODE, 16>(ctx, p, wdata, nw, xp, splits);
+    switch (plan.bn) {
+        case 256: return launch_tc<FMT, MODE, 256>(ctx, p, wdata, nw, xp, plan);
+        case 128: return launch_tc<FMT, MODE, 128>(ctx, p, wdata, nw, xp, plan);
+        case 64: return launch_tc<FMT, MODE, 64>(ctx, p, wdata, nw, xp, plan);
+        case 32: return launch_tc<FMT, MODE, 32>(ctx, p, wdata, nw, xp, plan);
+        default: return launch_tc<FMT, MODE, 16>(ctx, p, wdata, nw, xp, plan);
     }
 }
 

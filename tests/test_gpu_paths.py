@@ -185,6 +185,65 @@ def test_tc_swiglu_over_its_input(ctx, typ, M, rows, cols, at):
     assert torch.equal(own, buf[64 + at:64 + at + M * rows])
 
 
+@pytest.mark.parametrize("typ", [kf.KF_T_Q4, kf.KF_T_BINARY, kf.KF_T_BF16])
+@pytest.mark.parametrize("M,tc_bn,splits", [(16, 16, 8), (20, 32, 2), (45, 64, 4), (100, 128, 3), (130, 256, 2), (251, 256, 5), (257, 128, 7)])
+def test_tc_split_over_cluster_equals_workspace(ctx, typ, M, tc_bn, splits):
+    """A split whose parts meet in a cluster adds the same partial sums in the same order as one through the workspace (which gemv_exact keeps to): equal bits, every epilogue."""
+    import torch
+    import ctypes as C
+    rows, cols = 272, 8192
+    mk = lambda seed: (make_q(ctx, typ, rows, cols, seed) if typ != kf.KF_T_BF16 else _bf16_weight(ctx, rows, cols, seed))[0]  # noqa: E731
+    w, u = mk(5), mk(6)
+    dw = w.desc()
+    gu = (kf.TensorDesc * 2)(dw, u.desc())
+    x, r = torch.randn(M, cols, device="cuda").bfloat16(), torch.randn(M, rows, device="cuda").bfloat16()
+    ctx.set_int("tc_min_m", 1), ctx.set_int("tc_bn", tc_bn), ctx.set_int("gemv_splitk", splits)
+    outs = []
+    try:
+        for exact in (0, 1):
+            ctx.set_int("gemv_exact", exact)
+            y, yr, yg, yf = (torch.zeros(M, rows, device="cuda", dtype=t) for t in (torch.bfloat16, torch.bfloat16, torch.bfloat16, torch.float32))
+            torch.cuda.synchronize()
+            ctx.check(ctx.lib.kf_linear(ctx.h, _ptr(y), C.byref(dw), _ptr(x), M, kf.KF_EPI_NONE, None), "none")
+            ctx.check(ctx.lib.kf_linear(ctx.h, _ptr(yr), C.byref(dw), _ptr(x), M, kf.KF_EPI_RESIDUAL, _ptr(r)), "residual")
+            ctx.check(ctx.lib.kf_linear(ctx.h, _ptr(yf), C.byref(dw), _ptr(x), M, kf.KF_EPI_F32, None), "f32")
+            ctx.check(ctx.lib.kf_linear_swiglu(ctx.h, _ptr(yg), C.byref(gu[0]), C.byref(gu[1]), _ptr(x), M), "swiglu")
+            ctx.sync()
+            outs.append((y, yr, yg, yf))
+    finally:
+        ctx.set_int("tc_min_m", -1), ctx.set_int("tc_bn", 0), ctx.set_int("gemv_splitk", 0), ctx.set_int("gemv_exact", 0)
+    assert float(outs[0][3].abs().max()) > 0
+    for a, b in zip(*outs):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("typ", [kf.KF_T_Q4, kf.KF_T_BF16])
+@pytest.mark.parametrize("M,tc_bn", [(41, 16), (600, 128), (1100, 256)])
+def test_tc_several_items_per_cta(ctx, typ, M, tc_bn):
+    """Items that the epilogue warps finish alone, under the next one's main loop, and the last one, with the producers' help: 1e-5 of the rms covers the order of
+    fp32 sums, 2^-8 the rounding of a bf16 result."""
+    import torch
+    import ctypes as C
+    torch.backends.cuda.matmul.allow_tf32 = False
+    rows, cols = 6416, 256
+    w, wd = make_q(ctx, typ, rows, cols, 5) if typ != kf.KF_T_BF16 else _bf16_weight(ctx, rows, cols, 5)
+    dw = w.desc()
+    x, r = torch.randn(M, cols, device="cuda").bfloat16(), torch.randn(M, rows, device="cuda").bfloat16()
+    acc = x.float() @ wd.T
+    eps, tiny = 2.0 ** -8 * 1.001, 1e-5 * float(acc.square().mean().sqrt())
+    yr, yf = r.clone(), torch.zeros(M, rows, device="cuda")
+    torch.cuda.synchronize()
+    ctx.set_int("tc_bn", tc_bn), ctx.set_int("gemv_splitk", 1)
+    try:
+        ctx.check(ctx.lib.kf_linear(ctx.h, _ptr(yr), C.byref(dw), _ptr(x), M, kf.KF_EPI_RESIDUAL, _ptr(yr)), "residual")
+        ctx.check(ctx.lib.kf_linear(ctx.h, _ptr(yf), C.byref(dw), _ptr(x), M, kf.KF_EPI_F32, None), "f32")
+        ctx.sync()
+    finally:
+        ctx.set_int("tc_bn", 0), ctx.set_int("gemv_splitk", 0)
+    assert bool(((yf - acc).abs() <= tiny).all())
+    assert bool(((yr.float() - (r.float() + acc)).abs() <= eps * (acc.abs() + (r.float() + acc).abs()) * 1.02 + tiny).all())
+
+
 @pytest.mark.parametrize("tc_bn", [0, 64])
 def test_tc_split_as_asked(ctx, tc_bn):
     """gemv_splitk is taken as it is, up to the number of k stages (K = 5120 in 4 bits: 20 of 256), and so is the token tile beside it.  Sums of parts differ in
