@@ -8,11 +8,12 @@
 //     form y = g sigmoid(alpha g) (u + shift) with g = min(A x, limit), u = clamp(B x, -limit, limit);
 //   * "batch" form for a handful of rows: several weights, each with an input and an output of its own, in one launch.
 // A warp-per-output GEMV for a handful of rows (decode: every weight row is read once, 16-byte loads when the row length allows) and 64 x 64 shared-memory tile
-// kernels for panels: a cp.async ring with mma.sync m16n8k16 for bf16 activations, FFMA for float ones (which also takes bf16 rows of odd lengths).
+// kernels for panels: a cp.async ring with tcgen05 for bf16 activations, FFMA for float ones (mma.sync for bf16 rows of odd lengths).
 // No reference equivalent: the reference's SLP::Forw hands every shape to cuBLASLt (src/Device/CUDA/NeuronFuse.cu:305-381).
 #include <algorithm>
 
 #include "kf_common.cuh"
+#include "kf_tc.cuh"
 
 namespace {
 
@@ -457,135 +458,155 @@ __global__ void __launch_bounds__(256) kf_lin_tile_any_kernel(LinArgs a) {
     }
 }
 
-// bf16 activations: 64 slots x 64 outputs (of either weight, DUAL) per CTA, k in steps of 64 through a ring of stages filled by cp.async, 8 warps as 4 (m) x 2 (n) on
-// mma.sync m16n8k16.  The weights of a routed panel are the traffic (64 experts of 2 x 1408 x 2048: 738 MB), so the ring is there to keep bytes on their way: two
-// CTAs per SM, each with three of four 24 KB stages in flight (DUAL; 144 KB an SM, 96 of them weights) or five of six 16 KB stages (160 KB, 80 of them weights).
-// Fetching the next step through registers had 24 KB on its way: 291 us for those, 0.39 of the HBM rate, 177 here (0.64); the down projections 194 and 113 (0.50).  A warp whose 16 slots lie past the group's end only helps to load.
-// Rows lie as 128 bytes, 16-byte chunk c of row r at c ^ (r & 7): ldmatrix without conflicts.  A weight that is not 16-byte aligned (the table is on the device: only
-// the kernel sees it) is fetched element by element into the same places.
-template <bool DUAL>
-struct TileRing {
-    static constexpr int BK = 64, TILE = 64 * BK * 2, STAGE = (DUAL ? 3 : 2) * TILE, N = DUAL ? 4 : 6;
-    static constexpr size_t SMEM = (size_t)N * STAGE;
-};
+// bf16 activations: 128 weight rows (DUAL: 64 of either weight) x 64 slots per CTA on tcgen05, k in steps of 64.  The weights of a routed panel are the traffic (64
+// experts of 2 x 1408 x 2048: 738 MB), 48 slots each, so the CTA is built to keep bytes on their way: two CTAs per SM with four 24 KB stages each, filled by
+// cp.async (the table of weights is on the device, the rows of x are gathered: no tensor map), two to three of them in flight, 96 KB or more an SM; nothing
+// but the copies and one thread's matrix instructions in the loop.  On mma.sync, whose fragments went through ldmatrix, shared memory was as busy as DRAM (8
+// warps of 16 x 32 read 82 KB a step of 24 KB): 186 us for those and 118 for the down projections, 132 (0.85 of the copy rate) and 75 (0.75) here.
+// Rows lie as 128 bytes, 16-byte chunk c of row r at c ^ (r & 7): the K-major SWIZZLE_128B layout of the matrix descriptors.  A weight that is not 16-byte
+// aligned (only the kernel sees it) is fetched element by element into the same places.
+constexpr int kTileRows = 128, kTileStages = 4, kTileStage = (kTileRows + BM) * 128;  // weight rows, then slots, 128 bytes each
+constexpr size_t kTileSmem = (size_t)kTileStages * kTileStage + 1024;
+static_assert(kTileStages * kTileStage >= BM * kTileRows * 4, "the ring takes the fp32 results");
 __device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool ok) {
     asm volatile("cp.async.cg.shared.global.L2::256B [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
 }
 template <bool DUAL>
 __global__ void __launch_bounds__(256, 2) kf_lin_tile_kernel(LinArgs a) {
-    using R = TileRing<DUAL>;
-    constexpr int BK = R::BK;
-    extern __shared__ __align__(128) uint8_t tile_smem[];
-    const uint32_t ring = (uint32_t)__cvta_generic_to_shared(tile_smem);
+    constexpr int BK = 64, NS = kTileStages, OUTS = DUAL ? 64 : 128;  // outputs of a CTA
+    extern __shared__ uint8_t tile_raw[];
+    __shared__ uint64_t done[NS];  // the matrix instructions that read a stage have finished
+    __shared__ uint32_t tmem_smem;
+    uint8_t* const tile_smem = tile_raw + ((1024u - smem_u32(tile_raw)) & 1023u);
+    const uint32_t ring = smem_u32(tile_smem);
     const int g  = blockIdx.z;
     const int lo = a.offsets ? a.offsets[g] : 0, hi = a.offsets ? a.offsets[g + 1] : a.M;
-    const int n0 = blockIdx.x * BN, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int wm = warp & 3, wn = warp >> 2;             // warp tile: rows wm * 16, columns wn * 32
-    const int lr = tid >> 3, lc = tid & 7;                // this thread's loads: rows lr and lr + 32, chunk lc of each tile
+    const int n0 = blockIdx.x * OUTS, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (lo + (int)blockIdx.y * BM >= hi) return;  // the whole CTA: nothing to do
+    if (tid == 0) {
+        for (int i = 0; i < NS; i++) mbar_init(&done[i], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 64;" ::"r"(smem_u32(&tmem_smem)) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_smem;
+    const int lr = tid >> 3, lc = tid & 7;  // this thread's loads: rows lr, lr + 32, ... of either operand, chunk lc
     const int steps = (a.K + BK - 1) / BK;
+    const uint16_t* W[2] = {a.Wt0 ? a.Wt0[g] : a.W0, DUAL ? (a.Wt1 ? a.Wt1[g] : a.W1) : nullptr};
+    const bool wvec = ((uintptr_t)W[0] & 15) == 0 && (!DUAL || ((uintptr_t)W[1] & 15) == 0);
+    uint32_t it = 0;  // k-steps of the CTA so far: stage it % NS
     // a CTA walks the slot tiles blockIdx.y, blockIdx.y + gridDim.y, ... of its group: the grid is sized for the average group, not the worst
     for (int m0 = lo + blockIdx.y * BM; m0 < hi; m0 += gridDim.y * BM) {
-        const uint16_t* W[2] = {a.Wt0 ? a.Wt0[g] : a.W0, DUAL ? (a.Wt1 ? a.Wt1[g] : a.W1) : nullptr};
-        const bool wvec = ((uintptr_t)W[0] & 15) == 0 && (!DUAL || ((uintptr_t)W[1] & 15) == 0);
-        const uint16_t* xr[2];
-        bool xok[2], wok[2];
-        size_t woff[2];
+        const uint16_t *xr[2], *wr[4];
+        bool xok[2], wok[4];
 #pragma unroll
         for (int i = 0; i < 2; i++) {
-            const int s = m0 + lr + 32 * i, n = n0 + lr + 32 * i;
-            xok[i]  = s < hi, wok[i] = n < a.N;
-            xr[i]   = (const uint16_t*)a.x + (size_t)(xok[i] ? (a.src_row ? a.src_row[s] : s) : 0) * a.ldx + lc * 8;
-            woff[i] = (size_t)(wok[i] ? n : 0) * a.K + lc * 8;
+            const int s = m0 + lr + 32 * i;
+            xok[i] = s < hi;
+            xr[i]  = (const uint16_t*)a.x + (size_t)(xok[i] ? (a.src_row ? a.src_row[s] : s) : 0) * a.ldx + lc * 8;
         }
-        auto load = [&](int step) {
-            const uint32_t st = ring + (uint32_t)(step % R::N) * R::STAGE;
-            const int k       = step * BK + lc * 8;
-            const bool kok    = k < a.K;  // K is a multiple of 8
+#pragma unroll
+        for (int i = 0; i < 4; i++) {  // rows 0 .. 127 of the tile: DUAL 64 of W[0], then the same 64 of W[1]
+            const int n = n0 + (DUAL ? (lr + 32 * i) & 63 : lr + 32 * i);
+            wok[i] = n < a.N;
+            wr[i]  = W[DUAL ? i >> 1 : 0] + (size_t)(wok[i] ? n : 0) * a.K + lc * 8;
+        }
+        auto load = [&](int step, uint32_t stage) {
+            const uint32_t st = ring + stage * kTileStage;
+            const bool kok    = step * BK + lc * 8 < a.K;  // K is a multiple of 8
             const size_t kof  = (size_t)(kok ? step * BK : 0);
 #pragma unroll
-            for (int i = 0; i < 2; i++) {
-                const int r        = lr + 32 * i;
+            for (int i = 0; i < 4; i++) {
+                const int r = lr + 32 * i;
                 const uint32_t dst = st + (uint32_t)(r * 128 + ((lc ^ (r & 7)) << 4));
-                cp16(dst, xok[i] && kok ? xr[i] + kof : (const uint16_t*)a.x, xok[i] && kok);
-#pragma unroll
-                for (int w = 0; w < (DUAL ? 2 : 1); w++) {
-                    const bool ok = wok[i] && kok;
-                    if (wvec) {
-                        cp16(dst + (1 + w) * R::TILE, ok ? W[w] + woff[i] + kof : W[w], ok);
-                    } else {
-                        uint16_t* d = reinterpret_cast<uint16_t*>(tile_smem + (dst - ring) + (1 + w) * R::TILE);
-                        for (int e = 0; e < 8; e++) d[e] = ok ? W[w][woff[i] + kof + e] : (uint16_t)0;
-                    }
+                const bool ok = wok[i] && kok;
+                if (wvec) {
+                    cp16(dst, ok ? wr[i] + kof : W[0], ok);
+                } else {
+                    uint16_t* d = reinterpret_cast<uint16_t*>(tile_smem + (dst - ring));
+                    for (int e = 0; e < 8; e++) d[e] = ok ? wr[i][kof + e] : (uint16_t)0;
                 }
+            }
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const int r = lr + 32 * i;
+                cp16(st + (uint32_t)(kTileRows * 128 + r * 128 + ((lc ^ (r & 7)) << 4)), xok[i] && kok ? xr[i] + kof : (const uint16_t*)a.x, xok[i] && kok);
             }
         };
-        float acc[DUAL ? 2 : 1][16];
+        const uint32_t it0 = it;
 #pragma unroll
-        for (int w = 0; w < (DUAL ? 2 : 1); w++)
-#pragma unroll
-            for (int i = 0; i < 16; i++) acc[w][i] = 0.f;
-#pragma unroll
-        for (int i = 0; i < R::N - 1; i++) {
-            if (i < steps) load(i);
+        for (int i = 0; i < NS - 1; i++) {  // the stages are free: the slot tile before this one ended behind its last matrix instruction
+            if (i < steps) load(i, (it0 + i) % NS);
             asm volatile("cp.async.commit_group;" ::: "memory");
         }
-        const bool busy = m0 + wm * 16 < hi;
-        for (int step = 0; step < steps; step++) {
-            asm volatile("cp.async.wait_group %0;" ::"n"(R::N - 2) : "memory");
-            __syncthreads();  // this step's bytes are there for everybody, and everybody has left the stage that is filled next
-            if (step + R::N - 1 < steps) load(step + R::N - 1);
+        const int cols = min(BM, (hi - m0 + 15) & ~15);  // slots that the matrix instructions see
+        const uint32_t idesc = make_idesc_bf16(cols);
+        for (int step = 0; step < steps; step++, it++) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(NS - 2) : "memory");
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // what this thread has copied or stored is for the tensor cores to read
+            __syncthreads();
+            if (warp == 0) {
+                const uint32_t st = ring + (it % NS) * kTileStage;
+                const uint64_t ad = make_desc_sw128(st), bd = make_desc_sw128(st + kTileRows * 128);
+                tc_fence_after();
+#pragma unroll
+                for (int k = 0; k < BK / 16; k++) umma_ss(tmem, ad + (uint64_t)(2 * k), bd + (uint64_t)(2 * k), idesc, (step > 0 || k > 0) ? 1u : 0u);
+                umma_commit_a(smem_u32(&done[it % NS]));
+            }
+            if (step + NS - 1 < steps) {  // into the stage of the step before this one
+                if (step > 0) mbar_wait(&done[(it - 1) % NS], ((it - 1) / NS) & 1);
+                load(step + NS - 1, (it + NS - 1) % NS);
+            }
             asm volatile("cp.async.commit_group;" ::: "memory");
-            if (!busy) continue;
-            const uint8_t* xs = tile_smem + (size_t)(step % R::N) * R::STAGE;
-            auto at = [](const uint8_t* base, int row, int c) { return base + row * 128 + ((c ^ (row & 7)) << 4); };
+        }
+        mbar_wait(&done[(it - 1) % NS], ((it - 1) / NS) & 1);  // all of them: they finish in order
+        tc_fence_after();
+        // ---- accumulator -> shared memory [slot][row] -> y, the outputs of a slot side by side ----
+        float* res = reinterpret_cast<float*>(tile_smem);
+        const int row = (warp & 3) * 32 + lane;
+        for (int c0 = (warp >> 2) * 16; c0 < cols; c0 += 32) {
+            uint32_t v[16];
+            tmem_ld16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0, v);
 #pragma unroll
-            for (int kk = 0; kk < BK / 16; kk++) {
-                uint32_t af[4];
-                ldsm_x4(af, at(xs, wm * 16 + (lane & 15), kk * 2 + (lane >> 4)));
+            for (int j = 0; j < 16; j++) res[(c0 + j) * kTileRows + row] = __uint_as_float(v[j]);
+        }
+        tc_fence_before();
+        __syncthreads();
+        const bool quads = a.ldy % 4 == 0 && ((uintptr_t)a.y & 15) == 0;
+        for (int i = tid; i < (min(hi, m0 + BM) - m0) * (OUTS / 4); i += 256) {
+            const int t = i / (OUTS / 4), c = (i % (OUTS / 4)) * 4, n = n0 + c;
+            if (n >= a.N) continue;
+            float v[4];
 #pragma unroll
-                for (int j = 0; j < 4; j += 2) {
-                    const int nr = wn * 32 + j * 8 + (lane & 7) + (lane >> 4) * 8, c = kk * 2 + ((lane >> 3) & 1);
-#pragma unroll
-                    for (int w = 0; w < (DUAL ? 2 : 1); w++) {
-                        uint32_t bf[4];
-                        ldsm_x4(bf, at(xs + (1 + w) * R::TILE, nr, c));
-                        mma_bf16_16816(&acc[w][j * 4], af, bf);
-                        mma_bf16_16816(&acc[w][(j + 1) * 4], af, bf + 2);
-                    }
-                }
+            for (int e = 0; e < 4; e++) {
+                const float r0 = res[t * kTileRows + c + e];
+                v[e] = DUAL ? lin_pair(a, r0, res[t * kTileRows + (DUAL ? 64 : 0) + c + e]) : lin_act(r0, a.act);
+            }
+            const size_t at = (size_t)(m0 + t) * a.ldy + n;
+            const bool four = quads && n + 3 < a.N;
+            if ((DUAL || a.act) && a.out_act == 1) {
+                uint16_t* y = (uint16_t*)a.y + at;
+                if (four) *reinterpret_cast<uint2*>(y) = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]));
+                else
+                    for (int e = 0; e < 4 && n + e < a.N; e++) y[e] = f32_to_bf16_bits(v[e]);
+            } else {
+                float* y = (float*)a.y + at;
+                if (four) *reinterpret_cast<float4*>(y) = make_float4(v[0], v[1], v[2], v[3]);
+                else
+                    for (int e = 0; e < 4 && n + e < a.N; e++) y[e] = v[e];
             }
         }
-        const int gr = lane >> 2, tg = lane & 3;
-        const bool pairs = a.ldy % 2 == 0 && ((uintptr_t)a.y & 7) == 0;
-#pragma unroll
-        for (int j = 0; j < 4; j++)
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int s = m0 + wm * 16 + gr + 8 * h, n = n0 + wn * 32 + j * 8 + tg * 2;
-                if (s >= hi || n >= a.N) continue;
-                float v[2];
-#pragma unroll
-                for (int e = 0; e < 2; e++) v[e] = DUAL ? lin_pair(a, acc[0][j * 4 + 2 * h + e], acc[DUAL ? 1 : 0][j * 4 + 2 * h + e]) : lin_act(acc[0][j * 4 + 2 * h + e], a.act);
-                const size_t at = (size_t)s * a.ldy + n;
-                const bool two  = n + 1 < a.N;
-                if ((DUAL || a.act) && a.out_act == 1) {
-                    uint16_t* y = (uint16_t*)a.y + at;
-                    if (two && pairs) *reinterpret_cast<uint32_t*>(y) = pack_bf16x2(v[0], v[1]);
-                    else {
-                        y[0] = f32_to_bf16_bits(v[0]);
-                        if (two) y[1] = f32_to_bf16_bits(v[1]);
-                    }
-                } else {
-                    float* y = (float*)a.y + at;
-                    if (two && pairs) *reinterpret_cast<float2*>(y) = make_float2(v[0], v[1]);
-                    else {
-                        y[0] = v[0];
-                        if (two) y[1] = v[1];
-                    }
-                }
-            }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();  // the ring is free for the next slot tile
+        __syncthreads();  // the ring and the accumulator are free for the next slot tile
+    }
+    if (warp == 0) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 64;" ::"r"(tmem) : "memory");
     }
 }
 
@@ -601,10 +622,11 @@ int launch(kf_ctx* ctx, const LinArgs& a, int slots, int groups, bool gemv) {
         if (sizeof(TA) == 2 && a.K % 8 == 0 && a.ldx % 8 == 0 && ((uintptr_t)a.x & 15) == 0) {  // rows that can be fetched 16 bytes at a time
             static bool set[kf_ctx::kMaxDevices] = {};  // function attributes are per device (one flag per instantiation and device)
             if (!set[ctx->device]) {
-                KF_CUDA(ctx, cudaFuncSetAttribute(kf_lin_tile_kernel<DUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TileRing<DUAL>::SMEM));
+                KF_CUDA(ctx, cudaFuncSetAttribute(kf_lin_tile_kernel<DUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileSmem));
                 set[ctx->device] = true;
             }
-            kf_lin_tile_kernel<DUAL><<<grid, 256, TileRing<DUAL>::SMEM, ctx->stream>>>(a);
+            const int outs = DUAL ? kTileRows / 2 : kTileRows;
+            kf_lin_tile_kernel<DUAL><<<dim3((a.N + outs - 1) / outs, gy, groups), 256, kTileSmem, ctx->stream>>>(a);
         } else {
             kf_lin_tile_any_kernel<TA, DUAL><<<grid, 256, 0, ctx->stream>>>(a);
         }
