@@ -804,10 +804,11 @@ __global__ void __launch_bounds__(128, KF_PF_MINB) kf_attn_prefill_kernel(uint16
     }
 }
 
-// ---- QK-norm + RoPE + K/V append for big panels: one WARP per (token, head) (the block-per-head kernel of ops.cu needs 150 K tiny
-// blocks for a 2048-token panel and is scheduling bound: 80 us against 15 us here).  Same arithmetic; the sum of squares is taken in
-// warp-butterfly order as in the fused decode kernel.
-template <int DPL>
+// ---- QK-norm + RoPE + K/V append for big panels: one WARP per R rows (heads) of a token (the block-per-head kernel of ops.cu needs 150 K tiny
+// blocks for a 2048-token panel and is scheduling bound).  Same arithmetic; the sum of squares is taken in warp-butterfly order as in the fused decode
+// kernel.  Bound by latency, then by L2: the rows of a warp are fetched together and share the token's angles and the weights (1999 tokens of 32 + 8
+// heads: 24.0 us with one row a warp, 22.6 with four; few rows keep one).
+template <int DPL, int R>
 __global__ void __launch_bounds__(256) kf_qknorm_rope_kv_warp_kernel(uint16_t* __restrict__ q, const uint16_t* __restrict__ k,
                                                                      const uint16_t* __restrict__ v, const uint16_t* __restrict__ qw,
                                                                      const uint16_t* __restrict__ kw, uint16_t* __restrict__ kcache,
@@ -815,31 +816,53 @@ __global__ void __launch_bounds__(256) kf_qknorm_rope_kv_warp_kernel(uint16_t* _
                                                                      const int32_t* __restrict__ pos_dev, int M, int n_head, int n_kv, float eps,
                                                                      size_t seq_stride) {
     constexpr int HD = DPL * 32;
+    kf_grid_dependency_wait();
     kf_grid_launch_dependents();  // the attention behind us may set itself up; it waits for our end before it reads anything
     const int lane = threadIdx.x & 31;
+    const int per_tok = n_head + n_kv, warps = (per_tok + R - 1) / R;  // warps of a token
     const long long wid = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
-    const int per_tok   = n_head + n_kv;
-    if (wid >= (long long)M * per_tok) return;
-    const int m = (int)(wid / per_tok), h = (int)(wid % per_tok);
+    if (wid >= (long long)M * warps) return;
+    const int m = (int)(wid / warps), h0 = (int)(wid % warps) * R;
     const int pos = pos_dev[m];
-    const float2* cs_row = table + (size_t)pos * (HD / 2);
-    const bool is_q = h < n_head;
-    const int kvh   = h - n_head;
-    const uint16_t* src = is_q ? q + ((size_t)m * n_head + h) * HD : k + ((size_t)m * n_kv + kvh) * HD;
-    uint16_t* dst       = is_q ? q + ((size_t)m * n_head + h) * HD : kcache + (size_t)m * seq_stride + ((size_t)pos * n_kv + kvh) * HD;
-    float o[DPL];
-    norm_rope_row<DPL>(o, src, is_q ? qw : kw, cs_row, lane, eps);
-    if constexpr (DPL == 4)
-        *reinterpret_cast<uint2*>(dst + lane * 4) = make_uint2(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]));
-    else
-        *reinterpret_cast<uint32_t*>(dst + lane * 2) = pack_bf16x2(o[0], o[1]);
-    if (!is_q) {  // the V row of this kv head
-        const uint16_t* vs = v + ((size_t)m * n_kv + kvh) * HD + lane * DPL;
-        uint16_t* vd       = vcache + (size_t)m * seq_stride + ((size_t)pos * n_kv + kvh) * HD + lane * DPL;
-        if constexpr (DPL == 4)
-            *reinterpret_cast<uint2*>(vd) = *reinterpret_cast<const uint2*>(vs);
-        else
-            *reinterpret_cast<uint32_t*>(vd) = *reinterpret_cast<const uint32_t*>(vs);
+    float x[R][DPL], vv[R][DPL], w[2][DPL];
+    float2 cs[DPL];
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        const int h = min(h0 + r, per_tok - 1);
+        load_row<DPL>(x[r], (h < n_head ? q + ((size_t)m * n_head + h) * HD : k + ((size_t)m * n_kv + h - n_head) * HD) + lane * DPL);
+        if (h >= n_head) load_row<DPL>(vv[r], v + ((size_t)m * n_kv + h - n_head) * HD + lane * DPL);
+    }
+    if (qw && h0 < n_head) load_row<DPL>(w[0], qw + lane * DPL);
+    if (kw && h0 + R > n_head) load_row<DPL>(w[1], kw + lane * DPL);
+#pragma unroll
+    for (int d = 0; d < DPL; d++) cs[d] = table[(size_t)pos * (HD / 2) + (lane & 15) * DPL + d];
+    auto store = [&](uint16_t* dst, const float (&o)[DPL]) {
+        if constexpr (DPL == 4) *reinterpret_cast<uint2*>(dst + lane * 4) = make_uint2(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]));
+        else *reinterpret_cast<uint32_t*>(dst + lane * 2) = pack_bf16x2(o[0], o[1]);
+    };
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        const int h = h0 + r;
+        if (h >= per_tok) return;
+        const bool is_q = h < n_head;
+        if (is_q ? qw != nullptr : kw != nullptr) {
+            float ss = 0.f;
+#pragma unroll
+            for (int d = 0; d < DPL; d++) ss = fmaf(x[r][d], x[r][d], ss);
+            ss            = warp_sum(ss);
+            const float s = 1.0f / sqrtf(fmaf(ss, 1.0f / (float)HD, eps));
+#pragma unroll
+            for (int d = 0; d < DPL; d++) x[r][d] = bf16_bits_to_f32(f32_to_bf16_bits((x[r][d] * s) * (is_q ? w[0][d] : w[1][d])));  // the norm kernel's bf16 output
+        }
+        float o[DPL];
+#pragma unroll
+        for (int d = 0; d < DPL; d++) {  // half-split rotation: dim j pairs with j + HD/2, held by lane ^ 16
+            const float other = __shfl_xor_sync(0xffffffffu, x[r][d], 16);
+            o[d]              = lane < 16 ? fmaf(x[r][d], cs[d].x, -(other * cs[d].y)) : fmaf(other, cs[d].y, x[r][d] * cs[d].x);
+        }
+        const size_t row = (size_t)m * seq_stride + ((size_t)pos * n_kv + h - n_head) * HD;
+        store(is_q ? q + ((size_t)m * n_head + h) * HD : kcache + row, o);
+        if (!is_q) store(vcache + row, vv[r]);  // the V row of this kv head
     }
 }
 }  // namespace
@@ -1132,16 +1155,16 @@ extern "C" int kf_attn_sigmoid_prefill(kf_ctx* ctx, void* out, int ldo, const vo
 // warp-per-head variant of kf_qknorm_rope_kvappend for big panels (called from ops.cu); hd 64 / 128 only
 int kf_qknorm_rope_kv_warp(kf_ctx* ctx, void* q, const void* k, const void* v, const void* qw, const void* kw, void* kcache, void* vcache,
                            const void* table, const int32_t* pos_dev, int M, int n_head, int n_kv, int hd, float eps, size_t seq_stride) {
-    const long long warps = (long long)M * (n_head + n_kv);
+    // four rows a warp from two blocks of one-row warps per SM on; below that the GPU would not be full
+    const bool four = (long long)M * (n_head + n_kv) >= 16ll * ctx->sm_count;
+    const long long warps = (long long)M * (four ? (n_head + n_kv + 3) / 4 : n_head + n_kv);
     const unsigned blocks = (unsigned)((warps + 7) / 8);
-    if (hd == 128)
-        kf_qknorm_rope_kv_warp_kernel<4><<<blocks, 256, 0, ctx->stream>>>((uint16_t*)q, (const uint16_t*)k, (const uint16_t*)v, (const uint16_t*)qw,
-                                                                          (const uint16_t*)kw, (uint16_t*)kcache, (uint16_t*)vcache, (const float2*)table,
-                                                                          pos_dev, M, n_head, n_kv, eps, seq_stride);
-    else
-        kf_qknorm_rope_kv_warp_kernel<2><<<blocks, 256, 0, ctx->stream>>>((uint16_t*)q, (const uint16_t*)k, (const uint16_t*)v, (const uint16_t*)qw,
-                                                                          (const uint16_t*)kw, (uint16_t*)kcache, (uint16_t*)vcache, (const float2*)table,
-                                                                          pos_dev, M, n_head, n_kv, eps, seq_stride);
+    auto go = [&](auto kern) {
+        return kf_launch_pdl(ctx, kern, dim3(blocks), dim3(256), 0, (uint16_t*)q, (const uint16_t*)k, (const uint16_t*)v, (const uint16_t*)qw, (const uint16_t*)kw,
+                             (uint16_t*)kcache, (uint16_t*)vcache, (const float2*)table, pos_dev, M, n_head, n_kv, eps, seq_stride);
+    };
+    if (hd == 128) KF_CUDA(ctx, four ? go(kf_qknorm_rope_kv_warp_kernel<4, 4>) : go(kf_qknorm_rope_kv_warp_kernel<4, 1>));
+    else KF_CUDA(ctx, four ? go(kf_qknorm_rope_kv_warp_kernel<2, 4>) : go(kf_qknorm_rope_kv_warp_kernel<2, 1>));
     KF_LAUNCH_CHECK(ctx);
     return KF_OK;
 }

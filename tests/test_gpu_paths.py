@@ -557,7 +557,7 @@ def test_maps_of_steps_leave_those_of_weights(ctx):
 
 
 # ---------------------------------------------------------------------------------------------- tile matmul over expert-sorted slots
-@pytest.mark.parametrize("N,K", [(64, 64), (65, 72), (8, 8), (130, 200), (192, 448), (33, 512)])
+@pytest.mark.parametrize("N,K", [(64, 64), (65, 72), (8, 8), (130, 200), (192, 448), (33, 512), (257, 320)])
 @pytest.mark.parametrize("counts", [(64, 0, 1, 63, 65, 17), (200, 3, 0, 0, 1, 0), (16, 16, 16, 16, 16, 16)])
 @pytest.mark.parametrize("shift", [0, 1])
 def test_grouped_tiles(ctx, N, K, counts, shift):
@@ -601,6 +601,41 @@ def test_norm_of_several_tokens(ctx, typ, M, K):
         ws = [make_q(ctx, typ, n, K, n)[0] for n in (256, 128)]
     for a, b in zip(kf.rmsnorm_linear(ctx, ws, x, nw, M, 1e-6), kf.linear_multi(ctx, ws, xn, M)):
         assert np.array_equal(a.numpy(np.uint16), b.numpy(np.uint16))
+
+
+@pytest.mark.parametrize("typ", [kf.KF_T_Q4, kf.KF_T_SIGN, kf.KF_T_BINARY])
+@pytest.mark.parametrize("M,K", [(9, 128), (33, 2048), (10, 2176), (17, 4224), (66, 8192), (11, 8320)])
+def test_norm_in_front_of_panels(ctx, typ, M, K):
+    """RMSNorm written in the weights' k order has the bits of RMSNorm and the reordering, with rows that stay in registers (up to 8192) and that do not."""
+    x, nw = kf.fill_normal(ctx, M * K, M * K, 2.0), kf.fill_normal(ctx, K, 3, 0.5)
+    xn = kf.rmsnorm(ctx, x, nw, M, K, 1e-6)
+    ws = [make_q(ctx, typ, n, K, n)[0] for n in (256, 128)]
+    for a, b in zip(kf.rmsnorm_linear(ctx, ws, x, nw, M, 1e-6), kf.linear_multi(ctx, ws, xn, M)):
+        assert np.array_equal(a.numpy(np.uint16), b.numpy(np.uint16))
+
+
+@pytest.mark.parametrize("hd,n_head,n_kv,M", [(128, 32, 8, 300), (128, 6, 3, 1001), (64, 5, 1, 800), (64, 14, 2, 513)])
+@pytest.mark.parametrize("norm", [True, False])
+def test_qknorm_rows_per_warp(ctx, hd, n_head, n_kv, M, norm):
+    """Four rows of a token per warp give the bits of one row per warp (calls of 16 tokens)."""
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(M)
+    q, k, v = (torch.randn(M, n, hd, generator=g, device="cuda").bfloat16() for n in (n_head, n_kv, n_kv))
+    w = [torch.randn(hd, generator=g, device="cuda").bfloat16() for _ in range(2)]
+    table = torch.randn(M + 40, hd, generator=g, device="cuda")
+    pos = torch.randperm(M + 40, generator=g, device="cuda")[:M].int()
+    outs, used = [], M // 16 * 16
+    for step in (used, 16):
+        qq, kc, vc = q.clone(), torch.zeros(M + 40, n_kv, hd, device="cuda").bfloat16(), torch.zeros(M + 40, n_kv, hd, device="cuda").bfloat16()
+        torch.cuda.synchronize()
+        for m in range(0, used, step):
+            ctx.check(ctx.lib.kf_qknorm_rope_kvappend(ctx.h, _ptr(qq[m:]), _ptr(k[m:]), _ptr(v[m:]), _ptr(w[0]) if norm else None, _ptr(w[1]) if norm else None, _ptr(kc), _ptr(vc),
+                                                      _ptr(table), _ptr(pos[m:]), step, n_head, n_kv, hd, M + 40, 1e-6, 0), "qknorm")
+        ctx.sync()
+        outs.append((qq, kc, vc))
+    for a, b in zip(*outs):
+        assert torch.equal(a, b)
 
 
 # ---------------------------------------------------------------------------------------------- routing of a panel, weighted sum of the experts
