@@ -296,6 +296,7 @@ template <int FMT, int BN>
 struct Rings {
     static constexpr bool A_TMEM = FMT != TF_BF16;
     static constexpr int U       = BN <= 128 ? 2 : 1;  // k-blocks per ring stage: below 256 tokens the barrier traffic, not the MMA, paces a k-block
+    static constexpr bool HELP   = BN >= 128;  // the producers help with the last item: below that their way to the barrier takes longer than their share of the work (12 tokens x 3072 x 6144 + 0.9 us)
     static constexpr int NACC    = (A_TMEM && BN == 256) ? 1 : 2;
     static constexpr int A_BYTES = A_TMEM ? 0 : BM * 128;
     static constexpr int SUB     = A_BYTES + BN * 128;  // one k-block of a stage: [A tile (bf16 weights only)][B tile]
@@ -394,6 +395,8 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
     __shared__ uint64_t a_full[SA1], a_empty[SA1], b_full[SB], b_empty[SB], raw_full[RS1], raw_empty[RS1], tmem_full[NACC], tmem_empty[NACC];
     __shared__ uint32_t tmem_base_smem;
     __shared__ int last_flag;
+    __shared__ Item s_last;  // the CTA's last item, decoded while nobody waits for it
+    const int last_ait = (p.n_items - 1 - (int)blockIdx.x) / (int)gridDim.x, last_item = blockIdx.x + last_ait * gridDim.x;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
@@ -432,7 +435,6 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    if (warp == kXWarp && lane == 0) asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_x) : "memory");
     // producers: this thread's row of zero / step; scale / zero of the current group and of the next two (register queue; the loads run 1-2 groups ahead of
     // their use).  Those of the first item are asked for here: they take a DRAM round trip, as long as the first weights
     const int prow = (warp & 3) * 32 + lane, gpr = (p.K >> 7) >> p.gshift;
@@ -451,6 +453,7 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
             zq2 = __ldg(zrow + g2), sq2 = __ldg(srow + g2);
         }
     };
+    if (tid == kEpiWarp0 * 32) s_last = decode_item<KBR>(p, last_item);
     if (warp < kProducerWarps) fetch_gama(decode_item<KBR>(p, blockIdx.x));
     tc_fence_before();
     __syncthreads();
@@ -459,12 +462,12 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
     kf_grid_launch_dependents();
 
     // ============ the end of an item: TMEM -> registers -> output buffer in shared memory -> Y in 16-byte accesses, or partial sums of a split.  Runs on the
-    // four epilogue warps while the other roles work on the next item, and on these and the eight producer warps (three to a quarter of the lanes) for the
-    // CTA's last item, where nothing else is left to do.  Four warps took 4 us for the 256 tokens of an item and 10 with SwiGLU, in front of which the matrix
+    // four epilogue warps while the other roles work on the next item, and from 128 tokens on these and the eight producer warps (three to a quarter of the lanes)
+    // for the CTA's last item, where nothing else is left to do.  Four warps took 4 us for the 256 tokens of an item and 10 with SwiGLU, in front of which the matrix
     // instructions of the next item waited: there is no second accumulator beside 256 columns and the A ring (4-bit SwiGLU 51200 x 5120 at 2048 tokens 842 -> 757 us,
     // 6144 x 1024 at 700, one item per CTA, 22.2 -> 17.8) ============
-    const int last_ait  = (p.n_items - 1 - (int)blockIdx.x) / (int)gridDim.x, last_item = blockIdx.x + last_ait * gridDim.x;
-    const bool finisher = warp < kProducerWarps || warp >= kEpiWarp0;
+    constexpr int NFIN  = C::HELP ? 384 : 128;  // threads that finish the last item
+    const bool finisher = warp >= kEpiWarp0 || (C::HELP && warp < kProducerWarps);
     const int fin_t     = warp < kProducerWarps ? 128 + tid : tid - kEpiWarp0 * 32;  // 0 .. 127: epilogue warps
     const bool f32out   = p.epilogue == 4;
     constexpr int kRes  = 4;  // residual pieces in flight per thread
@@ -540,11 +543,9 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
         const bool direct = p.splits == 1 && p.staged;
         uint4 res[kRes];
         if (direct && p.epilogue == 1) fetch_res(res, w, m0, N, 0, min(cnt, round), 0, nthr);
-        if (warp >= kEpiWarp0) {
-            if (NACC == 2 && nthr == 128) mbar_wait_sleepy(&tmem_full[buf], (ait / NACC) & 1);  // a whole main loop away: poll politely
-            else mbar_wait(&tmem_full[buf], (ait / NACC) & 1);
-        }
-        epi_bar_sync(nthr);  // the output buffer is free; producers learn here that the accumulator is complete
+        // one warp polls, a whole main loop ahead and politely (four took issue slots from the producers: 6144 x 3072 at 12 tokens 18.3 -> 19.1 us); the others learn it here
+        if (warp == kEpiWarp0) mbar_wait_sleepy(&tmem_full[buf], (ait / NACC) & 1, NACC == 2 && nthr == 128 ? 200 : 20);
+        epi_bar_sync(nthr);  // the output buffer is free, the accumulator complete
         tc_fence_after();
         auto release = [&]() {  // the accumulator buffer may be overwritten by the next item
             tc_fence_before();
@@ -839,9 +840,9 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
             finish(w, ait, (warp - kEpiWarp0) * 32 + lane, 128);
         }
     }
-    if (finisher) {  // the last item: all twelve warps
+    if (finisher) {  // the last item
         if (warp < kProducerWarps) kf_grid_dependency_wait();
-        finish(decode_item<KBR>(p, last_item), last_ait, fin_t, 384);
+        finish(s_last, last_ait, fin_t, NFIN);
     }
     // ============ split over a cluster: every CTA has its partial sums in shared memory and adds up its share of the tokens, in the order of the parts.  Takes
     // 3 us, of which the reads from the other CTAs are half; through global memory, where the last CTA to arrive did it all, 4-bit 4096 x 12288 at 300 tokens
@@ -850,7 +851,7 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
         __syncwarp();
         cluster_arrive(), cluster_wait();
         if (finisher) {
-            const Item w  = decode_item<KBR>(p, last_item);
+            const Item w  = s_last;
             const int m0 = w.m0 * BN, cnt = min(BN, p.M - m0), N = p.Nw[w.wi];
             const int t0 = cnt * w.z / p.splits, t1 = cnt * (w.z + 1) / p.splits;
             const int round = C::OUT / (f32out ? 512 : 256);  // tokens that the output buffer takes
@@ -858,24 +859,24 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
             uint4 res[kRes];
             for (int r0 = t0; r0 < t1; r0 += round) {
                 const int r1 = min(t1, r0 + round);
-                if (r0 > t0) epi_bar_sync(384);
-                if (p.epilogue == 1 && p.staged) fetch_res(res, w, m0, N, r0, r1, 0, 384);
-                for (int t = r0 + (fin_t >> 5); t < r1; t += 24) {  // a warp adds up two tokens at a time
-                    const bool two = t + 12 < r1;
+                if (r0 > t0) epi_bar_sync(NFIN);
+                if (p.epilogue == 1 && p.staged) fetch_res(res, w, m0, N, r0, r1, 0, NFIN);
+                for (int t = r0 + (fin_t >> 5); t < r1; t += NFIN / 16) {  // a warp adds up two tokens at a time
+                    const bool two = t + NFIN / 32 < r1;
                     float4 s0 = make_float4(0.f, 0.f, 0.f, 0.f), s1 = s0;
 #pragma unroll 4
                     for (int z = 0; z < p.splits; z++) {
                         const float4 a = ld_cluster_f4(part + (uint32_t)(t * BM + lane * 4) * 4, z);
-                        const float4 c = ld_cluster_f4(part + (uint32_t)((two ? t + 12 : t) * BM + lane * 4) * 4, z);
+                        const float4 c = ld_cluster_f4(part + (uint32_t)((two ? t + NFIN / 32 : t) * BM + lane * 4) * 4, z);
                         s0.x += a.x, s0.y += a.y, s0.z += a.z, s0.w += a.w;
                         s1.x += c.x, s1.y += c.y, s1.z += c.z, s1.w += c.w;
                     }
                     put4(w, m0, N, r0, t, s0);
-                    if (two) put4(w, m0, N, r0, t + 12, s1);
+                    if (two) put4(w, m0, N, r0, t + NFIN / 32, s1);
                 }
                 if (p.staged) {
-                    epi_bar_sync(384);
-                    copy_out(res, w, m0, N, r0, r1, 384);
+                    epi_bar_sync(NFIN);
+                    copy_out(res, w, m0, N, r0, r1, NFIN);
                 }
             }
         }

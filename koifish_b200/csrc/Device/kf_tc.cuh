@@ -50,11 +50,11 @@ __device__ __forceinline__ void mbar_wait_a(uint32_t a, uint32_t parity) {
 }
 __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity) { mbar_wait_a(smem_u32(bar), parity); }
 // for the warps that wait a long time (epilogue): back off between polls so the spinning does not take issue slots from the producers
-__device__ __noinline__ void mbar_wait_sleepy(uint64_t* bar, uint32_t parity) {
+__device__ __noinline__ void mbar_wait_sleepy(uint64_t* bar, uint32_t parity, uint32_t ns) {
     const uint32_t a = smem_u32(bar);
-    for (uint32_t it = 0; it < (1u << 22); it++) {
+    for (uint32_t it = 0; it < (1u << 24); it++) {
         if (mbar_try(a, parity)) return;
-        __nanosleep(200);
+        __nanosleep(ns);
     }
     __trap();
 }
