@@ -108,8 +108,10 @@ extern "C" int kf_qknorm_rope_kvappend(kf_ctx* ctx, void* q, const void* k, cons
     if (!ctx || !q || !k || !v || !kcache || !vcache || !table || !pos_dev) return KF_ERR_BAD_ARG;
     KF_REQUIRE(ctx, M >= 1 && hd % 2 == 0 && hd / 2 <= 1024 && n_head % n_kv == 0 && max_seq > 0, "shape");
     // a warp per (token, head) or several, which starts under the projection's tail (attention.cu): 1 token of 64 + 8 heads deep in its context, whole attention block
-    // 59.3 us with a block per head, 56.8 so; a step of eight sequences through the 0.6B shape 1262 -> 1242
-    if (hd == 128 || hd == 64)
+    // 59.3 us with a block per head, 56.8 so.  Its lanes take hd / 32 elements at once; rows that start elsewhere go element by element below
+    const uintptr_t rows = (uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)qw | (uintptr_t)kw | (uintptr_t)kcache | (uintptr_t)vcache |
+                           (M > 1 ? (uintptr_t)seq_stride * 2 : 0);
+    if ((hd == 128 || hd == 64) && rows % (hd / 16) == 0)
         return kf_qknorm_rope_kv_warp(ctx, q, k, v, qw, kw, kcache, vcache, table, pos_dev, M, n_head, n_kv, hd, eps, seq_stride);
     dim3 grid(n_head + n_kv, M);
     kf_qknorm_rope_kv_kernel<<<grid, hd / 2, 0, ctx->stream>>>((uint16_t*)q, (const uint16_t*)k, (const uint16_t*)v, (const uint16_t*)qw,

@@ -638,6 +638,46 @@ def test_qknorm_rows_per_warp(ctx, hd, n_head, n_kv, M, norm):
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("hd,n_head,n_kv", [(128, 4, 2), (64, 3, 1)])
+@pytest.mark.parametrize("M", [1, 5, 16])
+@pytest.mark.parametrize("odd", ["none", "q", "k", "v", "qw", "kw", "kc", "vc", "stride"])
+def test_qknorm_at_any_element(ctx, hd, n_head, n_kv, M, odd):
+    """One operand, or the sequences of the cache, an odd number of elements on.  The fp32 sums of squares differ in their order from the oracle's (2^-20 of the norm),
+    which may move a normalised value over a rounding edge: one bf16 step (2^-7 at most) of either term of the rotation, and one of the result.  V is copied."""
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(M * hd)
+    rows = 7
+    stride = rows * n_kv * hd + (odd == "stride")
+
+    def at(name, n, values=None):
+        t = (torch.zeros(n + 1, device="cuda") if values is None else values).bfloat16()
+        return t[1:] if odd == name else t[:n]
+    rand = lambda name, n: at(name, n, torch.randn(n + 1, generator=g, device="cuda"))  # noqa: E731
+    q, k, v, qw, kw = rand("q", M * n_head * hd), rand("k", M * n_kv * hd), rand("v", M * n_kv * hd), rand("qw", hd), rand("kw", hd)
+    kc, vc = at("kc", M * stride), at("vc", M * stride)
+    table = torch.randn(rows, hd // 2, 2, generator=g, device="cuda")
+    pos = torch.randint(0, rows, (M,), generator=g, device="cuda", dtype=torch.int32)
+    q0 = q.clone()
+    torch.cuda.synchronize()
+    ctx.check(ctx.lib.kf_qknorm_rope_kvappend(ctx.h, _ptr(q), _ptr(k), _ptr(v), _ptr(qw), _ptr(kw), _ptr(kc), _ptr(vc), _ptr(table), _ptr(pos), M, n_head, n_kv, hd, rows,
+                                              1e-6, stride), "qknorm")
+    ctx.sync()
+    c, s = (table[pos.long(), :, i].double()[:, None] for i in (0, 1))
+
+    def check(got, x, w, heads):
+        x = x.view(M, heads, hd).double()
+        n = (x * torch.rsqrt(x.square().mean(2, keepdim=True) + 1e-6) * w.double()).bfloat16().double()
+        a, b = n[:, :, :hd // 2], n[:, :, hd // 2:]
+        want, size = torch.cat([a * c - b * s, a * s + b * c], 2), torch.cat([(a * c).abs() + (b * s).abs(), (a * s).abs() + (b * c).abs()], 2)
+        assert bool(((got.view(M, heads, hd).double() - want).abs() <= 2.0 ** -7 * (size + want.abs())).all())
+    check(q, q0, qw, n_head)
+    kept = [torch.stack([t[m * stride:m * stride + rows * n_kv * hd].view(rows, n_kv * hd)[int(pos[m])] for m in range(M)]) for t in (kc, vc)]
+    check(kept[0], k, kw, n_kv)
+    assert torch.equal(kept[1].reshape(-1), v)
+    assert int((vc != 0).sum()) == int((v != 0).sum())
+
+
 # ---------------------------------------------------------------------------------------------- routing of a panel, weighted sum of the experts
 @pytest.mark.parametrize("M,E,top,full", [(33, 8, 8, 0), (300, 7, 2, 1), (512, 64, 6, 0), (129, 256, 4, 1), (129, 257, 4, 1), (70, 300, 40, 0), (2049, 33, 1, 0), (5, 64, 6, 1)])
 def test_panel_routing(ctx, M, E, top, full):
