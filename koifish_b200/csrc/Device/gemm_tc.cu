@@ -14,9 +14,9 @@
 //     the expanded weights never touch shared memory, which stays free for the B operand;
 //   * warp 8  (1 thread): tcgen05.mma [D], [A in TMEM], B-descriptor; tcgen05.commit frees the stage / publishes the accumulator;
 //   * warps 11-14 (epilogue): tcgen05.ld the accumulator into shared memory (it then goes back to the MMA warp), then the final store (bf16 / +residual /
-//     SwiGLU / fp32) under the next item's main loop; the producers help with a CTA's last item.  With split-K the parts of a tile are the CTAs of a
-//     cluster, which add up through distributed shared memory, or, where these do not fit on the GPU at once, fp32 partials in global memory + an
-//     arrival counter; either way in the order of the parts (deterministic).
+//     SwiGLU / fp32) under the next item's main loop; the producers help with a CTA's last item, where it is not the part of a split whose parts are the
+//     CTAs of a cluster and meet in distributed shared memory (there from 128 tokens).  Splits that do not fit on the GPU as clusters leave fp32 partials in
+//     global memory + an arrival counter; either way the sums are taken in the order of the parts (deterministic).
 // bf16 weights need no expansion: warp 9 TMA-loads them straight into a swizzled A tile in shared memory (classic SS MMA).
 // The k order inside every 32-wide slot is the extraction-friendly permutation of gemv.cu; kf_tc_prepare_x permutes the activations
 // identically, so the contraction is unchanged.  Every barrier wait is bounded and traps instead of hanging the GPU.
@@ -291,12 +291,14 @@ __device__ __forceinline__ int slot_offset(int q) {
 
 // Ring depths.  The three rings are decoupled because their latencies differ: the raw ring hides DRAM latency (bytes in flight per SM
 // = RS x 8 KB must cover ~2 us x 44 GB/s), the B ring hides the L2 round trip of the (small, L2-resident) activation tiles, the A ring
-// only the on-chip producer -> MMA hand-off.  Sized so that shared memory, the epilogue's two output buffers included, stays below 226 KB and tensor memory within 512 columns.
+// only the on-chip producer -> MMA hand-off.  Sized so that shared memory, the epilogue's output buffer included, stays below 226 KB and tensor memory within 512 columns.
 template <int FMT, int BN>
 struct Rings {
     static constexpr bool A_TMEM = FMT != TF_BF16;
     static constexpr int U       = BN <= 128 ? 2 : 1;  // k-blocks per ring stage: below 256 tokens the barrier traffic, not the MMA, paces a k-block
-    static constexpr bool HELP   = BN >= 128;  // the producers help with the last item: below that their way to the barrier takes longer than their share of the work (12 tokens x 3072 x 6144 + 0.9 us)
+    // the producers take their share of a cluster's sums from 128 tokens on: below that their way there takes longer than the share (4-bit 3072 x 6144 at 12 tokens
+    // 12.65 -> 13.13 us with them, at 40 13.3 -> 14.1)
+    static constexpr int NSUM    = BN >= 128 ? 384 : 128;
     static constexpr int NACC    = (A_TMEM && BN == 256) ? 1 : 2;
     static constexpr int A_BYTES = A_TMEM ? 0 : BM * 128;
     static constexpr int SUB     = A_BYTES + BN * 128;  // one k-block of a stage: [A tile (bf16 weights only)][B tile]
@@ -395,8 +397,6 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
     __shared__ uint64_t a_full[SA1], a_empty[SA1], b_full[SB], b_empty[SB], raw_full[RS1], raw_empty[RS1], tmem_full[NACC], tmem_empty[NACC];
     __shared__ uint32_t tmem_base_smem;
     __shared__ int last_flag;
-    __shared__ Item s_last;  // the CTA's last item, decoded while nobody waits for it
-    const int last_ait = (p.n_items - 1 - (int)blockIdx.x) / (int)gridDim.x, last_item = blockIdx.x + last_ait * gridDim.x;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
@@ -436,7 +436,7 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     // producers: this thread's row of zero / step; scale / zero of the current group and of the next two (register queue; the loads run 1-2 groups ahead of
-    // their use).  Those of the first item are asked for here: they take a DRAM round trip, as long as the first weights
+    // their use)
     const int prow = (warp & 3) * 32 + lane, gpr = (p.K >> 7) >> p.gshift;
     const uint16_t *zrow = nullptr, *srow = nullptr;
     int gcur = 0;
@@ -453,8 +453,6 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
             zq2 = __ldg(zrow + g2), sq2 = __ldg(srow + g2);
         }
     };
-    if (tid == kEpiWarp0 * 32) s_last = decode_item<KBR>(p, last_item);
-    if (warp < kProducerWarps) fetch_gama(decode_item<KBR>(p, blockIdx.x));
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -462,12 +460,10 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
     kf_grid_launch_dependents();
 
     // ============ the end of an item: TMEM -> registers -> output buffer in shared memory -> Y in 16-byte accesses, or partial sums of a split.  Runs on the
-    // four epilogue warps while the other roles work on the next item, and from 128 tokens on these and the eight producer warps (three to a quarter of the lanes)
-    // for the CTA's last item, where nothing else is left to do.  Four warps took 4 us for the 256 tokens of an item and 10 with SwiGLU, in front of which the matrix
-    // instructions of the next item waited: there is no second accumulator beside 256 columns and the A ring (4-bit SwiGLU 51200 x 5120 at 2048 tokens 842 -> 757 us,
-    // 6144 x 1024 at 700, one item per CTA, 22.2 -> 17.8) ============
-    constexpr int NFIN  = C::HELP ? 384 : 128;  // threads that finish the last item
-    const bool finisher = warp >= kEpiWarp0 || (C::HELP && warp < kProducerWarps);
+    // four epilogue warps while the other roles work on the next item, and on these and the eight producer warps (three to a quarter of the lanes) for the CTA's
+    // last item, where nothing else is left to do.  Four warps took 4 us for the 256 tokens of an item and 10 with SwiGLU, in front of which the matrix instructions
+    // of the next item waited: there is no second accumulator beside 256 columns and the A ring (4-bit SwiGLU 51200 x 5120 at 2048 tokens 842 -> 726 us, 6144 x 1024
+    // at 700, one item per CTA, 22.0 -> 17.0).  Small token tiles gain as well: 12288 x 3072 at 40 tokens 18.9 -> 17.6 ============
     const int fin_t     = warp < kProducerWarps ? 128 + tid : tid - kEpiWarp0 * 32;  // 0 .. 127: epilogue warps
     const bool f32out   = p.epilogue == 4;
     constexpr int kRes  = 4;  // residual pieces in flight per thread
@@ -543,25 +539,15 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
         const bool direct = p.splits == 1 && p.staged;
         uint4 res[kRes];
         if (direct && p.epilogue == 1) fetch_res(res, w, m0, N, 0, min(cnt, round), 0, nthr);
-        // one warp polls, a whole main loop ahead and politely (four took issue slots from the producers: 6144 x 3072 at 12 tokens 18.3 -> 19.1 us); the others learn it here
-        if (warp == kEpiWarp0) mbar_wait_sleepy(&tmem_full[buf], (ait / NACC) & 1, NACC == 2 && nthr == 128 ? 200 : 20);
-        epi_bar_sync(nthr);  // the output buffer is free, the accumulator complete
+        epi_bar_sync(nthr);  // the output buffer is free
+        if (nthr == 128) mbar_wait_sleepy(&tmem_full[buf], (ait / NACC) & 1, NACC == 2 ? 200 : 20);  // a main loop away: poll politely
+        else mbar_wait(&tmem_full[buf], (ait / NACC) & 1);
         tc_fence_after();
         auto release = [&]() {  // the accumulator buffer may be overwritten by the next item
             tc_fence_before();
             __syncwarp();
             if (lane == 0 && warp >= kEpiWarp0) mbar_arrive(&tmem_empty[buf]);
         };
-        if (p.cluster) {
-            float* sums = reinterpret_cast<float*>(tiles);  // the rings are idle: this is the CTA's only item and its MMAs have completed
-            for (int c0 = part * 16; c0 < cnt; c0 += nparts * 16) {
-                uint32_t v[16];
-                tmem_ld16(tbase + (uint32_t)c0, v);
-#pragma unroll
-                for (int j = 0; j < 16; j++) sums[(c0 + j) * BM + row] = __uint_as_float(v[j]);
-            }
-            return;
-        }
         if (direct) {
             for (int r0 = 0; r0 < cnt; r0 += round) {
                 const int r1 = min(cnt, r0 + round);
@@ -655,6 +641,7 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
             const uint32_t full0 = smem_u32(&a_full[0]), empty0 = smem_u32(&a_empty[0]);
             const uint32_t rfull0 = smem_u32(&raw_full[0]), rempty0 = smem_u32(&raw_empty[0]);
             uint32_t s = 0, eph = 1, rs = 0, rph = 0;  // ring positions and the parities to wait for
+            fetch_gama(decode_item<KBR>(p, blockIdx.x));  // beside the first weights, which are as long on their way; in front of the barrier it held up the loaders (12288 x 3072 at 12 tokens + 0.4 us)
             for (int item = blockIdx.x; item < p.n_items; item += gridDim.x) {
                 const Item w = decode_item<KBR>(p, item);
                 if (item != (int)blockIdx.x) fetch_gama(w);
@@ -835,14 +822,32 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
     } else {
         kf_grid_dependency_wait();  // residual / workspace / counters may still be in use by the previous kernel
         uint32_t ait = 0;
+        const int last_item = blockIdx.x + (p.n_items - 1 - (int)blockIdx.x) / (int)gridDim.x * gridDim.x;
         for (int item = blockIdx.x; item < last_item; item += gridDim.x, ait++) {
             const Item w = decode_item<KBR>(p, item);
             finish(w, ait, (warp - kEpiWarp0) * 32 + lane, 128);
         }
     }
+    constexpr int NSUM  = C::NSUM;
+    const bool finisher = warp >= kEpiWarp0 || ((NSUM == 384 || !p.cluster) && warp < kProducerWarps);
     if (finisher) {  // the last item
         if (warp < kProducerWarps) kf_grid_dependency_wait();
-        finish(s_last, last_ait, fin_t, NFIN);
+        if (!p.cluster) {
+            const int last_ait = (p.n_items - 1 - (int)blockIdx.x) / (int)gridDim.x;
+            finish(decode_item<KBR>(p, blockIdx.x + last_ait * gridDim.x), last_ait, fin_t, 384);
+        } else {
+            if (NACC == 2 && NSUM == 128) mbar_wait_sleepy(&tmem_full[0], 0, 200);
+            else mbar_wait(&tmem_full[0], 0);
+            tc_fence_after();
+            const int quad = warp & 3, cnt = min(BN, p.M - decode_item<KBR>(p, blockIdx.x).m0 * BN);
+            float* sums    = reinterpret_cast<float*>(tiles) + quad * 32 + lane;  // the rings are idle: this is the CTA's only item and its MMAs have completed
+            for (int c0 = (fin_t >> 7) * 16; c0 < cnt; c0 += NSUM / 8) {
+                uint32_t v[16];
+                tmem_ld16(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, v);
+#pragma unroll
+                for (int j = 0; j < 16; j++) sums[(c0 + j) * BM] = __uint_as_float(v[j]);
+            }
+        }
     }
     // ============ split over a cluster: every CTA has its partial sums in shared memory and adds up its share of the tokens, in the order of the parts.  Takes
     // 3 us, of which the reads from the other CTAs are half; through global memory, where the last CTA to arrive did it all, 4-bit 4096 x 12288 at 300 tokens
@@ -851,7 +856,7 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
         __syncwarp();
         cluster_arrive(), cluster_wait();
         if (finisher) {
-            const Item w  = s_last;
+            const Item w  = decode_item<KBR>(p, blockIdx.x);
             const int m0 = w.m0 * BN, cnt = min(BN, p.M - m0), N = p.Nw[w.wi];
             const int t0 = cnt * w.z / p.splits, t1 = cnt * (w.z + 1) / p.splits;
             const int round = C::OUT / (f32out ? 512 : 256);  // tokens that the output buffer takes
@@ -859,24 +864,24 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
             uint4 res[kRes];
             for (int r0 = t0; r0 < t1; r0 += round) {
                 const int r1 = min(t1, r0 + round);
-                if (r0 > t0) epi_bar_sync(NFIN);
-                if (p.epilogue == 1 && p.staged) fetch_res(res, w, m0, N, r0, r1, 0, NFIN);
-                for (int t = r0 + (fin_t >> 5); t < r1; t += NFIN / 16) {  // a warp adds up two tokens at a time
-                    const bool two = t + NFIN / 32 < r1;
+                if (r0 > t0) epi_bar_sync(NSUM);
+                if (p.epilogue == 1 && p.staged) fetch_res(res, w, m0, N, r0, r1, 0, NSUM);
+                for (int t = r0 + (fin_t >> 5); t < r1; t += NSUM / 16) {  // a warp adds up two tokens at a time
+                    const bool two = t + NSUM / 32 < r1;
                     float4 s0 = make_float4(0.f, 0.f, 0.f, 0.f), s1 = s0;
 #pragma unroll 4
                     for (int z = 0; z < p.splits; z++) {
                         const float4 a = ld_cluster_f4(part + (uint32_t)(t * BM + lane * 4) * 4, z);
-                        const float4 c = ld_cluster_f4(part + (uint32_t)((two ? t + NFIN / 32 : t) * BM + lane * 4) * 4, z);
+                        const float4 c = ld_cluster_f4(part + (uint32_t)((two ? t + NSUM / 32 : t) * BM + lane * 4) * 4, z);
                         s0.x += a.x, s0.y += a.y, s0.z += a.z, s0.w += a.w;
                         s1.x += c.x, s1.y += c.y, s1.z += c.z, s1.w += c.w;
                     }
                     put4(w, m0, N, r0, t, s0);
-                    if (two) put4(w, m0, N, r0, t + NFIN / 32, s1);
+                    if (two) put4(w, m0, N, r0, t + NSUM / 32, s1);
                 }
                 if (p.staged) {
-                    epi_bar_sync(NFIN);
-                    copy_out(res, w, m0, N, r0, r1, NFIN);
+                    epi_bar_sync(NSUM);
+                    copy_out(res, w, m0, N, r0, r1, NSUM);
                 }
             }
         }

@@ -218,30 +218,37 @@ def test_tc_split_over_cluster_equals_workspace(ctx, typ, M, tc_bn, splits):
 
 
 @pytest.mark.parametrize("typ", [kf.KF_T_Q4, kf.KF_T_BF16])
-@pytest.mark.parametrize("M,tc_bn", [(41, 16), (600, 128), (1100, 256)])
-def test_tc_several_items_per_cta(ctx, typ, M, tc_bn):
-    """Items that the epilogue warps finish alone, under the next one's main loop, and the last one, with the producers' help: 1e-5 of the rms covers the order of
-    fp32 sums, 2^-8 the rounding of a bf16 result."""
+@pytest.mark.parametrize("M,tc_bn", [(41, 16), (300, 64), (600, 128), (1100, 256)])
+@pytest.mark.parametrize("splits", [1, 2, 3])
+def test_tc_several_items_per_cta(ctx, typ, M, tc_bn, splits):
+    """Items that the epilogue warps finish alone, under the next one's main loop, and the last one, with the producers' help; whole and in parts whose sums meet in the
+    workspace; every epilogue, and an output that starts at an odd element.  An fp32 sum of 1024 terms is off by 2^-24 * sqrt(1024) = 2e-6 of the rms; 4e-5 holds for
+    the largest of the seven million.  A bf16 result is rounded to 2^-8 of itself; SwiGLU takes the rounded gate and up, each of which may be one step off."""
     import torch
     import ctypes as C
-    torch.backends.cuda.matmul.allow_tf32 = False
-    rows, cols = 6416, 256
-    w, wd = make_q(ctx, typ, rows, cols, 5) if typ != kf.KF_T_BF16 else _bf16_weight(ctx, rows, cols, 5)
-    dw = w.desc()
+    rows, cols = 6416, 1024
+    mk = lambda seed: make_q(ctx, typ, rows, cols, seed) if typ != kf.KF_T_BF16 else _bf16_weight(ctx, rows, cols, seed)  # noqa: E731
+    (w, wd), (u, ud) = mk(5), mk(6)
+    gu = (kf.TensorDesc * 2)(w.desc(), u.desc())
     x, r = torch.randn(M, cols, device="cuda").bfloat16(), torch.randn(M, rows, device="cuda").bfloat16()
-    acc = x.float() @ wd.T
-    eps, tiny = 2.0 ** -8 * 1.001, 1e-5 * float(acc.square().mean().sqrt())
-    yr, yf = r.clone(), torch.zeros(M, rows, device="cuda")
+    acc, up = x.double() @ wd.double().T, x.double() @ ud.double().T
+    eps, tiny = 2.0 ** -8 * 1.001, 4e-5 * float(acc.square().mean().sqrt())
+    yr, yf, yg, yo = r.clone(), torch.zeros(M, rows, device="cuda"), torch.zeros_like(r), torch.zeros(M * rows + 1, device="cuda").bfloat16()[1:]
     torch.cuda.synchronize()
-    ctx.set_int("tc_bn", tc_bn), ctx.set_int("gemv_splitk", 1)
+    ctx.set_int("tc_min_m", 1), ctx.set_int("tc_bn", tc_bn), ctx.set_int("gemv_splitk", splits)
     try:
-        ctx.check(ctx.lib.kf_linear(ctx.h, _ptr(yr), C.byref(dw), _ptr(x), M, kf.KF_EPI_RESIDUAL, _ptr(yr)), "residual")
-        ctx.check(ctx.lib.kf_linear(ctx.h, _ptr(yf), C.byref(dw), _ptr(x), M, kf.KF_EPI_F32, None), "f32")
+        ctx.check(ctx.lib.kf_linear(ctx.h, _ptr(yr), C.byref(gu[0]), _ptr(x), M, kf.KF_EPI_RESIDUAL, _ptr(yr)), "residual")
+        ctx.check(ctx.lib.kf_linear(ctx.h, _ptr(yf), C.byref(gu[0]), _ptr(x), M, kf.KF_EPI_F32, None), "f32")
+        ctx.check(ctx.lib.kf_linear(ctx.h, _ptr(yo), C.byref(gu[0]), _ptr(x), M, kf.KF_EPI_NONE, None), "odd")
+        ctx.check(ctx.lib.kf_linear_swiglu(ctx.h, _ptr(yg), C.byref(gu[0]), C.byref(gu[1]), _ptr(x), M), "swiglu")
         ctx.sync()
     finally:
-        ctx.set_int("tc_bn", 0), ctx.set_int("gemv_splitk", 0)
-    assert bool(((yf - acc).abs() <= tiny).all())
-    assert bool(((yr.float() - (r.float() + acc)).abs() <= eps * (acc.abs() + (r.float() + acc).abs()) * 1.02 + tiny).all())
+        ctx.set_int("tc_min_m", -1), ctx.set_int("tc_bn", 0), ctx.set_int("gemv_splitk", 0)
+    assert bool(((yf.double() - acc).abs() <= tiny).all())
+    assert bool(((yo.view(M, rows).double() - acc).abs() <= eps * acc.abs() + tiny).all())
+    assert bool(((yr.double() - (r.double() + acc)).abs() <= eps * (acc.abs() + (r.double() + acc).abs()) * 1.02 + tiny).all())
+    want = acc * torch.sigmoid(acc) * up
+    assert bool(((yg.double() - want).abs() <= eps * (2 * want.abs() + 1.2 * (acc * up).abs()) * 1.02 + tiny * (1 + acc.abs() + up.abs())).all())
 
 
 @pytest.mark.parametrize("tc_bn", [0, 64])
