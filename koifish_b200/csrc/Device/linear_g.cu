@@ -7,8 +7,9 @@
 //   * DUAL form: two weight tables A, B of equal shape and y = silu(A x) * (B x), the gate / up pair of a gated feed-forward, or its clamped
 //     form y = g sigmoid(alpha g) (u + shift) with g = min(A x, limit), u = clamp(B x, -limit, limit);
 //   * "batch" form for a handful of rows: several weights, each with an input and an output of its own, in one launch.
-// A warp-per-output GEMV for a handful of rows (decode: every weight row is read once, 16-byte loads when the row length allows) and 64 x 64 shared-memory tile
-// kernels for panels: a cp.async ring with tcgen05 for bf16 activations, FFMA for float ones (mma.sync for bf16 rows of odd lengths).
+// A warp-per-output GEMV for a handful of rows (decode: every weight row is read once, 16-byte loads when the row length allows) and shared-memory tile kernels for
+// panels: a cp.async ring with tcgen05 for bf16 activations (128 weight rows x 64 slots; mma.sync on 64 x 64 where that leaves most SMs idle), 64 x 64 tiles with
+// FFMA for float ones (mma.sync for bf16 rows of odd lengths).
 // No reference equivalent: the reference's SLP::Forw hands every shape to cuBLASLt (src/Device/CUDA/NeuronFuse.cu:305-381).
 #include <algorithm>
 
@@ -468,6 +469,21 @@ __global__ void __launch_bounds__(256) kf_lin_tile_any_kernel(LinArgs a) {
 constexpr int kTileRows = 128, kTileStages = 4, kTileStage = (kTileRows + BM) * 128;  // weight rows, then slots, 128 bytes each
 constexpr size_t kTileSmem = (size_t)kTileStages * kTileStage + 1024;
 static_assert(kTileStages * kTileStage >= BM * kTileRows * 4, "the ring takes the fp32 results");
+// two neighbouring outputs, of which `left` exist
+__device__ __forceinline__ void store_pair(uint16_t* y, float v0, float v1, int left, bool pairs) {
+    if (pairs && left > 1) *reinterpret_cast<uint32_t*>(y) = pack_bf16x2(v0, v1);
+    else {
+        if (left > 0) y[0] = f32_to_bf16_bits(v0);
+        if (left > 1) y[1] = f32_to_bf16_bits(v1);
+    }
+}
+__device__ __forceinline__ void store_pair(float* y, float v0, float v1, int left, bool pairs) {
+    if (pairs && left > 1) *reinterpret_cast<float2*>(y) = make_float2(v0, v1);
+    else {
+        if (left > 0) y[0] = v0;
+        if (left > 1) y[1] = v1;
+    }
+}
 __device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool ok) {
     asm volatile("cp.async.cg.shared.global.L2::256B [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
 }
@@ -577,7 +593,7 @@ __global__ void __launch_bounds__(256, 2) kf_lin_tile_kernel(LinArgs a) {
         }
         tc_fence_before();
         __syncthreads();
-        const bool quads = a.ldy % 4 == 0 && ((uintptr_t)a.y & 15) == 0;
+        const bool quads = a.ldy % 4 == 0 && ((uintptr_t)a.y & 15) == 0, pairs = a.ldy % 2 == 0 && ((uintptr_t)a.y & 7) == 0;
         for (int i = tid; i < (min(hi, m0 + BM) - m0) * (OUTS / 4); i += 256) {
             const int t = i / (OUTS / 4), c = (i % (OUTS / 4)) * 4, n = n0 + c;
             if (n >= a.N) continue;
@@ -592,13 +608,11 @@ __global__ void __launch_bounds__(256, 2) kf_lin_tile_kernel(LinArgs a) {
             if ((DUAL || a.act) && a.out_act == 1) {
                 uint16_t* y = (uint16_t*)a.y + at;
                 if (four) *reinterpret_cast<uint2*>(y) = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]));
-                else
-                    for (int e = 0; e < 4 && n + e < a.N; e++) y[e] = f32_to_bf16_bits(v[e]);
+                else store_pair(y, v[0], v[1], a.N - n, pairs), store_pair(y + 2, v[2], v[3], a.N - n - 2, pairs);
             } else {
                 float* y = (float*)a.y + at;
                 if (four) *reinterpret_cast<float4*>(y) = make_float4(v[0], v[1], v[2], v[3]);
-                else
-                    for (int e = 0; e < 4 && n + e < a.N; e++) y[e] = v[e];
+                else store_pair(y, v[0], v[1], a.N - n, pairs), store_pair(y + 2, v[2], v[3], a.N - n - 2, pairs);
             }
         }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -607,6 +621,118 @@ __global__ void __launch_bounds__(256, 2) kf_lin_tile_kernel(LinArgs a) {
     if (warp == 0) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 64;" ::"r"(tmem) : "memory");
+    }
+}
+
+// One weight and few CTAs: 64 slots x 64 outputs per CTA, k in steps of 64 through a ring of six stages filled by cp.async, 8 warps as 4 (m) x 2 (n) on mma.sync
+// m16n8k16.  Twice as many CTAs as the kernel above and no tensor memory to set up (1 us); shared memory, which bounds this form where all warps multiply, has
+// little to do while a warp whose 16 slots lie past the group's end only helps to load.
+constexpr int kFewStages = 6, kFewTile = 64 * 128, kFewStage = 2 * kFewTile;
+constexpr size_t kFewSmem = (size_t)kFewStages * kFewStage;
+__global__ void __launch_bounds__(256, 2) kf_lin_tile_few_kernel(LinArgs a) {
+    constexpr int BK = 64, NS = kFewStages;
+    extern __shared__ __align__(128) uint8_t tile_smem[];
+    const uint32_t ring = smem_u32(tile_smem);
+    const int g  = blockIdx.z;
+    const int lo = a.offsets ? a.offsets[g] : 0, hi = a.offsets ? a.offsets[g + 1] : a.M;
+    const int n0 = blockIdx.x * BN, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int wm = warp & 3, wn = warp >> 2;             // warp tile: rows wm * 16, columns wn * 32
+    const int lr = tid >> 3, lc = tid & 7;                // this thread's loads: rows lr and lr + 32 of either operand, chunk lc
+    const int steps = (a.K + BK - 1) / BK;
+    for (int m0 = lo + blockIdx.y * BM; m0 < hi; m0 += gridDim.y * BM) {
+        const uint16_t* W = a.Wt0 ? a.Wt0[g] : a.W0;
+        const bool wvec = ((uintptr_t)W & 15) == 0;
+        const uint16_t* xr[2];
+        bool xok[2], wok[2];
+        size_t woff[2];
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int s = m0 + lr + 32 * i, n = n0 + lr + 32 * i;
+            xok[i]  = s < hi, wok[i] = n < a.N;
+            xr[i]   = (const uint16_t*)a.x + (size_t)(xok[i] ? (a.src_row ? a.src_row[s] : s) : 0) * a.ldx + lc * 8;
+            woff[i] = (size_t)(wok[i] ? n : 0) * a.K + lc * 8;
+        }
+        auto load = [&](int step) {
+            const uint32_t st = ring + (uint32_t)(step % NS) * kFewStage;
+            const int k       = step * BK + lc * 8;
+            const bool kok    = k < a.K;  // K is a multiple of 8
+            const size_t kof  = (size_t)(kok ? step * BK : 0);
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const int r        = lr + 32 * i;
+                const uint32_t dst = st + (uint32_t)(r * 128 + ((lc ^ (r & 7)) << 4));
+                cp16(dst, xok[i] && kok ? xr[i] + kof : (const uint16_t*)a.x, xok[i] && kok);
+                const bool ok = wok[i] && kok;
+                if (wvec) {
+                    cp16(dst + kFewTile, ok ? W + woff[i] + kof : W, ok);
+                } else {
+                    uint16_t* d = reinterpret_cast<uint16_t*>(tile_smem + (dst - ring) + kFewTile);
+                    for (int e = 0; e < 8; e++) d[e] = ok ? W[woff[i] + kof + e] : (uint16_t)0;
+                }
+            }
+        };
+        float acc[16];
+#pragma unroll
+        for (int i = 0; i < 16; i++) acc[i] = 0.f;
+#pragma unroll
+        for (int i = 0; i < NS - 1; i++) {
+            if (i < steps) load(i);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        }
+        const bool busy = m0 + wm * 16 < hi;
+        for (int step = 0; step < steps; step++) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(NS - 2) : "memory");
+            __syncthreads();  // this step's bytes are there for everybody, and everybody has left the stage that is filled next
+            if (step + NS - 1 < steps) load(step + NS - 1);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            if (!busy) continue;
+            const uint8_t* xs = tile_smem + (size_t)(step % NS) * kFewStage;
+            auto at = [](const uint8_t* base, int row, int c) { return base + row * 128 + ((c ^ (row & 7)) << 4); };
+#pragma unroll
+            for (int kk = 0; kk < BK / 16; kk++) {
+                uint32_t af[4];
+                ldsm_x4(af, at(xs, wm * 16 + (lane & 15), kk * 2 + (lane >> 4)));
+#pragma unroll
+                for (int j = 0; j < 4; j += 2) {
+                    const int nr = wn * 32 + j * 8 + (lane & 7) + (lane >> 4) * 8, c = kk * 2 + ((lane >> 3) & 1);
+                    uint32_t bf[4];
+                    ldsm_x4(bf, at(xs + kFewTile, nr, c));
+                    mma_bf16_16816(&acc[j * 4], af, bf);
+                    mma_bf16_16816(&acc[(j + 1) * 4], af, bf + 2);
+                }
+            }
+        }
+        const int gr = lane >> 2, tg = lane & 3;
+        const bool pairs = a.ldy % 2 == 0 && ((uintptr_t)a.y & 7) == 0;
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int s = m0 + wm * 16 + gr + 8 * h, n = n0 + wn * 32 + j * 8 + tg * 2;
+                if (s >= hi || n >= a.N) continue;
+                float v[2];
+#pragma unroll
+                for (int e = 0; e < 2; e++) v[e] = lin_act(acc[j * 4 + 2 * h + e], a.act);
+                const size_t at = (size_t)s * a.ldy + n;
+                const bool two  = n + 1 < a.N;
+                if (a.act && a.out_act == 1) {
+                    uint16_t* y = (uint16_t*)a.y + at;
+                    if (two && pairs) *reinterpret_cast<uint32_t*>(y) = pack_bf16x2(v[0], v[1]);
+                    else {
+                        y[0] = f32_to_bf16_bits(v[0]);
+                        if (two) y[1] = f32_to_bf16_bits(v[1]);
+                    }
+                } else {
+                    float* y = (float*)a.y + at;
+                    if (two && pairs) *reinterpret_cast<float2*>(y) = make_float2(v[0], v[1]);
+                    else {
+                        y[0] = v[0];
+                        if (two) y[1] = v[1];
+                    }
+                }
+            }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();  // the ring is free for the next slot tile
     }
 }
 
@@ -623,7 +749,17 @@ int launch(kf_ctx* ctx, const LinArgs& a, int slots, int groups, bool gemv) {
             static bool set[kf_ctx::kMaxDevices] = {};  // function attributes are per device (one flag per instantiation and device)
             if (!set[ctx->device]) {
                 KF_CUDA(ctx, cudaFuncSetAttribute(kf_lin_tile_kernel<DUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileSmem));
+                if (!DUAL) KF_CUDA(ctx, cudaFuncSetAttribute(kf_lin_tile_few_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFewSmem));
                 set[ctx->device] = true;
+            }
+            // 64 x 64 tiles while they do not outnumber the SMs (8 groups of 18 slots, 512 outputs over 1792: 13.7 us, 17.0 in 128 x 64; 16 groups of 60 slots, 256
+            // outputs: 15.5, 17.0), or the two places of every SM where most groups hold up to 16 slots, one row of warps (16 groups of 8 slots, 1024 outputs over 1024:
+            // 11.4, 12.0; with 20 slots each 13.1, 12.5; three times as many tiles as SMs, 9 slots: 13.1, 10.3)
+            const long long ctas = (long long)grid.x * gy * groups;
+            if (!DUAL && (ctas <= ctx->sm_count || (ctas <= 2 * ctx->sm_count && slots <= 8ll * groups))) {
+                kf_lin_tile_few_kernel<<<grid, 256, kFewSmem, ctx->stream>>>(a);
+                KF_LAUNCH_CHECK(ctx);
+                return KF_OK;
             }
             const int outs = DUAL ? kTileRows / 2 : kTileRows;
             kf_lin_tile_kernel<DUAL><<<dim3((a.N + outs - 1) / outs, gy, groups), 256, kTileSmem, ctx->stream>>>(a);

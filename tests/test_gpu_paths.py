@@ -564,11 +564,12 @@ def test_maps_of_steps_leave_those_of_weights(ctx):
 
 
 # ---------------------------------------------------------------------------------------------- tile matmul over expert-sorted slots
-@pytest.mark.parametrize("N,K", [(64, 64), (65, 72), (8, 8), (130, 200), (192, 448), (33, 512), (257, 320)])
+@pytest.mark.parametrize("N,K", [(64, 64), (65, 72), (8, 8), (130, 200), (192, 448), (33, 512), (257, 320), (1602, 72), (1727, 200), (3300, 328)])
 @pytest.mark.parametrize("counts", [(64, 0, 1, 63, 65, 17), (200, 3, 0, 0, 1, 0), (16, 16, 16, 16, 16, 16)])
 @pytest.mark.parametrize("shift", [0, 1])
 def test_grouped_tiles(ctx, N, K, counts, shift):
-    """Ragged outputs, reductions and slot tiles, empty experts, gathered rows, weights that do not start on 16 bytes.  Products are exact in fp32 and the sums fp32:
+    """Ragged outputs, reductions and slot tiles, empty experts, gathered rows, weights that do not start on 16 bytes; outputs in 64 x 64 tiles (up to 257: fewer
+    tiles than SMs; 1602 with groups of 16: no more than twice as many) and in 128 x 64.  Products are exact in fp32 and the sums fp32:
     2^-24 * K terms of the rms, stated as 1e-5; the gate / up form rounds its result to bf16 once (2^-8)."""
     import torch
     torch.backends.cuda.matmul.allow_tf32 = False
