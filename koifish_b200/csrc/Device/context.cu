@@ -162,6 +162,12 @@ extern "C" int kf_ctx_get_int(kf_ctx* ctx, const char* key, int* value_out) {
         *value_out = ctx->gemv_exact;
     else if (!strcmp(key, "gemv_last_s"))
         *value_out = ctx->gemv_last_s;
+    else if (!strcmp(key, "tc_last_bn"))
+        *value_out = ctx->tc_last & 0xfff;
+    else if (!strcmp(key, "tc_last_split"))
+        *value_out = ctx->tc_last >> 12 & 0xffff;
+    else if (!strcmp(key, "tc_last_cluster"))
+        *value_out = ctx->tc_last >> 30;
     else if (!strcmp(key, "tp_fused"))
         *value_out = ctx->tp_fused;
     else if (!strcmp(key, "gemv_xg_min_m"))

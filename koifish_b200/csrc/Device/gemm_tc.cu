@@ -23,6 +23,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <atomic>
 #include <map>
 #include <tuple>
 
@@ -981,28 +982,28 @@ struct TcPlan {
     int bn, splits;
     bool cluster;
 };
-// CTAs of the kernel that can be resident in clusters of s (2 .. 8); 0 where the driver cannot say.  A property of the device: asked once.
+// CTAs of the kernel that can be resident in clusters of s (2 .. 8); 0 where the driver cannot say.  A property of the device, asked until it has answered; contexts of
+// several threads may ask at once.
 template <int FMT, int MODE, int BN>
 int cluster_ctas(const kf_ctx* ctx, int s) {
-    static int known[kf_ctx::kMaxDevices][9] = {};  // + 1
-    int& k = known[ctx->device][s];
-    if (k == 0) {
-        auto kern = kf_gemm_tc_kernel<FMT, MODE, BN>;
-        cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute attr[1];
-        attr[0].id               = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = (unsigned)s, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
-        cfg.gridDim = dim3((unsigned)(ctx->sm_count / s * s)), cfg.blockDim = dim3(kThreadsTC), cfg.dynamicSmemBytes = Rings<FMT, BN>::SMEM;
-        cfg.attrs = attr, cfg.numAttrs = 1;
-        int n = 0;
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Rings<FMT, BN>::SMEM) != cudaSuccess ||
-            cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
-            (void)cudaGetLastError();
-            n = 0;
-        }
-        k = n * s + 1;
+    static std::atomic<int> known[kf_ctx::kMaxDevices][9];  // + 1
+    std::atomic<int>& k = known[ctx->device][s];
+    if (const int had = k.load(std::memory_order_relaxed)) return had - 1;
+    auto kern = kf_gemm_tc_kernel<FMT, MODE, BN>;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id               = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)s, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)(ctx->sm_count / s * s)), cfg.blockDim = dim3(kThreadsTC), cfg.dynamicSmemBytes = Rings<FMT, BN>::SMEM;
+    cfg.attrs = attr, cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Rings<FMT, BN>::SMEM) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return 0;
     }
-    return k - 1;
+    k.store(n * s + 1, std::memory_order_relaxed);
+    return n * s;
 }
 template <int FMT, int MODE>
 int cluster_ctas(const kf_ctx* ctx, int bn, int s) {
@@ -1035,6 +1036,7 @@ int launch_tc(kf_ctx* ctx, GemmParams& p, const void* const* wdata, int nw, cons
     p.m_tiles = (p.M + BN - 1) / BN;
     const int base_items = p.n_tiles * p.m_tiles;
     p.splits = plan.splits, p.n_items = base_items * plan.splits, p.cluster = plan.cluster;
+    ctx->tc_last = BN | plan.splits << 12 | (plan.cluster ? 1 << 30 : 0);
     if (plan.splits > 1 && !plan.cluster) {
         int rc = kf_ensure_gemv_ws(ctx, (size_t)p.n_items * BN * BM * sizeof(float), base_items);
         if (rc) return rc;

@@ -44,6 +44,7 @@ struct kf_ctx {
     int tc_min_m = -1;  // token count from which kf_linear* use the tcgen05 GEMM: -1 = per weight type (linear.cu), 0 = never
     // tuning
     int tc_bn        = 0;  // token tile of the tcgen05 matmul (16, 32, 64, 128, 256); 0 = by modelled time
+    int tc_last      = 0;  // plan of its last launch: token tile | k-parts << 12 | parts in clusters << 30
     int gemv_splitk  = 0;
     int gemv_variant = 0;
     int gemv_cluster = 1;  // M = 1 split-K: 1 = merge the k-slices of a row block inside a thread-block cluster (DSMEM) when S <= 8; 2 = also cap S at 8; 0 = global workspace

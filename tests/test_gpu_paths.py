@@ -188,7 +188,8 @@ def test_tc_swiglu_over_its_input(ctx, typ, M, rows, cols, at):
 @pytest.mark.parametrize("typ", [kf.KF_T_Q4, kf.KF_T_BINARY, kf.KF_T_BF16])
 @pytest.mark.parametrize("M,tc_bn,splits", [(16, 16, 8), (20, 32, 2), (45, 64, 4), (100, 128, 3), (130, 256, 2), (251, 256, 5), (257, 128, 7)])
 def test_tc_split_over_cluster_equals_workspace(ctx, typ, M, tc_bn, splits):
-    """A split whose parts meet in a cluster adds the same partial sums in the same order as one through the workspace (which gemv_exact keeps to): equal bits, every epilogue."""
+    """A split whose parts meet in a cluster adds the same partial sums in the same order as one through the workspace (which gemv_exact keeps to): equal bits, every
+    epilogue.  The plan of the last launch tells which of the two ran."""
     import torch
     import ctypes as C
     rows, cols = 272, 8192
@@ -202,12 +203,15 @@ def test_tc_split_over_cluster_equals_workspace(ctx, typ, M, tc_bn, splits):
     try:
         for exact in (0, 1):
             ctx.set_int("gemv_exact", exact)
+            def ran(name, st):
+                ctx.check(st, name)
+                assert [ctx.get_int("tc_last_" + k) for k in ("bn", "split", "cluster")] == [tc_bn, splits, 1 - exact], name
             y, yr, yg, yf = (torch.zeros(M, rows, device="cuda", dtype=t) for t in (torch.bfloat16, torch.bfloat16, torch.bfloat16, torch.float32))
             torch.cuda.synchronize()
-            ctx.check(ctx.lib.kf_linear(ctx.h, _ptr(y), C.byref(dw), _ptr(x), M, kf.KF_EPI_NONE, None), "none")
-            ctx.check(ctx.lib.kf_linear(ctx.h, _ptr(yr), C.byref(dw), _ptr(x), M, kf.KF_EPI_RESIDUAL, _ptr(r)), "residual")
-            ctx.check(ctx.lib.kf_linear(ctx.h, _ptr(yf), C.byref(dw), _ptr(x), M, kf.KF_EPI_F32, None), "f32")
-            ctx.check(ctx.lib.kf_linear_swiglu(ctx.h, _ptr(yg), C.byref(gu[0]), C.byref(gu[1]), _ptr(x), M), "swiglu")
+            ran("none", ctx.lib.kf_linear(ctx.h, _ptr(y), C.byref(dw), _ptr(x), M, kf.KF_EPI_NONE, None))
+            ran("residual", ctx.lib.kf_linear(ctx.h, _ptr(yr), C.byref(dw), _ptr(x), M, kf.KF_EPI_RESIDUAL, _ptr(r)))
+            ran("f32", ctx.lib.kf_linear(ctx.h, _ptr(yf), C.byref(dw), _ptr(x), M, kf.KF_EPI_F32, None))
+            ran("swiglu", ctx.lib.kf_linear_swiglu(ctx.h, _ptr(yg), C.byref(gu[0]), C.byref(gu[1]), _ptr(x), M))
             ctx.sync()
             outs.append((y, yr, yg, yf))
     finally:
