@@ -14,9 +14,9 @@
 //     the expanded weights never touch shared memory, which stays free for the B operand;
 //   * warp 8  (1 thread): tcgen05.mma [D], [A in TMEM], B-descriptor; tcgen05.commit frees the stage / publishes the accumulator;
 //   * warps 11-14 (epilogue): tcgen05.ld the accumulator into shared memory (it then goes back to the MMA warp), then the final store (bf16 / +residual /
-//     SwiGLU / fp32) under the next item's main loop; the producers help with a CTA's last item, where it is not the part of a split whose parts are the
-//     CTAs of a cluster and meet in distributed shared memory (there from 128 tokens).  Splits that do not fit on the GPU as clusters leave fp32 partials in
-//     global memory + an arrival counter; either way the sums are taken in the order of the parts (deterministic).
+//     SwiGLU / fp32) under the next item's main loop; the producers help with a CTA's last item (from 64 tokens).  With split-K the parts of a tile are the CTAs of a
+//     cluster, which add up through distributed shared memory, or, where these do not fit on the GPU at once, fp32 partials in global memory + an
+//     arrival counter; either way in the order of the parts (deterministic).
 // bf16 weights need no expansion: warp 9 TMA-loads them straight into a swizzled A tile in shared memory (classic SS MMA).
 // The k order inside every 32-wide slot is the extraction-friendly permutation of gemv.cu; kf_tc_prepare_x permutes the activations
 // identically, so the contraction is unchanged.  Every barrier wait is bounded and traps instead of hanging the GPU.
@@ -73,6 +73,8 @@ struct GemmParams {
     int n_tiles, m_tiles, splits, n_items;
     int staged;                // outputs (and residual) may be accessed 16 bytes at a time
     int cluster;               // the parts of a split are the CTAs of a cluster, one item each
+    int item_lo, item_hi;      // item = (row tile * item_hi + hi) * item_lo + lo: token tile and part, the latter innermost in clusters
+    int part_raw, part_rem;    // raw stages of a part; the first part_rem have one more
     uint32_t lop_mask, lop_magic;
 };
 
@@ -297,8 +299,10 @@ template <int FMT, int BN>
 struct Rings {
     static constexpr bool A_TMEM = FMT != TF_BF16;
     static constexpr int U       = BN <= 128 ? 2 : 1;  // k-blocks per ring stage: below 256 tokens the barrier traffic, not the MMA, paces a k-block
-    // the producers take their share of a cluster's sums from 128 tokens on: below that their way there takes longer than the share (4-bit 3072 x 6144 at 12 tokens
-    // 12.65 -> 13.13 us with them, at 40 13.3 -> 14.1)
+    // threads that finish a CTA's last item, and its part of a cluster's sums: the producers help from 64 and from 128 tokens on.  Below that their way there takes
+    // longer than their share (4-bit 4096 x 1024 at 20 tokens, whole: tile of 16 8.3 us with them, 7.8 without, of 32 8.05 and 7.8; tile of 64 at 40 tokens 8.5 and
+    // 8.8; 3072 x 6144 in clusters, at 12 tokens 13.1 and 12.65, at 40 14.1 and 13.3)
+    static constexpr int NFIN    = BN >= 64 ? 384 : 128;
     static constexpr int NSUM    = BN >= 128 ? 384 : 128;
     static constexpr int NACC    = (A_TMEM && BN == 256) ? 1 : 2;
     static constexpr int A_BYTES = A_TMEM ? 0 : BM * 128;
@@ -321,21 +325,18 @@ struct Item {
     int wi;               // weight of the launch
     int kb0, kb1;         // k-block range
 };
+// In front of every role's first and last step: two divisions (five, with the ranges of the parts taken apart here, cost 0.5 us: 4-bit 4096 x 1024 at 20 tokens 8.6 -> 7.8
+// with the help above, 4096 x 2048 in clusters at 12 8.9 -> 8.0)
 template <int KBR>
 __device__ __forceinline__ Item decode_item(const GemmParams& p, int item) {
     Item it;
-    const int u  = p.cluster ? item / p.splits : item;
-    const int mt = u % p.m_tiles;
-    const int t  = u / p.m_tiles;
-    it.z         = p.cluster ? item % p.splits : t % p.splits;
-    const int tn = p.cluster ? t : t / p.splits;
+    const int t = item / p.item_lo, lo = item % p.item_lo, tn = t / p.item_hi, hi = t % p.item_hi;
+    const int mt = p.cluster ? hi : lo;
+    it.z         = p.cluster ? lo : hi;
     it.wi = p.epilogue == kEpiGlu ? 0 : (tn >= p.tile0[1] ? 1 : 0) + (tn >= p.tile0[2] ? 1 : 0);
     it.n0 = p.epilogue == kEpiGlu ? tn * (BM / 2) : (tn - p.tile0[it.wi]) * BM, it.m0 = mt, it.tile = tn * p.m_tiles + mt;  // m0 = token-tile index (the caller scales it by BN)
-    const int nkb  = p.K / BK;
-    const int nraw = (nkb + KBR - 1) / KBR;
-    const int base = nraw / p.splits, rem = nraw % p.splits;
-    const int r0 = it.z * base + min(it.z, rem), r1 = r0 + base + (it.z < rem ? 1 : 0);
-    it.kb0 = r0 * KBR, it.kb1 = min(r1 * KBR, nkb);
+    const int r0 = it.z * p.part_raw + min(it.z, p.part_rem), r1 = r0 + p.part_raw + (it.z < p.part_rem ? 1 : 0);
+    it.kb0 = r0 * KBR, it.kb1 = min(r1 * KBR, p.K / BK);
     return it;
 }
 
@@ -461,10 +462,10 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
     kf_grid_launch_dependents();
 
     // ============ the end of an item: TMEM -> registers -> output buffer in shared memory -> Y in 16-byte accesses, or partial sums of a split.  Runs on the
-    // four epilogue warps while the other roles work on the next item, and on these and the eight producer warps (three to a quarter of the lanes) for the CTA's
-    // last item, where nothing else is left to do.  Four warps took 4 us for the 256 tokens of an item and 10 with SwiGLU, in front of which the matrix instructions
-    // of the next item waited: there is no second accumulator beside 256 columns and the A ring (4-bit SwiGLU 51200 x 5120 at 2048 tokens 842 -> 726 us, 6144 x 1024
-    // at 700, one item per CTA, 22.0 -> 17.0).  Small token tiles gain as well: 12288 x 3072 at 40 tokens 18.9 -> 17.6 ============
+    // four epilogue warps while the other roles work on the next item, and from 64 tokens on these and the eight producer warps (three to a quarter of the lanes) for
+    // the CTA's last item, where nothing else is left to do.  Four warps took 4 us for the 256 tokens of an item and 10 with SwiGLU, in front of which the matrix
+    // instructions of the next item waited: there is no second accumulator beside 256 columns and the A ring (4-bit SwiGLU 51200 x 5120 at 2048 tokens 836 -> 736 us,
+    // 6144 x 1024 at 700, one item per CTA, 22.1 -> 16.5) ============
     const int fin_t     = warp < kProducerWarps ? 128 + tid : tid - kEpiWarp0 * 32;  // 0 .. 127: epilogue warps
     const bool f32out   = p.epilogue == 4;
     constexpr int kRes  = 4;  // residual pieces in flight per thread
@@ -829,13 +830,13 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
             finish(w, ait, (warp - kEpiWarp0) * 32 + lane, 128);
         }
     }
-    constexpr int NSUM  = C::NSUM;
-    const bool finisher = warp >= kEpiWarp0 || ((NSUM == 384 || !p.cluster) && warp < kProducerWarps);
+    constexpr int NFIN  = C::NFIN, NSUM = C::NSUM;
+    const bool finisher = warp >= kEpiWarp0 || ((p.cluster ? NSUM : NFIN) == 384 && warp < kProducerWarps);
     if (finisher) {  // the last item
         if (warp < kProducerWarps) kf_grid_dependency_wait();
         if (!p.cluster) {
             const int last_ait = (p.n_items - 1 - (int)blockIdx.x) / (int)gridDim.x;
-            finish(decode_item<KBR>(p, blockIdx.x + last_ait * gridDim.x), last_ait, fin_t, 384);
+            finish(decode_item<KBR>(p, blockIdx.x + last_ait * gridDim.x), last_ait, fin_t, NFIN);
         } else {
             if (NACC == 2 && NSUM == 128) mbar_wait_sleepy(&tmem_full[0], 0, 200);
             else mbar_wait(&tmem_full[0], 0);
@@ -1036,6 +1037,9 @@ int launch_tc(kf_ctx* ctx, GemmParams& p, const void* const* wdata, int nw, cons
     p.m_tiles = (p.M + BN - 1) / BN;
     const int base_items = p.n_tiles * p.m_tiles;
     p.splits = plan.splits, p.n_items = base_items * plan.splits, p.cluster = plan.cluster;
+    p.item_lo = plan.cluster ? plan.splits : p.m_tiles, p.item_hi = plan.cluster ? p.m_tiles : plan.splits;
+    const int nraw = (p.K / BK + F::KBR - 1) / F::KBR;
+    p.part_raw = nraw / plan.splits, p.part_rem = nraw % plan.splits;
     ctx->tc_last = BN | plan.splits << 12 | (plan.cluster ? 1 << 30 : 0);
     if (plan.splits > 1 && !plan.cluster) {
         int rc = kf_ensure_gemv_ws(ctx, (size_t)p.n_items * BN * BM * sizeof(float), base_items);
