@@ -1079,9 +1079,12 @@ int launch_tc(kf_ctx* ctx, GemmParams& p, const void* const* wdata, int nw, cons
 // Token tile and k-split by their modelled time: waves x (k-blocks x time per k-block + epilogue) + the fix-up of split sums.  The times per k-block of 64 are
 // measured ones (us; 4-bit and bf16 weights, the former stand for all that are expanded; below 64 tokens the weights' bytes or their expansion, above the matrix instructions).  Splitting pays for few row tiles and a
 // handful of tokens only: 1024 x 3072 at 16 tokens 9.9 us in 8 parts against 15.7 whole, at 256 tokens 34 against 17.  (The rule before it charged BN / 16
-// k-blocks for the fix-up: 1024 x 3072 at 256 tokens went into 12 parts and took 91 us, now 17.5.)  Parts that fit on the GPU as clusters cost 1 us more and
-// no second pass: swept over six shapes of the 0.6B and 8B blocks at 12 to 2000 tokens, the choice is within 8 % of the best tile and split.  The
-// reference-exact arithmetic keeps the earlier rule and the order of sums it was compared in.
+// k-blocks for the fix-up: 1024 x 3072 at 256 tokens went into 12 parts and took 91 us, now 15.)  Several token tiles of up to 64 fetch and expand the same weights
+// beside one another, which costs a tenth of a k-block's time for each but the first.  Parts that fit on the GPU as clusters cost no second pass, but the placement
+// of the clusters, two barriers and the sum: 2.5 to 7 us, a little more where SwiGLU waits behind it, less for bf16 weights.  (At 1 + 0.006 BN, 1-bit SwiGLU 7680 x
+// 1536 at 40 tokens went into two parts of 64, 12.2 us, now whole, 10.1; 4-bit 4096 x 2048 at 12 is in four, 8.0, against 8.8 whole.)  Swept over 14 shapes of the 0.6B to
+// 32B blocks at 12 to 700 tokens in four types, the choice is 1 % behind the best tile and split in the mean, more than 5 % in 23 of 262 cases, 18 % at most.
+// The reference-exact arithmetic keeps the earlier rule and the order of sums it was compared in.
 template <int FMT, int MODE>
 int launch_tc_bn(kf_ctx* ctx, GemmParams& p, const void* const* wdata, int nw, const void* xp) {
     constexpr int KBR = Fmt<FMT>::KBR;
@@ -1092,8 +1095,8 @@ int launch_tc_bn(kf_ctx* ctx, GemmParams& p, const void* const* wdata, int nw, c
         const int by_m = p.M > 128 ? 256 : p.M > 64 ? 128 : p.M > 32 ? 64 : p.M > 16 ? 32 : 16;  // one token tile where the panel fits one
         if (ctx->tc_bn > 0 ? b != ctx->tc_bn : ctx->gemv_exact ? b != by_m : ((b < 256 && p.M > 8 * b) || (b > 16 && p.M <= b / 2))) continue;
         static const double kb_packed[5] = {0.235, 0.235, 0.24, 0.26, 0.42}, kb_bf16[5] = {0.09, 0.10, 0.16, 0.24, 0.39};
-        const double t_kb = FMT == TF_BF16 ? kb_bf16[i] : kb_packed[i];
-        const int items   = tiles * ((p.M + b - 1) / b);
+        const int m_tiles = (p.M + b - 1) / b, items = tiles * m_tiles;
+        const double t_kb = (FMT == TF_BF16 ? kb_bf16[i] : kb_packed[i]) * (b <= 64 ? 1.0 + 0.1 * (m_tiles - 1) : 1.0);
         const int given = std::min(ctx->gemv_splitk, nraw);  // > 0: the split asked for
         for (int s = given > 0 ? given : 1; s <= (given > 0 ? given : std::min(16, nraw)); s++) {
             const int waves = (items * s + ctx->sm_count - 1) / ctx->sm_count, len = (nraw + s - 1) / s * KBR;
@@ -1102,11 +1105,10 @@ int launch_tc_bn(kf_ctx* ctx, GemmParams& p, const void* const* wdata, int nw, c
                 if (c < best * 0.95) best = c, plan = {b, s, false};
                 continue;
             }
-            const double t = waves * (len * t_kb + 0.5 + 0.006 * b + (s > 1 ? 0.5 + 0.02 * b : 0.0)) + (s > 1 ? b * (0.03 + 0.008 * s) : 0.0);
-            if (t < best * 0.98) best = t, plan = {b, s, false};
-            if (s == 1 || s > 8 || items * s > ctx->sm_count) continue;
-            const double tc = len * t_kb + 0.5 + 0.003 * b + 1.0 + 0.006 * b;
-            if (tc < best * 0.98 && items * s <= cluster_ctas<FMT, MODE>(ctx, b, s)) best = tc, plan = {b, s, true};
+            const bool cluster = s > 1 && s <= 8 && items * s <= ctx->sm_count && items * s <= cluster_ctas<FMT, MODE>(ctx, b, s);
+            const double t = cluster ? len * t_kb + 2.2 + 0.02 * b + 0.03 * (s - 2) + (p.epilogue == kEpiGlu ? 0.005 * b : 0.0) - (FMT == TF_BF16 ? 0.3 + 0.002 * b : 0.0)
+                                     : waves * (len * t_kb + 0.5 + 0.006 * b + (s > 1 ? 0.5 + 0.02 * b : 0.0)) + (s > 1 ? b * (0.05 + 0.008 * s) : 0.0);
+            if (t < best * 0.97) best = t, plan = {b, s, cluster};
         }
     }
     switch (plan.bn) {
