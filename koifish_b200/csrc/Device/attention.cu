@@ -804,8 +804,8 @@ __global__ void __launch_bounds__(128, KF_PF_MINB) kf_attn_prefill_kernel(uint16
     }
 }
 
-// ---- QK-norm + RoPE + K/V append for big panels: one WARP per R rows (heads) of a token (the block-per-head kernel of ops.cu needs 150 K tiny
-// blocks for a 2048-token panel and is scheduling bound).  Same arithmetic; the sum of squares is taken in warp-butterfly order as in the fused decode
+// ---- QK-norm + RoPE + K/V append for heads of 64 and 128, any number of tokens: one WARP per R rows (heads) of a token (the block-per-head kernel of ops.cu needs
+// 150 K tiny blocks for a 2048-token panel and is scheduling bound; for a handful of tokens it starts only behind the projection).  Same arithmetic; the sum of squares is taken in warp-butterfly order as in the fused decode
 // kernel.  Bound by latency, then by L2: the rows of a warp are fetched together and share the token's angles and the weights (1999 tokens of 32 + 8
 // heads: 24.0 us with one row a warp, 22.6 with four; few rows keep one).
 template <int DPL, int R>
@@ -1152,7 +1152,7 @@ extern "C" int kf_attn_sigmoid_prefill(kf_ctx* ctx, void* out, int ldo, const vo
     return KF_OK;
 }
 
-// warp-per-head variant of kf_qknorm_rope_kvappend for big panels (called from ops.cu); hd 64 / 128 only
+// warp-per-head variant of kf_qknorm_rope_kvappend (called from ops.cu): hd 64 / 128, operands and sequences that start on hd / 16 bytes
 int kf_qknorm_rope_kv_warp(kf_ctx* ctx, void* q, const void* k, const void* v, const void* qw, const void* kw, void* kcache, void* vcache,
                            const void* table, const int32_t* pos_dev, int M, int n_head, int n_kv, int hd, float eps, size_t seq_stride) {
     // four rows a warp from two blocks of one-row warps per SM on; below that the GPU would not be full

@@ -463,7 +463,7 @@ __global__ void __launch_bounds__(256) kf_lin_tile_any_kernel(LinArgs a) {
 // experts of 2 x 1408 x 2048: 738 MB), 48 slots each, so the CTA is built to keep bytes on their way: two CTAs per SM with four 24 KB stages each, filled by
 // cp.async (the table of weights is on the device, the rows of x are gathered: no tensor map), two to three of them in flight, 96 KB or more an SM; nothing
 // but the copies and one thread's matrix instructions in the loop.  On mma.sync, whose fragments went through ldmatrix, shared memory was as busy as DRAM (8
-// warps of 16 x 32 read 82 KB a step of 24 KB): 186 us for those and 118 for the down projections, 132 (0.85 of the copy rate) and 75 (0.75) here.
+// warps of 16 x 32 read 82 KB a step of 24 KB): 177 us for those and 113 for the down projections, 130 (0.86 of the copy rate) and 75 (0.77) here.
 // Rows lie as 128 bytes, 16-byte chunk c of row r at c ^ (r & 7): the K-major SWIZZLE_128B layout of the matrix descriptors.  A weight that is not 16-byte
 // aligned (only the kernel sees it) is fetched element by element into the same places.
 constexpr int kTileRows = 128, kTileStages = 4, kTileStage = (kTileRows + BM) * 128;  // weight rows, then slots, 128 bytes each
