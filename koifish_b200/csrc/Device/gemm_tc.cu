@@ -7,10 +7,10 @@
 //
 // Work item = [128 weight rows] x [BN tokens] x [one K range (split-K)].  The weights are the A operand (UMMA_M = 128), the tokens
 // the B operand (UMMA_N = BN), BK = 64.  One CTA per SM walks the items round-robin; its 15 warps are specialised:
-//   * warp 9  (1 thread): TMA of the PACKED weight bytes, 64 B per row per stage, into a raw ring (SWIZZLE_64B, conflict-free reads);
+//   * warp 9  (1 thread): TMA of the PACKED weight bytes, up to 128 B per row per stage, into a raw ring (swizzled over the row, conflict-free reads);
 //   * warp 10 (1 thread): TMA of the activation tile (already permuted, see below) into the B ring (SWIZZLE_128B, K-major);
-//   * warps 0-7 (producers, thread = weight row x 32-weight slot): raw bytes -> the reference's bit-exact bf16 weights (the same
-//     two-rounding arithmetic as gemv.cu) -> tcgen05.st into the A ring that lives in TENSOR MEMORY (lane = row, 2 weights / column);
+//   * warps 0-7 (producers, thread = weight row; two teams take the raw stages in turn): raw bytes -> the reference's bit-exact bf16 weights (one rounding or two, as
+//     gemv.cu; times a power of two that the sums get back) -> tcgen05.st into the A ring that lives in TENSOR MEMORY (lane = row, 2 weights / column);
 //     the expanded weights never touch shared memory, which stays free for the B operand;
 //   * warp 8  (1 thread): tcgen05.mma [D], [A in TMEM], B-descriptor; tcgen05.commit frees the stage / publishes the accumulator;
 //   * warps 11-14 (epilogue): tcgen05.ld the accumulator into shared memory (it then goes back to the MMA warp), then the final store (bf16 / +residual /
@@ -24,13 +24,15 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <map>
 #include <tuple>
+#include <type_traits>
 
 #include "kf_common.cuh"
 #include "kf_tc.cuh"
 
-// tuning experiments (bit 0: no expansion, 1: no TMEM store, 2: no scale / zero fetch in the loop ...): debug builds only
+// tuning experiments (bit 0: no expansion, 1: no TMEM store, 3: no weight copies, 4: no activation copies): debug builds only
 // (KF_NVCC_DEFS="-DKF_DEBUG_KNOBS -DKF_TC_EXP=n"); a release build compiles them out
 #if !defined(KF_DEBUG_KNOBS) || !defined(KF_TC_EXP)
 #undef KF_TC_EXP
@@ -40,22 +42,17 @@
 namespace {
 
 enum { TF_BF16 = 0, TF_F8 = 1, TF_Q4 = 2, TF_Q2 = 3, TF_Q1 = 4 };
-enum { TM_PLAIN = 0, TM_AFFINE = 1, TM_AFFINE_SYM = 2, TM_SCALE = 3, TM_AFFINE_FMA = 4 };  // _FMA: one bf16 rounding (ctx deq_fma, default), see kf_common.cuh
+enum { TM_PLAIN = 0, TM_AFFINE = 1, TM_SCALE = 3, TM_AFFINE_FMA = 4 };  // _FMA: one bf16 rounding (ctx deq_fma, default), see kf_common.cuh
 
 constexpr int BM = 128;    // weight rows per item (UMMA M)
 constexpr int BK = 64;     // k per stage: 64 bf16 = one 128-byte swizzle row of the B tile
-#ifndef KF_TC_RAWB
-#define KF_TC_RAWB 128
-#endif
-#ifndef KF_TC_RAWB_LOWBIT
-#define KF_TC_RAWB_LOWBIT 64
-#endif
-// packed bytes per weight row per raw stage (64: SWIZZLE_64B, 128: SWIZZLE_128B).  A K split ends on a raw-stage boundary, and 128 bytes
-// are 512 / 1024 weights of the 2- / 1-bit formats: too coarse to balance 148 SMs (1-bit 25600x5120 at 32 tokens: 71 us, 38 us with 64)
+// packed bytes per weight row per raw stage: four k-blocks of the 4-, 2- and 1-bit formats (the swizzle spans a row), two of the 8-bit one.  A K split ends on a raw-stage
+// boundary, and more than 256 weights are too coarse to balance 148 SMs (1-bit 25600x5120 at 32 tokens with 128 bytes: 71 us, 38 us with 64)
 template <int FMT>
-__host__ __device__ constexpr int raw_bytes() { return (FMT == 3 || FMT == 4) ? KF_TC_RAWB_LOWBIT : KF_TC_RAWB; }  // TF_Q2, TF_Q1
+__host__ __device__ constexpr int raw_bytes() { return FMT == 4 ? 32 : FMT == 3 ? 64 : 128; }  // TF_Q1, TF_Q2
 constexpr int kProducerWarps = 8, kMmaWarp = 8, kRawWarp = 9, kXWarp = 10, kEpiWarp0 = 11;
 constexpr int kThreadsTC = 15 * 32;
+constexpr int kTeams = 2;  // of four producer warps
 
 constexpr int kEpiGlu = 2;  // epilogue: y = silu(w0 x) * (w1 x); an item takes 64 rows of either weight
 constexpr int kMaxW = 3;  // weights of one launch (Q/K/V, gate/up): same type, same K, their row tiles share one item space
@@ -75,7 +72,9 @@ struct GemmParams {
     int cluster;               // the parts of a split are the CTAs of a cluster, one item each
     int item_lo, item_hi;      // item = (row tile * item_hi + hi) * item_lo + lo: token tile and part, the latter innermost in clusters
     int part_raw, part_rem;    // raw stages of a part; the first part_rem have one more
-    uint32_t lop_mask, lop_magic;
+    uint32_t fold2;            // qbias as bf16x2 (types without a zero)
+    int bias;                  // qbias does not fold into the zero: it is taken off the codes
+    uint32_t qsub[8];          // qbias as a number of each code field, bf16x2
 };
 
 template <int FMT>
@@ -222,28 +221,45 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t local, int cta_rank) {
     return v;
 }
 
-__device__ __forceinline__ uint32_t and_or3(uint32_t a, uint32_t b, uint32_t c) {
-    uint32_t d;
-    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-    return d;
-}
-// one pair of codes -> bf16x2 weights, bit-exact w.r.t. the reference (see gemv.cu deq_pair)
-template <int MODE>
-__device__ __forceinline__ uint32_t tdeq(uint32_t reg, int shift, uint32_t step2, uint32_t zero2, uint32_t nb2, uint32_t bias2, uint32_t mask,
-                                         uint32_t magic) {
-    const uint32_t v = and_or3(reg >> shift, mask, magic);
-    if (MODE == TM_AFFINE_FMA) {  // zero2 holds -zero: RN(step * k - zero), ONE rounding (fma.rn.bf16, as the reference built for sm_90+)
-        __nv_bfloat162 k = __hsub2_rn(u32_as_bf162(v), u32_as_bf162(bias2));
-        return bf162_as_u32(__hfma2(k, u32_as_bf162(step2), u32_as_bf162(zero2)));
+// Codes -> bf16 weights without a shift or a conversion: a code field that lies in the low byte of a 16-bit half IS the bf16 number code * 2^(bit - 133) (exponents 0 and
+// 1 share their scale, so all 256 patterns are linear), so one AND picks a pair of codes out of a register (of the register >> 8 for the upper bytes) and one bf16 fma
+// with step * 2^(133 - bit - 24) and -zero * 2^-24 rounds exactly as RN(step * code - zero) does, 2^24 smaller; the sums get the factor back (kUnscale, exact) on
+// their way out of tensor memory.  Two instructions a pair instead of four and a shift, which run at half rate on two pipes: steps stay below 2^19, weights matter
+// down to 2^-102.  (4-bit SwiGLU 51200 x 5120 at 45 tokens, with the leaner producer loop below and its larger stages: 65.5 -> 40.8 us, at 16 tokens 64 -> 38.4; ternary
+// 24576 x 4096 at 45 36 -> 24.4.)
+constexpr int kWShift     = 24;
+constexpr float kUnscale  = 16777216.0f;
+template <int BITS>
+__host__ __device__ constexpr int n_fields() { return BITS <= 4 ? 8 / BITS : 1; }  // code fields of a byte
+// per group: the multiplier of each field and -zero (one fma) or zero (two roundings), scaled
+template <int FMT, int MODE>
+struct Gama {
+    static constexpr int BITS = FMT == TF_Q4 ? 4 : FMT == TF_Q2 ? 2 : FMT == TF_Q1 ? 1 : 8, NF = n_fields<BITS>();
+    uint32_t s[NF], z;
+    // fold: qbias as a bf16x2 power of two or zero, whose product with the step is exact (types without a zero of their own)
+    __device__ __forceinline__ void set(uint32_t zero, uint32_t step, uint32_t fold2) {
+        const uint32_t st2   = __byte_perm(step, 0u, 0x1010), z2 = __byte_perm(zero, 0u, 0x1010);
+        const auto down      = [](uint32_t v, int e) {  // v * 2^e
+            const uint32_t p = (uint32_t)(127 + e) << 7;
+            return bf162_as_u32(__hmul2_rn(u32_as_bf162(v), u32_as_bf162(p | p << 16)));
+        };
+        s[0] = down(st2, 133 - kWShift);
+#pragma unroll
+        for (int f = 1; f < NF; f++) s[f] = down(s[0], -f * BITS);
+        if (MODE == TM_SCALE) z = down(bf162_as_u32(__hmul2_rn(u32_as_bf162(st2), u32_as_bf162(fold2))), -kWShift) ^ 0x80008000u;
+        else z = down(z2, -kWShift) ^ (MODE == TM_AFFINE_FMA ? 0x80008000u : 0u);
     }
-    if (MODE == TM_AFFINE) {
-        __nv_bfloat162 p = __hfma2(u32_as_bf162(v), u32_as_bf162(step2), u32_as_bf162(nb2));
-        return bf162_as_u32(__hsub2_rn(p, u32_as_bf162(zero2)));
-    }
-    __nv_bfloat162 k = __hsub2_rn(u32_as_bf162(v), u32_as_bf162(bias2));
-    __nv_bfloat162 p = __hmul2_rn(u32_as_bf162(step2), k);  // ternary / binary: exactly {-step, 0, step} / {0, step}
-    if (MODE == TM_SCALE) return bf162_as_u32(p);
-    return bf162_as_u32(__hsub2_rn(p, u32_as_bf162(zero2)));
+};
+// the codes at field f of both halves of `reg` -> bf16x2 weights * 2^-24.  BIAS: qbias (as a number of that field, qf) comes off the codes first
+template <int FMT, int MODE, bool BIAS>
+__device__ __forceinline__ uint32_t tdeq(uint32_t reg, int f, const Gama<FMT, MODE>& g, uint32_t qf) {
+    constexpr int BITS = Gama<FMT, MODE>::BITS;
+    uint32_t v         = reg & (((1u << BITS) - 1u) * 0x00010001u << (f * BITS));
+    if (BIAS) v = bf162_as_u32(__hsub2_rn(u32_as_bf162(v), u32_as_bf162(qf)));  // a small integer of the field: exact
+    if (MODE == TM_AFFINE_FMA || (MODE == TM_SCALE && !BIAS)) return bf162_as_u32(__hfma2(u32_as_bf162(v), u32_as_bf162(g.s[f]), u32_as_bf162(g.z)));
+    const __nv_bfloat162 q = __hmul2_rn(u32_as_bf162(v), u32_as_bf162(g.s[f]));  // RN(step * k)
+    if (MODE == TM_SCALE) return bf162_as_u32(q);
+    return bf162_as_u32(__hsub2_rn(q, u32_as_bf162(g.z)));  // RN(that - zero)
 }
 __device__ __forceinline__ uint32_t tf8_pair(uint32_t reg, uint32_t sel) {
     uint32_t h2 = __byte_perm(reg, 0u, sel);
@@ -251,45 +267,21 @@ __device__ __forceinline__ uint32_t tf8_pair(uint32_t reg, uint32_t sel) {
     return bf162_as_u32(__hmul2_rn(u32_as_bf162(t), u32_as_bf162(0x77807780u)));
 }
 
-// Expand the 32 weights of one slot (codes in `w`, memory order) into 16 bf16x2 registers in the permuted k order.
-template <int FMT, int MODE>
-__device__ __forceinline__ void expand_slot(uint32_t (&o)[16], const uint32_t* w, uint32_t step2, uint32_t zero2, uint32_t nb2, uint32_t bias2,
-                                            uint32_t mask, uint32_t magic) {
-    if constexpr (FMT == TF_Q4) {  // 4 registers, first codes in the LAST register, nibble c_j at bits [31-4j : 28-4j]
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const uint32_t r = w[3 - u];
-            o[4 * u + 0] = tdeq<MODE>(r, 0, step2, zero2, nb2, bias2, mask, magic);
-            o[4 * u + 1] = tdeq<MODE>(r, 4, step2, zero2, nb2, bias2, mask, magic);
-            o[4 * u + 2] = tdeq<MODE>(r, 8, step2, zero2, nb2, bias2, mask, magic);
-            o[4 * u + 3] = tdeq<MODE>(r, 12, step2, zero2, nb2, bias2, mask, magic);
-        }
-    } else if constexpr (FMT == TF_Q2) {  // 2 registers
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const uint32_t r = w[1 - (u >> 1)];
-            const int b      = 8 * (u & 1);
-            o[4 * u + 0] = tdeq<MODE>(r, b + 0, step2, zero2, nb2, bias2, mask, magic);
-            o[4 * u + 1] = tdeq<MODE>(r, b + 2, step2, zero2, nb2, bias2, mask, magic);
-            o[4 * u + 2] = tdeq<MODE>(r, b + 4, step2, zero2, nb2, bias2, mask, magic);
-            o[4 * u + 3] = tdeq<MODE>(r, b + 6, step2, zero2, nb2, bias2, mask, magic);
-        }
-    } else if constexpr (FMT == TF_Q1) {  // 1 register
-#pragma unroll
-        for (int p = 0; p < 16; p++) o[p] = tdeq<MODE>(w[0], p, step2, zero2, nb2, bias2, mask, magic);
-    } else {  // F8: 8 registers, natural order
+// Expand the 32 weights of one slot (codes in `w`, memory order) into 16 bf16x2 registers in the permuted k order.  qsub: qbias as a number of each field
+template <int FMT, int MODE, bool BIAS>
+__device__ __forceinline__ void expand_slot(uint32_t* o, const uint32_t* w, const Gama<FMT, MODE>& g, const uint32_t* qsub) {
+    if constexpr (FMT == TF_F8) {  // 8 registers, natural order
 #pragma unroll
         for (int r = 0; r < 8; r++) o[2 * r] = tf8_pair(w[r], 0x1404u), o[2 * r + 1] = tf8_pair(w[r], 0x3424u);
+    } else {  // 4 / 2 / 1 registers, first codes in the LAST; o[p] takes the fields at bits b = p * BITS .. of both halves of its register
+        constexpr int BITS = Gama<FMT, MODE>::BITS, PR = 16 / BITS, NF = Gama<FMT, MODE>::NF;
+#pragma unroll
+        for (int p = 0; p < 16; p++) {
+            const uint32_t r = w[16 / PR - 1 - p / PR];
+            const int i      = p % PR;
+            o[p] = tdeq<FMT, MODE, BIAS>(i < NF ? r : __byte_perm(r, 0u, 0x4321), i % NF, g, BIAS ? qsub[i % NF] : 0u);
+        }
     }
-}
-
-// byte offset of 32-weight slot q inside the 64-byte raw row of a stage (PackedQ.hpp:160-211: the first codes sit in word.high)
-template <int FMT>
-__device__ __forceinline__ int slot_offset(int q) {
-    if (FMT == TF_Q4) return 16 * q;
-    if (FMT == TF_Q2) return 16 * (q >> 1) + 8 * (1 - (q & 1));
-    if (FMT == TF_Q1) return 16 * (q >> 2) + 12 - 4 * (q & 3);
-    return 32 * q;  // F8
 }
 
 // Ring depths.  The three rings are decoupled because their latencies differ: the raw ring hides DRAM latency (bytes in flight per SM
@@ -298,7 +290,8 @@ __device__ __forceinline__ int slot_offset(int q) {
 template <int FMT, int BN>
 struct Rings {
     static constexpr bool A_TMEM = FMT != TF_BF16;
-    static constexpr int U       = BN <= 128 ? 2 : 1;  // k-blocks per ring stage: below 256 tokens the barrier traffic, not the MMA, paces a k-block
+    // k-blocks per stage of the A and B rings: a poll and two commits cost the MMA warp as much as eight small matrix instructions
+    static constexpr int U       = BN == 256 ? 1 : BN == 128 || FMT == TF_BF16 || FMT == TF_F8 ? 2 : 4;
     // threads that finish a CTA's last item, and its part of a cluster's sums: the producers help from 64 and from 128 tokens on.  Below that their way there takes
     // longer than their share (4-bit 4096 x 1024 at 20 tokens, whole: tile of 16 8.3 us with them, 7.8 without, of 32 8.05 and 7.8; tile of 64 at 40 tokens 8.5 and
     // 8.8; 3072 x 6144 in clusters, at 12 tokens 13.1 and 12.65, at 40 14.1 and 13.3)
@@ -309,15 +302,20 @@ struct Rings {
     static constexpr int SUB     = A_BYTES + BN * 128;  // one k-block of a stage: [A tile (bf16 weights only)][B tile]
     static constexpr int STAGE   = U * SUB;
     static constexpr int SA      = !A_TMEM ? 0 : (BN <= 64 ? 12 : 8) / U;
-    static constexpr int SB      = (A_TMEM ? (BN == 16 ? 32 : BN == 32 ? 16 : BN == 64 ? 10 : BN == 128 ? 6 : 3)
+    static constexpr int SB      = (A_TMEM ? (BN == 16 ? 32 : BN == 32 ? 20 : BN == 64 ? 12 : BN == 128 ? 6 : 3)
                                            : (BN == 16 ? 10 : BN == 32 ? 10 : BN == 64 ? 8 : BN == 128 ? 6 : 4)) / U;
     static constexpr int RAWB    = raw_bytes<FMT>();
-    static constexpr int RS      = !A_TMEM ? 0 : (BN <= 64 ? 128 : BN == 128 ? 96 : 64) * 1024 / (BM * RAWB);
+    static constexpr int RS      = !A_TMEM ? 0 : (BN <= 64 ? 96 : BN == 128 ? 96 : 64) * 1024 / (BM * 128) * (RAWB < 128 ? 2 : 1);
+
     // output buffer: the item's whole accumulator in bf16 where there is only one in tensor memory, which then goes back to the MMA warp after ~1.5 us of draining
     static constexpr int OUT     = BN == 16 ? 8 * 1024 : A_TMEM && BN > 64 ? BN * 256 : 16 * 1024;  // at least one read of tensor memory in fp32
     static constexpr size_t SMEM = (size_t)SB * STAGE + (size_t)RS * BM * RAWB + OUT + 1024;
     static_assert((size_t)SB * STAGE + (size_t)RS * BM * RAWB >= (size_t)BN * BM * 4, "the rings take the partial sums of a split over a cluster");
     static_assert(SMEM <= 226 * 1024, "shared memory budget");
+    // A barrier's phase is one bit: a producer that waits for a stage must know that the use before the one it waits for is over.  Raw stages: the slots belong to the
+    // teams, so that use was its own.  A stages: it has waited, at its last one, for a stage at most SA later
+    static_assert(RS % kTeams == 0, "every team has raw stages of its own");
+    static_assert(!A_TMEM || (kTeams - 1) * (Fmt<FMT>::KBR / U) + 1 <= SA, "a team is never two rounds of the A ring ahead");
 };
 
 struct Item {
@@ -426,9 +424,9 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
     };
     constexpr int WKB = A_TMEM ? KBR : U, WRING = A_TMEM ? RS1 : SB;  // k-blocks of a weight stage, stages of its ring
     if (warp == kRawWarp && lane == 0) {
-        for (int s = 0; s < SA; s++) mbar_init(&a_full[s], kProducerWarps), mbar_init(&a_empty[s], 1);  // one arrival per producer WARP
+        for (int s = 0; s < SA; s++) mbar_init(&a_full[s], 4), mbar_init(&a_empty[s], 1);  // one arrival per producer WARP of a team
         for (int s = 0; s < SB; s++) mbar_init(&b_full[s], A_TMEM ? 1 : 2), mbar_init(&b_empty[s], 1);
-        for (int s = 0; s < RS; s++) mbar_init(&raw_full[s], 1), mbar_init(&raw_empty[s], kProducerWarps);
+        for (int s = 0; s < RS; s++) mbar_init(&raw_full[s], 1), mbar_init(&raw_empty[s], 4);
         for (int s = 0; s < NACC; s++) mbar_init(&tmem_full[s], 1), mbar_init(&tmem_empty[s], 4);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -437,28 +435,11 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    // producers: this thread's row of zero / step; scale / zero of the current group and of the next two (register queue; the loads run 1-2 groups ahead of
-    // their use)
-    const int prow = (warp & 3) * 32 + lane, gpr = (p.K >> 7) >> p.gshift;
-    const uint16_t *zrow = nullptr, *srow = nullptr;
-    int gcur = 0;
-    uint32_t zq0 = 0, sq0 = 0, zq1 = 0, sq1 = 0, zq2 = 0, sq2 = 0;
-    auto fetch_gama = [&](const Item& w) {
-        if constexpr (MODE != TM_PLAIN) {
-            const int seg  = glu ? prow >> 6 : w.wi;
-            const int grow = min(w.n0 + (glu ? prow & 63 : prow), p.Nw[seg] - 1);
-            zrow = p.zero[seg] + (size_t)grow * gpr, srow = p.step[seg] + (size_t)grow * gpr;
-            gcur = (w.kb0 >> 1) >> p.gshift;
-            const int g1 = min(gcur + 1, gpr - 1), g2 = min(gcur + 2, gpr - 1);
-            zq0 = __ldg(zrow + gcur), sq0 = __ldg(srow + gcur);
-            zq1 = __ldg(zrow + g1), sq1 = __ldg(srow + g1);
-            zq2 = __ldg(zrow + g2), sq2 = __ldg(srow + g2);
-        }
-    };
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = tmem_base_smem;
+    // all 512 columns start at address 0: a constant keeps the MMA warp's operands in uniform registers, a value out of shared memory would be moved there for each instruction
+    const uint32_t tmem_base = TMEM_COLS == 512 ? 0u : tmem_base_smem;
     kf_grid_launch_dependents();
 
     // ============ the end of an item: TMEM -> registers -> output buffer in shared memory -> Y in 16-byte accesses, or partial sums of a split.  Runs on the
@@ -468,6 +449,7 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
     // 6144 x 1024 at 700, one item per CTA, 22.1 -> 16.5) ============
     const int fin_t     = warp < kProducerWarps ? 128 + tid : tid - kEpiWarp0 * 32;  // 0 .. 127: epilogue warps
     const bool f32out   = p.epilogue == 4;
+    auto sum_of         = [](uint32_t v) { return __uint_as_float(v) * (MODE == TM_PLAIN ? 1.0f : kUnscale); };
     constexpr int kRes  = 4;  // residual pieces in flight per thread
     // the residual of pieces j0 .. j0 + kRes - 1 of this thread: piece i = token t0 + i / 16, rows 8 (i % 16) ..
     auto fetch_res = [&](uint4 (&res)[kRes], const Item& w, int m0, int N, int t0, int t1, int j0, int nthr) {
@@ -563,8 +545,9 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
                     else tmem_ld32(tbase + (uint32_t)c0, v);
 #pragma unroll
                     for (int j = 0; j < TC; j++) {
-                        if (f32out) *reinterpret_cast<uint32_t*>(outs + (c0 - r0 + j) * 512 + row * 4) = v[j];
-                        else *reinterpret_cast<uint16_t*>(outs + (c0 - r0 + j) * 256 + row * 2) = f32_to_bf16_bits(__uint_as_float(v[j]));  // the reference's GEMM output is bf16 (gemm.cu:124-126)
+                        const float sum = sum_of(v[j]);
+                        if (f32out) *reinterpret_cast<float*>(outs + (c0 - r0 + j) * 512 + row * 4) = sum;
+                        else *reinterpret_cast<uint16_t*>(outs + (c0 - r0 + j) * 256 + row * 2) = f32_to_bf16_bits(sum);  // the reference's GEMM output is bf16 (gemm.cu:124-126)
                     }
                 }
                 if (r1 == cnt) release();
@@ -580,11 +563,11 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
             if (p.splits > 1) {
 #pragma unroll
                 for (int j = 0; j < 16; j++)
-                    if (c0 + j < cnt) wsp[(size_t)(c0 + j) * BM + row] = __uint_as_float(v[j]);
+                    if (c0 + j < cnt) wsp[(size_t)(c0 + j) * BM + row] = sum_of(v[j]);
             } else if (w.n0 + row < N) {
                 float acc[16];
 #pragma unroll
-                for (int j = 0; j < 16; j++) acc[j] = __uint_as_float(v[j]);
+                for (int j = 0; j < 16; j++) acc[j] = sum_of(v[j]);
                 store_cols<16>(p, p.y[w.wi], N, acc, m0 + c0, cnt - c0, w.n0 + row);
             }
         }
@@ -630,110 +613,128 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
 
     if (warp < kProducerWarps) {
         if constexpr (A_TMEM) {
-            // ============ producers: thread = (weight row, 32-weight slot of the k-block): raw bytes -> bf16 -> TMEM ============
-            const int quad = warp & 3, slot = warp >> 2;
-            const int row  = prow;
-            const uint32_t bias2 = pack_bf16x2((float)(128 + p.qbias), (float)(128 + p.qbias));
-            // TMA swizzle of the raw stage: the 16-byte chunk index is XORed with address bits [7,9) (64-byte rows) / [7,10) (128-byte rows)
-            const uint32_t rsw   = RAWB == 64 ? (uint32_t)((row >> 1) & 3) : (uint32_t)(row & 7);
-            constexpr int UNIT = KBR >= 2 ? 2 : 1;  // k-blocks expanded together (independent work for the scheduler)
-            constexpr int NW   = F::SLOTB / 4;      // registers of one packed slot
-            const uint32_t raw_thread = smem_u32(raws) + (uint32_t)(row * RAWB);
-            const uint32_t a_thread   = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(A_COL0 + slot * 16);
+            // ============ producers: raw bytes -> bf16 -> TMEM.  Teams of four warps take the raw stages in turn; a warp expands all of a stage for 32 weight rows
+            // (thread = row).  What bounds them is the number of instructions: with the two slots of 32 weights on two warps, a poll of the free A stage and a wait for the
+            // stores per two k-blocks, and zero / step fetched by both warps, 440 clk a k-block were spent where the bytes take 187; now 250.  A second set of eight warps
+            // gained nothing once the loop was lean (41.4 us against 40.9) ============
+            constexpr int NW = F::SLOTB / 4;                           // registers of one packed slot of 32 weights
+            constexpr int SPR = KBR / U, TEAMS = kTeams;  // A stages of a raw stage
+            const int quad = warp & 3, team = warp >> 2;
+            const int row = quad * 32 + lane, gpr = (p.K >> 7) >> p.gshift;
+            // the row's first byte in a raw stage.  TMA swizzle: the 16-byte chunk index is XORed with address bits [7,8) (32-byte rows) / [7,9) (64) / [7,10) (128)
+            const uint32_t rsw     = RAWB == 32 ? (uint32_t)((row >> 2) & 1) : RAWB == 64 ? (uint32_t)((row >> 1) & 3) : (uint32_t)(row & 7);
+            const uint32_t raw_row = smem_u32(raws) + (uint32_t)(row * RAWB) + (rsw << 4);
+            const uint32_t a_row   = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)A_COL0;
             const uint32_t full0 = smem_u32(&a_full[0]), empty0 = smem_u32(&a_empty[0]);
             const uint32_t rfull0 = smem_u32(&raw_full[0]), rempty0 = smem_u32(&raw_empty[0]);
-            uint32_t s = 0, eph = 1, rs = 0, rph = 0;  // ring positions and the parities to wait for
-            fetch_gama(decode_item<KBR>(p, blockIdx.x));  // beside the first weights, which are as long on their way; in front of the barrier it held up the loaders (12288 x 3072 at 12 tokens + 0.4 us)
-            for (int item = blockIdx.x; item < p.n_items; item += gridDim.x) {
-                const Item w = decode_item<KBR>(p, item);
-                if (item != (int)blockIdx.x) fetch_gama(w);
-                uint32_t step2 = 0, zero2 = 0, nb2 = 0;
-                if (MODE != TM_PLAIN) {
-                    step2 = __byte_perm(sq0, 0u, 0x1010), zero2 = __byte_perm(zq0, 0u, 0x1010) ^ (MODE == TM_AFFINE_FMA ? 0x80008000u : 0u);
-                    if (MODE == TM_AFFINE) nb2 = bf162_as_u32(__hmul2_rn(u32_as_bf162(step2), u32_as_bf162(0xC300C300u)));
+            // zero / step of the groups in a raw stage; fetched a round ahead (the first beside the first weights, which are as long on their way)
+            constexpr int GN = KBR / 2;
+            uint32_t zn[GN] = {}, sn[GN] = {};
+            const uint16_t *zrow = nullptr, *srow = nullptr;
+            auto rows_of = [&](const Item& w) {
+                if constexpr (MODE != TM_PLAIN) {
+                    const int seg  = glu ? row >> 6 : w.wi;
+                    const int grow = min(w.n0 + (glu ? row & 63 : row), p.Nw[seg] - 1);
+                    zrow = p.zero[seg] + (size_t)grow * gpr, srow = p.step[seg] + (size_t)grow * gpr;
                 }
-                const int r1 = (w.kb1 + KBR - 1) / KBR;
-                for (int r = w.kb0 / KBR; r < r1; r++) {
-                    // ---- this thread's slots of the raw stage: one per k-block ----
-                    mbar_wait_a(rfull0 + rs * 8, rph);
-                    const uint32_t src = raw_thread + rs * RAW_BYTES;
-                    uint32_t wreg[KBR][NW];
+            };
+            auto fetch_gama = [&](int r) {
+                if constexpr (MODE != TM_PLAIN) {
 #pragma unroll
-                    for (int kin = 0; kin < KBR; kin++) {
-                        const int boff = slot_offset<FMT>(kin * 2 + slot);
-                        if constexpr (F::SLOTB == 32) {
-                            lds128(src + ((((uint32_t)(boff >> 4) + 0) ^ rsw) << 4), &wreg[kin][0]);
-                            lds128(src + ((((uint32_t)(boff >> 4) + 1) ^ rsw) << 4), &wreg[kin][4]);
-                        } else if constexpr (F::SLOTB == 16) {
-                            lds128(src + (((uint32_t)(boff >> 4) ^ rsw) << 4), &wreg[kin][0]);
-                        } else if constexpr (F::SLOTB == 8) {
-                            lds64(src + (((uint32_t)(boff >> 4) ^ rsw) << 4) + (boff & 15), &wreg[kin][0]);
-                        } else {
-                            wreg[kin][0] = lds32(src + (((uint32_t)(boff >> 4) ^ rsw) << 4) + (boff & 15));
-                        }
+                    for (int j = 0; j < GN; j++) {
+                        const int g = min((r * (KBR / 2) + j) >> p.gshift, gpr - 1);
+                        zn[j] = __ldg(zrow + g), sn[j] = __ldg(srow + g);
                     }
-                    const uint32_t rdone = rempty0 + rs * 8;
-                    if (++rs == RS) rs = 0, rph ^= 1;
+                }
+            };
+            auto produce = [&](auto bias) {
+                uint32_t a0 = 0, raw0 = 0;  // A and raw stages of the items so far
+                Item w = decode_item<KBR>(p, blockIdx.x);
+                auto first = [&]() { return w.kb0 / KBR + (int)(((uint32_t)team + raw0) % (uint32_t)TEAMS); };  // the team's first raw stage of an item
+                rows_of(w), fetch_gama(first());
+                for (int item = blockIdx.x; item < p.n_items;) {
+                    const int rb = w.kb0 / KBR, re = (w.kb1 + KBR - 1) / KBR, kend = w.kb1;
+                    int r = first();
+                    const uint32_t a1 = a0 + (uint32_t)((r - rb) * SPR), raw1 = raw0 + (uint32_t)(r - rb);
+                    uint32_t s = a1 % SA, eph = (a1 / SA & 1u) ^ 1u, rs = raw1 % RS, rph = raw1 / RS & 1u;
+                    a0 += (uint32_t)(w.kb1 - w.kb0 + U - 1) / U, raw0 += (uint32_t)(re - rb);
+                    auto next_item = [&]() {  // and its first zero / step
+                        item += gridDim.x;
+                        if (item < p.n_items) w = decode_item<KBR>(p, item), rows_of(w), fetch_gama(first());
+                    };
+                    if (r >= re) next_item();
+                    while (r < re) {
+                        const int nk = kend - r * KBR;  // k-blocks from here to the end of the part: an even number
+                        mbar_wait_a(rfull0 + rs * 8, rph);
+                        const uint32_t src = raw_row + rs * RAW_BYTES;
+                        uint32_t zc[GN], sc[GN];
 #pragma unroll
-                    for (int kin = 0; kin < KBR; kin += UNIT) {
-                        const int kb = r * KBR + kin;
-                        if (KBR > 2 && kb >= w.kb1) break;  // ragged last raw stage (K is a multiple of 128: never splits a unit)
-                        if (MODE != TM_PLAIN) {
-                            const int gi = (kb >> 1) >> p.gshift;
-                            if (gi != gcur) {  // rotate the queue, fetch two groups ahead
-                                gcur = gi;
-                                zq0 = zq1, sq0 = sq1, zq1 = zq2, sq1 = sq2;
-                                const int g2 = min(gi + 2, gpr - 1);
-#if !(KF_TC_EXP & 4)
-                                zq2 = __ldg(zrow + g2), sq2 = __ldg(srow + g2);
-#endif
-                                step2 = __byte_perm(sq0, 0u, 0x1010), zero2 = __byte_perm(zq0, 0u, 0x1010) ^ (MODE == TM_AFFINE_FMA ? 0x80008000u : 0u);
-                                if (MODE == TM_AFFINE) nb2 = bf162_as_u32(__hmul2_rn(u32_as_bf162(step2), u32_as_bf162(0xC300C300u)));
+                        for (int j = 0; j < GN; j++) zc[j] = zn[j], sc[j] = sn[j];
+                        r += TEAMS;
+                        if (r < re) fetch_gama(r);
+                        else next_item();
+                        Gama<FMT, MODE> gm;
+#pragma unroll
+                        for (int k = 0; k < KBR; k++) {
+                            if (KBR > 2 && (k & 1) == 0 && k >= nk) break;
+                            uint32_t v[2 * NW];  // both slots of the k-block, the first codes in the last register of each
+                            if constexpr (F::SLOTB >= 16) {
+#pragma unroll
+                                for (int c = 0; c < NW / 2; c++) lds128(src ^ (uint32_t)((k * (NW / 2) + c) << 4), &v[4 * c]);
+                            } else if constexpr (F::SLOTB == 8) {  // 16 bytes a k-block, the first slot in their upper half
+                                uint32_t q[4];
+                                lds128(src ^ (uint32_t)(k << 4), q);
+                                v[0] = q[2], v[1] = q[3], v[2] = q[0], v[3] = q[1];
+                            } else {  // 8 bytes a k-block, likewise in 16
+                                uint32_t q[2];
+                                lds64((src ^ (uint32_t)(k >> 1 << 4)) + ((k & 1) ? 0 : 8), q);
+                                v[0] = q[1], v[1] = q[0];
                             }
-                        }
-                        uint32_t o[UNIT][16];
-#pragma unroll
-                        for (int u = 0; u < UNIT; u++) {
+                            if (MODE != TM_PLAIN && (k & 1) == 0) gm.set(zc[k / 2], sc[k / 2], p.fold2);
+                            uint32_t o[32];
 #if KF_TC_EXP & 1
-                            for (int i = 0; i < 16; i++) o[u][i] = wreg[kin + u][i % NW] ^ step2;
+                            for (int i = 0; i < 32; i++) o[i] = v[i % (2 * NW)] ^ gm.z;
 #else
-                            expand_slot<FMT, MODE>(o[u], wreg[kin + u], step2, zero2, nb2, bias2, p.lop_mask, p.lop_magic);
+                            expand_slot<FMT, MODE, decltype(bias)::value>(o, &v[0], gm, p.qsub);
+                            expand_slot<FMT, MODE, decltype(bias)::value>(o + 16, &v[NW], gm, p.qsub);
 #endif
-                        }
-                        uint32_t sfull[UNIT];
-#pragma unroll
-                        for (int u = 0; u < UNIT; u++) {
-                            if (u % U == 0) {
+                            if (k % U == 0) {
                                 mbar_wait_a(empty0 + s * 8, eph);
                                 tc_fence_after();
                             }
 #if KF_TC_EXP & 2
-                            asm volatile("" ::"r"(o[u][0] ^ o[u][5] ^ o[u][10] ^ o[u][15]));
+                            asm volatile("" ::"r"(o[0] ^ o[5] ^ o[10] ^ o[15] ^ o[17] ^ o[22] ^ o[27] ^ o[31]));
 #else
-                            tmem_st16(a_thread + s * (32 * U) + (u % U) * 32, o[u]);
+                            tmem_st32(a_row + s * (32 * U) + (k % U) * 32, o);
 #endif
-                            sfull[u] = full0 + s * 8;
-                            if (u % U == U - 1)
+                            // The raw stage goes back to the loader with its last A stage: tcgen05.wait::st cannot complete before the weights it stores have been
+                            // computed, so every byte of the stage has reached its register.  An arrival right behind the shared-memory loads is no such proof: it
+                            // overtakes loads that still queue in the load / store unit (behind a burst of zero / step fetches at the start of an item), the loader
+                            // refills the stage and lanes expand the bytes of the stage RS further on (4-bit 8192 x 5120 at 2048 tokens: every call wrong).  One
+                            // arrival per warp: per-thread arrivals on one barrier word serialise in the shared-memory atomic unit.
+                            if (k % U == U - 1 || (k & 1 && k + 1 >= nk)) {
+                                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                                tc_fence_before();
+                                __syncwarp();
+                                if (lane == 0) {
+                                    mbar_arrive_a(full0 + s * 8);
+                                    if (k == KBR - 1 || (k & 1 && k + 1 >= nk)) mbar_arrive_a(rempty0 + rs * 8);
+                                }
                                 if (++s == SA) s = 0, eph ^= 1;
+                            }
                         }
-                        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) {
-#pragma unroll
-                            for (int u = U - 1; u < UNIT; u += U) mbar_arrive_a(sfull[u]);
-                        }
+                        rs += TEAMS;
+                        if (rs >= RS) rs -= RS, rph ^= 1;
+                        // over the other teams' stages
+                        constexpr int OVER = (TEAMS - 1) * SPR;
+                        s += OVER % SA;
+                        if (s >= SA) s -= SA, eph ^= 1;
+                        if (OVER / SA & 1) eph ^= 1;
                     }
-                    // Hand the stage back to the loader only now: tcgen05.wait::st above cannot complete before the weights it stores have been
-                    // computed, so every byte of the stage has reached its register.  An arrival right behind the shared-memory loads is
-                    // no such proof: it overtakes loads that still queue in the load / store unit (behind a burst of zero / step fetches at the
-                    // start of an item), the loader refills the stage and lanes expand the bytes of the stage RS further on (4-bit 8192 x 5120 at
-                    // 2048 tokens: every call wrong).  One arrival per warp: 256 per-thread arrivals on one barrier word serialise in the
-                    // shared-memory atomic unit.
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive_a(rdone);
                 }
-            }
+            };
+            if (p.bias) produce(std::true_type());
+            else produce(std::false_type());
         }
     } else if (warp == kRawWarp) {
         if (lane == 0) {
@@ -760,10 +761,10 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
 #if KF_TC_EXP & 16
                     mbar_arrive(&b_full[s]);
 #else
-                    mbar_arrive_expect_tx(&b_full[s], U * B_BYTES);
+                    mbar_arrive_expect_tx(&b_full[s], min(U, w.kb1 - kb) * B_BYTES);
 #pragma unroll
                     for (int u = 0; u < U; u++)
-                        tma_load_2d(tiles + (size_t)s * STAGE + u * SUB + A_BYTES, &tm_x, (kb + u) * BK, w.m0 * BN, &b_full[s]);
+                        if (u < 2 || kb + u < w.kb1) tma_load_2d(tiles + (size_t)s * STAGE + u * SUB + A_BYTES, &tm_x, (kb + u) * BK, w.m0 * BN, &b_full[s]);
 #endif
                     it++;
                 }
@@ -775,6 +776,7 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
         constexpr uint32_t idesc = make_idesc_bf16(BN);
         uint32_t ait = 0;
         uint32_t sa = 0, aph = 0, sb = 0, bph = 0;  // ring positions and the parities to wait for
+        uint32_t okb = 0, oka = A_TMEM ? 0 : 1;
         const uint32_t bfull0 = smem_u32(&b_full[0]), bempty0 = smem_u32(&b_empty[0]);
         const uint32_t afull0 = smem_u32(&a_full[0]), aempty0 = smem_u32(&a_empty[0]);
         const uint32_t tiles0 = smem_u32(tiles);
@@ -785,23 +787,17 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
             tc_fence_after();
             const uint32_t tmem_d = tmem_base + (uint32_t)(buf * BN);
             uint32_t acc = 0;
-            for (int kb = w.kb0; kb < w.kb1; kb += U) {
-                {  // both polls are issued before either result is consumed (a try_wait takes ~90 cycles even when complete)
-                    const uint32_t ab = bfull0 + sb * 8, aa = afull0 + (A_TMEM ? sa : 0) * 8;
-                    const uint32_t okb = mbar_try(ab, bph), oka = A_TMEM ? mbar_try(aa, aph) : 1u;
-                    if (!okb) mbar_wait_slow(ab, bph);
-                    if (!oka) mbar_wait_slow(aa, aph);
-                }
+            auto stage = [&](auto blocks) {
+                if (!okb) mbar_wait_a(bfull0 + sb * 8, bph);
+                if (!oka) mbar_wait_a(afull0 + sa * 8, aph);
                 tc_fence_after();
 #pragma unroll
-                for (int u = 0; u < U; u++) {
+                for (int u = 0; u < decltype(blocks)::value; u++) {
                     const uint32_t st_addr = tiles0 + sb * STAGE + u * SUB;
                     const uint64_t bdesc   = make_desc_sw128(st_addr + A_BYTES);
                     if constexpr (A_TMEM) {
                         const uint32_t ta = tmem_base + (uint32_t)(A_COL0 + sa * (32 * U) + u * 32);
-#pragma unroll
-                        for (int k = 0; k < ((KF_TC_EXP & 32) ? 0 : BK / 16); k++)  // 16 bf16 of K per MMA: +32 bytes in the swizzle row / +8 TMEM columns
-                            umma_ts(tmem_d, ta + (uint32_t)(k * 8), bdesc + (uint64_t)(2 * k), idesc, (k > 0 || u > 0) ? 1u : acc);
+                        umma_ts_x4(tmem_d, ta, bdesc, idesc, u > 0 ? 1u : acc);
                     } else {
                         const uint64_t adesc = make_desc_sw128(st_addr);
 #pragma unroll
@@ -816,8 +812,13 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
                 if constexpr (A_TMEM) {
                     umma_commit_a(aempty0 + sa * 8);
                     if (++sa == SA) sa = 0, aph ^= 1;
+                    oka = mbar_test(afull0 + sa * 8, aph);
                 }
-            }
+                okb = mbar_test(bfull0 + sb * 8, bph);  // the next stage's state, asked for ahead of the loop's bookkeeping (a poll takes ~90 cycles)
+            };
+            int kb = w.kb0;
+            for (; kb + U <= w.kb1; kb += U) stage(std::integral_constant<int, U>());
+            if (U > 2 && kb < w.kb1) stage(std::integral_constant<int, 2>());  // K is a multiple of 128
             umma_commit_a(smem_u32(&tmem_full[buf]));
             ait++;
         }
@@ -847,7 +848,7 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
                 uint32_t v[16];
                 tmem_ld16(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, v);
 #pragma unroll
-                for (int j = 0; j < 16; j++) sums[(c0 + j) * BM] = __uint_as_float(v[j]);
+                for (int j = 0; j < 16; j++) sums[(c0 + j) * BM] = sum_of(v[j]);
             }
         }
     }
@@ -1052,7 +1053,7 @@ int launch_tc(kf_ctx* ctx, GemmParams& p, const void* const* wdata, int nw, cons
         const int j = i < nw ? i : 0;  // unused slots repeat the first weight (never dereferenced)
         if (A_TMEM)
             rc = kf_tmap_2d(ctx, &tm_w[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, wdata[j], (uint64_t)p.K * F::BITS / 8, (uint64_t)p.Nw[j], F::RAWB, glu ? BM / 2 : BM,
-                            F::RAWB == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, true);
+                            F::RAWB == 32 ? CU_TENSOR_MAP_SWIZZLE_32B : F::RAWB == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, true);
         else
             rc = kf_tmap_2d(ctx, &tm_w[i], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, wdata[j], (uint64_t)p.K, (uint64_t)p.Nw[j], BK, glu ? BM / 2 : BM,
                             CU_TENSOR_MAP_SWIZZLE_128B, true);
@@ -1126,12 +1127,20 @@ int tc_format(const kf_tensor_desc* w, int* fmt, int* mode, int deq_fma) {
     switch (w->type) {
         case KF_T_BF16: *fmt = TF_BF16, *mode = TM_PLAIN; return KF_OK;
         case KF_T_F8E5M2: *fmt = TF_F8, *mode = TM_PLAIN; return KF_OK;
-        case KF_T_Q4: *fmt = TF_Q4, *mode = deq_fma ? TM_AFFINE_FMA : w->qbias == 0 ? TM_AFFINE : TM_AFFINE_SYM; return KF_OK;
-        case KF_T_Q2: *fmt = TF_Q2, *mode = deq_fma ? TM_AFFINE_FMA : w->qbias == 0 ? TM_AFFINE : TM_AFFINE_SYM; return KF_OK;
+        case KF_T_Q4: *fmt = TF_Q4, *mode = deq_fma ? TM_AFFINE_FMA : TM_AFFINE; return KF_OK;
+        case KF_T_Q2: *fmt = TF_Q2, *mode = deq_fma ? TM_AFFINE_FMA : TM_AFFINE; return KF_OK;
         case KF_T_SIGN: *fmt = TF_Q2, *mode = TM_SCALE; return KF_OK;
         case KF_T_BINARY: *fmt = TF_Q1, *mode = TM_SCALE; return KF_OK;
     }
     return KF_ERR_UNSUPPORTED;
+}
+
+// the bf16 number q * 2^(bit - 133), |q| < 256
+uint32_t field_bf16(int q, int bit) {
+    const float v = std::ldexp((float)q, bit - 133);  // exact, also below the normal range
+    uint32_t u;
+    memcpy(&u, &v, 4);
+    return u >> 16;
 }
 
 }  // namespace
@@ -1203,7 +1212,12 @@ int kf_gemm_tc_multi(kf_ctx* ctx, int n, void* const* y, const kf_tensor_desc* w
     const void* wdata[kMaxW] = {};
     p.residual = (const uint16_t*)residual, p.M = M, p.K = K;
     p.qbias = w[0].qbias, p.epilogue = epilogue;
-    p.lop_mask = fmt == TF_Q4 ? 0x000F000Fu : fmt == TF_Q2 ? 0x00030003u : 0x00010001u, p.lop_magic = 0x43004300u;
+    if (mode != TM_PLAIN) {
+        const int q = w[0].qbias, bits = fmt == TF_Q4 ? 4 : fmt == TF_Q2 ? 2 : 1;
+        p.bias = mode == TM_SCALE ? (q & (q - 1)) != 0 : q != 0;
+        for (int f = 0; f < 8 / bits; f++) p.qsub[f] = field_bf16(q, f * bits) * 0x00010001u;
+        p.fold2 = field_bf16(q, 133) * 0x00010001u;
+    }
     for (int i = 0; i < n; i++) {
         int f2, m2;
         KF_REQUIRE(ctx, y[i] && !tc_format(&w[i], &f2, &m2, ctx->deq_fma) && f2 == fmt && m2 == mode && w[i].cols == K && w[i].group == w[0].group &&
@@ -1231,9 +1245,7 @@ int kf_gemm_tc_multi(kf_ctx* ctx, int n, void* const* y, const kf_tensor_desc* w
     KF_TC_CASE(TF_Q4, TM_AFFINE_FMA)
     KF_TC_CASE(TF_Q2, TM_AFFINE_FMA)
     KF_TC_CASE(TF_Q4, TM_AFFINE)
-    KF_TC_CASE(TF_Q4, TM_AFFINE_SYM)
     KF_TC_CASE(TF_Q2, TM_AFFINE)
-    KF_TC_CASE(TF_Q2, TM_AFFINE_SYM)
     KF_TC_CASE(TF_Q2, TM_SCALE)
     KF_TC_CASE(TF_Q1, TM_SCALE)
     KF_TC_CASE(TF_F8, TM_PLAIN)

@@ -119,6 +119,40 @@ def _ptr(t):
     return t.data_ptr()
 
 
+@pytest.mark.parametrize("fma", [0, 1])
+@pytest.mark.parametrize("typ,bits,qbias", [(kf.KF_T_Q4, 4, 0), (kf.KF_T_Q4, 4, 8), (kf.KF_T_Q4, 4, 117), (kf.KF_T_Q2, 2, 0), (kf.KF_T_Q2, 2, -2), (kf.KF_T_SIGN, 2, 0), (kf.KF_T_SIGN, 2, 1),
+                                            (kf.KF_T_SIGN, 2, 3), (kf.KF_T_BINARY, 1, 0), (kf.KF_T_BINARY, 1, 1)])
+@pytest.mark.parametrize("M,rows,cols", [(9, 16, 128), (40, 144, 640), (128, 272, 384), (256, 128, 1152)])
+def test_tc_weights_bit_for_bit(ctx, typ, bits, qbias, fma, M, rows, cols):
+    """Each token picks one column, so the result is the weight itself: the codes that the matmul expands inside its own number format round as kf_dequant does, for steps
+    from 2^-40 to 2^15, zeros of any size beside them, codes with and without a bias, and reductions that end inside a stage."""
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(3 * M + bits + qbias)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    data = torch.randint(0, 256, (rows, cols * bits // 8), generator=g, device="cuda", dtype=torch.uint8)
+    n = rows * cols // 128
+    step = (rnd(n) * torch.exp2(torch.randint(-40, 16, (n,), generator=g, device="cuda").float())).bfloat16()
+    zero = (rnd(n) * 4 * step.float()).bfloat16() if typ in (kf.KF_T_Q4, kf.KF_T_Q2) else torch.zeros(n, device="cuda").bfloat16()
+    step[::17], zero[::13] = 0, 0
+    gama = torch.cat([torch.ones(rows + cols, device="cuda").bfloat16(), zero, step]).contiguous()
+    desc = kf.TensorDesc(data.data_ptr(), gama.data_ptr(), rows, cols, typ, 128, qbias, None, None)
+    import ctypes as C
+    w, y = torch.zeros(rows, cols, device="cuda").bfloat16(), torch.zeros(M, rows, device="cuda").bfloat16()
+    k = (torch.arange(M, device="cuda") * 37 + 5) % cols
+    x = torch.zeros(M, cols, device="cuda").bfloat16()
+    x[torch.arange(M, device="cuda"), k] = 1
+    torch.cuda.synchronize()
+    ctx.set_int("deq_fma", fma), ctx.set_int("tc_min_m", 1)
+    try:
+        ctx.check(ctx.lib.kf_dequant(ctx.h, C.byref(desc), w.data_ptr()), "dequant")
+        ctx.check(ctx.lib.kf_linear(ctx.h, y.data_ptr(), C.byref(desc), x.data_ptr(), M, kf.KF_EPI_NONE, None), "linear")
+        ctx.sync()
+    finally:
+        ctx.set_int("deq_fma", 1), ctx.set_int("tc_min_m", -1)
+    assert bool((y.float() == w[:, k].T.float()).all())
+
+
 @pytest.mark.parametrize("typ", [kf.KF_T_Q4, kf.KF_T_BINARY, kf.KF_T_F8E5M2, kf.KF_T_BF16])
 @pytest.mark.parametrize("M,tc_bn,splits", [(9, 16, 1), (9, 32, 3), (17, 16, 2), (33, 64, 0), (64, 32, 5), (65, 128, 1), (129, 64, 1), (130, 256, 2), (255, 128, 3),
                                             (257, 0, 0), (300, 256, 1)])
