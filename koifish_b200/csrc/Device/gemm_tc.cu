@@ -1078,14 +1078,15 @@ int launch_tc(kf_ctx* ctx, GemmParams& p, const void* const* wdata, int nw, cons
     return KF_OK;
 }
 // Token tile and k-split by their modelled time: waves x (k-blocks x time per k-block + epilogue) + the fix-up of split sums.  The times per k-block of 64 are
-// measured ones (us; 4-bit and bf16 weights, the former stand for all that are expanded; below 64 tokens the weights' bytes or their expansion, above the matrix
+// measured ones (us; the 4-, 2- and 1-bit types share theirs; below 64 tokens the weights' bytes or their expansion, above the matrix
 // instructions).  Splitting pays for few row tiles and a handful of tokens only: 1024 x 3072 at 16 tokens 9.9 us in 8 parts against 15.7 whole, at 256 tokens 34 against
 // 17.  (The rule before it charged BN / 16 k-blocks for the fix-up: 1024 x 3072 at 256 tokens went into 12 parts and took 91 us.)  Parts that fit on the GPU as clusters
 // cost no second pass, but the placement of the clusters, two barriers and the sum: 2.5 to 7 us, less for bf16 weights (the same for SwiGLU in the
 // epilogue, so that it has the bits of gate and up written out first); a
 // split through the workspace has a fixed cost of its own, which shows where it is one wave; so does the fetching of the same weights by several small token tiles.  Swept
 // over 124 shapes, five types and 8 to 1000 tokens, every tile and up to 12 parts: the choice is 1.5 % behind the best in the mean, more than 5 % in 45 of 372 cases;
-// with clusters at 1 us + 0.006 BN it was 2.0 % and 58 (1-bit SwiGLU 7680 x 1536 at 40 tokens went into two parts of 64, 12.2 us; whole 10.5).  The reference-exact
+// with clusters at 1 us + 0.006 BN it was 2.0 % and 58 (1-bit SwiGLU 7680 x 1536 at 40 tokens went into two parts of 64, 12.2 us; whole 10.5).  The packed types were swept
+// again with their lighter expansion, 90 shapes: 0.7 % behind the best, 5 cases above 5 %, with the earlier prices 2.8 % and 17.  The reference-exact
 // arithmetic keeps the earlier rule and the order of sums it was compared in.
 template <int FMT, int MODE>
 int launch_tc_bn(kf_ctx* ctx, GemmParams& p, const void* const* wdata, int nw, const void* xp) {
@@ -1096,9 +1097,10 @@ int launch_tc_bn(kf_ctx* ctx, GemmParams& p, const void* const* wdata, int nw, c
     for (int b = 16, i = 0; b <= 256; b *= 2, i++) {
         const int by_m = p.M > 128 ? 256 : p.M > 64 ? 128 : p.M > 32 ? 64 : p.M > 16 ? 32 : 16;  // one token tile where the panel fits one
         if (ctx->tc_bn > 0 ? b != ctx->tc_bn : ctx->gemv_exact ? b != by_m : ((b < 256 && p.M > 8 * b) || (b > 16 && p.M <= b / 2))) continue;
-        static const double kb_packed[5] = {0.235, 0.235, 0.24, 0.26, 0.42}, kb_bf16[5] = {0.09, 0.10, 0.16, 0.24, 0.39};
+        static const double kb_packed[5] = {0.154, 0.154, 0.15, 0.219, 0.361}, kb_f8[5] = {0.235, 0.235, 0.24, 0.26, 0.42}, kb_bf16[5] = {0.09, 0.10, 0.16, 0.24, 0.39};
+        constexpr bool PACKED = FMT != TF_BF16 && FMT != TF_F8;
         const int m_tiles = (p.M + b - 1) / b, items = tiles * m_tiles;
-        const double t_kb0 = FMT == TF_BF16 ? kb_bf16[i] : kb_packed[i];
+        const double t_kb0 = FMT == TF_BF16 ? kb_bf16[i] : FMT == TF_F8 ? kb_f8[i] : kb_packed[i];
         const int given = std::min(ctx->gemv_splitk, nraw);  // > 0: the split asked for
         for (int s = given > 0 ? given : 1; s <= (given > 0 ? given : std::min(16, nraw)); s++) {
             const int waves = (items * s + ctx->sm_count - 1) / ctx->sm_count, len = (nraw + s - 1) / s * KBR;
@@ -1108,9 +1110,9 @@ int launch_tc_bn(kf_ctx* ctx, GemmParams& p, const void* const* wdata, int nw, c
                 continue;
             }
             const bool cluster = s > 1 && s <= 8 && items * s <= ctx->sm_count && items * s <= cluster_ctas<FMT, MODE>(ctx, b, s);
-            const double t_kb = t_kb0 * (waves == 1 && b <= 64 ? 1.0 + 0.033 * (m_tiles - 1) : 1.0);
-            const double t = cluster ? len * t_kb + 2.5 + 0.017 * b + 0.03 * (s - 2) - (FMT == TF_BF16 ? 0.2 + 0.0025 * b : 0.0)
-                                     : waves * (len * t_kb + 0.5 + 0.006 * b + (s > 1 ? 0.5 + 0.02 * b : 0.0)) + (s > 1 ? b * (0.03 + 0.008 * s) + (waves == 1 ? 1.5 : 0.0) : 0.0);
+            const double t_kb = t_kb0 * (waves == 1 && b <= 64 ? 1.0 + (PACKED ? 0.045 : 0.033) * (m_tiles - 1) : 1.0);
+            const double t = cluster ? len * t_kb + (PACKED ? 2.9 : 2.5) + 0.017 * b + 0.03 * (s - 2) - (FMT == TF_BF16 ? 0.2 + 0.0025 * b : 0.0)
+                                     : waves * (len * t_kb + (PACKED ? 0.6 : 0.5) + 0.006 * b + (s > 1 ? 0.5 + 0.02 * b : 0.0)) + (s > 1 ? b * (0.03 + 0.008 * s) + (waves == 1 ? 1.5 : 0.0) : 0.0);
             if (t < best * 0.98) best = t, plan = {b, s, cluster};
         }
     }
