@@ -14,6 +14,11 @@
 #include "kf_common.cuh"
 
 namespace {
+// first of `len` positions of part `i` of n: floor(i * len / n) without a 64-bit division (a hundred instructions each at the head of every CTA)
+__device__ __forceinline__ int split_at(int i, int len, int n) {
+    const unsigned d = (unsigned)len / (unsigned)n, r = (unsigned)len - d * (unsigned)n;
+    return (int)((unsigned)i * d + (unsigned)i * r / (unsigned)n);
+}
 constexpr int kAttnWarps = 4;
 constexpr int kTokBatch  = 8;  // cache rows in flight per warp (fused kernel: the first batch is requested before the dependency wait)
 
@@ -41,7 +46,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32) kf_attn_decode_kernel(uint16_
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int kvh = h / (n_head / n_kv), kv_dim = n_kv * HD;
     const int len = pos_dev[m] + 1;
-    const int t0 = (int)(((long long)split * len) / nsplit), t1 = (int)(((long long)(split + 1) * len) / nsplit);
+    const int t0 = split_at(split, len, nsplit), t1 = split_at(split + 1, len, nsplit);
 
     float qf[DPL];
     load_row<DPL>(qf, q + ((size_t)m * n_head + h) * HD + lane * DPL);
@@ -185,7 +190,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32) kf_attn_fused_kernel(uint16_t
     // of cached K / V rows (rows < pos were written by earlier tokens).  Under programmatic dependent launch these loads overlap the
     // predecessor's tail.
     const int pos = pos_dev[m], len = pos + 1;
-    const int t0 = (int)(((long long)split * len) / nsplit), t1 = (int)(((long long)(split + 1) * len) / nsplit);
+    const int t0 = split_at(split, len, nsplit), t1 = split_at(split + 1, len, nsplit);
     const float2* cs_row  = table + (size_t)pos * (HD / 2);
     const uint16_t* kbase = kc + (size_t)m * seq_stride + (size_t)kvh * HD + lane * DPL;
     const uint16_t* vbase = vc + (size_t)m * seq_stride + (size_t)kvh * HD + lane * DPL;
@@ -203,6 +208,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32) kf_attn_fused_kernel(uint16_t
     int tb = t0 + warp * kTokBatch;
     if (tb < t1) load_batch(tb);
     kf_grid_dependency_wait();  // q / k / v come from the QKV GEMV right before us
+    q = behind_wait(q), k = behind_wait(k), v = behind_wait(v);
 
     float qf[DPL], knew[DPL], vnew[DPL];
     norm_rope_row<DPL>(qf, q + ((size_t)m * n_head + h) * HD, qw, cs_row, lane, eps);
@@ -355,7 +361,7 @@ __global__ void __launch_bounds__(kClusterWarpsMax * 32) kf_attn_cluster_kernel(
     if (nsplit > 1) cluster_arrive();  // matched by the wait in front of the first remote store: by then every CTA of the cluster runs
     // ---- independent of the QKV GEMV: position, slice, rotation table row and ALL cached rows of this warp's first pass ----
     const int pos = pos_dev[m], len = pos + 1;
-    const int t0 = (int)(((long long)split * len) / nsplit), t1 = (int)(((long long)(split + 1) * len) / nsplit);
+    const int t0 = split_at(split, len, nsplit), t1 = split_at(split + 1, len, nsplit);
     const float2* cs_row  = table + (size_t)pos * (HD / 2);
     const uint16_t* kbase = kc + (size_t)m * seq_stride + (size_t)kvh * HD + lane * DPL;
     const uint16_t* vbase = vc + (size_t)m * seq_stride + (size_t)kvh * HD + lane * DPL;
@@ -370,6 +376,7 @@ __global__ void __launch_bounds__(kClusterWarpsMax * 32) kf_attn_cluster_kernel(
     int tb = t0 + warp * kWarpTok;
     if (tb < t1) load_pass(tb);
     kf_grid_dependency_wait();  // q / k / v come from the QKV GEMV right before us
+    q = behind_wait(q), k = behind_wait(k), v = behind_wait(v);
 
     float qf[DPL], knew[DPL], vnew[DPL];
     norm_rope_row<DPL>(qf, q + ((size_t)m * n_head + h) * HD, qw, cs_row, lane, eps);
@@ -817,12 +824,13 @@ __global__ void __launch_bounds__(256) kf_qknorm_rope_kv_warp_kernel(uint16_t* _
                                                                      size_t seq_stride) {
     constexpr int HD = DPL * 32;
     kf_grid_dependency_wait();
+    k = behind_wait(k), v = behind_wait(v);
     kf_grid_launch_dependents();  // the attention behind us may set itself up; it waits for our end before it reads anything
     const int lane = threadIdx.x & 31;
     const int per_tok = n_head + n_kv, warps = (per_tok + R - 1) / R;  // warps of a token
-    const long long wid = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (wid >= (long long)M * warps) return;
-    const int m = (int)(wid / warps), h0 = (int)(wid % warps) * R;
+    const unsigned wid = blockIdx.x * 8 + (threadIdx.x >> 5);
+    const int m = (int)(wid / (unsigned)warps), h0 = (int)(wid - (unsigned)m * warps) * R;
+    if (m >= M) return;
     const int pos = pos_dev[m];
     float x[R][DPL], vv[R][DPL], w[2][DPL];
     float2 cs[DPL];

@@ -131,6 +131,7 @@ __global__ void __launch_bounds__(256) kf_permute_x_kernel(uint16_t* __restrict_
     const int lane = threadIdx.x & 31;
     const size_t i0 = (size_t)blockIdx.x * (256 * kPermPieces) + threadIdx.x;
     kf_grid_dependency_wait();    // x comes from the kernel before us ...
+    x = behind_wait(x);
     kf_grid_launch_dependents();  // ... and only behind it may the matmul start to stream its weights (they might have been written there as well)
     uint4 v[kPermPieces];
 #pragma unroll
@@ -155,6 +156,7 @@ __global__ void __launch_bounds__(256) kf_rmsnorm_permute_kernel(uint16_t* __res
     constexpr int NV = NC > 0 ? NC : 1;
     uint4 v[NV], g[NV];
     kf_grid_dependency_wait();  // as above
+    x = behind_wait(x);
     kf_grid_launch_dependents();
     const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)blockIdx.x * dim);
     uint4* orow     = reinterpret_cast<uint4*>(xp + (size_t)blockIdx.x * dim);

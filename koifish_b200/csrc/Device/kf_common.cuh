@@ -233,6 +233,14 @@ __device__ __forceinline__ uint16_t kf_deq_scalar(int k, uint16_t step, uint16_t
 }
 __device__ __forceinline__ uint32_t bf162_as_u32(__nv_bfloat162 v) { return *reinterpret_cast<uint32_t*>(&v); }
 
+// A pointer to what the kernel before this one writes, for reading behind kf_grid_dependency_wait().  A load through a `const __restrict__` parameter promises the compiler
+// that nobody writes there while the kernel runs, so it may move the load in front of the wait -- and did, once a slow division between the two was gone (the decode
+// attention read the queries of the step before).  What comes out of this it cannot have before.
+template <typename T>
+__device__ __forceinline__ T* behind_wait(T* p) {
+    asm volatile("" : "+l"(p) : : "memory");
+    return p;
+}
 // streaming 128-bit load: weights are read exactly once per token -> do not allocate in L1
 __device__ __forceinline__ uint4 ldg_stream_v4(const void* p) {
     uint4 r;
