@@ -160,6 +160,8 @@ extern "C" int kf_ctx_get_int(kf_ctx* ctx, const char* key, int* value_out) {
         *value_out = ctx->deq_fma;
     else if (!strcmp(key, "gemv_exact"))
         *value_out = ctx->gemv_exact;
+    else if (!strcmp(key, "gemv_i8_max_m"))
+        *value_out = ctx->gemv_i8_max_m;
     else if (!strcmp(key, "gemv_last_s"))
         *value_out = ctx->gemv_last_s;
     else if (!strcmp(key, "tc_last_bn"))
@@ -190,6 +192,8 @@ extern "C" int kf_ctx_set_int(kf_ctx* ctx, const char* key, int value) {
         ctx->gemv_variant = value;
     else if (!strcmp(key, "gemv_cluster"))
         ctx->gemv_cluster = value;
+    else if (!strcmp(key, "gemv_i8_max_m"))
+        ctx->gemv_i8_max_m = value < 0 ? 0 : value > 2 ? 2 : value;
     else if (!strcmp(key, "gemv_exact"))
         ctx->gemv_exact = value;
     else if (!strcmp(key, "tp_fused"))

@@ -1132,6 +1132,11 @@ int kf_gemv_small(kf_ctx* ctx, int n, void* const* y, const kf_tensor_desc* w, c
         const int rc = kf_gemv_tma(ctx, n, y, w, x, M, epilogue, residual, norm_w, norm_eps);
         if (rc != 1) return rc;
     }
+    // a split, a tile, a merge or a staging that was asked for is one of this kernel's
+    if (!ctx->gemv_exact && ctx->gemv_splitk <= 0 && ctx->gemv_variant == 0 && ctx->gemv_cluster == 1 && ctx->gemv_xg_min_m >= 0) {
+        const int rc = kf_gemv_i8(ctx, n, y, w, x, M, epilogue, residual, norm_w, norm_eps);
+        if (rc != 1) return rc;
+    }
     return gemv_dispatch(ctx, n, y, w, x, M, epilogue, residual, norm_w, norm_eps);
 }
 

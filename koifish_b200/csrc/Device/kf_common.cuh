@@ -52,6 +52,7 @@ struct kf_ctx {
     // cannot unpack bit-exact bf16 weights at the HBM rate) -- logits within the stated tolerance ; 1: the in-kernel dequant reproduces the
     // reference's bf16 roundings bit for bit (weights identical to kf_dequant / GetDataX inside the matmul), ~0.57 of the HBM peak
     int gemv_exact   = 0;
+    int gemv_i8_max_m = 2;  // tokens up to which the decode arithmetic runs on the integer tensor cores (gemv_i8.cu); 0 = never
     int gemv_last_s  = 0;  // read-only: k-split of the most recent dequant-GEMV launch (tools/gemv_bench.py records it)
     // rounding of the reference's dequant expression (step * k - zero) in bf16 (CU_Q128toX_, T.cu:274), pinned against the reference kernel
     // compiled both ways (oracle/ref_kernels.cu): 1 = ONE rounding, fma.rn.bf16 -- what nvcc's default -fmad=true (implied by the
@@ -148,6 +149,9 @@ int kf_tmap_count(const kf_ctx* ctx, bool weights);
 // gemv_tma.cu: KF_OK = launched, 1 = request not covered by this kernel (caller falls back to gemv.cu), < 0 = error
 int kf_gemv_tma(kf_ctx* ctx, int n, void* const* y, const kf_tensor_desc* w, const void* x, int M, int epilogue, const void* residual,
                 const void* norm_w, float norm_eps);
+// gemv_i8.cu: likewise, integer tensor cores
+int kf_gemv_i8(kf_ctx* ctx, int n, void* const* y, const kf_tensor_desc* w, const void* x, int M, int epilogue, const void* residual, const void* norm_w,
+               float norm_eps);
 int kf_ensure_gemv_ws(kf_ctx* ctx, size_t bytes, int counters);
 // KF_ERR_CUDA when a bounded wait of a kernel ran out since the last time it was asked; the counters such a kernel left half way are cleared first
 int kf_wait_status(kf_ctx* ctx);

@@ -28,6 +28,101 @@ def make_q(ctx, typ, rows, cols, seed=5):
     return w, bf16_tensor(kf.dequant(ctx, w), rows, cols).float()
 
 
+# ---------------------------------------------------------------------------------------------- one and two tokens on the integer tensor cores
+@pytest.mark.parametrize("typ,bits", [(kf.KF_T_Q4, 4), (kf.KF_T_Q2, 2), (kf.KF_T_SIGN, 2), (kf.KF_T_BINARY, 1)])
+@pytest.mark.parametrize("M", [1, 2])
+@pytest.mark.parametrize("rows,cols", [(8192, 384), (4112, 640), (2064, 1024), (1040, 1152), (64, 17024), (5120, 8320)])
+@pytest.mark.parametrize("wide", [0, 12])
+def test_gemv_i8(ctx, typ, bits, M, rows, cols, wide):
+    """Every epilogue, with and without the norm in front, over runs of tiles that end inside a warp's share, odd numbers of k-steps, zeros and steps that start anywhere in their
+    blocks, and K in halves.  The group sums are exact; an activation is off by 2^(b - 30) of its group's largest, which `wide` puts 2^12 above the rest, where b is the highest bit
+    that a code lies at in its byte; G groups are added up in fp32.  A bf16 result (8 significant bits) is off by one rounding more, the residual form by two, SwiGLU by those of
+    gate and up."""
+    import ctypes as C
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(rows + cols + M)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    qbias = 1 if typ == kf.KF_T_SIGN else 0
+
+    def weight():
+        data = torch.randint(0, 256, (rows, cols * bits // 8), generator=g, device="cuda", dtype=torch.uint8)
+        n = rows * cols // 128
+        step = (rnd(n).abs() * 0.02 + 0.002).bfloat16()
+        zero = (rnd(n) * 0.05).bfloat16() if typ in (kf.KF_T_Q4, kf.KF_T_Q2) else torch.zeros(n, device="cuda").bfloat16()
+        gama = torch.cat([torch.ones(rows + cols, device="cuda").bfloat16(), zero, step]).contiguous()
+        per = 8 // bits
+        b = data.view(rows, -1, 16).flip(2).reshape(rows, -1)
+        q = torch.stack([(b >> (8 - bits * (j + 1))) & ((1 << bits) - 1) for j in range(per)], 2).view(rows, -1, 128)
+        w = step.double().view(rows, -1, 1) * (q.double() - qbias) - zero.double().view(rows, -1, 1)
+        high = (step.double().abs() * ((1 << bits) - 1 + qbias)).view(rows, -1)  # of a weight without its zero, by group
+        return kf.TensorDesc(data.data_ptr(), gama.data_ptr(), rows, cols, typ, 128, qbias, None, None), w.view(rows, cols), (high, high + zero.double().abs().view(rows, -1), data, gama)
+
+    (dw, w, keep0), (du, u, keep1) = weight(), weight()
+    x = rnd(M, cols)
+    x[:, 5::128] *= 2.0 ** wide
+    x, nw = x.bfloat16(), (rnd(cols) * 0.1 + 1).bfloat16()
+    s = 1 / torch.sqrt(x.float().square().mean(1, keepdim=True) + 1e-6)
+    xn = ((x.float() * s) * nw.float()).bfloat16()  # off by one bf16 rounding where the sum of squares is taken in another order: bounded below by its share of the sum
+    r = rnd(M, rows).bfloat16()
+    ys = {k: torch.zeros(M, rows, device="cuda", dtype=torch.float32 if k == "f32" else torch.bfloat16) for k in ("none", "res", "f32", "glu", "norm")}
+    gu, two = (kf.TensorDesc * 2)(dw, du), (C.c_void_p * 2)(ys["glu"].data_ptr(), ys["glu"].data_ptr())
+    one, yn = (kf.TensorDesc * 1)(dw), (C.c_void_p * 1)(ys["norm"].data_ptr())
+    torch.cuda.synchronize()
+    for _ in range(2):
+        ys["res"].copy_(r)
+        torch.cuda.synchronize()
+        ctx.check(ctx.lib.kf_linear(ctx.h, ys["none"].data_ptr(), C.byref(dw), x.data_ptr(), M, kf.KF_EPI_NONE, None), "none")
+        ctx.check(ctx.lib.kf_linear(ctx.h, ys["res"].data_ptr(), C.byref(dw), x.data_ptr(), M, kf.KF_EPI_RESIDUAL, ys["res"].data_ptr()), "residual")
+        ctx.check(ctx.lib.kf_linear(ctx.h, ys["f32"].data_ptr(), C.byref(dw), x.data_ptr(), M, kf.KF_EPI_F32, None), "f32")
+        ctx.check(ctx.lib.kf_rmsnorm_linear(ctx.h, 2, two, gu, x.data_ptr(), nw.data_ptr(), 1e-6, M, 2), "swiglu")
+        ctx.check(ctx.lib.kf_rmsnorm_linear(ctx.h, 1, yn, one, x.data_ptr(), nw.data_ptr(), 1e-6, M, 0), "norm")
+        ctx.sync()
+    top_bit = {4: 4, 2: 6, 1: 7}[bits]
+
+    def slip(v, keep):
+        a = v.double().abs().view(M, -1, 128)
+        return 2.0 ** (top_bit - 30) * 128 * (a.amax(2) @ keep[0].T) + (cols // 128 + 8) * 2.0 ** -24 * (a.sum(2) @ keep[1].T)
+
+    want, eps, tiny = x.double() @ w.T, 2.0 ** -8 * 1.001, slip(x, keep0)
+    assert bool(((ys["f32"].double() - want).abs() <= tiny).all())
+    assert bool(((ys["none"].double() - want).abs() <= eps * want.abs() + tiny).all())
+    assert bool(((ys["res"].double() - (r.double() + want)).abs() <= eps * (want.abs() + (r.double() + want).abs()) * 1.02 + tiny).all())
+    xd, top = xn.double(), xn.double().abs().amax(1, keepdim=True)
+    slack = 2.0 ** -8 * top * torch.maximum(w.abs().amax(1), u.abs().amax(1)) * 2  # two activations rounded the other way
+    nrm, nmag = xd @ w.T, slip(xn, keep0) + slack
+    assert bool(((ys["norm"].double() - nrm).abs() <= eps * nrm.abs() + nmag).all())
+    up, umag = xd @ u.T, slip(xn, keep1) + slack
+    glu = nrm * torch.sigmoid(nrm) * up
+    bound = 1.1 * (eps * nrm.abs() + nmag) * (up.abs() + umag) + (nrm.abs() + nmag) * (eps * up.abs() + umag) + 1.1 * eps * glu.abs()
+    assert bool(((ys["glu"].double() - glu).abs() <= bound * 1.02).all())
+
+
+@pytest.mark.parametrize("typ", [kf.KF_T_Q4, kf.KF_T_SIGN, kf.KF_T_BINARY])
+def test_gemv_i8_special_values(ctx, typ):
+    """Infinities and NaN have no fixed-point form: the rows they reach are not finite.  Groups of zeros and of the smallest numbers stay what they are."""
+    import ctypes as C
+    import torch
+    rows, cols = 1024, 1024
+    w, wd = make_q(ctx, typ, rows, cols)
+    d = w.desc()
+    for bad in (float("inf"), float("-inf"), float("nan")):
+        x, y = torch.zeros(1, cols, device="cuda").bfloat16(), torch.zeros(1, rows, device="cuda")
+        x[0, 300] = bad
+        torch.cuda.synchronize()
+        ctx.check(ctx.lib.kf_linear(ctx.h, y.data_ptr(), C.byref(d), x.data_ptr(), 1, kf.KF_EPI_F32, None), "linear")
+        ctx.sync()
+        assert not bool(torch.isfinite(y).any())
+    x, y = torch.zeros(1, cols, device="cuda").bfloat16(), torch.zeros(1, rows, device="cuda")
+    x[0, 130] = 2.0 ** -120
+    x[0, 700] = 2.0 ** 100
+    torch.cuda.synchronize()
+    ctx.check(ctx.lib.kf_linear(ctx.h, y.data_ptr(), C.byref(d), x.data_ptr(), 1, kf.KF_EPI_F32, None), "linear")
+    ctx.sync()
+    # the weights are 0.02: rounded to bf16 in wd (2^-9), not so inside the matmul
+    assert bool(((y.double() - x.double() @ wd.double().T).abs() <= 2.0 ** 100 * 0.2 * 2.0 ** -8).all())
+
+
 # ---------------------------------------------------------------------------------------------- long reductions in the tcgen05 matmul
 @pytest.mark.parametrize("plan", [0, 1])
 @pytest.mark.parametrize("rows,cols,M", [(5120, 8192, 2048), (10240, 25600, 45), (2560, 25600, 128), (51200, 5120, 45), (1024, 25600, 300)])
