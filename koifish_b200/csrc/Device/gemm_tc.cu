@@ -53,6 +53,7 @@ __host__ __device__ constexpr int raw_bytes() { return FMT == 4 ? 32 : FMT == 3 
 constexpr int kProducerWarps = 8, kMmaWarp = 8, kRawWarp = 9, kXWarp = 10, kEpiWarp0 = 11;
 constexpr int kThreadsTC = 15 * 32;
 constexpr int kTeams = 2;  // of four producer warps
+constexpr int kNaturalBN = 128;  // token tiles from which activations may come in their own order
 
 constexpr int kEpiGlu = 2;  // epilogue: y = silu(w0 x) * (w1 x); an item takes 64 rows of either weight
 constexpr int kMaxW = 3;  // weights of one launch (Q/K/V, gate/up): same type, same K, their row tiles share one item space
@@ -74,6 +75,7 @@ struct GemmParams {
     int part_raw, part_rem;    // raw stages of a part; the first part_rem have one more
     uint32_t fold2;            // qbias as bf16x2 (types without a zero)
     int bias;                  // qbias does not fold into the zero: it is taken off the codes
+    int natural;               // the activations are in their own order: the expanded weights are put into it
     uint32_t qsub[8];          // qbias as a number of each code field, bf16x2
 };
 
@@ -286,9 +288,29 @@ __device__ __forceinline__ void expand_slot(uint32_t* o, const uint32_t* w, cons
     }
 }
 
+// The same 32 weights from the permuted into their own order, in place: one byte permute a pair.  Register p of a word's P holds elements 2 P - 1 - p and P - 1 - p.
+template <int FMT>
+__device__ __forceinline__ void natural_order(uint32_t* o) {
+    constexpr int P = 16 / Gama<FMT, TM_AFFINE>::BITS;
+    if constexpr (FMT != TF_F8) {
+#pragma unroll
+        for (int b = 0; b < 16; b += P) {
+            uint32_t n[P];
+#pragma unroll
+            for (int j = 0; j < P; j++) {
+                const int p = (j < P / 2 ? P : 2 * P) - 1 - 2 * j;
+                n[j] = __byte_perm(o[b + p], o[b + p - 1], j < P / 2 ? 0x7632 : 0x5410);
+            }
+#pragma unroll
+            for (int j = 0; j < P; j++) o[b + j] = n[j];
+        }
+    }
+}
+
 // Ring depths.  The three rings are decoupled because their latencies differ: the raw ring hides DRAM latency (bytes in flight per SM
-// = RS x 8 KB must cover ~2 us x 44 GB/s), the B ring hides the L2 round trip of the (small, L2-resident) activation tiles, the A ring
-// only the on-chip producer -> MMA hand-off.  Sized so that shared memory, the epilogue's output buffer included, stays below 226 KB and tensor memory within 512 columns.
+// = RS x 8 or 16 KB must cover ~2 us x 44 GB/s; at 256 tokens a stage lasts a microsecond and two do), the B ring hides the L2 round trip of the (small, L2-resident)
+// activation tiles (a fourth one at 256 tokens: 4-bit SwiGLU 51200 x 5120 at 200 96.3 -> 94.4 us), the A ring only the on-chip producer -> MMA hand-off.  Sized so that
+// shared memory, the epilogue's output buffer included, stays below 226 KB and tensor memory within 512 columns.
 template <int FMT, int BN>
 struct Rings {
     static constexpr bool A_TMEM = FMT != TF_BF16;
@@ -304,10 +326,10 @@ struct Rings {
     static constexpr int SUB     = A_BYTES + BN * 128;  // one k-block of a stage: [A tile (bf16 weights only)][B tile]
     static constexpr int STAGE   = U * SUB;
     static constexpr int SA      = !A_TMEM ? 0 : (BN <= 64 ? 12 : 8) / U;
-    static constexpr int SB      = (A_TMEM ? (BN == 16 ? 32 : BN == 32 ? 20 : BN == 64 ? 12 : BN == 128 ? 6 : 3)
+    static constexpr int SB      = (A_TMEM ? (BN == 16 ? 32 : BN == 32 ? 20 : BN == 64 ? 12 : BN == 128 ? 6 : FMT == TF_F8 ? 3 : 4)
                                            : (BN == 16 ? 10 : BN == 32 ? 10 : BN == 64 ? 8 : BN == 128 ? 6 : 4)) / U;
     static constexpr int RAWB    = raw_bytes<FMT>();
-    static constexpr int RS      = !A_TMEM ? 0 : (BN <= 64 ? 96 : BN == 128 ? 96 : 64) * 1024 / (BM * 128) * (RAWB < 128 ? 2 : 1);
+    static constexpr int RS      = !A_TMEM ? 0 : (BN <= 128 ? 96 : FMT == TF_F8 ? 64 : 32) * 1024 / (BM * 128) * (RAWB < 128 ? 2 : 1);
 
     // output buffer: the item's whole accumulator in bf16 where there is only one in tensor memory, which then goes back to the MMA warp after ~1.5 us of draining
     static constexpr int OUT     = BN == 16 ? 8 * 1024 : A_TMEM && BN > 64 ? BN * 256 : 16 * 1024;  // at least one read of tensor memory in fp32
@@ -699,6 +721,9 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
 #else
                             expand_slot<FMT, MODE, decltype(bias)::value>(o, &v[0], gm, p.qsub);
                             expand_slot<FMT, MODE, decltype(bias)::value>(o + 16, &v[NW], gm, p.qsub);
+                            if constexpr (BN >= kNaturalBN) {  // below, the branch alone costs the producers 4 % (51200 x 5120 at 45 tokens 49.3 -> 51.2 us)
+                                if (p.natural) natural_order<FMT>(o), natural_order<FMT>(o + 16);
+                            }
 #endif
                             if (k % U == 0) {
                                 mbar_wait_a(empty0 + s * 8, eph);
@@ -1099,10 +1124,11 @@ int launch_tc_bn(kf_ctx* ctx, GemmParams& p, const void* const* wdata, int nw, c
     for (int b = 16, i = 0; b <= 256; b *= 2, i++) {
         const int by_m = p.M > 128 ? 256 : p.M > 64 ? 128 : p.M > 32 ? 64 : p.M > 16 ? 32 : 16;  // one token tile where the panel fits one
         if (ctx->tc_bn > 0 ? b != ctx->tc_bn : ctx->gemv_exact ? b != by_m : ((b < 256 && p.M > 8 * b) || (b > 16 && p.M <= b / 2))) continue;
+        if (p.natural && b < kNaturalBN) continue;
         static const double kb_packed[5] = {0.154, 0.154, 0.15, 0.219, 0.361}, kb_f8[5] = {0.235, 0.235, 0.24, 0.26, 0.42}, kb_bf16[5] = {0.09, 0.10, 0.16, 0.24, 0.39};
         constexpr bool PACKED = FMT != TF_BF16 && FMT != TF_F8;
         const int m_tiles = (p.M + b - 1) / b, items = tiles * m_tiles;
-        const double t_kb0 = FMT == TF_BF16 ? kb_bf16[i] : FMT == TF_F8 ? kb_f8[i] : kb_packed[i];
+        const double t_kb0 = FMT == TF_BF16 ? kb_bf16[i] : FMT == TF_F8 ? kb_f8[i] : kb_packed[i] * (p.natural && b == 128 ? 1.25 : 1.0);
         const int given = std::min(ctx->gemv_splitk, nraw);  // > 0: the split asked for
         for (int s = given > 0 ? given : 1; s <= (given > 0 ? given : std::min(16, nraw)); s++) {
             const int waves = (items * s + ctx->sm_count - 1) / ctx->sm_count, len = (nraw + s - 1) / s * KBR;
@@ -1204,7 +1230,7 @@ int kf_tc_same_order(const kf_tensor_desc* a, const kf_tensor_desc* b) {
     return fa == fb ? 0 : 1;
 }
 
-// xp: activations as returned by kf_tc_prepare_x for weights of this type.  n <= 3 weights of the SAME storage type, K and group share
+// xp: activations as returned by kf_tc_prepare_x for weights of this type, or in their own order anywhere but in its scratch (packed types: more work in the producers).  n <= 3 weights of the SAME storage type, K and group share
 // one launch (their row tiles form one item space): Q/K/V and gate/up cost one kernel each instead of three / two.
 int kf_gemm_tc_multi(kf_ctx* ctx, int n, void* const* y, const kf_tensor_desc* w, const void* xp, int M, int epilogue, const void* residual) {
     KF_REQUIRE(ctx, n >= 1 && n <= kMaxW && y && w && xp && M >= 1, "args");
@@ -1241,7 +1267,8 @@ int kf_gemm_tc_multi(kf_ctx* ctx, int n, void* const* y, const kf_tensor_desc* w
         p.gshift = gs;
     }
     if (epilogue == 1) KF_REQUIRE(ctx, residual && n == 1, "residual: single weight");
-    p.staged = ((uintptr_t)residual & 15) == 0;
+    p.natural = fmt != TF_BF16 && fmt != TF_F8 && xp != ctx->xperm;
+    p.staged  = ((uintptr_t)residual & 15) == 0;
     for (int i = 0; i < n; i++) p.staged = p.staged && ((uintptr_t)y[i] & 15) == 0;
     if (epilogue == kEpiGlu) KF_REQUIRE(ctx, n == 2 && w[0].rows == w[1].rows && y[0] == y[1] && p.staged, "SwiGLU: gate and up of equal shape, one 16-byte aligned output");
 #define KF_TC_CASE(F, MD) \

@@ -138,8 +138,14 @@ static int linear_any(kf_ctx* ctx, int n, void* const* y, const kf_tensor_desc* 
             if (rc) return rc;
             xin = ctx->xnorm;
         }
-        // the activations in the k order of the weights' type: prepared once, shared by every weight of the same type
-        rc = kf_tc_prepare_x(ctx, &w[0], xin, M, &xp);
+        // the activations in the k order of the weights' type: prepared once, shared by every weight of the same type.  A single packed weight takes panels of more than 128
+        // tokens as they are: there its producers wait for the matrix instructions and can put the weights into order instead, which saves a launch (1024 x 3072 at 700 tokens
+        // 14.3 -> 11.6 us, 4096 x 4096 at 1999 56.0 -> 53.6); below that they pace the matmul.  Not where the result lies over the activations, which other items still
+        // read, nor with a tile or split that was asked for, whose sums are compared with those of the other order
+        const bool packed = w[0].type == KF_T_Q4 || w[0].type == KF_T_Q2 || w[0].type == KF_T_SIGN || w[0].type == KF_T_BINARY;
+        const uintptr_t xa = (uintptr_t)xin, xe = xa + (size_t)M * K * 2, ya = (uintptr_t)y[0], ye = ya + (size_t)M * w[0].rows * (epilogue == KF_EPI_F32 ? 4 : 2);
+        if (n == 1 && !norm_w && packed && M > 128 && !ctx->gemv_exact && ctx->tc_bn <= 0 && ctx->gemv_splitk <= 0 && xa % 16 == 0 && (ye <= xa || xe <= ya)) xp = xin;
+        else rc = kf_tc_prepare_x(ctx, &w[0], xin, M, &xp);
         if (rc) return rc;
     }
     // gate, up and CU_swiglu_v0 in one launch; not where the matmul reads x itself (bf16 and 8-bit weights without a norm) and the result lies over it: an item
