@@ -1138,6 +1138,8 @@ int launch_tc_bn(kf_ctx* ctx, GemmParams& p, const void* const* wdata, int nw, c
                 continue;
             }
             const bool cluster = s > 1 && s <= 8 && items * s <= ctx->sm_count && items * s <= cluster_ctas<FMT, MODE>(ctx, b, s);
+            // a workspace cannot grow inside a graph capture: a split that was not asked for is not chosen there before an eager call has sized it
+            if (s > 1 && !cluster && given <= 0 && ctx->capturing && ((size_t)items * s * b * BM * sizeof(float) > ctx->gemv_ws_bytes || items > ctx->gemv_cnt_n)) continue;
             const double t_kb = t_kb0 * (waves == 1 && b <= 64 ? 1.0 + (PACKED ? 0.045 : 0.033) * (m_tiles - 1) : 1.0);
             const double t = cluster ? len * t_kb + (PACKED ? 2.9 : 2.5) + 0.017 * b + 0.03 * (s - 2) - (FMT == TF_BF16 ? 0.2 + 0.0025 * b : 0.0)
                                      : waves * (len * t_kb + (PACKED ? 0.6 : 0.5) + 0.006 * b + (s > 1 ? 0.5 + 0.02 * b : 0.0)) + (s > 1 ? b * (0.03 + 0.008 * s) + (waves == 1 ? 1.5 : 0.0) : 0.0);
