@@ -227,12 +227,12 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t local, int cta_rank) {
 
 // Codes -> bf16 weights without a shift or a conversion: a code field that lies in the low byte of a 16-bit half IS the bf16 number code * 2^(bit - 133) (exponents 0 and
 // 1 share their scale, so all 256 patterns are linear), so one AND picks a pair of codes out of a register (of the register >> 8 for the upper bytes) and one bf16 fma
-// with step * 2^(133 - bit - 24) and -zero * 2^-24 rounds exactly as RN(step * code - zero) does, 2^24 smaller; the sums get the factor back (kUnscale, exact) on
-// their way out of tensor memory.  Two instructions a pair instead of four and a shift, which run at half rate on two pipes: steps stay below 2^19, weights matter
-// down to 2^-102.  (4-bit SwiGLU 51200 x 5120 at 45 tokens, with the leaner producer loop below and its larger stages: 65.5 -> 40.8 us, at 16 tokens 64 -> 38.4; ternary
+// with step * 2^(133 - bit - 60) and -zero * 2^-60 rounds exactly as RN(step * code - zero) does, 2^60 smaller; the sums get the factor back (kUnscale, exact) on
+// their way out of tensor memory.  Two instructions a pair instead of four and a shift, which run at half rate on two pipes; 60 leaves as much room above as below: steps
+// up to 2^54, weights exact down to 2^-66.  (4-bit SwiGLU 51200 x 5120 at 45 tokens, with the leaner producer loop below and its larger stages: 65.5 -> 40.8 us, at 16 tokens 64 -> 38.4; ternary
 // 24576 x 4096 at 45 36 -> 24.4.)
-constexpr int kWShift     = 24;
-constexpr float kUnscale  = 16777216.0f;
+constexpr int kWShift    = 60;
+constexpr float kUnscale = 1152921504606846976.0f;  // 2^60
 template <int BITS>
 __host__ __device__ constexpr int n_fields() { return BITS <= 4 ? 8 / BITS : 1; }  // code fields of a byte
 // per group: the multiplier of each field and -zero (one fma) or zero (two roundings), scaled
@@ -254,7 +254,7 @@ struct Gama {
         else z = down(z2, -kWShift) ^ (MODE == TM_AFFINE_FMA ? 0x80008000u : 0u);
     }
 };
-// the codes at field f of both halves of `reg` -> bf16x2 weights * 2^-24.  BIAS: qbias (as a number of that field, qf) comes off the codes first
+// the codes at field f of both halves of `reg` -> bf16x2 weights * 2^-60.  BIAS: qbias (as a number of that field, qf) comes off the codes first
 template <int FMT, int MODE, bool BIAS>
 __device__ __forceinline__ uint32_t tdeq(uint32_t reg, int f, const Gama<FMT, MODE>& g, uint32_t qf) {
     constexpr int BITS = Gama<FMT, MODE>::BITS;

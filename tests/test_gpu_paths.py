@@ -220,14 +220,14 @@ def _ptr(t):
 @pytest.mark.parametrize("M,rows,cols", [(9, 16, 128), (40, 144, 640), (128, 272, 384), (256, 128, 1152)])
 def test_tc_weights_bit_for_bit(ctx, typ, bits, qbias, fma, M, rows, cols):
     """Each token picks one column, so the result is the weight itself: the codes that the matmul expands inside its own number format round as kf_dequant does, for steps
-    from 2^-40 to 2^15, zeros of any size beside them, codes with and without a bias, and reductions that end inside a stage."""
+    from 2^-40 to 2^50, zeros of any size beside them, codes with and without a bias, and reductions that end inside a stage."""
     import torch
     g = torch.Generator(device="cuda")
     g.manual_seed(3 * M + bits + qbias)
     rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
     data = torch.randint(0, 256, (rows, cols * bits // 8), generator=g, device="cuda", dtype=torch.uint8)
     n = rows * cols // 128
-    step = (rnd(n) * torch.exp2(torch.randint(-40, 16, (n,), generator=g, device="cuda").float())).bfloat16()
+    step = (rnd(n) * torch.exp2(torch.randint(-40, 50, (n,), generator=g, device="cuda").float())).bfloat16()
     zero = (rnd(n) * 4 * step.float()).bfloat16() if typ in (kf.KF_T_Q4, kf.KF_T_Q2) else torch.zeros(n, device="cuda").bfloat16()
     step[::17], zero[::13] = 0, 0
     gama = torch.cat([torch.ones(rows + cols, device="cuda").bfloat16(), zero, step]).contiguous()
