@@ -9,7 +9,7 @@ GQA attention, O GEMV+residual, RMSNorm, gate/up GEMV+SwiGLU, down GEMV+residual
   value  : tokens/s with everything resident in HBM, K CUDA-graph replays timed with CUDA events on the launching stream.
   e2e    : tokens/s through the reference-facing C ABI (kf_model_forward) with HOST buffers: token id + position H2D and the
            logits + next token D2H inside the timed region, every step.
-  roofline: the dominant kernel (kf_gemv_kernel, the fused unpack+dequant GEMV): algorithmic bytes per launch / its average
+  roofline: the dominant kernel (kf_gemv_i8_kernel, the fused unpack+dequant GEMV of one token; kf_gemv_kernel with gemv_exact): algorithmic bytes per launch / its average
            launch duration (CUDA events over a graph holding exactly the step's GEMV launches), vs the measured HBM peak.
   cpu_baseline: the CPU oracle ("port") timed on this box's host cores on a bounded sample of the same workload.
 N > 1: tensor parallel (one process per GPU, NCCL all-reduce per block), strong scaling of the same single-sequence decode.
@@ -96,7 +96,7 @@ class ClockSampler:
         return {"sm_mhz": sm[len(sm) // 2] if sm else None, "sm_max_mhz": max(mx) if mx else None, "reasons": sorted(reasons), "samples": len(sm)}
 
 
-GEMV_SOURCES = ("koifish_b200/csrc/Device/gemv.cu", "koifish_b200/csrc/Device/kf_common.cuh")
+GEMV_SOURCES = ("koifish_b200/csrc/Device/gemv_i8.cu", "koifish_b200/csrc/Device/gemv.cu", "koifish_b200/csrc/Device/kf_common.cuh")
 TRAFFIC_FILE = "profiles/r02_traffic_decode.json"
 
 
@@ -396,7 +396,7 @@ def main():
             pass
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak, "traffic": traffic,
                 "traffic_source": traffic_src,
-                "kernel": "kf_gemv_kernel (fused unpack+dequant GEMV, M=1, %s)" % ("in-kernel dequant to the reference's bf16 weights" if gemv_exact else "fp16-code tensor-core arithmetic, group affine on fp32 sums"), "launches_per_step": n_gemv,
+                "kernel": "kf_gemv_kernel (fused unpack+dequant GEMV, M=1, in-kernel dequant to the reference's bf16 weights)" if gemv_exact else "kf_gemv_i8_kernel (fused unpack+dequant GEMV, M=1, codes x fixed-point activations on the integer tensor cores, group affine on fp32)", "launches_per_step": n_gemv,
                 "algorithmic_bytes_per_launch": per_launch_bytes, "avg_launch_us": per_launch_s * 1e6, "gemv_share_of_step": gemv_ms_pass / ms_step,
                 "peak_source": peak_src, "frac_of_8TBps": achieved / 8000.0,
                 "step_gbps_all_kernels": step_alg_bytes / (ms_step / 1e3) / 1e9, "step_frac_of_peak": step_alg_bytes / (ms_step / 1e3) / 1e9 / peak}
