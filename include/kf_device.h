@@ -95,7 +95,7 @@ uint64_t kf_launch_count(kf_ctx* ctx);
  * every replay; callers that capture their own graphs with kf_graph_begin / kf_graph_end must do the same. */
 uint64_t kf_scratch_generation(kf_ctx* ctx);
 /* tuning knobs for sweeps: "gemv_splitk" (0 = heuristic), "gemv_variant", "gemv_exact" (0: factored dequant, NOT reference-exact),
- * "gemv_cluster" (single-token split-K merged inside a thread-block cluster), "attn_split", "attn_warps", "pdl" (programmatic
+ * "gemv_i8_max_m" (tokens up to which packed weights run on the integer tensor cores, 0 .. 2), "gemv_cluster" (single-token split-K merged inside a thread-block cluster), "attn_split", "attn_warps", "pdl" (programmatic
  * dependent launch), "deq_fma" (1, default: the dequant expression step*k - zero rounds ONCE in bf16, as the reference's kernel does when built
  * for sm_90+; 0: twice, as its -fmad=false / pre-sm_90 builds), "gemv_tma" (1: decode GEMVs of 4-bit weights take the persistent
  * TMA-fed stream-K kernel; 0, default: the cp.async kernel, which is faster), "gemv_tma_occ" (CTAs per SM, 1 or 2), "gemv_tma_smem_kb" (shared-memory budget),
