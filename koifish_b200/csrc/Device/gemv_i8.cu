@@ -254,7 +254,7 @@ __global__ void __launch_bounds__(kThreads, 2) kf_gemv_i8_kernel(const __grid_co
         amax = max(amax, __shfl_xor_sync(quad, amax, 1)), amax = max(amax, __shfl_xor_sync(quad, amax, 2));
         sum += __shfl_xor_sync(quad, sum, 1), sum += __shfl_xor_sync(quad, sum, 2);
         const int e = (int)(amax >> 7);                                           // biased exponent of the largest
-        const int scale = amax == 0 ? 0 : max(-97, min(126, 156 - e));            // 156 = 127 + 29
+        const int scale = amax == 0 ? 0 : max(-98, min(126, 156 - e));            // 156 = 127 + 29 ; at -97 the largest finite number, 255 * 2^23, would wrap in the digits below
         if (tt == 0) sx[s * MX + m] = make_float2(sum, __uint_as_float((uint32_t)(127 - scale) << 23));
         // infinities and NaN have no fixed-point form: they come back through the group's scale, which multiplies every sum that the group takes part in
         if (tt == 0 && amax >= 0x7f80u) sx[s * MX + m] = make_float2(sum, __uint_as_float(0x7fc00000u));

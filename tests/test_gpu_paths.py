@@ -123,6 +123,69 @@ def test_gemv_i8_special_values(ctx, typ):
     assert bool(((y.double() - x.double() @ wd.double().T).abs() <= 2.0 ** 100 * 0.2 * 2.0 ** -8).all())
 
 
+def pack_codes(codes, bits):
+    """[rows, cols] codes -> bytes of 128-bit words, the first code of a word in its most significant bits"""
+    import torch
+    rows, cols = codes.shape
+    c = codes.view(rows, -1, 8 // bits).to(torch.uint8)
+    b = torch.zeros_like(c[:, :, 0])
+    for j in range(8 // bits):
+        b |= c[:, :, j] << (8 - bits * (j + 1))
+    return b.view(rows, -1, 16).flip(2).contiguous().view(rows, -1)
+
+
+@pytest.mark.parametrize("typ,bits", [(kf.KF_T_Q4, 4), (kf.KF_T_Q2, 2), (kf.KF_T_SIGN, 2), (kf.KF_T_BINARY, 1)])
+@pytest.mark.parametrize("M", [1, 2])
+@pytest.mark.parametrize("kind", ["top"])
+def test_gemv_i8_activations_of_any_size(ctx, typ, bits, M, kind):
+    """Activations keep all their bits whatever stands beside them.  In every second row the code that meets the large activation is zero, so that nothing but the others shows: one
+    far above the rest of its group, the largest finite numbers of either sign at every place of a group (every field of a byte), numbers far below one, and whole groups of them
+    between groups far above one.  A product is exact; what is rounded are the fp32 sums: those of a group (none where it is a whole number, eight matrix instructions of 16
+    products otherwise), over the groups, and of its activations, which step * bias and zero multiply."""
+    import ctypes as C
+    import torch
+    rows, cols = 1024, 16384 if kind.startswith("top") else 1024
+    G, qbias = cols // 128, 1 if typ == kf.KF_T_SIGN else 0
+    g = torch.Generator(device="cuda")
+    g.manual_seed(bits * 10 + M)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    q = torch.randint(0, 2 ** bits, (rows, cols), generator=g, device="cuda")
+    x, grp = rnd(M, G, 128), torch.arange(G, device="cuda")
+    big = torch.zeros(G, 128, dtype=torch.bool, device="cuda")
+    if kind == "2^-100 and 2^60":
+        big[::2] = True
+        x[:, ::2] *= 2.0 ** 60
+        x[:, 1::2] *= 2.0 ** -100
+    elif kind == "2^-100":
+        x[:, 1:] *= 2.0 ** -100
+        x[:, 0] = 0
+    else:
+        big[grp, (grp * 37 + 5) % 128] = True  # 37 is odd: every place of a group in 128 groups
+        if kind == "top and others":
+            big[grp, (grp * 37 + 69) % 128] = True  # their sum is no number
+        x = x.bfloat16().float()
+        if kind == "top":
+            x[:] = 0
+        sign = 1 - 2 * (grp // 3 % 2).float()
+        x[:, big] = ((torch.finfo(torch.bfloat16).max if kind.startswith("top") else 2.0 ** float(kind[2:])) * sign).repeat_interleave(int(big[0].sum()))
+    q[1::2] *= ~big.view(1, cols)
+    if kind == "top":
+        q[1::4] = (q[::4] + 1) % 2 ** bits  # nothing else to be seen there
+    x = x.view(M, cols).bfloat16()
+    n = rows * G
+    step, zero = (rnd(n).abs() * 2.0 ** -18 + 2.0 ** -20).bfloat16(), torch.zeros(n, device="cuda").bfloat16()
+    gama, data = torch.cat([torch.ones(rows + cols, device="cuda").bfloat16(), zero, step]).contiguous(), pack_codes(q, bits)
+    d, y = kf.TensorDesc(data.data_ptr(), gama.data_ptr(), rows, cols, typ, 128, qbias, None, None), torch.zeros(M, rows, device="cuda")
+    torch.cuda.synchronize()
+    ctx.check(ctx.lib.kf_linear(ctx.h, y.data_ptr(), C.byref(d), x.data_ptr(), M, kf.KF_EPI_F32, None), "linear")
+    ctx.sync()
+    st = step.double().view(rows, G, 1)
+    want = x.double() @ (st * (q.double() - qbias).view(rows, G, 128)).view(rows, cols).T
+    mag = x.double().abs() @ (st * (q.double() + qbias).view(rows, G, 128)).view(rows, cols).T
+    # a limb's part of a number is at most three times the number
+    assert bool(torch.isfinite(y).all()) and bool(((y.double() - want).abs() <= 3 * (G + 64) * 2.0 ** -23 * mag + 2.0 ** -145).all())
+
+
 # ---------------------------------------------------------------------------------------------- long reductions in the tcgen05 matmul
 @pytest.mark.parametrize("plan", [0, 1])
 @pytest.mark.parametrize("rows,cols,M", [(5120, 8192, 2048), (10240, 25600, 45), (2560, 25600, 128), (51200, 5120, 45), (1024, 25600, 300)])
