@@ -9,9 +9,14 @@
 // the activations with three k-steps of weights in flight.  Here
 //   * a register holds FOUR codes: the bytes of `word & mask` are unsigned 8-bit operands of mma.sync.m16n8k32 (u8 x s8 -> s32), code * 2^bit where the field lies bit bits up in its
 //     byte, and the activation that meets it is staged 2^-bit smaller: 16 ANDs and 4 matrix instructions a tile for every width;
-//   * an activation is a fixed-point number of 30 bits below the largest of its group of 128 k, in four signed 8-bit limbs, which are four of the eight columns of the matrix
-//     instruction (two tokens fit).  All products and the sums of a group are exact integers; what is rounded is the
-//     activation, at 2^-30 of its group's largest (2^-26 under 4-bit, 2^-24 and 2^-23 under the highest fields of 2- and 1-bit codes), and the fp32 sum over the groups;
+//   * an activation is a whole number below 2^31 in units of its group of 128 k, in four signed 8-bit limbs, which are four of the eight columns of the matrix
+//     instruction (two tokens fit).  All products and the sums of a group are exact integers; what is rounded is the fp32 sum over the groups;
+//   * the 8 bits of a bf16 number are whole down to 2^-23 of the group's largest under the lowest field of a byte, down to 2^-19, 2^-17 and 2^-16 under the highest of 4-, 2- and
+//     1-bit codes.  A k-step with a number that is not (of a SwiGLU's outputs one group in 190, 90 and 57, of normal ones hardly any), with infinities or NaN, or with numbers
+//     that together leave the range, keeps its activations as they are, as bf16 pairs in the room of two limbs, and goes through mma.sync.m16n8k16 on codes as bf16 numbers: no
+//     activation loses a bit that it has above 2^-180 of the largest.  The loop that asks for such steps runs in the CTAs that hold one (5120 x 25600: 18.3 us, 19.1 with the question
+//     everywhere, 18.1 without such steps; ternary 4096 x 12288 at two tokens behind a SwiGLU 10.3 without, 10.8).  Against 64 bits the fp32 sums are off by 1e-7, whatever the
+//     activations (gemv.cu: 3e-7 for normal ones, 2e-6 for a SwiGLU's, 1e-5 with outliers of 2^14);
 //   * zero and code bias, which multiply the group's plain sum of activations, take one fma per row, group and token on the lanes that fetched them;
 //   * a CTA takes a run of 16-row tiles, and its eight warps equal shares of the run's k-steps: no barrier between the first copy and the last sum.  Every lane streams its own
 //     words through a ring in shared memory (cp.async), started before the kernel waits for its predecessor.  A k-step costs a warp 45 instructions beside 18 for its share of the
@@ -24,6 +29,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <type_traits>
 
 #include "kf_common.cuh"
 
@@ -101,11 +107,31 @@ __host__ __device__ constexpr int mma_elem(int i, int q, int e) {
     return per * (Fmt<FMT>::NW - 1 - mma_word<FMT>(i, q)) + (per - 1) - (8 * e + mma_bit<FMT>(i, q)) / Fmt<FMT>::BITS;
 }
 
+// A step in bf16: register p of 16 holds codes pair_elem(p) (its lower half) and pair_elem(p) - 16 / BITS
+template <int FMT>
+__host__ __device__ constexpr int pair_elem(int p) {
+    const int per = 32 / Fmt<FMT>::BITS;
+    return per * (Fmt<FMT>::NW - 1 - p / (per / 2)) + per - 1 - p % (per / 2);
+}
+template <int FMT>
+__device__ __forceinline__ uint32_t pair_codes(const uint32_t (&w)[Fmt<FMT>::NW], int p) {
+    constexpr int half = 16 / Fmt<FMT>::BITS;
+    constexpr uint32_t mask = ((1u << Fmt<FMT>::BITS) - 1u) * 0x00010001u;
+    const uint32_t v = ((w[p / half] >> (p % half * Fmt<FMT>::BITS)) & mask) | 0x43004300u;  // 128 + code
+    return bf162_as_u32(__hsub2_rn(u32_as_bf162(v), u32_as_bf162(0x43004300u)));
+}
+__device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
 // MX: tokens (1, 2) ; D: chunks in flight per warp
 template <int FMT, int MX, int D>
 __global__ void __launch_bounds__(kThreads, 2) kf_gemv_i8_kernel(const __grid_constant__ IParams p) {
     using F             = Fmt<FMT>;
     constexpr int NC    = 4 * MX;                   // columns staged: token * 4 + limb
+    constexpr int NF    = 8 / F::BITS;              // code fields of a byte
     constexpr int STEPB = 16 * F::BITS, CH = kCh;      // bytes of a row's k-step, k-steps of a chunk
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ float s_red[MX * 8], s_scale[MX];
@@ -182,7 +208,7 @@ __global__ void __launch_bounds__(kThreads, 2) kf_gemv_i8_kernel(const __grid_co
 
     // ---- activations.  Item = 32 consecutive values of a token (what one lane's codes of a k-step meet); the four lanes of a quad hold a group of 128 ----
     uint4* xs  = reinterpret_cast<uint4*>(smem);                       // [step][h][column][t]: operands of matrix instructions 2 h, 2 h + 1
-    float2* sx = reinterpret_cast<float2*>(smem + p.off_sx);           // [step][token] {sum of the group, 2^-scale}
+    float2* sx = reinterpret_cast<float2*>(smem + p.off_sx);           // [step][token] {sum of the group, 2^-scale} ; in bf16: {sum * 2^scale, -2^-scale}
     const int items = MX * nc * CH * 4;
     uint4 xv[4];
     auto load_x = [&](int it) {
@@ -192,6 +218,7 @@ __global__ void __launch_bounds__(kThreads, 2) kf_gemv_i8_kernel(const __grid_co
         for (int i = 0; i < 4; i++) xv[i] = s < n ? __ldg(gp + i) : make_uint4(0, 0, 0, 0);
     };
     if (tid < items) load_x(tid);  // beside the sums below
+    int any_wide = 0;
     if (p.norm_w) {  // the scale of each token, in the order of kf_rmsnorm_kernel (ops.cu): 256 threads
         if (tid < 256) {
             float ss[MX];
@@ -242,53 +269,92 @@ __global__ void __launch_bounds__(kThreads, 2) kf_gemv_i8_kernel(const __grid_co
                 for (int j = 0; j < 4; j++) v[4 * i + j] = pack_bf16x2((bf16lo(v[4 * i + j]) * sc) * bf16lo(ww[j]), (bf16hi(v[4 * i + j]) * sc) * bf16hi(ww[j]));
             }
         }
-        // the power of two that puts the group's largest magnitude into [2^29, 2^30), and the group's sum
+        // the power of two that puts the group's largest magnitude into [2^30, 2^31), one lower where that is 255 * 2^23, which the digits below cannot hold.  Beside it the least
+        // exponent of its numbers less the place that each meets in a byte (elements 2 i and 2 i + 1 always the same two; a zero less one is the largest there is)
         const unsigned quad = 0xFu << (lane & ~3);
-        uint32_t amax = 0;
+        uint32_t amax = 0, low[NF / 2];
         float sum = 0.f;
 #pragma unroll
+        for (int c = 0; c < NF / 2; c++) low[c] = 0xffffffffu;
+#pragma unroll
         for (int i = 0; i < 16; i++) {
-            amax = max(amax, max(v[i] & 0x7fffu, (v[i] >> 16) & 0x7fffu));
+            amax = __vmaxu2(amax, v[i] & 0x7fff7fffu);
+            low[i % (NF / 2)] = __viaddmin_u16x2(v[i] & 0x7fff7fffu, 0xffffffffu, low[i % (NF / 2)]);
             sum += bf16lo(v[i]), sum += bf16hi(v[i]);
         }
-        amax = max(amax, __shfl_xor_sync(quad, amax, 1)), amax = max(amax, __shfl_xor_sync(quad, amax, 2));
+        int least = 512;
+#pragma unroll
+        for (int c = 0; c < NF / 2; c++) {
+            const int hi = F::BITS * (NF - 1 - 2 * c), lo = hi - F::BITS;  // the first codes are the highest
+            least = min(least, min((int)(low[c] >> 7 & 0x1ffu) - hi, (int)(low[c] >> 23) - lo));
+        }
+        amax = max(amax & 0xffffu, amax >> 16) | (uint32_t)(1023 - least) << 16;
+        amax = __vmaxu2(amax, __shfl_xor_sync(quad, amax, 1)), amax = __vmaxu2(amax, __shfl_xor_sync(quad, amax, 2));
+        least = 1023 - (int)(amax >> 16), amax &= 0xffffu;
+        const int e = (int)(amax >> 7);                        // biased exponent of the largest
+        const int scale = min(100, 157 - (int)((amax + 1) >> 7));  // 157 = 127 + 30 ; so that a step times 2^-scale stays a normal number
+        float f[NF];                                               // 2^scale for each place a field may lie at
+#pragma unroll
+        for (int b = 0; b < NF; b++) f[b] = __uint_as_float((uint32_t)(127 + scale - b * F::BITS) << 23);
         sum += __shfl_xor_sync(quad, sum, 1), sum += __shfl_xor_sync(quad, sum, 2);
-        const int e = (int)(amax >> 7);                                           // biased exponent of the largest
-        const int scale = amax == 0 ? 0 : max(-98, min(126, 156 - e));            // 156 = 127 + 29 ; at -97 the largest finite number, 255 * 2^23, would wrap in the digits below
-        if (tt == 0) sx[s * MX + m] = make_float2(sum, __uint_as_float((uint32_t)(127 - scale) << 23));
-        // infinities and NaN have no fixed-point form: they come back through the group's scale, which multiplies every sum that the group takes part in
-        if (tt == 0 && amax >= 0x7f80u) sx[s * MX + m] = make_float2(sum, __uint_as_float(0x7fc00000u));
-        float f[F::BITS == 4 ? 2 : F::BITS == 2 ? 4 : 8];                         // 2^scale for each bit a field may lie at
+        // Does every number come out whole?  Those with all their 8 bits above one do; infinities, NaN and numbers whose sum is none do not.  (Asking the others one by one spares half of
+        // these steps and takes longer.)  One token's group decides for the step
+        int wide = e >= 246 || least < 134 - scale;
+        if (MX == 2) wide |= __shfl_xor_sync(0xFFu << (lane & ~7), wide, 4);
+        any_wide |= wide;
+        // a step that does not fit: bf16 pairs as the code pairs meet them, in the place of limbs 0 and 1, the largest in [2^63, 2^64) ; marked by the sign
+        float inv = __uint_as_float((uint32_t)(127 - scale) << 23);
+        if (__builtin_expect(wide, 0)) {
+            const int up      = min(100, 190 - e);  // 190 = 127 + 63
+            const uint32_t by = (uint32_t)(127 + up) * 0x00800080u;
 #pragma unroll
-        for (int b = 0; b < (int)(sizeof(f) / 4); b++) f[b] = __uint_as_float((uint32_t)(127 + scale - b * F::BITS) << 23);
+            for (int i = 0; i < 16; i++) v[i] = bf162_as_u32(__hmul2_rn(u32_as_bf162(v[i]), u32_as_bf162(by)));
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-            uint32_t o[4][4];  // [limb][instruction, k half]
-#pragma unroll
-            for (int c = 0; c < 4; c++) {
-                const int i = 2 * h + (c >> 1), qq = c & 1;
+            for (int i = 0; i < 4; i++) {
                 uint32_t w[4];
 #pragma unroll
-                for (int b = 0; b < 4; b++) {
-                    const int el = mma_elem<FMT>(i, qq, b);
-                    const float a = (el & 1) ? bf16hi(v[el >> 1]) : bf16lo(v[el >> 1]);
-                    // signed digits in base 256: adding 128 to the lower three makes them bytes without borrow, flipping their top bits takes it off again
-                    w[b] = ((uint32_t)__float2int_rn(a * f[mma_bit<FMT>(i, qq) / F::BITS]) + 0x00808080u) ^ 0x00808080u;
+                for (int c = 0; c < 4; c++) {
+                    const int lo = pair_elem<FMT>(4 * i + c), hi = lo - 16 / F::BITS;
+                    w[c] = __byte_perm(v[lo >> 1], v[hi >> 1], ((lo & 1) ? 0x32 : 0x10) | ((hi & 1) ? 0x7600 : 0x5400));
                 }
-                const uint32_t l01 = __byte_perm(w[0], w[1], 0x5140), h01 = __byte_perm(w[2], w[3], 0x5140);
-                const uint32_t l23 = __byte_perm(w[0], w[1], 0x7362), h23 = __byte_perm(w[2], w[3], 0x7362);
-                o[0][c] = __byte_perm(l01, h01, 0x5410), o[1][c] = __byte_perm(l01, h01, 0x7632);
-                o[2][c] = __byte_perm(l23, h23, 0x5410), o[3][c] = __byte_perm(l23, h23, 0x7632);
+                xs[((s * 2 + (i >> 1)) * NC + 4 * m + (i & 1)) * 4 + tt] = make_uint4(w[0], w[1], w[2], w[3]);
             }
+            sum = 0.f;
 #pragma unroll
-            for (int l = 0; l < 4; l++) xs[((s * 2 + h) * NC + 4 * m + l) * 4 + tt] = make_uint4(o[l][0], o[l][1], o[l][2], o[l][3]);
+            for (int i = 0; i < 16; i++) sum += bf16lo(v[i]), sum += bf16hi(v[i]);
+            sum += __shfl_xor_sync(quad, sum, 1), sum += __shfl_xor_sync(quad, sum, 2);
+            inv = -__uint_as_float((uint32_t)(127 - up) << 23);
+        } else {
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                uint32_t o[4][4];  // [limb][instruction, k half]
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    const int i = 2 * h + (c >> 1), qq = c & 1;
+                    uint32_t w[4];
+#pragma unroll
+                    for (int b = 0; b < 4; b++) {
+                        const int el = mma_elem<FMT>(i, qq, b);
+                        const float a = (el & 1) ? bf16hi(v[el >> 1]) : bf16lo(v[el >> 1]);
+                        // signed digits in base 256: adding 128 to the lower three makes them bytes without borrow, flipping their top bits takes it off again
+                        w[b] = ((uint32_t)__float2int_rn(a * f[mma_bit<FMT>(i, qq) / F::BITS]) + 0x00808080u) ^ 0x00808080u;
+                    }
+                    const uint32_t l01 = __byte_perm(w[0], w[1], 0x5140), h01 = __byte_perm(w[2], w[3], 0x5140);
+                    const uint32_t l23 = __byte_perm(w[0], w[1], 0x7362), h23 = __byte_perm(w[2], w[3], 0x7362);
+                    o[0][c] = __byte_perm(l01, h01, 0x5410), o[1][c] = __byte_perm(l01, h01, 0x7632);
+                    o[2][c] = __byte_perm(l23, h23, 0x5410), o[3][c] = __byte_perm(l23, h23, 0x7632);
+                }
+#pragma unroll
+                for (int l = 0; l < 4; l++) xs[((s * 2 + h) * NC + 4 * m + l) * 4 + tt] = make_uint4(o[l][0], o[l][1], o[l][2], o[l][3]);
+            }
         }
+        if (tt == 0) sx[s * MX + m] = make_float2(sum, inv);
     }
-    __syncthreads();
+    any_wide = __syncthreads_or(any_wide);
 
     // ---- the stream: k-steps of this warp, each lane's words as it copied them ----
     float* part = reinterpret_cast<float*>(smem + p.off_part);  // [tile + warp][token][16 rows]: a warp's sums of a tile (the pairs lie on a path, so the index is their own)
-    {
+    auto stream = [&](auto with_bf16) {
         float acc[4], z[MX];
         auto clear = [&]() {
 #pragma unroll
@@ -312,10 +378,14 @@ __global__ void __launch_bounds__(kThreads, 2) kf_gemv_i8_kernel(const __grid_co
                 asm volatile("ld.shared.u16 %0, [%1];" : "=r"(gv[j]) : "r"(gring + ((gat + 2 * j) & (kGB * 16 - 1))) : "memory");
             }
             int d[CH][4];
+            float2 sv[CH][MX];
 #pragma unroll
-            for (int j = 0; j < CH; j++)
+            for (int j = 0; j < CH; j++) {
 #pragma unroll
                 for (int c = 0; c < 4; c++) d[j][c] = 0;
+#pragma unroll
+                for (int m = 0; m < MX; m++) sv[j][m] = sx[(k + j) * MX + m];
+            }
             const uint32_t xk = xbase + (uint32_t)(k * (2 * NC * 64));
 #pragma unroll
             for (int h = 0; h < 2; h++) {
@@ -335,6 +405,31 @@ __global__ void __launch_bounds__(kThreads, 2) kf_gemv_i8_kernel(const __grid_co
                     }
                 }
             }
+            if (decltype(with_bf16)::value && fminf(sv[0][0].y, sv[CH - 1][0].y) < 0.f) {  // a step in bf16 (CH is two)
+#pragma unroll
+                for (int j = 0; j < CH; j++) {
+                    if (sv[j][0].y >= 0.f) continue;
+                    const float val = bf16_bits_to_f32(gv[j]);
+#pragma unroll
+                    for (int m = 0; m < MX; m++) z[m] = fmaf(-val * sv[j][m].y, sv[j][m].x, z[m]), sv[j][m].x = 0.f;
+                    const float gs = MX == 2 && (t & 2) ? sv[j][MX - 1].y : sv[j][0].y;
+                    const float stepa = __shfl_sync(0xffffffffu, val, (lane & ~3) | 1), stepb = __shfl_sync(0xffffffffu, val, (lane & ~3) | 3);
+                    float fd[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        uint32_t xb[4];  // the column's token as the limbs have it: columns 0 and 4, which even lanes hold the sums of, are those of tokens 0 and 1
+                        lds(xb, xk + (uint32_t)(((2 * j + (i >> 1)) * NC + (i & 1) - (g & 3)) * 64));
+#pragma unroll
+                        for (int c = 0; c < 2; c++) {
+                            const int pr = 4 * i + 2 * c;
+                            mma_bf16(fd, pair_codes<FMT>(wa[j], pr), pair_codes<FMT>(wb[j], pr), pair_codes<FMT>(wa[j], pr + 1), pair_codes<FMT>(wb[j], pr + 1), xb[2 * c], xb[2 * c + 1]);
+                        }
+                    }
+                    if (!(t & 1)) acc[0] = fmaf(-stepa * gs, fd[0], acc[0]), acc[2] = fmaf(-stepb * gs, fd[2], acc[2]);
+#pragma unroll
+                    for (int c = 0; c < 4; c++) d[j][c] = 0;
+                }
+            }
             copy(slot);  // its words are in the matrix instructions' registers
             slot = slot + 1 == D ? 0 : slot + 1;
 #pragma unroll
@@ -342,10 +437,9 @@ __global__ void __launch_bounds__(kThreads, 2) kf_gemv_i8_kernel(const __grid_co
                 // past the slice's end the ring holds what was there: the sum of activations and the scale are zero, which an infinity or NaN would survive
                 const float val = j > 0 && k + j >= n ? 0.f : bf16_bits_to_f32(gv[j]);
                 const float stepa = __shfl_sync(0xffffffffu, val, (lane & ~3) | 1), stepb = __shfl_sync(0xffffffffu, val, (lane & ~3) | 3);
-                float2 sv[MX];
 #pragma unroll
-                for (int m = 0; m < MX; m++) sv[m] = sx[(k + j) * MX + m], z[m] = fmaf(val, sv[m].x, z[m]);
-                const float gs = MX == 2 && (t & 2) ? sv[MX - 1].y : sv[0].y;  // of this lane's columns' token
+                for (int m = 0; m < MX; m++) z[m] = fmaf(val, sv[j][m].x, z[m]);
+                const float gs = MX == 2 && (t & 2) ? sv[j][MX - 1].y : sv[j][0].y;  // of this lane's columns' token
                 const float fa = stepa * gs, fb = stepb * gs;
                 acc[0] = fmaf(fa, (float)d[j][0], acc[0]), acc[1] = fmaf(fa, (float)d[j][1], acc[1]);
                 acc[2] = fmaf(fb, (float)d[j][2], acc[2]), acc[3] = fmaf(fb, (float)d[j][3], acc[3]);
@@ -372,7 +466,9 @@ __global__ void __launch_bounds__(kThreads, 2) kf_gemv_i8_kernel(const __grid_co
                 if (k >= n) k = 0, tile++, gnext += glen, gat = gnext + goff;
             }
         }
-    }
+    };
+    if (any_wide) stream(std::true_type());
+    else stream(std::false_type());
     cp_async_wait<0>();
     __syncthreads();
 
