@@ -227,12 +227,15 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t local, int cta_rank) {
 
 // Codes -> bf16 weights without a shift or a conversion: a code field that lies in the low byte of a 16-bit half IS the bf16 number code * 2^(bit - 133) (exponents 0 and
 // 1 share their scale, so all 256 patterns are linear), so one AND picks a pair of codes out of a register (of the register >> 8 for the upper bytes) and one bf16 fma
-// with step * 2^(133 - bit - 60) and -zero * 2^-60 rounds exactly as RN(step * code - zero) does, 2^60 smaller; the sums get the factor back (kUnscale, exact) on
-// their way out of tensor memory.  Two instructions a pair instead of four and a shift, which run at half rate on two pipes; 60 leaves as much room above as below: steps
-// up to 2^54, weights exact down to 2^-66.  (4-bit SwiGLU 51200 x 5120 at 45 tokens, with the leaner producer loop below and its larger stages: 65.5 -> 40.8 us, at 16 tokens 64 -> 38.4; ternary
-// 24576 x 4096 at 45 36 -> 24.4.)
-constexpr int kWShift    = 60;
-constexpr float kUnscale = 1152921504606846976.0f;  // 2^60
+// with step * 2^(133 - bit - 7) and -zero * 2^-7 rounds exactly as RN(step * code - zero) does, 2^7 smaller; the sums get the factor back (kUnscale, exact) on
+// their way out of tensor memory.  Two instructions a pair instead of four and a shift, which run at half rate on two pipes.  (4-bit SwiGLU 51200 x 5120 at 45 tokens, with the leaner
+// producer loop below and its larger stages: 65.5 -> 40.8 us, at 16 tokens 64 -> 38.4; ternary 24576 x 4096 at 45 36 -> 24.4.  The question for larger steps: 41.0 -> 41.8, 38.6 ->
+// 38.9 and nothing.)
+// With 2^-7 a step has to stay below four; stages with one of two or more (or that is no number) take the long way below, which holds every step.  A smaller factor would leave more of
+// them to it, a larger one takes bits from the smallest weights: now all of 2^-119 and above keep theirs, and what is lost below is less than 2^-126.
+constexpr int kWShift       = 7;
+constexpr float kUnscale    = 128.f;
+constexpr uint32_t kFarStep = 0x4000u;  // the bit of the exponent that says so
 template <int BITS>
 __host__ __device__ constexpr int n_fields() { return BITS <= 4 ? 8 / BITS : 1; }  // code fields of a byte
 // per group: the multiplier of each field and -zero (one fma) or zero (two roundings), scaled
@@ -254,7 +257,7 @@ struct Gama {
         else z = down(z2, -kWShift) ^ (MODE == TM_AFFINE_FMA ? 0x80008000u : 0u);
     }
 };
-// the codes at field f of both halves of `reg` -> bf16x2 weights * 2^-60.  BIAS: qbias (as a number of that field, qf) comes off the codes first
+// the codes at field f of both halves of `reg` -> bf16x2 weights * 2^-7.  BIAS: qbias (as a number of that field, qf) comes off the codes first
 template <int FMT, int MODE, bool BIAS>
 __device__ __forceinline__ uint32_t tdeq(uint32_t reg, int f, const Gama<FMT, MODE>& g, uint32_t qf) {
     constexpr int BITS = Gama<FMT, MODE>::BITS;
@@ -269,6 +272,24 @@ __device__ __forceinline__ uint32_t tf8_pair(uint32_t reg, uint32_t sel) {
     uint32_t h2 = __byte_perm(reg, 0u, sel);
     uint32_t t  = ((h2 >> 3) & 0x0FE00FE0u) | (h2 & 0x80008000u);
     return bf162_as_u32(__hmul2_rn(u32_as_bf162(t), u32_as_bf162(0x77807780u)));
+}
+
+// Any step: the codes as numbers, qbias (q2) off them, the arithmetic at its own scale, then 2^-7 -> the same 16 registers as below
+template <int FMT, int MODE>
+__device__ __forceinline__ void expand_slot_far(uint32_t* o, const uint32_t* w, uint32_t zero, uint32_t step, uint32_t q2) {
+    constexpr int BITS = Gama<FMT, MODE>::BITS, PR = 16 / BITS;
+    const uint32_t st2 = __byte_perm(step, 0u, 0x1010), z2 = __byte_perm(zero, 0u, 0x1010) ^ (MODE == TM_AFFINE_FMA ? 0x80008000u : 0u);
+    constexpr uint32_t down2 = (uint32_t)(127 - kWShift) * 0x00800080u;
+#pragma unroll
+    for (int p = 0; p < 16; p++) {
+        const uint32_t v = w[16 / PR - 1 - p / PR] >> (p % PR * BITS) & ((1u << BITS) - 1u) * 0x00010001u;
+        const __nv_bfloat162 k = __hsub2_rn(__hsub2_rn(u32_as_bf162(v | 0x43004300u), u32_as_bf162(0x43004300u)), u32_as_bf162(q2));
+        __nv_bfloat162 x;
+        if (MODE == TM_AFFINE_FMA) x = __hfma2(k, u32_as_bf162(st2), u32_as_bf162(z2));
+        else x = __hmul2_rn(k, u32_as_bf162(st2));
+        if (MODE == TM_AFFINE) x = __hsub2_rn(x, u32_as_bf162(z2));
+        o[p] = bf162_as_u32(__hmul2_rn(x, u32_as_bf162(down2)));
+    }
 }
 
 // Expand the 32 weights of one slot (codes in `w`, memory order) into 16 bf16x2 registers in the permuted k order.  qsub: qbias as a number of each field
@@ -671,25 +692,30 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
                     }
                 }
             };
-            auto produce = [&](auto bias) {
-                uint32_t a0 = 0, raw0 = 0;  // A and raw stages of the items so far
-                Item w = decode_item<KBR>(p, blockIdx.x);
-                auto first = [&]() { return w.kb0 / KBR + (int)(((uint32_t)team + raw0) % (uint32_t)TEAMS); };  // the team's first raw stage of an item
-                rows_of(w), fetch_gama(first());
-                for (int item = blockIdx.x; item < p.n_items;) {
-                    const int rb = w.kb0 / KBR, re = (w.kb1 + KBR - 1) / KBR, kend = w.kb1;
-                    int r = first();
-                    const uint32_t a1 = a0 + (uint32_t)((r - rb) * SPR), raw1 = raw0 + (uint32_t)(r - rb);
-                    uint32_t s = a1 % SA, eph = (a1 / SA & 1u) ^ 1u, rs = raw1 % RS, rph = raw1 / RS & 1u;
-                    a0 += (uint32_t)(w.kb1 - w.kb0 + U - 1) / U, raw0 += (uint32_t)(re - rb);
-                    auto next_item = [&]() {  // and its first zero / step
-                        item += gridDim.x;
-                        if (item < p.n_items) w = decode_item<KBR>(p, item), rows_of(w), fetch_gama(first());
-                    };
-                    if (r >= re) next_item();
+            enum { kPlainWay, kBias, kFar };
+            uint32_t a0 = 0, raw0 = 0;  // A and raw stages of the items so far
+            int item = blockIdx.x, r = 0, re = 0, kend = 0;  // the item to open next, the raw stage of the one at hand, its end and that of its k-blocks
+            uint32_t s = 0, eph = 0, rs = 0, rph = 0;
+            Item w = decode_item<KBR>(p, item);
+            auto first = [&]() { return w.kb0 / KBR + (int)(((uint32_t)team + raw0) % (uint32_t)TEAMS); };  // the team's first raw stage of an item
+            auto next_item = [&]() {  // and its first zero / step
+                item += gridDim.x;
+                if (item < p.n_items) w = decode_item<KBR>(p, item), rows_of(w), fetch_gama(first());
+            };
+            rows_of(w), fetch_gama(first());
+            // the stages from the one at hand: to the end, or (not kFar) up to one with a step that the quick expansion does not hold
+            auto produce = [&](auto way) {
+                constexpr int WAY = decltype(way)::value;
+                for (;;) {
                     while (r < re) {
                         const int nk = kend - r * KBR;  // k-blocks from here to the end of the part: an even number
                         mbar_wait_a(rfull0 + rs * 8, rph);
+                        if constexpr (MODE != TM_PLAIN && WAY != kFar) {  // in any row of the warp
+                            uint32_t top = 0;
+#pragma unroll
+                            for (int j = 0; j < GN; j++) top |= sn[j];
+                            if (__any_sync(0xffffffffu, top & kFarStep)) return;
+                        }
                         const uint32_t src = raw_row + rs * RAW_BYTES;
                         uint32_t zc[GN], sc[GN];
 #pragma unroll
@@ -714,13 +740,18 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
                                 lds64((src ^ (uint32_t)(k >> 1 << 4)) + ((k & 1) ? 0 : 8), q);
                                 v[0] = q[1], v[1] = q[0];
                             }
-                            if (MODE != TM_PLAIN && (k & 1) == 0) gm.set(zc[k / 2], sc[k / 2], p.fold2);
+                            if (WAY != kFar && MODE != TM_PLAIN && (k & 1) == 0) gm.set(zc[k / 2], sc[k / 2], p.fold2);
                             uint32_t o[32];
 #if KF_TC_EXP & 1
                             for (int i = 0; i < 32; i++) o[i] = v[i % (2 * NW)] ^ gm.z;
 #else
-                            expand_slot<FMT, MODE, decltype(bias)::value>(o, &v[0], gm, p.qsub);
-                            expand_slot<FMT, MODE, decltype(bias)::value>(o + 16, &v[NW], gm, p.qsub);
+                            if constexpr (WAY == kFar) {
+                                expand_slot_far<FMT, MODE>(o, &v[0], zc[k / 2], sc[k / 2], p.fold2);
+                                expand_slot_far<FMT, MODE>(o + 16, &v[NW], zc[k / 2], sc[k / 2], p.fold2);
+                            } else {
+                                expand_slot<FMT, MODE, WAY == kBias>(o, &v[0], gm, p.qsub);
+                                expand_slot<FMT, MODE, WAY == kBias>(o + 16, &v[NW], gm, p.qsub);
+                            }
                             if constexpr (BN >= kNaturalBN) {  // below, the branch alone costs the producers 4 % (51200 x 5120 at 45 tokens 49.3 -> 51.2 us)
                                 if (p.natural) natural_order<FMT>(o), natural_order<FMT>(o + 16);
                             }
@@ -758,10 +789,19 @@ __global__ void __launch_bounds__(kThreadsTC, 1)
                         if (s >= SA) s -= SA, eph ^= 1;
                         if (OVER / SA & 1) eph ^= 1;
                     }
+                    if (item >= p.n_items) return;
+                    const int rb = w.kb0 / KBR;
+                    re = (w.kb1 + KBR - 1) / KBR, kend = w.kb1, r = first();
+                    const uint32_t a1 = a0 + (uint32_t)((r - rb) * SPR), raw1 = raw0 + (uint32_t)(r - rb);
+                    s = a1 % SA, eph = (a1 / SA & 1u) ^ 1u, rs = raw1 % RS, rph = raw1 / RS & 1u;
+                    a0 += (uint32_t)(w.kb1 - w.kb0 + U - 1) / U, raw0 += (uint32_t)(re - rb);
+                    if (r >= re) next_item();
                 }
             };
-            if (p.bias) produce(std::true_type());
-            else produce(std::false_type());
+            if (MODE != TM_PLAIN && p.bias) produce(std::integral_constant<int, kBias>());
+            else produce(std::integral_constant<int, kPlainWay>());
+            // a loop of its own: within the one above, on its branch, the same code costs 4 % where the branch is never taken (51200 x 5120 at 45 tokens 41.1 -> 42.8 us)
+            if constexpr (MODE != TM_PLAIN) produce(std::integral_constant<int, kFar>());
         }
     } else if (warp == kRawWarp) {
         if (lane == 0) {

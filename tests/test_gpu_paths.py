@@ -279,7 +279,7 @@ def _ptr(t):
 @pytest.mark.parametrize("typ,bits,qbias", [(kf.KF_T_Q4, 4, 0), (kf.KF_T_Q4, 4, 8), (kf.KF_T_Q4, 4, 117), (kf.KF_T_Q2, 2, 0), (kf.KF_T_Q2, 2, -2), (kf.KF_T_SIGN, 2, 0), (kf.KF_T_SIGN, 2, 1),
                                             (kf.KF_T_SIGN, 2, 3), (kf.KF_T_BINARY, 1, 0), (kf.KF_T_BINARY, 1, 1)])
 @pytest.mark.parametrize("M,rows,cols", [(9, 16, 128), (40, 144, 640), (128, 272, 384), (256, 128, 1152)])
-def test_tc_weights_bit_for_bit(ctx, typ, bits, qbias, fma, M, rows, cols):
+def test_tc_weights_bit_for_bit(ctx, typ, bits, qbias, fma, M, rows, cols, lo=-40, hi=50):
     """Each token picks one column, so the result is the weight itself: the codes that the matmul expands inside its own number format round as kf_dequant does, for steps
     from 2^-40 to 2^50, zeros of any size beside them, codes with and without a bias, and reductions that end inside a stage."""
     import torch
@@ -288,7 +288,7 @@ def test_tc_weights_bit_for_bit(ctx, typ, bits, qbias, fma, M, rows, cols):
     rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
     data = torch.randint(0, 256, (rows, cols * bits // 8), generator=g, device="cuda", dtype=torch.uint8)
     n = rows * cols // 128
-    step = (rnd(n) * torch.exp2(torch.randint(-40, 50, (n,), generator=g, device="cuda").float())).bfloat16()
+    step = (rnd(n) * torch.exp2(torch.randint(lo, hi, (n,), generator=g, device="cuda").float())).bfloat16()
     zero = (rnd(n) * 4 * step.float()).bfloat16() if typ in (kf.KF_T_Q4, kf.KF_T_Q2) else torch.zeros(n, device="cuda").bfloat16()
     step[::17], zero[::13] = 0, 0
     gama = torch.cat([torch.ones(rows + cols, device="cuda").bfloat16(), zero, step]).contiguous()
@@ -307,6 +307,14 @@ def test_tc_weights_bit_for_bit(ctx, typ, bits, qbias, fma, M, rows, cols):
     finally:
         ctx.set_int("deq_fma", 1), ctx.set_int("tc_min_m", -1)
     assert bool((y.float() == w[:, k].T.float()).all())
+
+
+@pytest.mark.parametrize("fma", [0, 1])
+@pytest.mark.parametrize("typ,bits,qbias", [(kf.KF_T_Q4, 4, 0), (kf.KF_T_Q4, 4, 8), (kf.KF_T_Q2, 2, 0), (kf.KF_T_SIGN, 2, 1), (kf.KF_T_SIGN, 2, 3), (kf.KF_T_BINARY, 1, 0)])
+@pytest.mark.parametrize("M,rows,cols,lo,hi", [(20, 144, 640, -110, -40), (256, 128, 1152, -110, 118), (9, 272, 640, 50, 118), (40, 144, 640, -1, 5), (100, 144, 1152, -20, 118)])
+def test_tc_weights_of_any_step(ctx, typ, bits, qbias, fma, M, rows, cols, lo, hi):
+    """As above over the range of bf16: groups whose steps lie beyond what the quick expansion holds beside groups that it takes, in the same rows and the same stages."""
+    test_tc_weights_bit_for_bit(ctx, typ, bits, qbias, fma, M, rows, cols, lo, hi)
 
 
 @pytest.mark.parametrize("typ", [kf.KF_T_Q4, kf.KF_T_BINARY, kf.KF_T_F8E5M2, kf.KF_T_BF16])
