@@ -96,19 +96,6 @@ class ClockSampler:
         return {"sm_mhz": sm[len(sm) // 2] if sm else None, "sm_max_mhz": max(mx) if mx else None, "reasons": sorted(reasons), "samples": len(sm)}
 
 
-GEMV_SOURCES = ("koifish_b200/csrc/Device/gemv_i8.cu", "koifish_b200/csrc/Device/gemv.cu", "koifish_b200/csrc/Device/kf_common.cuh")
-TRAFFIC_FILE = "profiles/r02_traffic_decode.json"
-
-
-def kernel_digest():
-    """sha256 over the sources of the dominant kernel: a committed ncu traffic figure is only reported for the kernel it was taken from"""
-    import hashlib
-    h = hashlib.sha256()
-    for rel in GEMV_SOURCES:
-        h.update(open(os.path.join(ROOT, rel), "rb").read())
-    return h.hexdigest()[:16]
-
-
 def gemv_algorithmic_bytes(rows, cols, bits, group, M):
     """N*K*bits/8 + (N*K/G)*4 [packed types] + 2*M*K + 2*M*N"""
     b = rows * cols * bits / 8.0 + 2.0 * M * cols + 2.0 * M * rows
@@ -379,23 +366,7 @@ def main():
     achieved = per_launch_bytes / per_launch_s / 1e9
     kv_bytes_tok = 2.0 * info.n_layers * (args.ctx + args.steps // 2) * KD * 2
     step_alg_bytes = alg_bytes + head_bytes + kv_bytes_tok
-    # measured DRAM bytes per launch of the same kernel in the same decode step (one ncu pass, tools/gpu_traffic.sh), if committed
-    traffic, traffic_src = None, None
-    if world == 1 and args.workload == "qwen3-32b-q4" and not args.layers:
-        try:
-            tf = json.load(open(os.path.join(ROOT, TRAFFIC_FILE)))
-            if tf.get("kernel_digest") != kernel_digest() or tf.get("gemv_exact") != gemv_exact:
-                traffic_src = "%s is stale (taken from kernel digest %s / gemv_exact %s, this build is %s / %s): not reported" % (
-                    TRAFFIC_FILE, tf.get("kernel_digest"), tf.get("gemv_exact"), kernel_digest(), gemv_exact)
-            else:
-                t = tf["kernels"]["kf_gemv_kernel"]
-                traffic = t["avg_dram_read_bytes"] + t["avg_dram_write_bytes"]
-                traffic_src = "%s (ncu dram__bytes_read.sum + dram__bytes_write.sum, avg of %d launches, kernel digest %s)" % (
-                    TRAFFIC_FILE, t["launches"], tf["kernel_digest"])
-        except Exception:
-            pass
-    roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak, "traffic": traffic,
-                "traffic_source": traffic_src,
+    roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "kernel": "kf_gemv_kernel (fused unpack+dequant GEMV, M=1, in-kernel dequant to the reference's bf16 weights)" if gemv_exact else "kf_gemv_i8_kernel (fused unpack+dequant GEMV, M=1, codes x fixed-point activations on the integer tensor cores, group affine on fp32)", "launches_per_step": n_gemv,
                 "algorithmic_bytes_per_launch": per_launch_bytes, "avg_launch_us": per_launch_s * 1e6, "gemv_share_of_step": gemv_ms_pass / ms_step,
                 "peak_source": peak_src, "frac_of_8TBps": achieved / 8000.0,

@@ -15,7 +15,7 @@
 //     accumulate -- the accumulation type cuBLASLt uses in the reference).  Tensor-core *throughput* is irrelevant here (the op
 //     is bandwidth bound, the MMA pipe runs at < 20 %); the MMA is used because it takes bf16 pairs without an unpack-to-fp32
 //     and does the 16x8x16 FMAs in one issue slot -- the kernel is issue-slot limited, not DRAM limited, once the loads are
-//     deep enough (profiles/r01_ncu_gemv_q4_v1.txt);
+//     deep enough;
 //   * the k-order inside a 128-wide group is permuted to make code extraction cheap (nibbles 16 bits apart form one bf16x2
 //     register); the activations are staged in shared memory in the same permuted order, so no weight is ever shuffled;
 //   * per-group zero/step are staged once per CTA in shared memory with wide batched loads;
@@ -35,10 +35,10 @@ enum { MODE_PLAIN = 0, MODE_AFFINE = 1, MODE_AFFINE_SYM = 2, MODE_SCALE = 3, MOD
 // MODE_FAST (4 / 2 / 1-bit, the DEFAULT for decode: ctx knob gemv_exact = 0): the codes go to the tensor cores as fp16 SUBNORMALS.  A code
 // field that lies inside the low 10 bits of a 16-bit half IS the fp16 number c * 2^b * 2^-24 (exponent field 0: no implicit one, no offset to
 // cancel), so ONE LOP3 (`word & mask`, mask an immediate) turns two packed codes into an MMA operand pair; the fields above bit 9 come down
-// with one byte permute (>> 8) per register.  mma.sync handles fp16 subnormals exactly (tools/ubench/hmma_subnormal.cu).  The activation that
+// with one byte permute (>> 8) per register.  mma.sync handles fp16 subnormals exactly (profiles/r02_hmma_subnormal.txt).  The activation that
 // meets the field at bit b is staged as fp16 x * 2^-b (exact), with a power-of-two scale per 128-k group that puts the group's largest
 // magnitude in [2^13, 2^14).  Per weight that is 0.56 .. 0.62 integer-pipe instructions instead of 3 (shift + LOP3 + bf16 subtract of the
-// bf16 forms; a funnel shift alone costs ~5 clk per warp instruction and scheduler on B200, tools/ubench/deq_rate2.cu: the bit-exact forms
+// bf16 forms; a funnel shift alone costs ~5 clk per warp instruction and scheduler on B200, profiles/r02_ubench_deq_rate2.txt: the bit-exact forms
 // need 432 clk per [128 x 128] tile, MORE than the tile's bytes take at the HBM rate).  The group's step / zero / code bias are applied to
 // the fp32 group sums, y += step * (sum c x - qbias Sx) - zero Sx: the reference's affine dequant without its per-weight bf16 rounding (for
 // the yyang ternary / binary types, whose weights step * k are exact in bf16, that is the SAME arithmetic as the reference's).
@@ -1004,7 +1004,7 @@ int gemv_dispatch(kf_ctx* ctx, int n, void* const* y, const kf_tensor_desc* w, c
     // ---- tile shape: 32 rows per warp (RT = 2) when there are enough rows to keep every SM busy, else 16 -------------------------
     int rt = 1;
     if (M <= 8 && fmt != FMT_BF16 && fmt != FMT_F8) {
-        rt = 1;  // measured (profiles/r01_gemv_sweep_v4.txt): 16 rows per warp is never slower than 32 on B200
+        rt = 1;  // measured: 16 rows per warp is never slower than 32 on B200
         (void)total_rows;
         if (ctx->gemv_variant == 2) rt = 2;
     }

@@ -6,7 +6,7 @@
 // (src/Device/CUDA/NeuronFuse.cu:305-381), with the neighbouring CU_rms_infer / CU_swiglu_v0 / CU_add3 launches folded in.
 //
 // The op is HBM-bound on paper (0.53 B / weight, every packed byte read once).  What actually limited the first form of the cp.async kernel (gemv.cu) was the
-// ALU pipe: tools/ubench/deq_rate*.cu measure, from registers only, 432 clk per [128 rows x 128 k] tile and SM for the bit-exact bf16
+// ALU pipe: profiles/r02_ubench_deq_rate*.txt, from registers only: 432 clk per [128 rows x 128 k] tile and SM for the bit-exact bf16
 // unpack (SHF + LOP3 + HSUB2 + HFMA2 per pair of weights; a funnel shift alone costs ~5 clk per warp instruction and scheduler on this
 // part) -- MORE than the 392 clk the tile's bytes take at the measured HBM rate.  Hence two arithmetic modes (template MODE):
 //   DM_FAST (default)  the codes go to the tensor cores as fp16 numbers 1024 + c / 1024 + 16 c, built with ONE LOP3 each (both nibbles of
