@@ -824,7 +824,7 @@ __global__ void __launch_bounds__(256) kf_qknorm_rope_kv_warp_kernel(uint16_t* _
                                                                      size_t seq_stride) {
     constexpr int HD = DPL * 32;
     kf_grid_dependency_wait();
-    k = behind_wait(k), v = behind_wait(v);
+    k = behind_wait(k), v = behind_wait(v), pos_dev = behind_wait(pos_dev);
     kf_grid_launch_dependents();  // the attention behind us may set itself up; it waits for our end before it reads anything
     const int lane = threadIdx.x & 31;
     const int per_tok = n_head + n_kv, warps = (per_tok + R - 1) / R;  // warps of a token

@@ -94,6 +94,7 @@ __global__ void __launch_bounds__((4 * SETS + 1) * 32, 3 - SETS)
     }
     kf_grid_launch_dependents();
     kf_grid_dependency_wait();  // queries, the rows of the current position, positions, workspace
+    q = behind_wait(q), pos_dev = behind_wait(pos_dev);
     // the launch was sized from a hint: a sequence that needs them takes longer runs, so any length is covered; one without positions has one empty run, whose
     // result is what an empty softmax gives (0 / 0)
     auto shape = [&](int m, int& chunk, int& len) {

@@ -117,6 +117,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     const uint32_t tmem = tmem_base_smem;
     kf_grid_launch_dependents();
     kf_grid_dependency_wait();  // queries, cache rows and the position come from the kernels before us
+    pos_dev = behind_wait(pos_dev);
     const int pos0 = pos_dev[0], kv_len = min(pos0 + min(M, q0 + kQ), max_seq), n_tiles = (kv_len + kKV - 1) / kKV;
 
     if (warp < 8) {

@@ -68,6 +68,7 @@ __global__ void __launch_bounds__(256) kf_awq_gemv_kernel(float* __restrict__ pa
     const int word = blockIdx.x * 32 + wl, W8 = OC / 8;
     const int groups = IC / 128, g0 = (int)(((long long)blockIdx.y * groups) / S), g1 = (int)(((long long)(blockIdx.y + 1) * groups) / S);
     kf_grid_dependency_wait();
+    x = behind_wait(x);
     float acc[MT][8];
 #pragma unroll
     for (int m = 0; m < MT; m++)
@@ -117,6 +118,7 @@ __global__ void __launch_bounds__(256) kf_awq_gemv_kernel(float* __restrict__ pa
 __global__ void __launch_bounds__(256) kf_awq_reduce_kernel(void* __restrict__ y, const float* __restrict__ partial, const uint16_t* __restrict__ residual,
                                                             size_t n, int S, int epi) {
     kf_grid_dependency_wait();
+    partial = behind_wait(partial), residual = behind_wait(residual);
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float s = 0.f;

@@ -262,6 +262,7 @@ template <int FMT, int MODE, int MX>
 __device__ __forceinline__ void gemv_stage_x(uint4* __restrict__ dstx, float4* __restrict__ dstsx, const GemvParams& p, int s_begin, int nsteps,
                                              float* s_red, float* s_scale) {
     const int tid = threadIdx.x, lane = tid & 31;
+    const uint16_t* const px = behind_wait(p.x);
     // ---- optional fused RMSNorm: the same arithmetic, in the same order, as kf_rmsnorm_kernel (ops.cu).  Bound by latency: a token is two loads a thread.  The sums of
     //      up to eight tokens are formed side by side, their loads travel together and they share two block barriers; one token after the other cost a memory
     //      round trip and two barriers each (28 layers of 1024 x 3072, 8 tokens, 112 of these matmuls: step 1579 -> 1254 us; bits unchanged) ------------------
@@ -275,7 +276,7 @@ __device__ __forceinline__ void gemv_stage_x(uint4* __restrict__ dstx, float4* _
             for (int i = tid * 8; i < p.K; i += kThreads * 8) {
                 uint4 v[TB8];
 #pragma unroll
-                for (int m = 0; m < TB8; m++) v[m] = m0 + m < p.M ? __ldg(reinterpret_cast<const uint4*>(p.x + (size_t)(m0 + m) * p.K + i)) : make_uint4(0, 0, 0, 0);
+                for (int m = 0; m < TB8; m++) v[m] = m0 + m < p.M ? __ldg(reinterpret_cast<const uint4*>(px + (size_t)(m0 + m) * p.K + i)) : make_uint4(0, 0, 0, 0);
 #pragma unroll
                 for (int m = 0; m < TB8; m++) {
                     const uint32_t q[4] = {v[m].x, v[m].y, v[m].z, v[m].w};
@@ -310,7 +311,7 @@ __device__ __forceinline__ void gemv_stage_x(uint4* __restrict__ dstx, float4* _
             uint32_t src[KT / 2];
             if (m < p.M) {
                 const size_t k0 = (size_t)(s_begin + s) * KSTEP + tt * KT;
-                const uint4* gp = reinterpret_cast<const uint4*>(p.x + (size_t)m * p.K + k0);
+                const uint4* gp = reinterpret_cast<const uint4*>(px + (size_t)m * p.K + k0);
 #pragma unroll
                 for (int i = 0; i < KT / 8; i++) {
                     uint4 v = __ldg(gp + i);
@@ -526,6 +527,8 @@ __global__ void __launch_bounds__(kThreads, (NT >= 4 ? 1 : NT == 1 ? KF_GEMV_OCC
     //      residual) and writes buffers the predecessor may still be using (split-K workspace, y): wait for it to finish.  Under
     //      programmatic dependent launch this CTA may have been running for a while already, with its weight stream in flight -------
     kf_grid_dependency_wait();
+    const uint4* const xg   = XG ? behind_wait(p.xg) : nullptr;
+    const float4* const sxg = XG ? behind_wait(p.sxg) : nullptr;
 
     // ---- optional fused RMSNorm + the activations of this k-slice into shared memory, permuted to the fragment order ------------------
     if constexpr (!XG)
@@ -611,7 +614,7 @@ __global__ void __launch_bounds__(kThreads, (NT >= 4 ? 1 : NT == 1 ? KF_GEMV_OCC
             }
             float4 sv[NT][2];  // MODE_FAST: {-, 2^-24 Sx, 2^24 / scale} of this k-step's group for the thread's two token columns
             if (MODE == MODE_FAST) {
-                const float4* sx4 = XG ? p.sxg + (size_t)(s_begin + s) * MX
+                const float4* sx4 = XG ? sxg + (size_t)(s_begin + s) * MX
                                        : reinterpret_cast<const float4*>(reinterpret_cast<const uint8_t*>(smem) + p.sx_off) + s * MX;
 #pragma unroll
                 for (int nt = 0; nt < NT; nt++) {
@@ -633,7 +636,7 @@ __global__ void __launch_bounds__(kThreads, (NT >= 4 ? 1 : NT == 1 ? KF_GEMV_OCC
 #pragma unroll
                 for (int nt = 0; nt < NT; nt++) {
                     if constexpr (XG)
-                        xb[nt] = __ldg(p.xg + (((size_t)(s_begin + s) * UNITS + u) * MX + (MX >= 8 ? nt * 8 : 0)) * 4 + xlane);
+                        xb[nt] = __ldg(xg + (((size_t)(s_begin + s) * UNITS + u) * MX + (MX >= 8 ? nt * 8 : 0)) * 4 + xlane);
                     else
                         xb[nt] = smem[((s * UNITS + u) * MX + (MX >= 8 ? nt * 8 : 0)) * 4 + xlane];
                 }

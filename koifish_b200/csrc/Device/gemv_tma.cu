@@ -218,12 +218,13 @@ kf_gemv_tma_kernel(const __grid_constant__ TMaps tm, const TParams p) {
 
     // ---- everything above touched nothing the previous kernel writes.  From here on we read x / residual and write y / ws ----------
     kf_grid_dependency_wait();
+    const uint16_t* const px = behind_wait(p.x);
 
     // ---- optional fused RMSNorm: the arithmetic and summation order of kf_rmsnorm_kernel (ops.cu: 256 threads), bit for bit ----------
     if (p.norm_w) {
         for (int m = 0; m < p.M; m++) {
             if (tid < 256) {
-                const uint16_t* xr = p.x + (size_t)m * p.K;
+                const uint16_t* xr = px + (size_t)m * p.K;
                 float ss = 0.f;
                 for (int i = tid * 8; i < p.K; i += 256 * 8) {
                     const uint4 v = __ldg(reinterpret_cast<const uint4*>(xr + i));
@@ -343,7 +344,7 @@ kf_gemv_tma_kernel(const __grid_constant__ TMaps tm, const TParams p) {
                 uint32_t src[16];
                 if (m < p.M && wb + slot >= u0) {
                     const size_t k0 = (size_t)ks * 128 + tt * 32;
-                    const uint4* gp = reinterpret_cast<const uint4*>(p.x + (size_t)m * p.K + k0);
+                    const uint4* gp = reinterpret_cast<const uint4*>(px + (size_t)m * p.K + k0);
 #pragma unroll
                     for (int i = 0; i < 4; i++) {
                         const uint4 v = __ldg(gp + i);

@@ -111,6 +111,7 @@ __global__ void __launch_bounds__(256) kf_nf4_gemv_kernel(void* __restrict__ y, 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int row  = blockIdx.x * 8 + warp;
     kf_grid_dependency_wait();
+    x = behind_wait(x), residual = behind_wait(residual);
     if (row >= rows) return;
     {
         const uint16_t* lr = lut + (size_t)row * 16;
