@@ -106,7 +106,7 @@ uint64_t kf_scratch_generation(kf_ctx* ctx);
  * kf_attn_decode_gqa may take, default 4 s; when one runs out the kernel ends and kf_ctx_sync -- or the next of these calls -- returns KF_ERR_CUDA, once, and the
  * context is usable again), "attn_drop" (n > 0: the n-th thread block of these kernels loads nothing, so that its waits run out; for tests) */
 int kf_ctx_set_int(kf_ctx* ctx, const char* key, int value);
-int kf_ctx_get_int(kf_ctx* ctx, const char* key, int* value_out); /* gqa_min_ctx, tc_min_m, pdl, attn_split; attn_tc_error, attn_gqa_error (waits for the stream): not 0 when a bounded wait of these kernels ran out and has not been reported yet; tmap_weights: tensor maps of weights held; tc_last_bn, tc_last_split, tc_last_cluster: token tile, k-parts and whether these met in clusters, of the last tcgen05 GEMM */
+int kf_ctx_get_int(kf_ctx* ctx, const char* key, int* value_out); /* gqa_min_ctx, tc_min_m, pdl, attn_split; attn_tc_error, attn_gqa_error (waits for the stream): not 0 when a bounded wait of these kernels ran out and has not been reported yet; tmap_weights: tensor maps of weights held; gemv_last_s, gemv_last_kernel: k-parts and file (0 gemv.cu, 1 gemv_tma.cu, 2 gemv_i8.cu) of the last skinny matmul; tc_last_bn, tc_last_split, tc_last_cluster: token tile, k-parts and whether these met in clusters, of the last tcgen05 GEMM */
 
 /* ---- device memory (huTensor::Alloc_1, src/Device/CUDA/huTensor.cu:70-103) ---- */
 int kf_malloc(kf_ctx* ctx, size_t bytes, void** dev_out);

@@ -164,6 +164,8 @@ extern "C" int kf_ctx_get_int(kf_ctx* ctx, const char* key, int* value_out) {
         *value_out = ctx->gemv_i8_max_m;
     else if (!strcmp(key, "gemv_last_s"))
         *value_out = ctx->gemv_last_s;
+    else if (!strcmp(key, "gemv_last_kernel"))
+        *value_out = ctx->gemv_last_kernel;
     else if (!strcmp(key, "tc_last_bn"))
         *value_out = ctx->tc_last & 0xfff;
     else if (!strcmp(key, "tc_last_split"))

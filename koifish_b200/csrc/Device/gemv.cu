@@ -1098,7 +1098,7 @@ int gemv_dispatch(kf_ctx* ctx, int n, void* const* y, const kf_tensor_desc* w, c
     if (M == 1 && ctx->gemv_cluster == 2 && ctx->gemv_splitk <= 0 && S > 8 && S_min <= 8) S = 8;
     p.cluster    = (M <= 8 && ctx->gemv_cluster > 0 && S >= 2 && S <= 8 && (M == 1 || (p.steps_total + S - 1) / S <= 16 || ctx->gemv_splitk > 0)) ? 1 : 0;
     p.S          = S;
-    ctx->gemv_last_s = S;
+    ctx->gemv_last_s = S, ctx->gemv_last_kernel = 0;
     p.nsteps_max = (p.steps_total + S - 1) / S;  // floor/ceil slicing never exceeds ceil(steps/S)
     if (S > 1 && !p.cluster) {
         int rc = kf_ensure_gemv_ws(ctx, (size_t)S * rb * std::max(8, MXs) * rows_cta * sizeof(float), rb);
@@ -1133,6 +1133,7 @@ int kf_gemv_small(kf_ctx* ctx, int n, void* const* y, const kf_tensor_desc* w, c
 #endif
     if (M <= 8) {  // the persistent TMA-fed stream-K kernel covers the decode shapes (4-bit, group 128, K % 512 == 0)
         const int rc = kf_gemv_tma(ctx, n, y, w, x, M, epilogue, residual, norm_w, norm_eps);
+        if (rc == KF_OK) ctx->gemv_last_kernel = 1;
         if (rc != 1) return rc;
     }
     // a split, a tile, a merge or a staging that was asked for is one of this kernel's

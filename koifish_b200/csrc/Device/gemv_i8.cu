@@ -647,6 +647,6 @@ int kf_gemv_i8(kf_ctx* ctx, int n, void* const* y, const kf_tensor_desc* w, cons
     }
     if (!best.S) return 1;
     p.S = best.S, p.clusters = best.clusters;
-    ctx->gemv_last_s = best.S;
+    ctx->gemv_last_s = best.S, ctx->gemv_last_kernel = 2;
     return fmt == IF_Q4 ? launch_tokens<IF_Q4>(ctx, p, best) : fmt == IF_Q2 ? launch_tokens<IF_Q2>(ctx, p, best) : launch_tokens<IF_Q1>(ctx, p, best);
 }

@@ -54,6 +54,7 @@ struct kf_ctx {
     int gemv_exact   = 0;
     int gemv_i8_max_m = 2;  // tokens up to which the decode arithmetic runs on the integer tensor cores (gemv_i8.cu); 0 = never
     int gemv_last_s  = 0;  // read-only: k-split of the most recent dequant-GEMV launch (tools/gemv_bench.py records it)
+    int gemv_last_kernel = 0;  // read-only: file of that launch: 0 gemv.cu, 1 gemv_tma.cu, 2 gemv_i8.cu
     // rounding of the reference's dequant expression (step * k - zero) in bf16 (CU_Q128toX_, T.cu:274), pinned against the reference kernel
     // compiled both ways (oracle/ref_kernels.cu): 1 = ONE rounding, fma.rn.bf16 -- what nvcc's default -fmad=true (implied by the
     // reference's -use_fast_math) generates on sm_90+, i.e. what the reference computes on a B200 ; 0 = TWO roundings (bf16 multiply, then

@@ -75,6 +75,7 @@ def test_gemv_i8(ctx, typ, bits, M, rows, cols, wide):
         ctx.check(ctx.lib.kf_linear(ctx.h, ys["none"].data_ptr(), C.byref(dw), x.data_ptr(), M, kf.KF_EPI_NONE, None), "none")
         ctx.check(ctx.lib.kf_linear(ctx.h, ys["res"].data_ptr(), C.byref(dw), x.data_ptr(), M, kf.KF_EPI_RESIDUAL, ys["res"].data_ptr()), "residual")
         ctx.check(ctx.lib.kf_linear(ctx.h, ys["f32"].data_ptr(), C.byref(dw), x.data_ptr(), M, kf.KF_EPI_F32, None), "f32")
+        assert ctx.get_int("gemv_last_kernel") == 2
         ctx.check(ctx.lib.kf_rmsnorm_linear(ctx.h, 2, two, gu, x.data_ptr(), nw.data_ptr(), 1e-6, M, 2), "swiglu")
         ctx.check(ctx.lib.kf_rmsnorm_linear(ctx.h, 1, yn, one, x.data_ptr(), nw.data_ptr(), 1e-6, M, 0), "norm")
         ctx.sync()
@@ -98,7 +99,7 @@ def test_gemv_i8(ctx, typ, bits, M, rows, cols, wide):
 
 @pytest.mark.parametrize("typ", [kf.KF_T_Q4, kf.KF_T_SIGN, kf.KF_T_BINARY])
 def test_gemv_i8_special_values(ctx, typ):
-    """Infinities and NaN have no fixed-point form: the rows they reach are not finite.  Groups of zeros and of the smallest numbers stay what they are."""
+    """Infinities and NaN have no fixed-point form: the rows they reach are not finite, and the call after is as ever."""
     import ctypes as C
     import torch
     rows, cols = 1024, 1024
@@ -110,15 +111,38 @@ def test_gemv_i8_special_values(ctx, typ):
         torch.cuda.synchronize()
         ctx.check(ctx.lib.kf_linear(ctx.h, y.data_ptr(), C.byref(d), x.data_ptr(), 1, kf.KF_EPI_F32, None), "linear")
         ctx.sync()
-        assert not bool(torch.isfinite(y).any())
-    x, y = torch.zeros(1, cols, device="cuda").bfloat16(), torch.zeros(1, rows, device="cuda")
-    x[0, 130] = 2.0 ** -120
-    x[0, 700] = 2.0 ** 100
+        assert not bool(torch.isfinite(y).any()) and ctx.get_int("gemv_last_kernel") == 2
+        x[0, 300] = 1
+        torch.cuda.synchronize()
+        ctx.check(ctx.lib.kf_linear(ctx.h, y.data_ptr(), C.byref(d), x.data_ptr(), 1, kf.KF_EPI_F32, None), "linear")
+        ctx.sync()
+        # one bf16 rounding of the weight in wd (2^-9), none inside the matmul but those of fp32
+        assert bool(((y[0] - wd[:, 300]).abs() <= 2.0 ** -8 * wd[:, 300].abs() + 2.0 ** -20 * wd.abs().max()).all())
+
+
+@pytest.mark.parametrize("M,rows,cols,knobs,kernel", [(1, 256, 4096, {}, 2), (1, 240, 4096, {}, 0), (1, 8192, 256, {}, 0), (1, 8192, 128, {}, 0), (2, 25600, 5120, {}, 2), (2, 25616, 5120, {}, 0),
+                                                      (3, 4096, 4096, {}, 0), (1, 4096, 4096, {"gemv_exact": 1}, 0), (1, 4096, 4096, {"gemv_i8_max_m": 0}, 0),
+                                                      (2, 4096, 4096, {"gemv_i8_max_m": 1}, 0), (1, 4096, 4096, {"gemv_splitk": 2}, 0)])
+def test_gemv_i8_dispatch(ctx, M, rows, cols, knobs, kernel):
+    """What stays with gemv.cu: few tiles, k of 128 and 256, two tokens over the largest 4-bit weights, more tokens, and what is asked for.  Either way the result is the matmul's."""
+    import ctypes as C
+    import torch
+    w, wd = make_q(ctx, kf.KF_T_Q4, rows, cols)
+    d, x, y = w.desc(), torch.randn(M, cols, device="cuda").bfloat16(), torch.zeros(M, rows, device="cuda")
     torch.cuda.synchronize()
-    ctx.check(ctx.lib.kf_linear(ctx.h, y.data_ptr(), C.byref(d), x.data_ptr(), 1, kf.KF_EPI_F32, None), "linear")
-    ctx.sync()
-    # the weights are 0.02: rounded to bf16 in wd (2^-9), not so inside the matmul
-    assert bool(((y.double() - x.double() @ wd.double().T).abs() <= 2.0 ** 100 * 0.2 * 2.0 ** -8).all())
+    had = {k: ctx.get_int(k) if k != "gemv_splitk" else 0 for k in knobs}
+    for k, v in knobs.items():
+        ctx.set_int(k, v)
+    try:
+        ctx.check(ctx.lib.kf_linear(ctx.h, y.data_ptr(), C.byref(d), x.data_ptr(), M, kf.KF_EPI_F32, None), "linear")
+        ctx.sync()
+    finally:
+        for k, v in had.items():
+            ctx.set_int(k, v)
+    assert ctx.get_int("gemv_last_kernel") == kernel
+    want = x.double() @ wd.double().T
+    # bf16 weights in wd (2^-9 each, in either direction), the activations of gemv.cu in fp16
+    assert float((y.double() - want).norm() / want.norm()) <= 2.0 ** -8
 
 
 def pack_codes(codes, bits):
@@ -134,7 +158,7 @@ def pack_codes(codes, bits):
 
 @pytest.mark.parametrize("typ,bits", [(kf.KF_T_Q4, 4), (kf.KF_T_Q2, 2), (kf.KF_T_SIGN, 2), (kf.KF_T_BINARY, 1)])
 @pytest.mark.parametrize("M", [1, 2])
-@pytest.mark.parametrize("kind", ["2^14", "2^18", "2^40", "top", "top and others", "2^-100", "2^-100 and 2^60"])
+@pytest.mark.parametrize("kind", ["2^14", "2^18", "2^40", "top", "top and others", "2^-100", "2^-120 and less", "2^-100 and 2^60"])
 def test_gemv_i8_activations_of_any_size(ctx, typ, bits, M, kind):
     """Activations keep all their bits whatever stands beside them.  In every second row the code that meets the large activation is zero, so that nothing but the others shows: one
     far above the rest of its group, the largest finite numbers of either sign at every place of a group (every field of a byte), numbers far below one, and whole groups of them
@@ -154,8 +178,9 @@ def test_gemv_i8_activations_of_any_size(ctx, typ, bits, M, kind):
         big[::2] = True
         x[:, ::2] *= 2.0 ** 60
         x[:, 1::2] *= 2.0 ** -100
-    elif kind == "2^-100":
-        x[:, 1:] *= 2.0 ** -100
+    elif kind.startswith("2^-1"):
+        x[:, 1:] *= 2.0 ** -100 if kind == "2^-100" else 2.0 ** -120
+        x[:, 2] *= 2.0 ** -9  # the latter among the subnormal numbers
         x[:, 0] = 0
     else:
         big[grp, (grp * 37 + 5) % 128] = True  # 37 is odd: every place of a group in 128 groups
@@ -171,7 +196,8 @@ def test_gemv_i8_activations_of_any_size(ctx, typ, bits, M, kind):
         q[1::4] = (q[::4] + 1) % 2 ** bits  # nothing else to be seen there
     x = x.view(M, cols).bfloat16()
     n = rows * G
-    step, zero = (rnd(n).abs() * 2.0 ** -18 + 2.0 ** -20).bfloat16(), torch.zeros(n, device="cuda").bfloat16()
+    up = 2.0 ** 20 if kind == "2^-120 and less" else 1.0
+    step, zero = ((rnd(n).abs() * 2.0 ** -18 + 2.0 ** -20) * up).bfloat16(), torch.zeros(n, device="cuda").bfloat16()
     gama, data = torch.cat([torch.ones(rows + cols, device="cuda").bfloat16(), zero, step]).contiguous(), pack_codes(q, bits)
     d, y = kf.TensorDesc(data.data_ptr(), gama.data_ptr(), rows, cols, typ, 128, qbias, None, None), torch.zeros(M, rows, device="cuda")
     torch.cuda.synchronize()
@@ -180,6 +206,7 @@ def test_gemv_i8_activations_of_any_size(ctx, typ, bits, M, kind):
     st = step.double().view(rows, G, 1)
     want = x.double() @ (st * (q.double() - qbias).view(rows, G, 128)).view(rows, cols).T
     mag = x.double().abs() @ (st * (q.double() + qbias).view(rows, G, 128)).view(rows, cols).T
+    assert ctx.get_int("gemv_last_kernel") == 2
     # a limb's part of a number is at most three times the number
     assert bool(torch.isfinite(y).all()) and bool(((y.double() - want).abs() <= 3 * (G + 64) * 2.0 ** -23 * mag + 2.0 ** -145).all())
 
