@@ -67,7 +67,7 @@ struct GemmParams {
     float* ws;                 // split-K partials
     unsigned* cnt;             // split-K arrival counters (self-resetting)
     int M, N, K;
-    int qbias, gshift, epilogue;
+    int gshift, epilogue;
     int n_tiles, m_tiles, splits, n_items;
     int staged;                // outputs (and residual) may be accessed 16 bytes at a time
     int cluster;               // the parts of a split are the CTAs of a cluster, one item each
@@ -1283,7 +1283,7 @@ int kf_gemm_tc_multi(kf_ctx* ctx, int n, void* const* y, const kf_tensor_desc* w
     memset(&p, 0, sizeof(p));
     const void* wdata[kMaxW] = {};
     p.residual = (const uint16_t*)residual, p.M = M, p.K = K;
-    p.qbias = w[0].qbias, p.epilogue = epilogue;
+    p.epilogue = epilogue;
     if (mode != TM_PLAIN) {
         const int q = w[0].qbias, bits = fmt == TF_Q4 ? 4 : fmt == TF_Q2 ? 2 : 1;
         p.bias = mode == TM_SCALE ? (q & (q - 1)) != 0 : q != 0;

@@ -220,29 +220,27 @@ __global__ void __launch_bounds__(kThreads, 2) kf_gemv_i8_kernel(const __grid_co
     if (tid < items) load_x(tid);  // beside the sums below
     int any_wide = 0;
     if (p.norm_w) {  // the scale of each token, in the order of kf_rmsnorm_kernel (ops.cu): 256 threads
-        if (tid < 256) {
-            float ss[MX];
+        float ss[MX];
 #pragma unroll
-            for (int m = 0; m < MX; m++) ss[m] = 0.f;
-            for (int i = tid * 8; i < p.K; i += 256 * 8) {
-                uint4 v[MX];
+        for (int m = 0; m < MX; m++) ss[m] = 0.f;
+        for (int i = tid * 8; i < p.K; i += kThreads * 8) {
+            uint4 v[MX];
 #pragma unroll
-                for (int m = 0; m < MX; m++) v[m] = __ldg(reinterpret_cast<const uint4*>(px + (size_t)m * p.K + i));
-#pragma unroll
-                for (int m = 0; m < MX; m++) {
-                    const uint32_t w[4] = {v[m].x, v[m].y, v[m].z, v[m].w};
-#pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        const float a = bf16lo(w[j]), b = bf16hi(w[j]);
-                        ss[m] = fmaf(a, a, ss[m]), ss[m] = fmaf(b, b, ss[m]);
-                    }
-                }
-            }
+            for (int m = 0; m < MX; m++) v[m] = __ldg(reinterpret_cast<const uint4*>(px + (size_t)m * p.K + i));
 #pragma unroll
             for (int m = 0; m < MX; m++) {
-                ss[m] = warp_sum(ss[m]);
-                if (lane == 0) s_red[m * 8 + warp] = ss[m];
+                const uint32_t w[4] = {v[m].x, v[m].y, v[m].z, v[m].w};
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const float a = bf16lo(w[j]), b = bf16hi(w[j]);
+                    ss[m] = fmaf(a, a, ss[m]), ss[m] = fmaf(b, b, ss[m]);
+                }
             }
+        }
+#pragma unroll
+        for (int m = 0; m < MX; m++) {
+            ss[m] = warp_sum(ss[m]);
+            if (lane == 0) s_red[m * 8 + warp] = ss[m];
         }
         __syncthreads();
         if (tid < MX) {
@@ -556,14 +554,13 @@ int launch_depth(kf_ctx* ctx, const IParams& p, size_t smem) {
     KF_LAUNCH_CHECK(ctx);
     return KF_OK;
 }
-// bytes in flight per SM: warps x depth x 2 KB (1 KB of 1-bit weights)
+// bytes in flight per CTA: warps x depth x 2, 1 or half a KB (4-, 2- and 1-bit weights)
 template <int FMT, int MX>
 int launch_fmt(kf_ctx* ctx, const IParams& p, const IPlan& plan) {
     switch (plan.depth) {
         case 2: return launch_depth<FMT, MX, 2>(ctx, p, plan.smem);
         case 3: return launch_depth<FMT, MX, 3>(ctx, p, plan.smem);
-        case 4: return launch_depth<FMT, MX, 4>(ctx, p, plan.smem);
-        default: return launch_depth<FMT, MX, 6>(ctx, p, plan.smem);
+        default: return launch_depth<FMT, MX, 4>(ctx, p, plan.smem);
     }
 }
 template <int FMT>
@@ -633,7 +630,7 @@ int kf_gemv_i8(kf_ctx* ctx, int n, void* const* y, const kf_tensor_desc* w, cons
         for (size_t room : {on_sm == 2 ? kTwo : kEarly, kHalfSM, kMost}) {
             late = room == kMost;  // one CTA an SM, and the next kernel starts only behind this one
             if (late && (on_sm == 2 || (M == 2 && fmt != IF_Q4))) break;
-            for (int d : {6, 4, 3, 2})
+            for (int d : {4, 3, 2})
                 if (!depth && ring + kWarps * slot * d <= room && blocks(d, ns) <= kGB && blocks(d, n0) <= kGB) depth = d;
             if (depth) break;
         }
