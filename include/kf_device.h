@@ -120,7 +120,10 @@ int kf_d2d_2d(kf_ctx* ctx, void* dst_dev, size_t dst_pitch, const void* src_dev,
 int kf_host_alloc(size_t bytes, void** host_out); /* pinned */
 int kf_host_free(void* host);
 
-/* ---- CUDA graph capture of a launch sequence (no reference equivalent: it launches ~40 kernels/layer eagerly) ---- */
+/* ---- CUDA graph capture of a launch sequence (no reference equivalent: it launches ~40 kernels/layer eagerly) ----
+ *      A tcgen05 matmul of packed, 8-bit or bf16 weights may cut K into parts whose sums meet in a workspace of the context.  The workspace cannot grow inside a
+ *      capture: where an eager call has not made room for it, the captured matmul is planned without that cut.  Its fp32 sums are then added in another order
+ *      than the eager call's, and a bf16 result may be rounded the other way.  One eager step of the same shapes first gives the captured step the eager bits. */
 typedef struct kf_graph kf_graph;
 int kf_graph_begin(kf_ctx* ctx);
 int kf_graph_end(kf_ctx* ctx, kf_graph** out);

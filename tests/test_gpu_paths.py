@@ -410,6 +410,46 @@ def test_tc_swiglu_over_its_input(ctx, typ, M, rows, cols, at):
     assert torch.equal(own, buf[64 + at:64 + at + M * rows])
 
 
+def test_tc_split_inside_a_capture():
+    """A shape that an eager call cuts through the workspace: captured on a context without one it is planned whole or in clusters, captured after an eager call it has that call's
+    bits.  fp32 sums in one order or the other: each of K / 16 additions loses at most 2^-23 of a partial sum, which stays below six times the rms."""
+    import ctypes as C
+    import torch
+    rows, cols, M = 9600, 4608, 12
+    outs, plans = [], []
+    for eager_first in (False, True):
+        c = kf.Context(0)
+        w, wd = make_q(c, kf.KF_T_Q4, rows, cols)
+        d = w.desc()
+        g = torch.Generator(device="cuda")
+        g.manual_seed(3)
+        x, y, e = torch.randn(M, cols, generator=g, device="cuda").bfloat16(), torch.zeros(M, rows, device="cuda"), torch.zeros(M, rows, device="cuda")
+        small, s = torch.zeros(M, 16, device="cuda"), make_q(c, kf.KF_T_Q4, 16, cols)[0]
+        torch.cuda.synchronize()
+        ds = s.desc()
+        c.check(c.lib.kf_linear(c.h, _ptr(small), C.byref(ds), _ptr(x), M, kf.KF_EPI_F32, None), "scratch for the activations")
+        if eager_first:
+            c.check(c.lib.kf_linear(c.h, _ptr(e), C.byref(d), _ptr(x), M, kf.KF_EPI_F32, None), "eager")
+            assert c.get_int("tc_last_split") > 1 and not c.get_int("tc_last_cluster")
+        c.check(c.lib.kf_graph_begin(c.h), "begin")
+        rc, graph = c.lib.kf_linear(c.h, _ptr(y), C.byref(d), _ptr(x), M, kf.KF_EPI_F32, None), C.c_void_p()
+        plans.append((c.get_int("tc_last_split"), c.get_int("tc_last_cluster")))
+        c.check(c.lib.kf_graph_end(c.h, C.byref(graph)), "end")
+        c.check(rc, "captured")
+        for _ in range(2):
+            c.check(c.lib.kf_graph_launch(c.h, graph), "launch")
+        c.sync()
+        if eager_first:
+            assert torch.equal(y, e)
+        outs.append(y)
+        c.lib.kf_graph_destroy(graph)
+        c.close()
+    assert plans[0] != plans[1] and (plans[0][0] == 1 or plans[0][1] == 1)
+    want = x.double() @ wd.double().T
+    for y in outs:
+        assert bool(((y.double() - want).abs() <= cols // 16 * 2.0 ** -23 * 6 * want.square().mean().sqrt()).all())
+
+
 @pytest.mark.parametrize("typ", [kf.KF_T_Q4, kf.KF_T_BINARY, kf.KF_T_BF16])
 @pytest.mark.parametrize("M,tc_bn,splits", [(16, 16, 8), (20, 32, 2), (45, 64, 4), (100, 128, 3), (130, 256, 2), (251, 256, 5), (257, 128, 7)])
 def test_tc_split_over_cluster_equals_workspace(ctx, typ, M, tc_bn, splits):
