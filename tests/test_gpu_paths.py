@@ -410,6 +410,29 @@ def test_tc_swiglu_over_its_input(ctx, typ, M, rows, cols, at):
     assert torch.equal(own, buf[64 + at:64 + at + M * rows])
 
 
+@pytest.mark.parametrize("typ", [kf.KF_T_Q4, kf.KF_T_SIGN, kf.KF_T_BINARY])
+@pytest.mark.parametrize("at", [0, 8, 1024, -1024, 200 * 1024 - 8, 200 * 1024])
+def test_tc_single_weight_over_its_input(ctx, typ, at):
+    """One packed weight and more than 128 tokens: activations are read as they lie, by every item, so not where the result lies over them, `at` elements behind their start.  fp32 sums
+    in one order or the other (1e-5 of the rms), one bf16 rounding."""
+    import ctypes as C
+    import torch
+    M, n = 200, 1024
+    w, wd = make_q(ctx, typ, n, n)
+    d = w.desc()
+    g = torch.Generator(device="cuda")
+    g.manual_seed(7)
+    x = torch.randn(M, n, generator=g, device="cuda").bfloat16()
+    buf = torch.zeros(3 * M * n, device="cuda").bfloat16()
+    for _ in range(3):
+        buf[M * n:2 * M * n] = x.view(-1)
+        torch.cuda.synchronize()
+        ctx.check(ctx.lib.kf_linear(ctx.h, _ptr(buf[M * n + at:]), C.byref(d), _ptr(buf[M * n:]), M, kf.KF_EPI_NONE, None), "linear over x")
+        ctx.sync()
+        y, want = buf[M * n + at:2 * M * n + at].view(M, n).double(), x.double() @ wd.double().T
+        assert bool(((y - want).abs() <= 2.0 ** -8 * 1.001 * want.abs() + 1e-5 * want.square().mean().sqrt()).all())
+
+
 def test_tc_split_inside_a_capture():
     """A shape that an eager call cuts through the workspace: captured on a context without one it is planned whole or in clusters, captured after an eager call it has that call's
     bits.  fp32 sums in one order or the other: each of K / 16 additions loses at most 2^-23 of a partial sum, which stays below six times the rms."""
