@@ -14,17 +14,19 @@
 //   * the 8 bits of a bf16 number are whole down to 2^-23 of the group's largest under the lowest field of a byte, down to 2^-19, 2^-17 and 2^-16 under the highest of 4-, 2- and
 //     1-bit codes.  A k-step with a number that is not (of a SwiGLU's outputs one group in 190, 90 and 57, of normal ones hardly any), with infinities or NaN, or with numbers
 //     that together leave the range, keeps its activations as they are, as bf16 pairs in the room of two limbs, and goes through mma.sync.m16n8k16 on codes as bf16 numbers: no
-//     activation loses a bit that it has above 2^-180 of the largest.  The loop that asks for such steps runs in the CTAs that hold one (5120 x 25600: 18.3 us, 19.1 with the question
-//     everywhere, 18.1 without such steps; ternary 4096 x 12288 at two tokens behind a SwiGLU 10.3 without, 10.8).  Against 64 bits the fp32 sums are off by 1e-7, whatever the
-//     activations (gemv.cu: 3e-7 for normal ones, 2e-6 for a SwiGLU's, 1e-5 with outliers of 2^14);
+//     activation loses a bit that it has above 2^-180 of the largest.  The loop that asks for such steps runs in the CTAs that hold one, and their staging lies out of line.  (5120 x
+//     25600: 18.6 us, 18.9 with the question everywhere, 18.2 without such steps; ternary 4096 x 12288 at two tokens behind a SwiGLU 10.3 without, 10.8; 32B decode 209.4 tokens/s without,
+//     204 with both loops in the other order and nothing out of line, 206.4 so.)  Against 64 bits the fp32 sums are off by 1e-7, whatever the activations (gemv.cu: 3e-7 for normal ones,
+//     2e-6 for a SwiGLU's, 1e-5 with outliers of 2^14);
 //   * zero and code bias, which multiply the group's plain sum of activations, take one fma per row, group and token on the lanes that fetched them;
 //   * a CTA takes a run of 16-row tiles, and its eight warps equal shares of the run's k-steps: no barrier between the first copy and the last sum.  Every lane streams its own
 //     words through a ring in shared memory (cp.async), started before the kernel waits for its predecessor.  A k-step costs a warp 45 instructions beside 18 for its share of the
 //     copies and the loop; two CTAs an SM hide their latency, one leaves the issue slots 70 % idle;
 //   * a warp's sums of a tile go to shared memory and are added in the order of the warps; K is cut in halves over a cluster of two CTAs where tiles are few or the staged activations
 //     too many, and the leader adds them in order: bit-reproducible.
-// Measured against gemv.cu, us a launch in a chain of its own kind: 4-bit SwiGLU 51200 x 5120 at one token 31.5 -> 28.5 (4.9 TB/s), 5120 x 25600 21.4 -> 17.8, 10240 x 5120 11.4 -> 9.7,
-// 5120 x 8192 9.2 -> 7.6; ternary SwiGLU 24576 x 4096 at two tokens 16.2 -> 14.2, 4096 x 12288 12.1 -> 10.2; Qwen3-32B decode in 4 bits 185 -> 207 tokens/s.
+// Measured against gemv.cu, us a launch in a chain of its own kind: 4-bit SwiGLU 51200 x 5120 at one token 31.9 -> 29.3 (4.75 TB/s), 5120 x 25600 21.2 -> 18.6, 10240 x 5120 11.5 -> 9.9,
+// 5120 x 8192 9.2 -> 7.5; ternary SwiGLU 24576 x 4096 at two tokens 16.2 -> 14.0, 4096 x 12288 12.1 -> 9.9; binary 24576 x 4096 at one token 14.3 -> 11.4; Qwen3-32B decode in 4 bits
+// 185 -> 206 tokens/s.
 #include <string.h>
 
 #include <algorithm>
@@ -124,6 +126,33 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// A group as bf16 pairs at their places, times 2^up so that the largest lies in [2^63, 2^64) -> {sum of its numbers, -2^-up}
+template <int FMT, int MX>
+__device__ __noinline__ float2 stage_wide(uint4 v0, uint4 v1, uint4 v2, uint4 v3, uint4* at, int e) {
+    constexpr int BITS = Fmt<FMT>::BITS;
+    uint32_t v[16] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w, v2.x, v2.y, v2.z, v2.w, v3.x, v3.y, v3.z, v3.w};
+    const int up      = min(100, 190 - e);  // 190 = 127 + 63
+    const uint32_t by = (uint32_t)(127 + up) * 0x00800080u;
+    const unsigned quad = 0xFu << (threadIdx.x & 28);
+#pragma unroll
+    for (int i = 0; i < 16; i++) v[i] = bf162_as_u32(__hmul2_rn(u32_as_bf162(v[i]), u32_as_bf162(by)));
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        uint32_t w[4];
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const int lo = pair_elem<FMT>(4 * i + c), hi = lo - 16 / BITS;
+            w[c] = __byte_perm(v[lo >> 1], v[hi >> 1], ((lo & 1) ? 0x32 : 0x10) | ((hi & 1) ? 0x7600 : 0x5400));
+        }
+        at[((i >> 1) * 4 * MX + (i & 1)) * 4] = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+    float sum = 0.f;
+#pragma unroll
+    for (int i = 0; i < 16; i++) sum += bf16lo(v[i]), sum += bf16hi(v[i]);
+    sum += __shfl_xor_sync(quad, sum, 1), sum += __shfl_xor_sync(quad, sum, 2);
+    return make_float2(sum, -__uint_as_float((uint32_t)(127 - up) << 23));
 }
 
 // MX: tokens (1, 2) ; D: chunks in flight per warp
@@ -300,28 +329,12 @@ __global__ void __launch_bounds__(kThreads, 2) kf_gemv_i8_kernel(const __grid_co
         int wide = e >= 246 || least < 134 - scale;
         if (MX == 2) wide |= __shfl_xor_sync(0xFFu << (lane & ~7), wide, 4);
         any_wide |= wide;
-        // a step that does not fit: bf16 pairs as the code pairs meet them, in the place of limbs 0 and 1, the largest in [2^63, 2^64) ; marked by the sign
+        // a step that does not fit: bf16 pairs as the code pairs meet them, in the place of limbs 0 and 1 ; marked by the sign
         float inv = __uint_as_float((uint32_t)(127 - scale) << 23);
         if (__builtin_expect(wide, 0)) {
-            const int up      = min(100, 190 - e);  // 190 = 127 + 63
-            const uint32_t by = (uint32_t)(127 + up) * 0x00800080u;
-#pragma unroll
-            for (int i = 0; i < 16; i++) v[i] = bf162_as_u32(__hmul2_rn(u32_as_bf162(v[i]), u32_as_bf162(by)));
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                uint32_t w[4];
-#pragma unroll
-                for (int c = 0; c < 4; c++) {
-                    const int lo = pair_elem<FMT>(4 * i + c), hi = lo - 16 / F::BITS;
-                    w[c] = __byte_perm(v[lo >> 1], v[hi >> 1], ((lo & 1) ? 0x32 : 0x10) | ((hi & 1) ? 0x7600 : 0x5400));
-                }
-                xs[((s * 2 + (i >> 1)) * NC + 4 * m + (i & 1)) * 4 + tt] = make_uint4(w[0], w[1], w[2], w[3]);
-            }
-            sum = 0.f;
-#pragma unroll
-            for (int i = 0; i < 16; i++) sum += bf16lo(v[i]), sum += bf16hi(v[i]);
-            sum += __shfl_xor_sync(quad, sum, 1), sum += __shfl_xor_sync(quad, sum, 2);
-            inv = -__uint_as_float((uint32_t)(127 - up) << 23);
+            const float2 r = stage_wide<FMT, MX>(make_uint4(v[0], v[1], v[2], v[3]), make_uint4(v[4], v[5], v[6], v[7]), make_uint4(v[8], v[9], v[10], v[11]), make_uint4(v[12], v[13], v[14], v[15]),
+                                                 xs + (s * 2 * NC + 4 * m) * 4 + tt, e);
+            sum = r.x, inv = r.y;
         } else {
 #pragma unroll
             for (int h = 0; h < 2; h++) {
@@ -465,8 +478,8 @@ __global__ void __launch_bounds__(kThreads, 2) kf_gemv_i8_kernel(const __grid_co
             }
         }
     };
-    if (any_wide) stream(std::true_type());
-    else stream(std::false_type());
+    if (!any_wide) stream(std::false_type());
+    else stream(std::true_type());
     cp_async_wait<0>();
     __syncthreads();
 
@@ -596,9 +609,10 @@ int kf_gemv_i8(kf_ctx* ctx, int n, void* const* y, const kf_tensor_desc* w, cons
     p.nseg = n, p.x = (const uint16_t*)x, p.residual = (const uint16_t*)residual, p.norm_w = (const uint16_t*)norm_w, p.norm_eps = norm_eps;
     p.M = M, p.K = K, p.ksteps = K / 128, p.tiles = tiles, p.unit = epilogue == EPI_SWIGLU ? 2 : 1, p.qbias = w[0].qbias, p.epilogue = epilogue;
 
-    // Where gemv.cu is no slower.  Two tokens over the largest 4-bit weights: its activations take half the shared memory (51200 x 5120: 34.0 us there, 34.9 here; 5120 x 25600
-    // 22.4 and 22.2).  A handful of tiles: nothing but the launch to gain (256 x 2048: 3.7 and 3.5 us), and a step of several sequences, which is gemv.cu's, keeps the bits of
-    // single ones.  (Three and four tokens take two matrix instructions here and gain nothing: 3968 x 3328 at four 6.3 us there and 6.8 here.)
+    // What gemv.cu answers.  Two tokens over the largest 4-bit weights: its activations take half the shared memory (51200 x 5120, 128000 steps: 34.0 us there, 35.4 here; 24576 x 4096,
+    // 49152 steps: 17.3 and 16.0).  Weights of small models (a handful of tiles): 0.1 to 0.5 us are to be had here (at one token 256 x 2048 3.1 there and 2.85 here, 1024 x 896 3.2 and
+    // 2.85), but a step of several sequences, which is gemv.cu's, then keeps the bits of single ones.  (Three and four tokens take two matrix instructions here and gain nothing: 3968 x
+    // 3328 at four 6.3 us there and 6.8 here.)
     const long long steps = (long long)tiles * p.ksteps;
     if (steps < 512 || (M == 2 && fmt == IF_Q4 && steps > 64000)) return 1;
 
@@ -606,8 +620,8 @@ int kf_gemv_i8(kf_ctx* ctx, int n, void* const* y, const kf_tensor_desc* w, cons
     const int units = tiles / p.unit;
     constexpr int ch  = kCh;
     const size_t slot = (size_t)ch * 32 * 8 * bits;
-    // blocks of zeros or steps that the chunks in flight and the one in work can meet: those of a run of entries, and the two ends of each tile in it (K = 128 and 256 meet too many:
-    // gemv.cu)
+    // blocks of zeros or steps that the chunks in flight and the one in work can meet, at most: those of a run of entries, and the two ends of each tile in it (K = 128 and 256 meet too
+    // many: gemv.cu).  The bound is one block above what ten entries of long rows meet, so that four chunks are in flight for slices of 7 and 8 steps alone, three or two elsewhere
     auto blocks = [&](int depth, int ns) {
         const int steps = (depth + 1) * ch, chunks = (ns + ch - 1) / ch, tiles_met = (depth + 1 - 2) / chunks + 2;
         return std::min(tiles_met * ((2 * ns + 14) / 16 + 1), (2 * steps + 15) / 16 + 2 * tiles_met - 1);
@@ -628,7 +642,9 @@ int kf_gemv_i8(kf_ctx* ctx, int n, void* const* y, const kf_tensor_desc* w, cons
         int depth = 0;
         bool late = false;
         for (size_t room : {on_sm == 2 ? kTwo : kEarly, kHalfSM, kMost}) {
-            late = room == kMost;  // one CTA an SM, and the next kernel starts only behind this one
+            // one CTA an SM, and the next kernel starts only behind this one.  Not at two tokens where there are tiles for two CTAs an SM, whose activations then leave no room for a
+            // plan (K from about 18000): gemv.cu, as fast (5120 x 25600 at two: 22.2 us in 4 bits there, 21.2 in 2, 20.1 in 1)
+            late = room == kMost;
             if (late && (on_sm == 2 || (M == 2 && fmt != IF_Q4))) break;
             for (int d : {4, 3, 2})
                 if (!depth && ring + kWarps * slot * d <= room && blocks(d, ns) <= kGB && blocks(d, n0) <= kGB) depth = d;

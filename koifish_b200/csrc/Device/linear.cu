@@ -60,11 +60,11 @@ static int linear_panels(kf_ctx* ctx, int n, void* const* y, const kf_tensor_des
     return KF_OK;
 }
 
-// Token count from which the tensor-core kernel beats the skinny one (measured on B200): bf16 weights always (TMA streams them at the
-// full HBM rate), everything else from 9 tokens.  Launch by launch the packed formats cross over between 12 and 16 tokens
-// (profiles/r01_tc_crossover.txt), but inside the model the tensor-core path also shares one launch between Q/K/V and between gate/up,
-// and the skinny kernel's 16-token variant is its weakest: Qwen3-32B batch 12 decodes at 972 tok/s this way against 689
-// (profiles/r01_tc_crossover.txt, in-model table).  ctx knob tc_min_m: -1 auto, 0 never, n > 0 fixed threshold.
+// Token count from which the tensor-core kernel answers: bf16 weights always (TMA streams them at the full HBM rate), everything else from 9 tokens.  Above eight the skinny kernel has
+// only its weakest tile (us a launch at 12 tokens, 4 bits, skinny and tcgen05: 51200 x 5120 104.6 and 38.6, 4096 x 4096 13.9 and 10.0, 1024 x 3072 13.5 and 7.2; in the model the tcgen05
+// kernel also shares one launch between Q/K/V and between gate/up, Qwen3-32B batch 12 at 972 tok/s against 689).  At eight it is the size that decides: 51200 x 5120 40.4 and 38.1, 5120 x
+// 25600 31.0 and 25.9, but 10240 x 5120 17.4 and 17.0, 4096 x 4096 8.1 and 9.9, 6144 x 1024 6.2 and 6.9, 1024 x 3072 5.3 and 7.1; at three 35.6 and 38.6, 24.7 and 25.3, 6.5 and 9.9, 4.3
+// and 7.1 (profiles/skinny_vs_tcgen05.txt).  One line for all sizes keeps the layers of a step in one arithmetic.  ctx knob tc_min_m: -1 auto, 0 never, n > 0 fixed threshold.
 static bool use_tensor_cores(const kf_ctx* ctx, int n, const kf_tensor_desc* w, int M) {
     if (ctx->tc_min_m == 0) return false;
     for (int i = 0; i < n; i++) {

@@ -120,6 +120,29 @@ def test_gemv_i8_special_values(ctx, typ):
         assert bool(((y[0] - wd[:, 300]).abs() <= 2.0 ** -8 * wd[:, 300].abs() + 2.0 ** -20 * wd.abs().max()).all())
 
 
+@pytest.mark.parametrize("typ", [kf.KF_T_Q4, kf.KF_T_Q2, kf.KF_T_SIGN, kf.KF_T_BINARY])
+@pytest.mark.parametrize("rows,cols", [(4096, 4096), (2048, 5120)])
+def test_one_two_and_several_tokens_agree(ctx, typ, rows, cols):
+    """A token alone, in a pair and in a step of four take two kernels and two arithmetics.  gemv.cu holds activations in fp16, and its matrix instructions keep them to 2^-14 of a
+    code of one at the worst (sums of products), which bounds the difference."""
+    import ctypes as C
+    import torch
+    w, wd = make_q(ctx, typ, rows, cols)
+    d, g = w.desc(), torch.Generator(device="cuda")
+    g.manual_seed(11)
+    x, ys = torch.randn(4, cols, generator=g, device="cuda").bfloat16(), []
+    for m in (1, 2, 4):
+        y = torch.zeros(4, rows, device="cuda")
+        torch.cuda.synchronize()
+        for i in range(0, 4, m):
+            ctx.check(ctx.lib.kf_linear(ctx.h, _ptr(y[i:]), C.byref(d), _ptr(x[i:]), m, kf.KF_EPI_F32, None), "linear")
+        ctx.sync()
+        assert ctx.get_int("gemv_last_kernel") == (2 if m < 4 else 0)
+        ys.append(y)
+    slack = 2.0 ** -14 * (x.float().abs() @ wd.abs().T)
+    assert bool(((ys[0] - ys[2]).abs() <= slack).all()) and bool(((ys[1] - ys[2]).abs() <= slack).all())
+
+
 @pytest.mark.parametrize("M,rows,cols,knobs,kernel", [(1, 256, 4096, {}, 2), (1, 240, 4096, {}, 0), (1, 8192, 256, {}, 0), (1, 8192, 128, {}, 0), (2, 25600, 5120, {}, 2), (2, 25616, 5120, {}, 0),
                                                       (3, 4096, 4096, {}, 0), (1, 4096, 4096, {"gemv_exact": 1}, 0), (1, 4096, 4096, {"gemv_i8_max_m": 0}, 0),
                                                       (2, 4096, 4096, {"gemv_i8_max_m": 1}, 0), (1, 4096, 4096, {"gemv_splitk": 2}, 0)])
