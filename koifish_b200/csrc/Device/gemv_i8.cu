@@ -16,7 +16,8 @@
 //     that together leave the range, keeps its activations as they are, as bf16 pairs in the room of two limbs, and goes through mma.sync.m16n8k16 on codes as bf16 numbers: no
 //     activation loses a bit that it has above 2^-180 of the largest.  The loop that asks for such steps runs in the CTAs that hold one, and their staging lies out of line.  (5120 x
 //     25600: 18.6 us, 18.9 with the question everywhere, 18.2 without such steps; ternary 4096 x 12288 at two tokens behind a SwiGLU 10.3 without, 10.8; 32B decode 209.4 tokens/s without,
-//     204 with both loops in the other order and nothing out of line, 206.4 so.)  Against 64 bits the fp32 sums are off by 1e-7, whatever the activations (gemv.cu: 3e-7 for normal ones,
+//     204 with both loops in the other order and nothing out of line, 206.4 so.  Where a quarter of the k-steps are such, 4-bit matmuls take as long as gemv.cu (51200 x 5120 31.2 and 31.8
+//     us, 5120 x 25600 20.0 and 21.6), the others 3 to 7 % longer; where all are, 1.3 to 1.7 times as long: 50.9 and 30.9.)  Against 64 bits the fp32 sums are off by 1e-7, whatever the activations (gemv.cu: 3e-7 for normal ones,
 //     2e-6 for a SwiGLU's, 1e-5 with outliers of 2^14);
 //   * zero and code bias, which multiply the group's plain sum of activations, take one fma per row, group and token on the lanes that fetched them;
 //   * a CTA takes a run of 16-row tiles, and its eight warps equal shares of the run's k-steps: no barrier between the first copy and the last sum.  Every lane streams its own
